@@ -57,6 +57,21 @@ class Workspace:
         return self.buf.data_ptr()
 
 
+_native_ext = None
+
+
+def native():
+    """The native per-call host path (host/ops_native.cpp), built in-tree beside the library.  Like the library it is required:
+    there is no run without it.  Its functions return None for arguments they leave to the general routes below."""
+    global _native_ext
+    if _native_ext is None:
+        lib()
+        from . import _ops_native
+        _ops_native.init(binding.LIB_PATH, default_workspace)
+        _native_ext = _ops_native
+    return _native_ext
+
+
 _default_ws: dict[tuple, Workspace] = {}
 
 
@@ -93,9 +108,24 @@ class IntgemmTensor:
             raise Mi8Error(4, "storage too small for an intgemm8 tensor")
         self.storage = storage
         self.rows, self.cols = rows, cols
-        self.data = storage[:n].view(torch.int8).view(rows, cols)
-        self.quant_mult = storage[n:n + 4].view(torch.float32)
+        self._views = None
         self.shape = tuple(logical_shape) if logical_shape is not None else (rows, cols)
+
+    # The views are made when first asked for: an affine needs the storage's address only.
+    def _get_views(self):
+        if self._views is None:
+            n = self.rows * self.cols
+            self._views = native().intgemm_views(self.storage, self.rows, self.cols) or (
+                self.storage[:n].view(torch.int8).view(self.rows, self.cols), self.storage[n:n + 4].view(torch.float32))
+        return self._views
+
+    @property
+    def data(self) -> torch.Tensor:
+        return self._get_views()[0]
+
+    @property
+    def quant_mult(self) -> torch.Tensor:
+        return self._get_views()[1]
 
     @property
     def device(self):
@@ -152,6 +182,11 @@ def prepareB(w: torch.Tensor, w_is_nk: bool = False, ws: Workspace | None = None
         n, k = w.shape
     else:
         k, n = w.shape
+    if ws is None:
+        storage = native().prepare_b(w, k, n, bool(w_is_nk))
+        if isinstance(storage, torch.Tensor):
+            return IntgemmTensor(n, k, w.device, logical_shape=(k, n), storage=storage)
+        check(storage or 0)
     out = IntgemmTensor(n, k, w.device, logical_shape=(k, n))
     ws = ws or default_workspace(w.device)
     check(lib().mi8_prepare_b_f32(w.data_ptr(), k, n, int(w_is_nk), out.data.data_ptr(), out.quant_mult.data_ptr(),
@@ -257,6 +292,11 @@ def _affine_or_dot(a: torch.Tensor, b: IntgemmTensor, bias, transA: bool, transB
                    out_dtype=torch.float32, ws: Workspace | None = None, aq: IntgemmTensor | None = None) -> torch.Tensor:
     if not isinstance(b, IntgemmTensor):
         raise Mi8Error(1, f"Intgemm expects type of B to be a variant of intgemm not {type(b).__name__}")
+    if aq is None and ws is None and not transA and (out_dtype is torch.float32 or out_dtype is torch.float16):
+        out = native().affine(a, b.storage, b.cols, b.rows, bias, scale, relu, out_dtype is torch.float16)
+        if isinstance(out, torch.Tensor):
+            return out
+        check(out or 0)      # (None: arguments for the general route, which handles or rejects them)
     if aq is None:
         if transA:
             a = transpose(a)

@@ -8,7 +8,7 @@ import numpy as np
 import torch
 
 from .binding import check, lib
-from .ops import Workspace, _require_cuda, _stream_ptr, default_workspace
+from .ops import Workspace, _require_cuda, _stream_ptr, default_workspace, native
 
 
 class Packed8Weight:
@@ -34,6 +34,13 @@ class Packed8Weight:
 def prepareB(w: torch.Tensor) -> Packed8Weight:
     """marian-conv --gemm-type packed8avx512 for one weight: fp32 [K,N] on the device -> Packed8Weight (item + Bt)."""
     _require_cuda(w, "W")
+    got = native().p8_prepare_b(w)
+    if isinstance(got, tuple):
+        out = Packed8Weight.__new__(Packed8Weight)
+        out.K, out.N = w.shape
+        out.item, out.bt, out.scale_b, out.zp_b, out.off_b = got
+        return out
+    check(got or 0)          # (None: arguments for the general route)
     w = w.contiguous().float()
     K, N = w.shape
     L = lib()
@@ -75,6 +82,11 @@ def gemmInt8Packed(a: torch.Tensor, w: Packed8Weight, bias: torch.Tensor | None 
                    scratch: torch.Tensor | None = None, ws: Workspace | None = None) -> torch.Tensor:
     """C[M,N] = A[M,K] . B + bias with the arithmetic of the reference's gemmInt8Packed, in one ABI call."""
     _require_cuda(a, "A")
+    if out is None and scratch is None and ws is None:
+        c = native().p8_gemm(a, w.bt, w.scale_b, w.zp_b, w.off_b, bias)
+        if isinstance(c, torch.Tensor):
+            return c
+        check(c or 0)        # (None: arguments for the general route)
     a2 = a.reshape(-1, a.shape[-1]).contiguous()
     M, K = a2.shape
     L = lib()
