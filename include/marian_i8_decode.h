@@ -166,7 +166,7 @@ int mi8d_history_reuse(mi8d_decoder* d, unsigned out[2], int reset);
  *     Wq|Wk|Wv of an encoder layer, the SSRU's W|Wf) run as ONE GEMM launch over copies stored one behind the other;
  *   MI8D_OPT_QUANT_IN_GEMM (default 0): affines with K <= 1024 whose tiles fit one wave of CTAs quantise their
  *     activation while loading it (mi8_multiply_f32_slot) instead of through a quantisation launch;
- *   MI8D_OPT_FUSED_OUTPUT_MAX_ROWS (default 480): up to this many rows the output layer reduces its logits inside
+ *   MI8D_OPT_FUSED_OUTPUT_MAX_ROWS (default 0): up to this many rows the output layer reduces its logits inside
  *     the GEMM's write-back, above it the logits are written and read back by the log-softmax / top-k kernel;
  *   MI8D_OPT_SIDE_STREAM (default 1): the re-projection of the earlier history slabs runs on an internal stream;
  *   MI8D_OPT_ATTENTION_UNROLL (8 or 16, default 8; process-wide): key/value rows a thread keeps in flight;

@@ -13,12 +13,13 @@
 namespace mi8 {
 
 // exp(x): n = rint(x*log2(e)), r = x - n*ln2 (two-term), degree-6 Taylor polynomial, scaled by 2^n.
-__device__ __forceinline__ float det_expf(float x) {
-  if(x < -87.0f)
-    return 0.0f;
-  if(x > 88.0f)
-    x = 88.0f;
-  const float n = rintf(__fmul_rn(x, 1.44269504f));
+// The rounding to an integer is done by adding and subtracting 1.5 * 2^23 (|x * log2(e)| < 128, so the sum's last bit is worth
+// one: round to nearest even, as rintf), which also leaves n in the low bits of the sum: two additions and a shift on the main
+// pipes in place of a rounding and a conversion, which issue at a quarter of their rate.
+// (det_expf_nonpos: the same for x <= 0 or NaN, without the upper clamp.)
+__device__ __forceinline__ float det_expf_nonpos(float x) {
+  const float t = __fadd_rn(__fmul_rn(x, 1.44269504f), 12582912.0f);
+  const float n = __fadd_rn(t, -12582912.0f);
   float r = __fmaf_rn(n, -0.693145752f, x);
   r = __fmaf_rn(n, -1.42860677e-06f, r);
   float p = 1.3888889e-3f;
@@ -28,9 +29,10 @@ __device__ __forceinline__ float det_expf(float x) {
   p = __fmaf_rn(p, r, 0.5f);
   p = __fmaf_rn(p, r, 1.0f);
   p = __fmaf_rn(p, r, 1.0f);
-  const int e = static_cast<int>(n);
-  return __fmul_rn(p, __int_as_float((e + 127) << 23));
+  const float y = __fmul_rn(p, __int_as_float((__float_as_int(t) << 23) + 0x3f800000));
+  return x < -87.0f ? 0.0f : y;
 }
+__device__ __forceinline__ float det_expf(float x) { return det_expf_nonpos(x > 88.0f ? 88.0f : x); }
 
 // log(x) for finite x > 0 (normal numbers): x = m * 2^e with m in [sqrt(1/2), sqrt(2)),
 // log(m) = 2 atanh(s), s = (m-1)/(m+1), odd series up to s^11.

@@ -103,6 +103,32 @@ def test_attention_bit_exact(cuda_device, oracle, mode, rows, batch, length, hea
         assert np.abs(want[r0, sl] - w @ v[idx][:, sl].astype(np.float64)).max() < 1e-4
 
 
+@pytest.mark.parametrize("rows", [3, 400])                     # 1024 and 256 threads per row
+@pytest.mark.parametrize("vocab,k", [(128, 1), (129, 2), (1000, 8), (1027, 8), (4096, 4), (32000, 4)])
+def test_lse_topk_awkward_rows(cuda_device, oracle, rows, vocab, k):
+    """Masked entries (lowest finite value, -inf), whole blocks of them, fewer usable entries than k, equal values everywhere."""
+    L, check = _lib()
+    rng = np.random.default_rng(vocab)
+    lowest = np.finfo(np.float32).min
+    x = rng.standard_normal((rows, vocab)).astype(np.float32)
+    x[0] = lowest
+    x[0, [vocab - 1, vocab // 2]] = [0.5, 0.25]                # two entries, the rest masked by the lowest value
+    x[1] = 0.75                                                # every entry ties
+    x[2] = -np.inf
+    x[2, vocab // 3::max(1, vocab // 5)] = lowest              # a few entries of the lowest value among -inf
+    x[2, vocab - 1] = 1.0
+    if rows > 3:
+        x[3:, ::3] = -np.inf
+    ld = _dev(x, cuda_device)
+    cs = torch.empty(rows, k, device=cuda_device)
+    cw = torch.empty(rows, k, dtype=torch.int32, device=cuda_device)
+    check(L.mi8g_lse_topk(ld.data_ptr(), rows, vocab, k, None, cs.data_ptr(), cw.data_ptr(), _stream()))
+    torch.cuda.synchronize()
+    cs_w, cw_w = oracle.lse_topk(x, k)
+    assert np.array_equal(cs.cpu().numpy(), cs_w, equal_nan=True)
+    assert np.array_equal(cw.cpu().numpy(), cw_w)
+
+
 @pytest.mark.parametrize("rows,vocab,k", [(3, 512, 1), (8, 32000, 4), (5, 1000, 8), (2, 300, 3), (7, 5000, 3), (4, 4100, 8), (3, 32000, 1), (3, 1001, 2), (2, 130, 8),
                                            (600, 32000, 4)])
 def test_lse_topk_and_merge_bit_exact(cuda_device, oracle, rows, vocab, k):
