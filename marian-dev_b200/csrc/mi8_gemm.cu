@@ -164,9 +164,10 @@ __device__ __forceinline__ unsigned pack4_i8(const float4& v, float qm) {
 // element `base` of C, of which `valid` exist; `valid` may exceed CH) and stores it:
 // float(acc) * unquant (+ bias) as two separately rounded operations, then ReLU.  Each stage runs over
 // the whole chunk so the columns overlap in the pipeline.  Returns the running max|C| bit pattern.
+// `paired`: all lanes of the warp are here, lane pairs own column pairs and those are 4-byte aligned in a half-precision C.
 template <int CH>
 __device__ __forceinline__ unsigned write_back_chunk(const GemmParams& p, const int32_t (&v)[CH], size_t base, int valid, float unquant,
-                                                     float bias_n, unsigned out_max, void* c, int ldc, bool has_bias) {
+                                                     float bias_n, unsigned out_max, void* c, int ldc, bool has_bias, bool paired) {
   float f[CH];
 #pragma unroll
   for(int j = 0; j < CH; ++j)
@@ -196,10 +197,26 @@ __device__ __forceinline__ unsigned write_back_chunk(const GemmParams& p, const 
   }
   if(p.out_f16) {
     __half* dst = reinterpret_cast<__half*>(c) + base;
+    if(paired && valid >= CH) {
+      // Two rows at a time: neighbouring lanes hold neighbouring columns, so one exchange gives the even lane both columns of the
+      // first row and the odd lane both of the second, and each stores four bytes.  Half the store instructions, one conversion
+      // per two values and no test per row.  Affines into half precision, before -> after: 4096 x 512 x 32000 367 -> 141 us,
+      // 4096 x 256 x 32000 226 -> 114 us, 3937 x 1024 x 4096 58 -> 47 us, 4096 x 1024 x 32000 (bound by the operands' way from L2) 161 -> 157 us.
+      const bool odd = threadIdx.x & 1;
+      __half* pair_dst = odd ? dst - 1 + ldc : dst;
 #pragma unroll
-    for(int j = 0; j < CH; ++j)
-      if(j < valid)
-        dst[static_cast<size_t>(j) * ldc] = __float2half_rn(f[j]);
+      for(int j = 0; j < CH; j += 2) {
+        const __half2 h = __floats2half2_rn(f[j], f[j + 1]);
+        const unsigned own = *reinterpret_cast<const unsigned*>(&h);
+        const unsigned other = __shfl_xor_sync(0xffffffffu, own, 1);
+        *reinterpret_cast<unsigned*>(pair_dst + static_cast<size_t>(j) * ldc) = __byte_perm(own, other, odd ? 0x3276 : 0x5410);
+      }
+    } else {
+#pragma unroll
+      for(int j = 0; j < CH; ++j)
+        if(j < valid)
+          dst[static_cast<size_t>(j) * ldc] = __float2half_rn(f[j]);
+    }
   } else {
     float* dst = reinterpret_cast<float*>(c) + base;
     if(valid >= CH) {
@@ -562,6 +579,8 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       const float* seg_bias = p.seg_bias[seg];
       void* seg_c = p.seg_c[seg];
       const int ldc = p.seg_n;
+      // (segments are 128 columns wide or more: n_loc has the parity of the lane)
+      const bool paired = p.out_f16 && (ldc & 1) == 0 && (reinterpret_cast<uintptr_t>(seg_c) & 3u) == 0 && __all_sync(0xffffffffu, n_ok);
       if constexpr(kTopK > 0) {
         // Output layer: lane = query row n, columns = vocabulary entries m0 .. m0 + TM - 1; warp group g takes
         // the 128-column block g of the tile.  Value = float(acc) * unquant + bias[column], rounded as in the
@@ -745,7 +764,7 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
                                              p8_off_b, bias_n);
           } else if(n_ok)
             out_max = write_back_chunk<T::kChunk>(p, v, static_cast<size_t>(m0 + col0) * ldc + n_loc, cols_valid - col0, unquant, bias_n,
-                                                  out_max, seg_c, ldc, seg_bias != nullptr);
+                                                  out_max, seg_c, ldc, seg_bias != nullptr, paired);
         }
       }
       if(p.absmax_out != nullptr) {
@@ -1023,6 +1042,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       const float* seg_bias = p.seg_bias[seg];
       void* seg_c = p.seg_c[seg];
       const int ldc = p.seg_n;
+      const bool paired = p.out_f16 && (ldc & 1) == 0 && (reinterpret_cast<uintptr_t>(seg_c) & 3u) == 0 && __all_sync(0xffffffffu, n_ok);
       const float bias_n = (seg_bias != nullptr && n_ok) ? __ldg(seg_bias + n_loc) : 0.0f;
       float p8_scale_b = 0.0f;
       int p8_zp_b = 0, p8_off_b = 0;
@@ -1048,7 +1068,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
                                            p8_off_b, bias_n);
         } else if(n_ok)
           out_max = write_back_chunk<T::kChunk>(p, v, static_cast<size_t>(m0 + col0) * ldc + n_loc, cols_valid - col0, unquant, bias_n, out_max,
-                                                seg_c, ldc, seg_bias != nullptr);
+                                                seg_c, ldc, seg_bias != nullptr, paired);
       }
       if(p.absmax_out != nullptr) {
         out_max = __reduce_max_sync(0xffffffffu, out_max);

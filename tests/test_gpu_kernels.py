@@ -169,6 +169,13 @@ def test_cta_pair_kernel_many_tiles(cuda_device, oracle):
     _run_affine(cuda_device, oracle, 2100, 1024, 1000, True, False, 13, out_dtype=torch.float16, tile_m=512)
 
 
+@pytest.mark.parametrize("m,k,n,tile_m", [(31, 64, 128, 32), (33, 64, 130, 32), (32, 64, 255, 0), (64, 64, 96, 64), (300, 128, 1022, 256), (257, 1024, 258, 512),
+                                          (16, 2048, 34, 16)])
+def test_half_output_edges(cuda_device, oracle, m, k, n, tile_m):
+    """Half-precision write-back: whole and ragged row chunks, odd row strides and column counts that end inside a warp."""
+    _run_affine(cuda_device, oracle, m, k, n, True, False, m + n, out_dtype=torch.float16, tile_m=tile_m)
+
+
 @pytest.mark.parametrize("tile_m", [0, 64, 128, 256, 512])
 def test_rows_from_keeps_whole_tiles_below(cuda_device, oracle, tile_m):
     """Equal words: tiles wholly below the row limit keep the sentinel, every other row is computed; unequal
