@@ -35,8 +35,8 @@ if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
 KERNEL_NAMES = ["mi8_gemm_pair_kernel", "mi8_gemm_kernel", "quantize_slot_kernel", "attention1_kernel", "attention_enc_kernel",
-                "add_layernorm_kernel", "quantize_dual_kernel", "history_commit_kernel", "lse_topk_kernel",
-                "lse_merge_kernel", "nbest_merge_kernel", "embed_kernel", "ancestors_update_kernel", "gather_rows_kernel",
+                "add_layernorm_kernel", "quantize_dual_kernel", "lse_topk_kernel",
+                "lse_merge_kernel", "nbest_merge_kernel", "step_begin_kernel", "embed_ancestors_kernel", "embed_kernel", "gather_rows_kernel",
                 "ssru_cell_kernel", "mi8_absmax_kernel", "mi8_quantize_kernel", "mi8_transpose_quantize_kernel"]
 METRIC = "int8_decode_tgt_tokens_per_sec"
 UNIT = "tokens/s"

@@ -143,12 +143,13 @@ struct mi8d_decoder {
   int* anc[2] = {nullptr, nullptr};
   // beam-search bookkeeping (mi8d_search): per-step control words and n-best lists, device side and pinned host side
   int* s_ctrl = nullptr;            // [3 * max_rows + max_batch]: hypothesis rows, previous words, path scores (as bits), batch rows
-  int* s_out = nullptr;             // [3][max_batch * 8]: scores (as bits), beams, words
-  int* h_ctrl = nullptr;
-  int* h_out = nullptr;
+  int* h_ctrl = nullptr;            // pinned; read by the step's first kernel
+  int* h_out = nullptr;             // pinned, [3][max_batch * 8]: scores (as bits), beams, words, written by the step's last kernel
   float *blk_max = nullptr, *blk_sum = nullptr, *blk_topv = nullptr;   // per (row, 128-word block) partials of the output layer
   int* blk_topi = nullptr;
   bool keep_logits = false;
+  const int* step_ctrl = nullptr;   // set by mi8d_search around a step: pinned control words to bring to s_ctrl first, and how many
+  int n_step_ctrl = 0;
   unsigned* slots = nullptr;
   int n_slots = 0;
   // packed8avx512: scale, zero point and sum of every row of the activation quantised last
@@ -215,8 +216,7 @@ struct mi8d_decoder {
     blk_sum = arena.take<float>(R * nb);
     blk_topv = arena.take<float>(R * nb * 8);
     blk_topi = arena.take<int>(R * nb * 8);
-    s_ctrl = arena.take<int>(3 * R + B);
-    s_out = arena.take<int>(3 * B * 8);
+    s_ctrl = arena.take<int>(3 * R + B);   // (the arena rounds every array up to 256 bytes)
     cand_score = arena.take<float>(R * 8);
     cand_word = arena.take<int>(R * 8);
     for(int i = 0; i < 2; ++i) {
@@ -233,7 +233,7 @@ struct mi8d_decoder {
       enc_h = arena.take<float>(M * f);
       enc_aq = arena.take<int8_t>(M * (f > d ? f : d) + 256);
     }
-    n_slots = kSlotsPerLayer * c.dec_depth + 8 + 4 * c.enc_depth;
+    n_slots = kSlotsPerLayer * c.dec_depth + 8 + 4 * c.enc_depth + c.max_batch;
     slots = arena.take<unsigned>(n_slots);
     const size_t max_act_rows = R > B * S ? R : B * S;
     p8_scale_a = arena.take<float>(max_act_rows);
@@ -255,6 +255,7 @@ struct mi8d_decoder {
   }
 
   unsigned* layer_slot(int l, int which) const { return slots + 1 + kSlotsPerLayer * l + which; }
+  unsigned* arrivals() const { return slots + n_slots - cfg.max_batch; }   // per sentence: rows whose candidates are ready
   unsigned* input_slot(int l) const { return l == 0 ? slots : layer_slot(l - 1, kSlotOut); }
   unsigned* enc_slot(int l, int which) const { return slots + 1 + kSlotsPerLayer * cfg.dec_depth + 4 * l + which; }
 
@@ -587,7 +588,7 @@ int mi8d_create(const mi8d_config* cfg, void* arena, size_t arena_bytes, void* w
     cudaMemset(d->reuse_stats, 0, 2 * sizeof(unsigned));
   {
     // pinned host staging for the beam search's per-step upload and download
-    const size_t nc = 3 * static_cast<size_t>(cfg->max_rows) + cfg->max_batch, no = 3 * static_cast<size_t>(cfg->max_batch) * 8;
+    const size_t nc = 3 * static_cast<size_t>(cfg->max_rows) + cfg->max_batch + 3, no = 3 * static_cast<size_t>(cfg->max_batch) * 8;
     if(cudaHostAlloc(reinterpret_cast<void**>(&d->h_ctrl), nc * sizeof(int), cudaHostAllocDefault) != cudaSuccess ||
        cudaHostAlloc(reinterpret_cast<void**>(&d->h_out), no * sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
       cudaGetLastError();
@@ -988,7 +989,7 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
   const size_t slab_stride = static_cast<size_t>(SR) * dm;
   const size_t n_d = static_cast<size_t>(R) * dm;
 
-  MI8D_CUDA(cudaMemsetAsync(d->slots, 0, sizeof(unsigned) * d->n_slots, s));
+  MI8D_TRY(launch_step_begin(d->step_ctrl, d->s_ctrl, d->n_step_ctrl, d->slots, d->n_slots, s));
 
   // sentences that finished leave the batch: compact the encoder context, recompute cross K/V
   if(batch != d->batch) {
@@ -1026,24 +1027,27 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
     d->cross_valid = true;
   }
 
-  // Ancestor table of this step and, in the same launch, every layer's history abs-max over the earlier slabs; the
-  // producer of a layer's newest slab (embedding / the previous layer's last LayerNorm) adds that slab's maximum.
+  // layer-0 input: scaled embedding of the previous word (zero at the first step) + position t.  For self-attention also, in the same
+  // launch, the ancestor table of this step and every layer's history abs-max over the earlier slabs; the producer of a
+  // layer's newest slab (this embedding / the previous layer's last LayerNorm) adds that slab's maximum.
   const int anc_new = d->anc_cur ^ 1;
-  if(!c.ssru) {
+  float* x = c.ssru ? d->x_in : d->layers[0].slab + static_cast<size_t>(t) * slab_stride;
+  const int* words = t == 0 ? nullptr : prev_words;
+  const float* pos = d->positions + static_cast<size_t>(t) * dm;
+  const float emb_scale = sqrtf(static_cast<float>(dm));
+  if(c.ssru) {
+    MI8D_TRY(launch_embed(d->wemb, words, pos, 0, emb_scale, R, dm, x, nullptr, d->input_slot(0), s));
+  } else {
     const float* rowmax[16];
     unsigned* hslot[16];
     for(int l = 0; l < c.dec_depth; ++l) {
       rowmax[l] = d->layers[l].rowmax;
       hslot[l] = d->layer_slot(l, kSlotHistory);
     }
-    MI8D_TRY(launch_ancestors_update(d->anc[d->anc_cur], d->anc[anc_new], hyp_idx, t, R, SR, s, d->p8 ? 0 : c.dec_depth, rowmax, hslot));
+    MI8D_TRY(launch_embed_ancestors(d->wemb, words, pos, emb_scale, dm, x, d->layers[0].rowmax + static_cast<size_t>(t) * SR, d->input_slot(0),
+                                    d->layer_slot(0, kSlotHistory), d->anc[d->anc_cur], d->anc[anc_new], hyp_idx, t, R, SR, s,
+                                    d->p8 ? 0 : c.dec_depth, rowmax, hslot));
   }
-
-  // layer-0 input: scaled embedding of the previous word (zero at the first step) + position t
-  float* x = c.ssru ? d->x_in : d->layers[0].slab + static_cast<size_t>(t) * slab_stride;
-  float* x_rowmax = c.ssru ? nullptr : d->layers[0].rowmax + static_cast<size_t>(t) * SR;
-  MI8D_TRY(launch_embed(d->wemb, t == 0 ? nullptr : prev_words, d->positions + static_cast<size_t>(t) * dm, 0, sqrtf(static_cast<float>(dm)), R,
-                        dm, x, x_rowmax, d->input_slot(0), s, c.ssru ? nullptr : d->layer_slot(0, kSlotHistory)));
 
   const int cell_new = d->cell_cur ^ 1;
   float* aq_tail = reinterpret_cast<float*>(d->aq + n_d);
@@ -1161,21 +1165,32 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
   // without candidate lists (beam 6, 2 sentences of transformer-base: 16.2 ms a mini-batch with the reducing write-back, 15.2 ms
   // without; student, 16 sentences x beam 4: 7.3 and 7.0; 64 x 4 and 128 x 4 rows: level).  opt_fused_out_rows > 0 brings the other back.
   const bool fused_output = !d->p8 && !d->keep_logits && R <= d->opt_fused_out_rows && n_best >= 2;
+  StepEnd end;
+  end.beam = beam;
+  end.batch = batch;
+  end.arrivals = d->arrivals();
+  end.out_score = out_score;
+  end.out_beam = out_beam;
+  end.out_word = out_word;
+  if(!c.ssru && !d->p8) {   // remember which abs-max the stored keys/values of every layer now belong to
+    end.layers = c.dec_depth;
+    end.first = 1 + kSlotHistory;
+    end.stride = kSlotsPerLayer;
+    end.slots = d->slots;
+    end.prev_bits = d->prev_bits;
+    end.stats = d->reuse_stats;
+  }
   if(!fused_output) {
     MI8D_TRY(gemm_act(d, d->aq, R, d->out_w, false, d->logits, s));
-    MI8D_TRY(launch_lse_topk(d->logits, R, c.vocab, n_best, prev_scores, d->cand_score, d->cand_word, s));
+    MI8D_TRY(launch_lse_topk(d->logits, R, c.vocab, n_best, prev_scores, d->cand_score, d->cand_word, s, end));
   } else {
     // the GEMM's write-back reduces every 128-word block of a row; the logits never reach memory
     const int k_top = n_best <= 4 ? 4 : 8;
     MI8D_TRY(launch_gemm_logits(d->aq, aq_tail, d->out_w.bt, d->out_w.qm, R, c.vocab, dm, d->out_bias, 1.0f, k_top, d->blk_max, d->blk_sum,
                                 d->blk_topv, d->blk_topi, nullptr, s));
     MI8D_TRY(launch_lse_merge(d->blk_max, d->blk_sum, d->blk_topv, d->blk_topi, R, c.vocab, k_top, n_best, prev_scores, d->cand_score,
-                              d->cand_word, s));
+                              d->cand_word, s, end));
   }
-  MI8D_TRY(launch_nbest_merge(d->cand_score, d->cand_word, beam, batch, c.vocab, n_best, out_score, out_beam, out_word, s));
-
-  if(!c.ssru && !d->p8)   // remember which abs-max the stored keys/values of every layer now belong to
-    MI8D_TRY(launch_history_commit(d->prev_bits, d->slots, 1 + kSlotHistory, kSlotsPerLayer, c.dec_depth, d->reuse_stats, s));
   d->anc_cur = anc_new;
   d->cell_cur = cell_new;
   d->t = t + 1;
@@ -1255,7 +1270,8 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
       for(int a = 0; a < nb; ++a)
         hc[3 * R + a] = step_map[active[a]];
       const size_t n_up = static_cast<size_t>(3 * R + nb) * sizeof(int);
-      MI8D_CUDA(cudaMemcpyAsync(d->s_ctrl, hc, n_up, cudaMemcpyHostToDevice, s));
+      d->step_ctrl = hc;
+      d->n_step_ctrl = 3 * R + nb;
       up_bytes += n_up;
       hyp = d->s_ctrl;
       pw = d->s_ctrl + R;
@@ -1263,14 +1279,16 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
       bidx = d->s_ctrl + 3 * R;
     }
     const int cells = nb * n_best;
-    float* o_score = reinterpret_cast<float*>(d->s_out);
-    int* o_beam = d->s_out + cells;
-    int* o_word = d->s_out + 2 * cells;
+    // the step's last kernel writes the n-best lists straight into pinned host memory
+    float* o_score = reinterpret_cast<float*>(d->h_out);
+    int* o_beam = d->h_out + cells;
+    int* o_word = d->h_out + 2 * cells;
     const clk::time_point t_a = clk::now();
     rc = mi8d_step(d, hyp, pw, bidx, ps, tensor_beam, nb, n_best, o_score, o_beam, o_word, stream);
+    d->step_ctrl = nullptr;
+    d->n_step_ctrl = 0;
     if(rc != MI8_OK)
       return rc;
-    MI8D_CUDA(cudaMemcpyAsync(d->h_out, d->s_out, static_cast<size_t>(3 * cells) * sizeof(int), cudaMemcpyDeviceToHost, s));
     const clk::time_point t_b = clk::now();
     if(d->opt_blocking_wait == 2 && d->ev_step != nullptr) {
       // several searches (and ranks) share the host's cores: poll, and hand the core to another thread between polls - as

@@ -41,16 +41,9 @@ __device__ __forceinline__ unsigned max4u(unsigned m, const float4& v) {
 
 // out[r,:] = wemb[words[r],:] * scale + pos[(pos_mod ? r % pos_mod : 0),:]
 // (words == nullptr: zero embedding, the start symbol; pos_mod = source width for the encoder, 0 for a decoder step)
-__global__ void __launch_bounds__(kRowThreads)
-embed_kernel(const float* __restrict__ wemb, const int* __restrict__ words, const float* __restrict__ pos, int pos_mod, float scale,
-             int dim, float* __restrict__ out, float* __restrict__ rowmax, unsigned* absmax_slot, unsigned* absmax_slot2) {
-  pdl_launch_dependents();
-  const TraceHandles th = trace_open_all();
-  unsigned long long* const tb = th.first;
-  pdl_wait();
-  trace_stamp_start(th, kTrEmbed);
-  __shared__ unsigned red[kRowThreads / 32];
-  const int r = blockIdx.x;
+__device__ __forceinline__ void embed_row(int r, const float* __restrict__ wemb, const int* __restrict__ words, const float* __restrict__ pos,
+                                          int pos_mod, float scale, int dim, float* __restrict__ out, float* __restrict__ rowmax,
+                                          unsigned* absmax_slot, unsigned* absmax_slot2, unsigned* red) {
   const float4* src = words ? reinterpret_cast<const float4*>(wemb + static_cast<size_t>(words[r]) * dim) : nullptr;
   const float4* p4 = reinterpret_cast<const float4*>(pos + static_cast<size_t>(pos_mod ? r % pos_mod : 0) * dim);
   float4* dst = reinterpret_cast<float4*>(out + static_cast<size_t>(r) * dim);
@@ -75,8 +68,36 @@ embed_kernel(const float* __restrict__ wemb, const int* __restrict__ words, cons
     if(absmax_slot2)
       atomicMax(absmax_slot2, m);
   }
+}
+
+__global__ void __launch_bounds__(kRowThreads)
+embed_kernel(const float* __restrict__ wemb, const int* __restrict__ words, const float* __restrict__ pos, int pos_mod, float scale,
+             int dim, float* __restrict__ out, float* __restrict__ rowmax, unsigned* absmax_slot) {
+  pdl_launch_dependents();
+  const TraceHandles th = trace_open_all();
+  unsigned long long* const tb = th.first;
+  pdl_wait();
+  trace_stamp_start(th, kTrEmbed);
+  __shared__ unsigned red[kRowThreads / 32];
+  embed_row(blockIdx.x, wemb, words, pos, pos_mod, scale, dim, out, rowmax, absmax_slot, nullptr, red);
   trace_stamp(tb, kTrEmbed, 2);
   trace_stamp(th.last, kTrEmbed, 3);
+}
+
+// The beginning of a decoder step: brings the step's control words (hypothesis rows, previous words, path scores, batch rows)
+// from pinned host memory to the device and zeroes the abs-max slots and arrival counters.  One block, one round trip over
+// PCIe, in place of a copy and a memset between the host's decision and the first kernel.  With finish_step and
+// embed_ancestors_kernel below, which take three more commands out of a step: student, one sentence 4.95 -> 4.78 ms;
+// student, 16 x beam 4 6.80 -> 6.55 ms; transformer-base, 16 x beam 4 19.27 -> 19.08 ms; transformer-big level.
+__global__ void __launch_bounds__(1024)
+step_begin_kernel(const int* host_ctrl, int* __restrict__ ctrl, int n_ctrl, unsigned* __restrict__ slots, int n_slots) {
+  pdl_launch_dependents();
+  pdl_wait();
+  for(int i = threadIdx.x; i < n_slots; i += blockDim.x)
+    slots[i] = 0u;
+  const int4* src = reinterpret_cast<const int4*>(host_ctrl);   // (both arrays are 16-byte aligned and padded to whole vectors)
+  for(int i = threadIdx.x; i < (n_ctrl + 3) / 4; i += blockDim.x)
+    reinterpret_cast<int4*>(ctrl)[i] = __ldcv(src + i);
 }
 
 // out = LayerNorm(a + resid) * gamma + beta, one block of 256 threads per row; biased variance
@@ -277,15 +298,9 @@ struct HistMaxArgs {
   const float* rowmax[kMaxHistLayers];
   unsigned* slot[kMaxHistLayers];
 };
-__global__ void __launch_bounds__(256)
-ancestors_update_kernel(const int* __restrict__ anc_old, int* __restrict__ anc_new, const int* __restrict__ hyp,
-                        int t, int rows, int stride, const HistMaxArgs hist) {
-  pdl_launch_dependents();
-  const TraceHandles th = trace_open_all();
-  unsigned long long* const tb = th.first;
-  pdl_wait();
-  trace_stamp_start(th, kTrAncestors);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void ancestors_slice(int block, const int* __restrict__ anc_old, int* __restrict__ anc_new, const int* __restrict__ hyp,
+                                                int t, int rows, int stride, const HistMaxArgs& hist) {
+  const int i = block * static_cast<int>(blockDim.x) + threadIdx.x;
   const bool in = i < (t + 1) * rows;
   int tp = 0, src = 0;
   if(in) {
@@ -300,31 +315,27 @@ ancestors_update_kernel(const int* __restrict__ anc_old, int* __restrict__ anc_n
     if((threadIdx.x & 31) == 0 && m != 0u)
       atomicMax(hist.slot[l], m);
   }
-  trace_stamp(tb, kTrAncestors, 2);
-  trace_stamp(th.last, kTrAncestors, 3);
 }
 
-// prev_bits[l] = slots[first + l * stride]: remembers, per layer, the abs-max the stored keys/values belong to.
-// stats[0] counts (layer, step) pairs whose abs-max was unchanged, stats[1] all pairs.
-__global__ void history_commit_kernel(unsigned* __restrict__ prev_bits, const unsigned* __restrict__ slots, int first, int stride, int layers,
-                                      unsigned* __restrict__ stats) {
+// The two independent jobs at the start of a self-attention decoder's step in one launch: blocks [0, rows) embed the previous
+// words (layer 0's newest slab), the others update the ancestor table and start the layers' history abs-max.
+__global__ void __launch_bounds__(kRowThreads)
+embed_ancestors_kernel(const float* __restrict__ wemb, const int* __restrict__ words, const float* __restrict__ pos, float scale, int dim,
+                       float* __restrict__ out, float* __restrict__ rowmax, unsigned* absmax_slot, unsigned* absmax_slot2,
+                       const int* __restrict__ anc_old, int* __restrict__ anc_new, const int* __restrict__ hyp, int t, int rows, int stride,
+                       const HistMaxArgs hist) {
   pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
   pdl_wait();
-  trace_stamp_start(th, kTrCommit);
-  const int l = threadIdx.x;
-  if(l < layers) {
-    const unsigned now = slots[first + l * stride];
-    if(stats) {
-      if(prev_bits[l] == now)
-        atomicAdd(stats, 1u);
-      atomicAdd(stats + 1, 1u);
-    }
-    prev_bits[l] = now;
-  }
-  trace_stamp(tb, kTrCommit, 2);
-  trace_stamp(th.last, kTrCommit, 3);
+  trace_stamp_start(th, kTrEmbed);
+  __shared__ unsigned red[kRowThreads / 32];
+  if(static_cast<int>(blockIdx.x) < rows)
+    embed_row(blockIdx.x, wemb, words, pos, 0, scale, dim, out, rowmax, absmax_slot, absmax_slot2, red);
+  else
+    ancestors_slice(static_cast<int>(blockIdx.x) - rows, anc_old, anc_new, hyp, t, rows, stride, hist);
+  trace_stamp(tb, kTrEmbed, 2);
+  trace_stamp(th.last, kTrEmbed, 3);
 }
 
 // ---- single-query attention --------------------------------------------------------------------
@@ -637,6 +648,69 @@ __device__ __forceinline__ void topk_block_merge(float* s_v, int* s_i) {
   }
 }
 
+// The end of a step, run by whichever block of the output layer's last kernel finishes a sentence's last row (an arrival counter per
+// sentence, zeroed at the start of the step): the beam x k row candidates of sentence b (rows beam-major: row = j * batch + b)
+// become its k best, sorted; on ties the smaller flattened key (beam, word) first.  A candidate's place is the number of valid
+// candidates before it; places that stay empty get score -inf, beam 0, word 0.  Block 0 also remembers, per layer, the history
+// abs-max the stored keys/values now belong to (prev_bits[l] = slots[first + l * stride]; stats: pairs unchanged, all pairs).
+// In place of two launches, each of a launch's hand-over (6 us together in a transformer-base step).
+__device__ __forceinline__ void finish_step(const StepEnd& e, int r, int k, int vocab, const float* cand_score, const int* cand_word, float* c_v,
+                                            int* c_i, int* s_last) {
+  if(blockIdx.x == 0 && static_cast<int>(threadIdx.x) < e.layers) {
+    const unsigned now = e.slots[e.first + threadIdx.x * e.stride];
+    if(e.prev_bits[threadIdx.x] == now)
+      atomicAdd(e.stats, 1u);
+    atomicAdd(e.stats + 1, 1u);
+    e.prev_bits[threadIdx.x] = now;
+  }
+  if(e.arrivals == nullptr)
+    return;
+  const int b = r % e.batch;
+  __syncthreads();   // the row's candidates are written
+  if(threadIdx.x == 0) {
+    __threadfence();
+    *s_last = atomicAdd(e.arrivals + b, 1u) == static_cast<unsigned>(e.beam - 1) ? 1 : 0;
+    __threadfence();
+  }
+  __syncthreads();
+  if(!*s_last || threadIdx.x >= 32)
+    return;
+  const int n = e.beam * k;   // at most kMaxK * kMaxK
+  int valid = 0;
+  for(int c0 = 0; c0 < n; c0 += 32) {
+    const int c = c0 + threadIdx.x;
+    bool ok = false;
+    if(c < n) {
+      const int row = (c / k) * e.batch + b;
+      const float v = __ldcg(cand_score + row * k + c % k);
+      ok = v > -FLT_MAX;   // (not -inf: a dummy hypothesis; not the filler of a row with fewer than k entries)
+      c_v[c] = v;
+      c_i[c] = ok ? (c / k) * vocab + __ldcg(cand_word + row * k + c % k) : 0x7fffffff;
+    }
+    valid += __popc(__ballot_sync(0xffffffffu, ok));
+  }
+  __syncwarp();
+  for(int c = threadIdx.x; c < n; c += 32) {
+    const float v = c_v[c];
+    const int key = c_i[c];
+    if(v > -FLT_MAX) {
+      int place = 0;
+      for(int o = 0; o < n; ++o)
+        place += (c_v[o] > -FLT_MAX && better(c_v[o], c_i[o], v, key)) ? 1 : 0;
+      if(place < k) {
+        e.out_score[b * k + place] = v;
+        e.out_beam[b * k + place] = key / vocab;
+        e.out_word[b * k + place] = key % vocab;
+      }
+    }
+  }
+  for(int c = valid + threadIdx.x; c < k; c += 32) {
+    e.out_score[b * k + c] = -INFINITY;
+    e.out_beam[b * k + c] = 0;
+    e.out_word[b * k + c] = 0;
+  }
+}
+
 // Combines the per-block pairs (m_b, s_b) of one row, held in shared memory, into the row's log-sum-exp:
 // M = max_b m_b;  S = sum over b ascending of s_b * exp(m_b - M), product and sum rounded separately;
 // lse = M + log(S).  bm/bs: nb entries each; red: 33 floats.  Every thread returns the same value.
@@ -685,8 +759,8 @@ __device__ __forceinline__ float lse_from_blocks(float* bm, float* bs, int nb, f
 // kThreads: 1024 (one pass over 32000 logits) while there is at most a block per half SM, 256 otherwise.
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads)
-lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float* __restrict__ prev_scores, float* __restrict__ cand_score,
-                int* __restrict__ cand_word) {
+lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float* __restrict__ prev_scores, float* cand_score, int* cand_word,
+                const StepEnd end) {
   pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
@@ -698,6 +772,7 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
   __shared__ float red[33];
   __shared__ int pick[kMaxK];
   __shared__ int n_cand;
+  __shared__ int s_last;
   __shared__ float s_floor;
   const int r = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -857,6 +932,8 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
       }
     }
   }
+  __syncthreads();   // (c_v and c_i are reused)
+  finish_step(end, r, k, vocab, cand_score, cand_word, c_v, c_i, &s_last);
   trace_stamp(tb, kTrLseTopk, 2);
   trace_stamp(th.last, kTrLseTopk, 3);
 }
@@ -868,8 +945,8 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
 template <int KT>
 __global__ void __launch_bounds__(256)
 lse_merge_kernel(const float* __restrict__ blk_max, const float* __restrict__ blk_sum, const float* __restrict__ blk_topv,
-                 const int* __restrict__ blk_topi, int nb, int k, const float* __restrict__ prev_scores, float* __restrict__ cand_score,
-                 int* __restrict__ cand_word) {
+                 const int* __restrict__ blk_topi, int nb, int k, const float* __restrict__ prev_scores, float* cand_score, int* cand_word, int vocab,
+                 const StepEnd end) {
   pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
@@ -879,6 +956,7 @@ lse_merge_kernel(const float* __restrict__ blk_max, const float* __restrict__ bl
   __shared__ float s_v[256 * KT];
   __shared__ int s_i[256 * KT];
   __shared__ float red[33];
+  __shared__ int s_last;
   const int r = blockIdx.x;
   float* bm = lse_blocks;
   float* bs = lse_blocks + nb;
@@ -909,6 +987,8 @@ lse_merge_kernel(const float* __restrict__ blk_max, const float* __restrict__ bl
     cand_score[r * k + threadIdx.x] = __fadd_rn(__fadd_rn(s_v[threadIdx.x], -lse), ps);
     cand_word[r * k + threadIdx.x] = s_i[threadIdx.x];
   }
+  __syncthreads();   // (s_v and s_i are reused)
+  finish_step(end, r, k, vocab, cand_score, cand_word, s_v, s_i, &s_last);
   trace_stamp(tb, kTrLseMerge, 2);
   trace_stamp(th.last, kTrLseMerge, 3);
 }
@@ -1014,10 +1094,16 @@ void set_attention_block_heads(int h) { g_attention_block_heads = h; }
 
 // ------------------------------------------------------------------------------------------------ launchers
 int launch_embed(const float* wemb, const int* words, const float* pos, int pos_mod, float scale, int rows, int dim, float* out,
-                 float* rowmax, unsigned* slot, cudaStream_t s, unsigned* slot2) {
+                 float* rowmax, unsigned* slot, cudaStream_t s) {
   if(rows <= 0 || dim <= 0 || dim % 4 != 0 || dim > kRowThreads * 4 * kMaxVec || out == nullptr || pos == nullptr)
     return MI8_ERR_BAD_ARG;
-  launch_kernel(embed_kernel, dim3(rows), dim3(kRowThreads), 0, s, wemb, words, pos, pos_mod, scale, dim, out, rowmax, slot, slot2);
+  launch_kernel(embed_kernel, dim3(rows), dim3(kRowThreads), 0, s, wemb, words, pos, pos_mod, scale, dim, out, rowmax, slot);
+  count_launch();
+  return check_launch();
+}
+
+int launch_step_begin(const int* host_ctrl, int* ctrl, int n_ctrl, unsigned* slots, int n_slots, cudaStream_t s) {
+  launch_kernel(step_begin_kernel, dim3(1), dim3(1024), 0, s, host_ctrl, ctrl, n_ctrl, slots, n_slots);
   count_launch();
   return check_launch();
 }
@@ -1047,8 +1133,11 @@ int launch_quantize_slot(const float* x, size_t n, const unsigned* slot, int8_t*
   return check_launch();
 }
 
-int launch_ancestors_update(const int* anc_old, int* anc_new, const int* hyp, int t, int rows, int stride, cudaStream_t s,
-                            int hist_layers, const float* const* hist_rowmax, unsigned* const* hist_slot) {
+int launch_embed_ancestors(const float* wemb, const int* words, const float* pos, float scale, int dim, float* out, float* rowmax, unsigned* slot,
+                           unsigned* slot2, const int* anc_old, int* anc_new, const int* hyp, int t, int rows, int stride, cudaStream_t s,
+                           int hist_layers, const float* const* hist_rowmax, unsigned* const* hist_slot) {
+  if(rows <= 0 || dim <= 0 || dim % 4 != 0 || dim > kRowThreads * 4 * kMaxVec || out == nullptr || pos == nullptr)
+    return MI8_ERR_BAD_ARG;
   if(hist_layers < 0 || hist_layers > kMaxHistLayers)
     return MI8_ERR_UNSUPPORTED;
   HistMaxArgs hist;
@@ -1058,7 +1147,8 @@ int launch_ancestors_update(const int* anc_old, int* anc_new, const int* hyp, in
     hist.slot[l] = l < hist_layers ? hist_slot[l] : nullptr;
   }
   const int n = (t + 1) * rows;
-  launch_kernel(ancestors_update_kernel, dim3((n + 255) / 256), dim3(256), 0, s, anc_old, anc_new, hyp, t, rows, stride, hist);
+  launch_kernel(embed_ancestors_kernel, dim3(rows + (n + kRowThreads - 1) / kRowThreads), dim3(kRowThreads), 0, s, wemb, words, pos, scale, dim, out,
+                rowmax, slot, slot2, anc_old, anc_new, hyp, t, rows, stride, hist);
   count_launch();
   return check_launch();
 }
@@ -1083,14 +1173,6 @@ int launch_quantize_dual(const float* x, size_t n, const unsigned* slot_x, int8_
   bh = bh > hcap ? hcap : bh;
   launch_kernel(quantize_dual_kernel, dim3(static_cast<unsigned>(bx) + bh), dim3(256), 0, s, x, n, slot_x, q, qm_x, status,
                 static_cast<int>(bx), slabs, slab_rows, steps, rows_new, dim, slot_h, prev_bits, hq, qm_h);
-  count_launch();
-  return check_launch();
-}
-
-int launch_history_commit(unsigned* prev_bits, const unsigned* slots, int first, int stride, int layers, unsigned* stats, cudaStream_t s) {
-  if(layers > 64)
-    return MI8_ERR_UNSUPPORTED;
-  launch_kernel(history_commit_kernel, dim3(1), dim3(64), 0, s, prev_bits, slots, first, stride, layers, stats);
   count_launch();
   return check_launch();
 }
@@ -1159,7 +1241,7 @@ int launch_attention1(const float* q, const float* k, const float* v, const floa
 }
 
 int launch_lse_topk(const float* logits, int rows, int vocab, int k, const float* prev_scores, float* cand_score, int* cand_word,
-                    cudaStream_t s) {
+                    cudaStream_t s, const StepEnd& end) {
   if(rows <= 0 || vocab <= 0 || k < 1 || k > kMaxK)
     return MI8_ERR_BAD_ARG;
   const size_t smem = 2 * static_cast<size_t>((vocab + 127) / 128) * sizeof(float);
@@ -1167,15 +1249,15 @@ int launch_lse_topk(const float* logits, int rows, int vocab, int k, const float
     return MI8_ERR_UNSUPPORTED;
   // Few rows: 1024 threads each, so that a row of 32000 takes one pass. 
   if(rows <= 2 * sm_count())
-    launch_kernel(lse_topk_kernel<1024>, dim3(rows), dim3(1024), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word);
+    launch_kernel(lse_topk_kernel<1024>, dim3(rows), dim3(1024), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word, end);
   else
-    launch_kernel(lse_topk_kernel<256>, dim3(rows), dim3(256), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word);
+    launch_kernel(lse_topk_kernel<256>, dim3(rows), dim3(256), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word, end);
   count_launch();
   return check_launch();
 }
 
 int launch_lse_merge(const float* blk_max, const float* blk_sum, const float* blk_topv, const int* blk_topi, int rows, int vocab,
-                     int k_top, int k, const float* prev_scores, float* cand_score, int* cand_word, cudaStream_t s) {
+                     int k_top, int k, const float* prev_scores, float* cand_score, int* cand_word, cudaStream_t s, const StepEnd& end) {
   if(rows <= 0 || vocab <= 0 || k < 1 || k > k_top || (k_top != 4 && k_top != 8))
     return MI8_ERR_BAD_ARG;
   const int nb = (vocab + 127) / 128;
@@ -1184,10 +1266,10 @@ int launch_lse_merge(const float* blk_max, const float* blk_sum, const float* bl
     return MI8_ERR_UNSUPPORTED;
   if(k_top == 4)
     launch_kernel(lse_merge_kernel<4>, dim3(rows), dim3(256), smem, s, blk_max, blk_sum, blk_topv, blk_topi, nb, k, prev_scores, cand_score,
-                  cand_word);
+                  cand_word, vocab, end);
   else
     launch_kernel(lse_merge_kernel<8>, dim3(rows), dim3(256), smem, s, blk_max, blk_sum, blk_topv, blk_topi, nb, k, prev_scores, cand_score,
-                  cand_word);
+                  cand_word, vocab, end);
   count_launch();
   return check_launch();
 }

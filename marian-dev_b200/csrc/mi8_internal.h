@@ -154,6 +154,20 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
                    const float* scale_b, const int32_t* zp_b, const int32_t* off_b, int M, int N, int K, const float* bias, int relu,
                    float* c, int32_t* acc_out, void* ws, size_t ws_bytes, cudaStream_t stream, int force_tile_m, int force_splits);
 
+// What the last kernel of a decoder step does besides the rows' candidates: the n-best lists of the sentences (arrivals != nullptr; one
+// zeroed counter per sentence; the outputs may be pinned host memory) and the record of the history abs-max per layer (layers > 0).
+struct StepEnd {
+  int beam = 0, batch = 0;
+  unsigned* arrivals = nullptr;
+  float* out_score = nullptr;
+  int* out_beam = nullptr;
+  int* out_word = nullptr;
+  int layers = 0, first = 0, stride = 0;
+  const unsigned* slots = nullptr;
+  unsigned* prev_bits = nullptr;
+  unsigned* stats = nullptr;
+};
+
 // Output layer: GEMM whose write-back reduces every (row, block of 128 vocabulary entries) to its maximum, its sum
 // of exponentials and its k_top (4 or 8) best entries (blk_* arrays: [rows][ceil(vocab/128)] (x k_top)); then
 // launch_lse_merge turns those into the per-row candidates launch_lse_topk would have produced from the logits.
@@ -161,18 +175,22 @@ int launch_gemm_logits(const int8_t* aq, const float* d_qa, const int8_t* wq, co
                        const float* bias, float scale, int k_top, float* blk_max, float* blk_sum, float* blk_topv, int* blk_topi,
                        float* logits_out, cudaStream_t stream);
 int launch_lse_merge(const float* blk_max, const float* blk_sum, const float* blk_topv, const int* blk_topi, int rows, int vocab,
-                     int k_top, int k, const float* prev_scores, float* cand_score, int* cand_word, cudaStream_t s);
+                     int k_top, int k, const float* prev_scores, float* cand_score, int* cand_word, cudaStream_t s, const StepEnd& end = StepEnd());
 
 // decode-step glue (mi8_glue.cu)
-// slot2 (optional): a second 4-byte slot that receives the same maximum (the self-attention history's abs-max)
 int launch_embed(const float* wemb, const int* words, const float* pos, int pos_mod, float scale, int rows, int dim, float* out,
-                 float* rowmax, unsigned* slot, cudaStream_t s, unsigned* slot2 = nullptr);
+                 float* rowmax, unsigned* slot, cudaStream_t s);
+// host_ctrl: pinned host memory; ctrl and host_ctrl 16-byte aligned, room for whole 16-byte vectors
+int launch_step_begin(const int* host_ctrl, int* ctrl, int n_ctrl, unsigned* slots, int n_slots, cudaStream_t s);
+// slot2 (optional): a second 4-byte slot that receives the same maximum (the self-attention history's abs-max)
 int launch_add_layernorm(const float* a, const float* resid, const float* gamma, const float* beta, float eps, int rows, int dim,
                          float* out, float* rowmax, unsigned* slot, cudaStream_t s, unsigned* slot2 = nullptr);
 int launch_quantize_slot(const float* x, size_t n, const unsigned* slot, int8_t* q, float* d_qm, cudaStream_t s);
-// hist_layers > 0: also reduces, per layer, the maximum of rowmax over the earlier slabs' ancestor rows into hist_slot[l]
-int launch_ancestors_update(const int* anc_old, int* anc_new, const int* hyp, int t, int rows, int stride, cudaStream_t s,
-                            int hist_layers = 0, const float* const* hist_rowmax = nullptr, unsigned* const* hist_slot = nullptr);
+// the embedding of a step (slot2: the history's abs-max of layer 0) and the ancestor table; hist_layers > 0: also reduces, per layer, the
+// maximum of rowmax over the earlier slabs' ancestor rows into hist_slot[l]
+int launch_embed_ancestors(const float* wemb, const int* words, const float* pos, float scale, int dim, float* out, float* rowmax, unsigned* slot,
+                           unsigned* slot2, const int* anc_old, int* anc_new, const int* hyp, int t, int rows, int stride, cudaStream_t s,
+                           int hist_layers, const float* const* hist_rowmax, unsigned* const* hist_slot);
 // layer input x and the self-attention history quantised by one launch (see quantize_dual_kernel)
 int launch_quantize_dual(const float* x, size_t n, const unsigned* slot_x, int8_t* q, float* qm_x, const float* slabs, int slab_rows,
                          int steps, int rows_new, int dim, const unsigned* slot_h, const unsigned* prev_bits, int8_t* hq, float* qm_h,
@@ -183,12 +201,11 @@ void set_attention_block_heads(int h);
 int trace_set_glue(unsigned long long* buf);
 int trace_set_gemm(unsigned long long* buf);
 int trace_set_quant(unsigned long long* buf);
-int launch_history_commit(unsigned* prev_bits, const unsigned* slots, int first, int stride, int layers, unsigned* stats, cudaStream_t s);
 int launch_attention1(const float* q, const float* k, const float* v, const float* log_mask, int rows, int heads, int dim_head,
                       int len, int batch, int mode, float* out, unsigned* slot, cudaStream_t s, const int* anc = nullptr,
                       int anc_stride = 0, int kv_rows = 0);
 int launch_lse_topk(const float* logits, int rows, int vocab, int k, const float* prev_scores, float* cand_score, int* cand_word,
-                    cudaStream_t s);
+                    cudaStream_t s, const StepEnd& end = StepEnd());
 int launch_nbest_merge(const float* cand_score, const int* cand_word, int beam, int batch, int vocab, int k, float* out_score,
                        int* out_beam, int* out_word, cudaStream_t s);
 int launch_gather_rows(const float* in, const int* idx, int rows, int dim, float* out, cudaStream_t s);
