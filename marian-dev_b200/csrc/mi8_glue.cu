@@ -338,6 +338,35 @@ embed_ancestors_kernel(const float* __restrict__ wemb, const int* __restrict__ w
   trace_stamp(th.last, kTrEmbed, 3);
 }
 
+// The butterfly of the G threads of a head, for U positions at once: at the level that pairs lanes j and j ^ o the two
+// lanes split the positions still held between them - each sends the partial sums of the half it gives up and adds
+// what it receives to the half it keeps - so a level costs half as many shuffles and additions as the one before,
+// instead of one of each per position.  Every sum is "own + partner's" of the same two operands as in the plain
+// butterfly, hence the same bits.  Once a lane holds a single position the remaining levels are the plain butterfly.
+// Returns the first position lane j holds afterwards (its sum in d[0], with U > G the next U / G - 1 behind it).
+template <int G, int U>
+__device__ __forceinline__ int head_butterfly(float (&d)[U], int j) {
+  int pos = 0;
+#pragma unroll
+  for(int lvl = 0; ((G / 2) >> lvl) > 0; ++lvl) {
+    const int o = (G / 2) >> lvl;
+    const int c = (U >> lvl) > 1 ? (U >> lvl) : 1;   // positions a lane holds before this level
+    if(c > 1) {
+      const bool upper = (j & o) != 0;
+#pragma unroll
+      for(int i = 0; i < c / 2; ++i) {
+        const float send = upper ? d[i] : d[i + c / 2];
+        const float keep = upper ? d[i + c / 2] : d[i];
+        d[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, o));
+      }
+      pos += upper ? c / 2 : 0;
+    } else {
+      d[0] = __fadd_rn(d[0], __shfl_xor_sync(0xffffffffu, d[0], o));
+    }
+  }
+  return pos;
+}
+
 // ---- single-query attention --------------------------------------------------------------------
 // One block per query row; thread i owns elements 4i..4i+3 of the model dimension, i.e. a quarter-row
 // slice of head i / G with G = DH/4 threads per head.  For every key position the block reads the whole
@@ -410,29 +439,7 @@ attention1_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
       d[u] = __fmaf_rn(qv.z, kk[u].z, d[u]);
       d[u] = __fmaf_rn(qv.w, kk[u].w, d[u]);
     }
-    // The butterfly of the G threads of a head, for U positions at once: at the level that pairs lanes j and j ^ o the two
-    // lanes split the positions still held between them - each sends the partial sums of the half it gives up and adds
-    // what it receives to the half it keeps - so a level costs half as many shuffles and additions as the one before,
-    // instead of one of each per position.  Every sum is "own + partner's" of the same two operands as in the plain
-    // butterfly, hence the same bits.  Once a lane holds a single position the remaining levels are the plain butterfly.
-    int pos = 0;
-#pragma unroll
-    for(int lvl = 0; ((G / 2) >> lvl) > 0; ++lvl) {
-      const int o = (G / 2) >> lvl;
-      const int c = (U >> lvl) > 1 ? (U >> lvl) : 1;   // positions a lane holds before this level
-      if(c > 1) {
-        const bool upper = (j & o) != 0;
-#pragma unroll
-        for(int i = 0; i < c / 2; ++i) {
-          const float send = upper ? d[i] : d[i + c / 2];
-          const float keep = upper ? d[i + c / 2] : d[i];
-          d[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, o));
-        }
-        pos += upper ? c / 2 : 0;
-      } else {
-        d[0] = __fadd_rn(d[0], __shfl_xor_sync(0xffffffffu, d[0], o));
-      }
-    }
+    const int pos = head_butterfly<G, U>(d, j);
     // lanes that differ only in the bits of the plain levels hold the same position: the one with those bits clear writes
     // (with more positions than lanes a lane ends up holding U / G neighbouring positions)
     constexpr int kPlainMask = (U >= G) ? 0 : (G / U) - 1;
@@ -499,6 +506,185 @@ attention1_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     m_abs = __reduce_max_sync(0xffffffffu, m_abs);
     if((threadIdx.x & 31) == 0 && m_abs != 0u)
       atomicMax(absmax_slot, m_abs);
+  }
+  trace_stamp(tb, kTrAttention1, 2);
+  trace_stamp(th.last, kTrAttention1, 3);
+}
+
+// Cross-attention (mode 1) for all hypotheses of a sentence together.  attention1_kernel reads a sentence's keys and values once
+// per hypothesis (through L2) and waits for eight rows at a time.  Here a block serves 32 consecutive four-element slices
+// (32 / G heads) of one sentence, a warp per hypothesis: every key and value row is copied once into a ring of
+// kCrossStages x kCrossRows rows of shared memory, up to 32 rows ahead of their use and the first value rows during the softmax, and
+// read from there by all warps.  Arithmetic and order per (row, head): those of attention1_kernel.
+// A warp per hypothesis rather than one warp for all of them (each row read from shared memory once, four times the
+// registers): the small batches need the warps - 64 sentences x beam 4 x 512 are 256 warps that way, 11.8 us inside a step.
+// Bound by the chain of instructions of a warp and, where the keys and values of all layers exceed L2, by their read.
+// Inside a decoder step, attention1_kernel -> here: transformer-base 64 x beam 4 x 38 positions 11.7 -> 8.5 us, transformer-big 128 x beam 4
+// 15.1 -> 11 us; whole mini-batches: transformer-base, 64 x beam 4 40.7 -> 38.4 ms, big 46.4 -> 45.7 ms, four searches of big 219.5 -> 216.5 ms.
+constexpr int kCrossStages = 3;
+constexpr int kCrossRows = 16;     // rows per stage of the ring
+constexpr int kCrossU = 8;         // positions whose scores a warp sums at once
+constexpr int kCrossMaxBeams = 8;  // hypotheses per block
+
+__device__ __forceinline__ void prefetch_l2(const void* p, int bytes) {   // 16-byte aligned, a multiple of 16 bytes
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy16_async(void* smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+template <int DH>
+__global__ void __launch_bounds__(kCrossMaxBeams * 32)
+attention_cross_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                       const float* __restrict__ log_mask, int heads, int len, int rows, int batch, float scale, float* __restrict__ out,
+                       unsigned* absmax_slot) {
+  pdl_launch_dependents();
+  const TraceHandles th = trace_open_all();
+  unsigned long long* const tb = th.first;
+  constexpr int G = DH / 4, U = kCrossU, SR = kCrossRows;
+  constexpr int kWarpHeads = 32 / G;
+  static_assert(U <= G, "a lane holds one position after the butterfly");
+  extern __shared__ float4 cross_smem[];   // [stages][SR][32] rows, then per warp and head [len4] scores
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int j = lane % G;
+  const int dim = heads * DH;
+  const int slice = blockIdx.y * 32 + lane;   // this lane's four elements of the model dimension
+  const bool active = slice < dim / 4;        // (whole heads are active or not)
+  const int b = blockIdx.x;
+  const int r = (blockIdx.z * warps + warp) * batch + b;
+  const bool live = active && r < rows;
+  const int len4 = (len + 3) & ~3;
+  float* scores = reinterpret_cast<float*>(cross_smem + kCrossStages * SR * 32);
+  float* sc = scores + (warp * kWarpHeads + lane / G) * len4;
+  const size_t kv0 = static_cast<size_t>(b) * len * dim + 4 * slice;
+  const int tiles = (len + SR - 1) / SR;
+  // rows SR i .. SR i + SR - 1 of the keys (i < tiles), then of the values; the warps share the rows out
+  auto fetch = [&](int i) {
+    if(active && i < 2 * tiles) {
+      const int p0 = (i < tiles ? i : i - tiles) * SR;
+      const float* src = (i < tiles ? k : v) + kv0 + static_cast<size_t>(p0 + warp) * dim;
+      float4* dst = cross_smem + (i % kCrossStages) * (SR * 32) + lane;
+      const int n = min(SR, len - p0);
+      for(int u = warp; u < n; u += warps, src += static_cast<size_t>(warps) * dim)
+        copy16_async(dst + u * 32, src);
+    }
+    copy_commit();
+  };
+  // stage i is complete and the slot of stage i - 1 free again
+  auto advance = [&](int i) {
+    copy_wait<kCrossStages - 2>();
+    __syncthreads();
+    fetch(i + kCrossStages - 1);
+    return cross_smem + (i % kCrossStages) * (SR * 32) + lane;
+  };
+  // The keys and values were projected long before the preceding kernel: their way from HBM to L2 starts while that one runs.
+  // (A prefetch reads nothing into the program, so it may come before the wait even where they are still being written.)
+  {
+    const int bytes = min(512, (dim - static_cast<int>(blockIdx.y) * 128) * 4);
+    for(int i = threadIdx.x; i < 2 * len; i += blockDim.x)
+      prefetch_l2((i < len ? k : v) + (static_cast<size_t>(b) * len + (i < len ? i : i - len)) * dim + blockIdx.y * 128, bytes);
+  }
+  pdl_wait();
+  trace_stamp_start(th, kTrAttention1);
+#pragma unroll
+  for(int i = 0; i < kCrossStages - 1; ++i)
+    fetch(i);
+  const float4 qv = live ? __ldg(reinterpret_cast<const float4*>(q + static_cast<size_t>(r) * dim) + slice) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float* mask = log_mask ? log_mask + static_cast<size_t>(b) * len : nullptr;
+  constexpr int kPlainMask = (U >= G) ? 0 : (G / U) - 1;   // lanes that differ only in these bits hold the same position
+  for(int i = 0; i < tiles; ++i) {
+    const float4* src = advance(i);
+#pragma unroll
+    for(int h = 0; h < SR; h += U) {
+      if(i * SR + h < len) {
+        float d[U];
+#pragma unroll
+        for(int u = 0; u < U; ++u) {   // (rows past the end: whatever the ring holds; their sums are not written)
+          const float4 kk = src[(h + u) * 32];
+          d[u] = __fmul_rn(qv.x, kk.x);
+          d[u] = __fmaf_rn(qv.y, kk.y, d[u]);
+          d[u] = __fmaf_rn(qv.z, kk.z, d[u]);
+          d[u] = __fmaf_rn(qv.w, kk.w, d[u]);
+        }
+        const int p = i * SR + h + head_butterfly<G, U>(d, j);
+        if(active && (j & kPlainMask) == 0 && p < len) {
+          float s = __fmul_rn(d[0], scale);
+          if(mask)
+            s = __fadd_rn(s, __ldg(mask + p));
+          sc[p] = s;
+        }
+      }
+    }
+  }
+  __syncwarp();
+  float mx = -FLT_MAX, part = 0.f;
+  if(active)
+    for(int p = j; p < len; p += G)
+      mx = fmaxf(mx, sc[p]);
+#pragma unroll
+  for(int o = G / 2; o > 0; o >>= 1)
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if(active)
+    for(int p = j; p < len; p += G) {
+      const float e = det_expf(__fadd_rn(sc[p], -mx));
+      sc[p] = e;
+      part = __fadd_rn(part, e);
+    }
+#pragma unroll
+  for(int o = G / 2; o > 0; o >>= 1)
+    part = __fadd_rn(part, __shfl_xor_sync(0xffffffffu, part, o));
+  if(active)
+    for(int p = j; p < len; p += G)
+      sc[p] = __fdiv_rn(sc[p], part);
+  __syncwarp();
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for(int i = 0; i < tiles; ++i) {
+    const float4* src = advance(tiles + i);
+    const int n = active ? min(SR, len - i * SR) : 0;
+    const float* w = sc + i * SR;
+    int u = 0;
+    for(; u + 4 <= n; u += 4) {
+      const float4 w4 = *reinterpret_cast<const float4*>(w + u);
+      const float wu[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+      for(int e = 0; e < 4; ++e) {
+        const float4 vv = src[(u + e) * 32];
+        acc.x = __fmaf_rn(wu[e], vv.x, acc.x);
+        acc.y = __fmaf_rn(wu[e], vv.y, acc.y);
+        acc.z = __fmaf_rn(wu[e], vv.z, acc.z);
+        acc.w = __fmaf_rn(wu[e], vv.w, acc.w);
+      }
+    }
+    for(; u < n; ++u) {
+      const float4 vv = src[u * 32];
+      acc.x = __fmaf_rn(w[u], vv.x, acc.x);
+      acc.y = __fmaf_rn(w[u], vv.y, acc.y);
+      acc.z = __fmaf_rn(w[u], vv.z, acc.z);
+      acc.w = __fmaf_rn(w[u], vv.w, acc.w);
+    }
+  }
+  unsigned m_abs = 0u;
+  if(live) {
+    reinterpret_cast<float4*>(out + static_cast<size_t>(r) * dim)[slice] = acc;
+    m_abs = max4u(0u, acc);
+  }
+  if(absmax_slot) {   // one atomic per block: all go to one address
+    m_abs = __reduce_max_sync(0xffffffffu, m_abs);
+    unsigned* red = reinterpret_cast<unsigned*>(scores);   // (used up)
+    __syncthreads();
+    if(lane == 0)
+      red[warp] = m_abs;
+    __syncthreads();
+    if(warp == 0) {
+      m_abs = __reduce_max_sync(0xffffffffu, lane < warps ? red[lane] : 0u);
+      if(lane == 0 && m_abs != 0u)
+        atomicMax(absmax_slot, m_abs);
+    }
   }
   trace_stamp(tb, kTrAttention1, 2);
   trace_stamp(th.last, kTrAttention1, 3);
@@ -1209,6 +1395,23 @@ int launch_attention1(const float* q, const float* k, const float* v, const floa
         launch_kernel(attention_enc_kernel<64>, dim3(batch, heads), dim3(128), esmem, s, q, k, v, log_mask, heads, len, scale, out, slot);
       else
         launch_kernel(attention_enc_kernel<32>, dim3(batch, heads), dim3(128), esmem, s, q, k, v, log_mask, heads, len, scale, out, slot);
+      count_launch();
+      return check_launch();
+    }
+  }
+  if(mode == 1 && batch > 0 && (dim_head == 64 || dim_head == 32)) {
+    // the hypotheses of a sentence together; sentences so long that the scores leave no room for the ring within 48 KB go one
+    // row at a time below
+    const int beams = (rows + batch - 1) / batch;
+    const int groups = (beams + kCrossMaxBeams - 1) / kCrossMaxBeams, warps = (beams + groups - 1) / groups;
+    const int warp_heads = 128 / dim_head;
+    const size_t xsmem = kCrossStages * kCrossRows * 32 * sizeof(float4) + static_cast<size_t>(warps) * warp_heads * ((len + 3) & ~3) * sizeof(float);
+    if(xsmem <= 48 * 1024 && groups <= 65535) {
+      const dim3 xgrid(batch, (heads + warp_heads - 1) / warp_heads, groups);
+      if(dim_head == 64)
+        launch_kernel(attention_cross_kernel<64>, xgrid, dim3(warps * 32), xsmem, s, q, k, v, log_mask, heads, len, rows, batch, scale, out, slot);
+      else
+        launch_kernel(attention_cross_kernel<32>, xgrid, dim3(warps * 32), xsmem, s, q, k, v, log_mask, heads, len, rows, batch, scale, out, slot);
       count_launch();
       return check_launch();
     }

@@ -103,6 +103,35 @@ def test_attention_bit_exact(cuda_device, oracle, mode, rows, batch, length, hea
         assert np.abs(want[r0, sl] - w @ v[idx][:, sl].astype(np.float64)).max() < 1e-4
 
 
+@pytest.mark.parametrize("rows,batch,length,heads,dh", [
+    # rows a sentence's block serves (1..8, two blocks from 9 on), ragged row counts, a head group that is not full, lengths around
+    # the eight positions of a sum, the rows of a ring stage and of the ring, and lengths that take the one-row kernel
+    (5, 5, 7, 5, 64), (6, 3, 8, 3, 32), (9, 3, 9, 16, 64), (10, 2, 31, 8, 32), (12, 2, 32, 8, 64), (13, 2, 33, 16, 64), (4, 2, 48, 8, 64),
+    (7, 4, 257, 4, 64), (8, 2, 256, 8, 64), (8, 2, 512, 8, 64), (4, 4, 1, 1, 64), (16, 4, 128, 8, 32), (16, 4, 129, 8, 32),
+    (9, 1, 12, 8, 64), (17, 2, 500, 4, 32), (2, 2, 2000, 2, 64), (3, 1, 16, 2, 64), (3, 1, 17, 2, 64)])
+def test_cross_attention_rows_of_a_sentence_together(cuda_device, oracle, rows, batch, length, heads, dh):
+    L, check = _lib()
+    rng = np.random.default_rng(rows * length)
+    dim = heads * dh
+    q = rng.standard_normal((rows, dim)).astype(np.float32)
+    k = rng.standard_normal((batch * length, dim)).astype(np.float32)
+    v = rng.standard_normal((batch * length, dim)).astype(np.float32)
+    lens = rng.integers(1, length + 1, size=batch)
+    mask = np.where(np.arange(length)[None, :] < lens[:, None], 0.0, -99999999.0).astype(np.float32)
+    for m in (mask, None):
+        want = oracle.attention1(q, k, v, m, rows, heads, dh, length, batch, 1)
+        qd, kd, vd = _dev(q, cuda_device), _dev(k, cuda_device), _dev(v, cuda_device)
+        md = _dev(m, cuda_device) if m is not None else None
+        out = torch.full((rows + 1, dim), 7.0, device=cuda_device)
+        slot = torch.zeros(1, dtype=torch.int32, device=cuda_device)
+        check(L.mi8g_attention1(qd.data_ptr(), kd.data_ptr(), vd.data_ptr(), md.data_ptr() if md is not None else None, rows, heads, dh,
+                                length, batch, 1, out.data_ptr(), slot.data_ptr(), _stream()))
+        torch.cuda.synchronize()
+        assert np.array_equal(out[:rows].cpu().numpy(), want)
+        assert (out[rows] == 7.0).all()
+        assert slot.view(torch.float32).item() == np.abs(want).max()
+
+
 @pytest.mark.parametrize("rows", [3, 400])                     # 1024 and 256 threads per row
 @pytest.mark.parametrize("vocab,k", [(128, 1), (129, 2), (1000, 8), (1027, 8), (4096, 4), (32000, 4)])
 def test_lse_topk_awkward_rows(cuda_device, oracle, rows, vocab, k):
