@@ -66,7 +66,7 @@ struct EncLayerW {
 };
 struct DecLayerW {
   Aff self_q, self_k, self_v, self_o, rnn_w, rnn_wf, ctx_q, ctx_k, ctx_v, ctx_o, w1, w2;
-  Fused self_kv, rnn, ctx_kv;
+  Fused self_qkv, rnn, ctx_kv;
   Norm ln_self, ln_ctx, ln_ffn;
 };
 
@@ -89,7 +89,8 @@ struct LayerBufs {
   float* rowmax = nullptr;   // [max_steps][slab_rows]     max|x| per slab row
   float* kslab = nullptr;    // [max_steps][slab_rows][d]  projected keys / values of the slabs, valid for the
   float* vslab = nullptr;    //                            history abs-max remembered in prev_bits
-  int8_t* hq = nullptr;      // [max_steps][slab_rows][d]  quantised slabs + multiplier behind the last slab
+  int8_t* hq = nullptr;      // [max_steps][slab_rows][d]  quantised slabs, then [max_rows][d] the newest slab with the multiplier of
+                             // its own (the query projection's operand), then both multipliers (history's, own)
   float* cross_k = nullptr;  // [max_batch * max_src, d]
   float* cross_v = nullptr;
   float* cell[2] = {nullptr, nullptr};  // SSRU state, double-buffered [max_rows, d]
@@ -185,7 +186,7 @@ struct mi8d_decoder {
         L.rowmax = arena.take<float>(T * R);
         L.kslab = arena.take<float>(T * R * d);
         L.vslab = arena.take<float>(T * R * d);
-        L.hq = arena.take<int8_t>(T * R * d + 256);
+        L.hq = arena.take<int8_t>((T + 1) * R * d + 256);
       } else {
         L.cell[0] = arena.take<float>(R * d);
         L.cell[1] = arena.take<float>(R * d);
@@ -248,7 +249,7 @@ struct mi8d_decoder {
       for(auto& p : fused_enc)
         p = arena.take<int8_t>(3 * d * d);
       for(auto& p : fused_self)
-        p = arena.take<int8_t>(2 * d * d);
+        p = arena.take<int8_t>((c.ssru ? 2 : 3) * d * d);
       for(auto& p : fused_ctx)
         p = arena.take<int8_t>(2 * d * d);
     }
@@ -356,7 +357,7 @@ struct mi8d_decoder {
         ok = ok && aff(w.self_q, pre + "_Wq", pre + "_bq") && aff(w.self_k, pre + "_Wk", pre + "_bk") &&
              aff(w.self_v, pre + "_Wv", pre + "_bv") && aff(w.self_o, pre + "_Wo", pre + "_bo") && norm(w.ln_self, pre + "_Wo");
         if(ok)
-          copies = copies && fuse(w.self_kv, fused_self[l], {&w.self_k, &w.self_v}, s);
+          copies = copies && fuse(w.self_qkv, fused_self[l], {&w.self_q, &w.self_k, &w.self_v}, s);
       }
       const std::string pre = li + "_context", ffn = li + "_ffn";
       ok = ok && aff(w.ctx_q, pre + "_Wq", pre + "_bq") && aff(w.ctx_k, pre + "_Wk", pre + "_bk") && aff(w.ctx_v, pre + "_Wv", pre + "_bv") &&
@@ -423,44 +424,32 @@ int gemm(mi8d_decoder* d, const int8_t* a, int M, const Aff& w, bool relu, float
                      force_splits, absmax_out);
 }
 
-// The narrowest tile (activation rows) that covers an M x N product with at most `budget` CTAs; 0 = leave it to the plan.
-// Two GEMMs that run side by side on two streams each take half of the SMs this way (a CTA of this kernel fills an SM).
-int tile_within(int M, int N, int budget) {
-  if(M <= 64)
-    return 0;
-  for(int tm : {32, 64, 128, 256})
-    if(((N + 127) / 128) * ((M + tm - 1) / tm) <= budget)
-      return tm;
-  return 0;
-}
-
-// the same activation against the matrices of a fused group, one launch; outs[i] receives [M, f.n]
-int gemm_fused(mi8d_decoder* d, const int8_t* a, const float* qa, int M, const Fused& f, float* const* outs, cudaStream_t s,
-               int force_splits = 0, int a_rows_cap = 0, int a_row0 = 0, const unsigned* skip_a = nullptr,
-               const unsigned* skip_b = nullptr, int skip_rows_below = 0, int force_tile_m = 0) {
+// M rows of `a` against the matrices [first, last) of a fused group, one launch; outputs and the activation's details are the caller's
+GemmCall fused_call(mi8d_decoder* d, const int8_t* a, const Fused& f, int M, int first, int last, int a_rows_cap, cudaStream_t s) {
   GemmCall g;
   g.aq = a;
-  g.bt = f.bt;
+  g.bt = f.bt + static_cast<size_t>(first) * f.n * f.K;
   g.M = M;
-  g.N = f.nseg * f.n;
+  g.N = (last - first) * f.n;
   g.K = f.K;
-  g.d_qa = qa;
-  g.nseg = f.nseg;
-  for(int i = 0; i < f.nseg; ++i) {
-    g.seg_qb[i] = f.qm[i];
-    g.seg_bias[i] = f.bias[i];
-    g.seg_c[i] = outs[i];
+  g.nseg = last - first;
+  for(int i = first; i < last; ++i) {
+    g.seg_qb[i - first] = f.qm[i];
+    g.seg_bias[i - first] = f.bias[i];
   }
   g.ws = d->ws;
   g.ws_bytes = d->ws_bytes;
   g.stream = s;
-  g.force_splits = force_splits;
-  g.force_tile_m = force_tile_m;
   g.a_rows_cap = a_rows_cap;
-  g.a_row0 = a_row0;
-  g.skip_a = skip_a;
-  g.skip_b = skip_b;
-  g.skip_rows_below = skip_rows_below;
+  return g;
+}
+
+// the same activation against all matrices of a fused group; outs[i] receives [M, f.n]
+int gemm_fused(mi8d_decoder* d, const int8_t* a, const float* qa, int M, const Fused& f, float* const* outs, cudaStream_t s) {
+  GemmCall g = fused_call(d, a, f, M, 0, f.nseg, 0, s);
+  g.d_qa = qa;
+  for(int i = 0; i < f.nseg; ++i)
+    g.seg_c[i] = outs[i];
   return launch_gemm_call(g);
 }
 
@@ -1088,29 +1077,36 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
       // quantised and projected, otherwise everything is.  One launch quantises the layer input twice - with its own
       // multiplier for the query projection and, as the newest history slab, with the history's.
       const int steps = t + 1;
-      const int cap_rows = c.max_steps * c.max_rows;
-      float* hq_tail = reinterpret_cast<float*>(L.hq + static_cast<size_t>(cap_rows) * dm);
-      MI8D_TRY(launch_quantize_dual(x, n_d, x_slot, d->aq, aq_tail, L.slab, SR, steps, R, dm, sh, d->prev_bits + l, L.hq, hq_tail, s));
-      const bool fused = d->opt_fuse && w.self_kv.ready;
+      const int cap_rows = c.max_steps * c.max_rows;   // slabs of hq; the operand of the query projection lies behind them
+      int8_t* xq = L.hq + static_cast<size_t>(cap_rows) * dm;
+      float* hq_tail = reinterpret_cast<float*>(xq + static_cast<size_t>(c.max_rows) * dm);
+      float* xq_tail = hq_tail + 1;
+      MI8D_TRY(launch_quantize_dual(x, n_d, x_slot, xq, xq_tail, L.slab, SR, steps, R, dm, sh, d->prev_bits + l, L.hq, hq_tail, s));
+      const bool fused = d->opt_fuse && w.self_qkv.ready;
       float* kv_new[2] = {L.kslab + static_cast<size_t>(t) * slab_stride, L.vslab + static_cast<size_t>(t) * slab_stride};
-      float* kv_all[2] = {L.kslab, L.vslab};
-      // The key/value projections do not depend on the query projection: they run on the internal stream beside it.  Both
-      // sides then use tiles wide enough to fit half of the SMs each (a CTA of the GEMM fills an SM), so they really run
-      // at the same time; no split-K on either side, the two streams must not share the workspace's counters.
-      const bool side = d->overlap && d->opt_side_stream;
+      // Query, key and value projections of the newest slab are one launch (the query's segment takes its rows and multiplier from
+      // another place of hq).  The earlier slabs' keys and values, recomputed only when the abs-max changed, run before it, or
+      // beside it on the internal stream.  The internal stream gains where re-projections
+      // happen: transformer-base 64 x 4 37.4 against 37.9 ms on one stream, 16 x 4 18.1 against 18.8, transformer-big 44.2 against 44.9.
+      // (As three launches, the query's on its own stream beside the others with tiles for half of the SMs each: 38.4, 19.1 and 45.7 ms.)
+      const bool side = d->overlap && d->opt_side_stream && t > 0;
       cudaStream_t so = side ? d->side : s;
-      const int half = sm_count() / 2;
-      const int wide = wide_tile(d, R);
-      const int tile_q = std::max(side ? tile_within(R, w.self_q.N, half) : 0, wide);
-      const int tile_kv = std::max(side ? tile_within(R, 2 * w.self_k.N, half) : 0, wide);
       if(side) {
         MI8D_CUDA(cudaEventRecord(d->ev_fork, s));
         MI8D_CUDA(cudaStreamWaitEvent(so, d->ev_fork, 0));
       }
       if(t > 0) {
-        // earlier slabs: recomputed only when the abs-max changed (all tiles skipped otherwise)
+        // all tiles skipped when the stored results still hold; no split-K: the two streams must not share the workspace's counters
         if(fused) {
-          MI8D_TRY(gemm_fused(d, L.hq, hq_tail, t * SR, w.self_kv, kv_all, so, 1, cap_rows, 0, d->prev_bits + l, sh, t * SR));
+          GemmCall g = fused_call(d, L.hq, w.self_qkv, t * SR, 1, 3, cap_rows + c.max_rows, so);
+          g.d_qa = hq_tail;
+          g.seg_c[0] = L.kslab;
+          g.seg_c[1] = L.vslab;
+          g.force_splits = 1;
+          g.skip_a = d->prev_bits + l;
+          g.skip_b = sh;
+          g.skip_rows_below = t * SR;
+          MI8D_TRY(launch_gemm_call(g));
         } else {
           MI8D_TRY(launch_gemm(L.hq, w.self_k.bt, t * SR, w.self_k.N, w.self_k.K, hq_tail, w.self_k.qm, 1.0f, w.self_k.bias, 0, L.kslab, MI8_F32,
                                nullptr, d->ws, d->ws_bytes, so, 0, 1, nullptr, d->prev_bits + l, sh, t * SR));
@@ -1118,19 +1114,29 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
                                nullptr, d->ws, d->ws_bytes, so, 0, 1, nullptr, d->prev_bits + l, sh, t * SR));
         }
       }
-      // newest slab: always projected, as a problem of its own (R live rows)
-      if(fused) {
-        MI8D_TRY(gemm_fused(d, L.hq, hq_tail, R, w.self_kv, kv_new, so, 1, cap_rows, t * SR, nullptr, nullptr, 0, tile_kv));
-      } else {
-        const int8_t* a_new = L.hq + static_cast<size_t>(t) * slab_stride;
-        MI8D_TRY(launch_gemm(a_new, w.self_k.bt, R, w.self_k.N, w.self_k.K, hq_tail, w.self_k.qm, 1.0f, w.self_k.bias, 0, kv_new[0], MI8_F32,
-                             nullptr, d->ws, d->ws_bytes, so, 0, 1));
-        MI8D_TRY(launch_gemm(a_new, w.self_v.bt, R, w.self_v.N, w.self_v.K, hq_tail, w.self_v.qm, 1.0f, w.self_v.bias, 0, kv_new[1], MI8_F32,
-                             nullptr, d->ws, d->ws_bytes, so, 0, 1));
-      }
       if(side)
         MI8D_CUDA(cudaEventRecord(d->ev_join, so));
-      MI8D_TRY(gemm(d, d->aq, R, w.self_q, false, d->qbuf, s, nullptr, side ? 1 : 0, tile_q));
+      if(fused) {
+        GemmCall g = fused_call(d, L.hq, w.self_qkv, R, 0, 3, cap_rows + c.max_rows, s);
+        g.d_qa = hq_tail;
+        g.a_row0 = t * SR;
+        g.seg_row0[0] = cap_rows;
+        g.seg_qa[0] = xq_tail;
+        g.seg_c[0] = d->qbuf;
+        g.seg_c[1] = kv_new[0];
+        g.seg_c[2] = kv_new[1];
+        g.force_tile_m = wide_tile(d, R);
+        g.force_splits = g.force_tile_m != 0 ? 1 : 0;
+        MI8D_TRY(launch_gemm_call(g));
+      } else {
+        const int8_t* a_new = L.hq + static_cast<size_t>(t) * slab_stride;
+        MI8D_TRY(launch_gemm(xq, w.self_q.bt, R, w.self_q.N, w.self_q.K, xq_tail, w.self_q.qm, 1.0f, w.self_q.bias, 0, d->qbuf, MI8_F32,
+                             nullptr, d->ws, d->ws_bytes, s, 0, 1));
+        MI8D_TRY(launch_gemm(a_new, w.self_k.bt, R, w.self_k.N, w.self_k.K, hq_tail, w.self_k.qm, 1.0f, w.self_k.bias, 0, kv_new[0], MI8_F32,
+                             nullptr, d->ws, d->ws_bytes, s, 0, 1));
+        MI8D_TRY(launch_gemm(a_new, w.self_v.bt, R, w.self_v.N, w.self_v.K, hq_tail, w.self_v.qm, 1.0f, w.self_v.bias, 0, kv_new[1], MI8_F32,
+                             nullptr, d->ws, d->ws_bytes, s, 0, 1));
+      }
       if(side)
         MI8D_CUDA(cudaStreamWaitEvent(s, d->ev_join, 0));
       MI8D_TRY(launch_attention1(d->qbuf, L.kslab, L.vslab, nullptr, R, c.heads, dm / c.heads, steps, batch, 0, d->abuf, sa, s,

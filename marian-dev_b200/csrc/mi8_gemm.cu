@@ -113,12 +113,14 @@ struct GemmParams {
   // same activation in one launch (Wk|Wv of an attention block, Wq|Wk|Wv of the encoder): segment s covers
   // weight rows [s * seg_n, (s + 1) * seg_n), has its own multiplier, bias and output matrix [M, seg_n].
   // seg_n is a multiple of 128, so a tile never straddles two segments.  nseg == 1: the plain call
-  // (seg_n = N, seg_qb[0] = d_qb, seg_bias[0] = bias, seg_c[0] = c).
+  // (seg_n = N, seg_qb[0] = d_qb, seg_bias[0] = bias, seg_c[0] = c).  A segment may also take its activation rows from another
+  // place of the operand's buffer (seg_row0: their first row in the tensor map), quantised with a multiplier of its own (seg_qa).
   int nseg, seg_n;
+  int seg_row0[kMaxSegments];
+  const float* seg_qa[kMaxSegments];
   const float* seg_qb[kMaxSegments];
   const float* seg_bias[kMaxSegments];
   void* seg_c[kMaxSegments];
-  int a_row0;               // first row of the activation inside its tensor map (a slab of a larger buffer)
   int* rows_computed;       // optional (measurement): receives the number of activation rows this launch really computed
   int withhold_item;        // test hook: the producer leaves out the loads of this pipeline item (-1 = none)
   uint32_t spin_limit;      // bound of every barrier wait of this launch
@@ -372,6 +374,7 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       const WorkItem wi = decode_work(p, w);
       if(skip_on && (wi.m_tile + 1) * TM <= p.skip_rows_below)
         continue;
+      const int a_row0 = p.seg_row0[p.nseg > 1 ? (wi.n_tile * kTileN) / p.seg_n : 0];
       for(int kb = wi.kb_begin; kb < wi.kb_end; ++kb, ++it) {
         const uint32_t s = it % T::kStages;
         const uint32_t ph = (it / T::kStages) & 1u;
@@ -389,7 +392,7 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             tma_load_2d(st, &tmap_w, kb * kTileKBytes, wi.n_tile * kTileN, &ctl->full[s]);
           }
           if(!kQuantA)
-            tma_load_2d(st + T::kWBytes, &tmap_a, kb * kTileKBytes, p.a_row0 + wi.m_tile * TM, &ctl->full[s]);
+            tma_load_2d(st + T::kWBytes, &tmap_a, kb * kTileKBytes, a_row0 + wi.m_tile * TM, &ctl->full[s]);
         }
         __syncwarp();
       }
@@ -574,7 +577,7 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       if(!kP8 && kTopK == 0 && p.nseg > 1) {
         seg = (wi.n_tile * kTileN) / p.seg_n;
         n_loc = n - seg * p.seg_n;
-        unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(qa, *p.seg_qb[seg])), p.scale);
+        unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(*p.seg_qa[seg], *p.seg_qb[seg])), p.scale);
       }
       const float* seg_bias = p.seg_bias[seg];
       void* seg_c = p.seg_c[seg];
@@ -913,6 +916,8 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       const WorkItem wi = decode_work(p, w);
       if(skip_on && (wi.m_tile + 1) * T::kTM <= p.skip_rows_below)
         continue;
+      // (both CTAs' weight rows lie in one segment, or all segments share the activation: launch_gemm_call sees to it)
+      const int a_row0 = p.seg_row0[p.nseg > 1 ? (2 * wi.n_tile * kTileN) / p.seg_n : 0];
       for(int kb = wi.kb_begin; kb < wi.kb_end; ++kb, ++it) {
         const uint32_t s = it % T::kStages;
         const uint32_t ph = (it / T::kStages) & 1u;
@@ -930,7 +935,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             tma_load_2d_pair(st, &tmap_w, kb * kTileKBytes, (2 * wi.n_tile + static_cast<int>(rank)) * kTileN, full_addr(s));
           }
           tma_load_2d_pair(st + T::kWBytes, &tmap_a, kb * kTileKBytes,
-                           p.a_row0 + wi.m_tile * T::kTM + static_cast<int>(rank) * T::kHalfRows, full_addr(s));
+                           a_row0 + wi.m_tile * T::kTM + static_cast<int>(rank) * T::kHalfRows, full_addr(s));
         }
         __syncwarp();
       }
@@ -1037,7 +1042,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       if(!kP8 && p.nseg > 1) {
         seg = ((2 * wi.n_tile + static_cast<int>(rank)) * kTileN) / p.seg_n;
         n_loc = n - seg * p.seg_n;
-        unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(qa, *p.seg_qb[seg])), p.scale);
+        unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(*p.seg_qa[seg], *p.seg_qb[seg])), p.scale);
       }
       const float* seg_bias = p.seg_bias[seg];
       void* seg_c = p.seg_c[seg];
@@ -1695,8 +1700,9 @@ void finish_params(GemmParams& p) {
     p.rows_computed = t_profile.d_rows + t_profile.records.size();
 }
 void single_segment(GemmParams& p) {
-  p.a_row0 = 0;
   p.nseg = 1;
+  p.seg_row0[0] = 0;
+  p.seg_qa[0] = p.d_qa;
   p.seg_n = p.N;
   for(int i = 0; i < kMaxSegments; ++i) {
     p.seg_qb[i] = p.d_qb;
@@ -1996,8 +2002,19 @@ int launch_gemm_call(const GemmCall& g) {
     return MI8_ERR_BAD_ARG;
   if(K % 16 != 0 || (reinterpret_cast<uintptr_t>(g.aq) & 15u) || (reinterpret_cast<uintptr_t>(g.bt) & 15u))
     return MI8_ERR_MISALIGNED;
+  bool own_rows = false;   // segments with different activation rows
+  // a_rows_cap: the activation buffer is known to hold that many rows, so one descriptor serves every M up to
+  // it (rows past M inside the last tile are then real bytes instead of zero fill; their products are never stored)
+  for(int i = 0; i < g.nseg; ++i) {
+    const int row0 = g.seg_row0[i] < 0 ? g.a_row0 : g.seg_row0[i];
+    if(g.a_row0 < 0 || (row0 > 0 && g.a_rows_cap < row0 + M))
+      return MI8_ERR_BAD_ARG;
+    own_rows = own_rows || row0 != (g.seg_row0[0] < 0 ? g.a_row0 : g.seg_row0[0]);
+  }
   GemmPlan plan;
   int rc = make_gemm_plan(M, N, K, g.force_tile_m, g.force_splits, &plan);
+  if(rc == MI8_OK && plan.pair && own_rows && (N / g.nseg) % (2 * kTileN) != 0)   // a pair's 256 weight rows share their activation tile
+    rc = make_gemm_plan(M, N, K, 256, g.force_splits, &plan);
   if(rc != MI8_OK)
     return rc;
   if(plan.splits > 1) {
@@ -2008,10 +2025,6 @@ int launch_gemm_call(const GemmCall& g) {
   rc = get_kmajor_map(&tw, g.bt, N, K, kTileN);
   if(rc != MI8_OK)
     return rc;
-  // a_rows_cap: the activation buffer is known to hold that many rows, so one descriptor serves every M up to
-  // it (rows past M inside the last tile are then real bytes instead of zero fill; their products are never stored)
-  if(g.a_row0 < 0 || (g.a_row0 > 0 && g.a_rows_cap < g.a_row0 + M))
-    return MI8_ERR_BAD_ARG;
   rc = get_kmajor_map(&ta, g.aq, g.a_rows_cap > M ? g.a_rows_cap : M, K, plan.pair ? PairCfg::kHalfRows : plan.tile_m);
   if(rc != MI8_OK)
     return rc;
@@ -2060,8 +2073,9 @@ int launch_gemm_call(const GemmCall& g) {
     p.seg_qb[i] = g.seg_qb[i];
     p.seg_bias[i] = g.seg_bias[i];
     p.seg_c[i] = g.seg_c[i];
+    p.seg_row0[i] = g.seg_row0[i] < 0 ? g.a_row0 : g.seg_row0[i];
+    p.seg_qa[i] = g.seg_qa[i] != nullptr ? g.seg_qa[i] : g.d_qa;
   }
-  p.a_row0 = g.a_row0;
   finish_params(p);
 
   if(plan.pair)

@@ -97,6 +97,9 @@ struct GemmCall {
   int skip_rows_below = 0;
   int a_rows_cap = 0;   // rows the activation buffer holds (extent of its tensor map); 0 = M
   int a_row0 = 0;       // the M rows start at this row of the buffer `aq` points to (needs a_rows_cap >= a_row0 + M)
+  // per segment, where it differs: the first of its M activation rows (-1: a_row0) and their multiplier (null: d_qa)
+  int seg_row0[3] = {-1, -1, -1};
+  const float* seg_qa[3] = {nullptr, nullptr, nullptr};
 };
 int launch_gemm_call(const GemmCall& g);
 
