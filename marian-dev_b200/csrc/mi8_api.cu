@@ -197,10 +197,7 @@ int mi8_prepare_a_f32(const float* a, int rows, int cols, int8_t* q, float* d_qu
   if(rows == 0)
     return MI8_OK;
   const size_t n = static_cast<size_t>(rows) * static_cast<size_t>(cols);
-  int rc = launch_max_absolute(a, n, nullptr, d_quant_mult, workspace, workspace_bytes, as_stream(stream));
-  if(rc != MI8_OK)
-    return rc;
-  return launch_quantize(a, n, d_quant_mult, q, as_stream(stream));
+  return launch_prepare(a, n, d_quant_mult, q, workspace, workspace_bytes, as_stream(stream));
 }
 
 int mi8_prepare_b_f32(const float* w, int K, int N, int w_is_nk, int8_t* bt, float* d_quant_mult, void* workspace,
@@ -208,11 +205,11 @@ int mi8_prepare_b_f32(const float* w, int K, int N, int w_is_nk, int8_t* bt, flo
   if(K <= 0 || N <= 0 || d_quant_mult == nullptr)
     return MI8_ERR_BAD_ARG;
   const size_t n = static_cast<size_t>(K) * static_cast<size_t>(N);
+  if(w_is_nk)
+    return launch_prepare(w, n, d_quant_mult, bt, workspace, workspace_bytes, as_stream(stream));
   int rc = launch_max_absolute(w, n, nullptr, d_quant_mult, workspace, workspace_bytes, as_stream(stream));
   if(rc != MI8_OK)
     return rc;
-  if(w_is_nk)
-    return launch_quantize(w, n, d_quant_mult, bt, as_stream(stream));
   return launch_transpose_quantize(w, K, N, d_quant_mult, bt, as_stream(stream));
 }
 

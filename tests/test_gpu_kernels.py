@@ -169,6 +169,26 @@ def test_cta_pair_kernel_many_tiles(cuda_device, oracle):
     _run_affine(cuda_device, oracle, 2100, 1024, 1000, True, False, 13, out_dtype=torch.float16, tile_m=512)
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 16), (3, 16), (1, 8176), (2, 4096), (1, 8208), (2, 16368), (2, 16384), (1, 32784), (128, 1024), (1, 131088),
+                                       (256, 1024), (1, 262160)])
+@pytest.mark.parametrize("where", ["first", "last", "zero"])
+def test_prepare_a_of_small_tensors(cuda_device, rows, cols, where):
+    """Abs-max and quantisation in one launch: the ends of what one CTA and a cluster hold, the maximum in the first or last element, all zeros."""
+    ops = _ops()
+    rng = np.random.default_rng(rows + cols)
+    x = rng.uniform(-1, 1, (rows, cols)).astype(np.float32)
+    if where == "zero":
+        x[:] = 0
+    else:
+        x.reshape(-1)[0 if where == "first" else -1] = -3.5
+    aq = ops.prepareA(torch.from_numpy(x).to(cuda_device))
+    torch.cuda.synchronize()
+    qm = np.float32(1) if where == "zero" else np.float32(127) / np.abs(x).max()
+    assert np.float32(aq.quant_mult.item()) == qm
+    assert np.array_equal(aq.data.cpu().numpy().reshape(rows, cols), np.rint(x * qm).astype(np.int8))
+    assert ops.poll_status() == 0
+
+
 @pytest.mark.parametrize("m,k,n,tile_m", [(31, 64, 128, 32), (33, 64, 130, 32), (32, 64, 255, 0), (64, 64, 96, 64), (300, 128, 1022, 256), (257, 1024, 258, 512),
                                           (16, 2048, 34, 16)])
 def test_half_output_edges(cuda_device, oracle, m, k, n, tile_m):
