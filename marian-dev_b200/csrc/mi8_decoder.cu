@@ -474,8 +474,11 @@ int gemm_act(mi8d_decoder* d, const int8_t* q, int M, const Aff& w, bool relu, f
 // Int8::PrepareA of x (multiplier from the slot its producer reduced) followed by the affine: either the
 // quantisation kernel and the GEMM, or - with the option set and a shape that gives every CTA one tile - the GEMM
 // that quantises its operand while loading it.
+// `ready`: d->aq already holds the quantised x (see ln_quantises).
 int quant_gemm(mi8d_decoder* d, const float* x, int M, const unsigned* slot, const Aff& w, bool relu, float* c, cudaStream_t s,
-               unsigned* absmax_out = nullptr) {
+               unsigned* absmax_out = nullptr, bool ready = false) {
+  if(ready)
+    return gemm_act(d, d->aq, M, w, relu, c, s, absmax_out);
   float* qa = reinterpret_cast<float*>(d->aq + static_cast<size_t>(M) * w.K);
   if(!w.p8 && d->opt_cluster && M <= d->opt_cluster_max_rows && w.K <= d->opt_cluster_max_k && gemm_cq_supported(M, w.N, w.K, false)) {
     // the cluster GEMM: the CTAs of neighbouring weight tiles quantise the activation tile together (one launch, no int8 copy)
@@ -506,10 +509,20 @@ int add_ln(mi8d_decoder* d, const float* a, const float* resid, const Norm& n, i
   return launch_add_layernorm(a, resid, n.g, n.b, 1e-6f, rows, d->cfg.dim_emb, out, rowmax, slot, s, slot2);
 }
 
+// Whether a LayerNorm of `rows` rows whose result only feeds affines of its own multiplier also quantises it (into d->aq / enc_aq).
+bool ln_quantises(const mi8d_decoder* d, int rows) {
+  return !d->p8 && !d->opt_cluster && !d->opt_quant_in_gemm && add_layernorm_quant_supported(rows, d->cfg.dim_emb);
+}
+int add_ln_quant(mi8d_decoder* d, const float* a, const float* resid, const Norm& n, int rows, float* out, int8_t* q, cudaStream_t s) {
+  return launch_add_layernorm_quant(a, resid, n.g, n.b, 1e-6f, rows, d->cfg.dim_emb, out, q,
+                                    reinterpret_cast<float*>(q + static_cast<size_t>(rows) * d->cfg.dim_emb), s);
+}
+
 // out = LayerNorm(affine(x) + resid): the "dan" post-processing of a sub-layer's last affine (src/models/transformer.h:189-214).
 // One launch when the row fits a cluster (the cluster GEMM's LayerNorm write-back), else affine (into `tmp`) and LayerNorm.
+// `quant_next` (ln_quantises): the result is also quantised into d->aq for the next affine, and the slots and row maxima are left alone.
 int quant_gemm_ln(mi8d_decoder* d, const float* x, int M, const unsigned* slot, const Aff& w, const float* resid, const Norm& n, float* tmp,
-                  float* out, float* rowmax, unsigned* out_slot, cudaStream_t s, unsigned* out_slot2 = nullptr) {
+                  float* out, float* rowmax, unsigned* out_slot, cudaStream_t s, unsigned* out_slot2 = nullptr, bool quant_next = false) {
   if(!w.p8 && d->opt_cluster && d->opt_fused_ln && M <= d->opt_cluster_max_rows && w.K <= d->opt_cluster_max_k && w.N == d->cfg.dim_emb &&
      gemm_cq_supported(M, w.N, w.K, true)) {
     CqCall g;
@@ -534,6 +547,8 @@ int quant_gemm_ln(mi8d_decoder* d, const float* x, int M, const unsigned* slot, 
     return launch_gemm_cq(g);
   }
   MI8D_TRY(quant_gemm(d, x, M, slot, w, false, tmp, s));
+  if(quant_next)
+    return add_ln_quant(d, tmp, resid, n, M, out, d->aq, s);
   return add_ln(d, tmp, resid, n, M, out, rowmax, out_slot, s, out_slot2);
 }
 
@@ -904,13 +919,15 @@ int mi8d_encode(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
   // embeddings * sqrt(d) + positions 0..src-1 (src/models/transformer.h:93,110-114)
   float* x = d->enc_x[0];
   unsigned* x_slot = d->slots;
+  const bool lq = ln_quantises(d, M);
   MI8D_TRY(launch_embed(d->wemb, ids, d->positions, src, sqrtf(static_cast<float>(dm)), M, dm, x, nullptr, x_slot, s));
   for(int l = 0; l < c.enc_depth; ++l) {
     const EncLayerW& w = d->enc_w[l];
     unsigned *sa = d->enc_slot(l, 0), *s1 = d->enc_slot(l, 1), *s3 = d->enc_slot(l, 2);
     // q, keys and values are the same tensor: one quantisation serves the three projections, and with fused
     // weights one launch computes all three
-    MI8D_TRY(quantize_act(d, x, M, dm, x_slot, d->enc_aq, s));
+    if(l == 0 || !lq)
+      MI8D_TRY(quantize_act(d, x, M, dm, x_slot, d->enc_aq, s));
     if(d->opt_fuse && w.qkv.ready) {
       float* outs[3] = {d->enc_q, d->enc_k, d->enc_v};
       MI8D_TRY(gemm_fused(d, d->enc_aq, aq_tail, M, w.qkv, outs, s));
@@ -923,15 +940,22 @@ int mi8d_encode(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
     MI8D_TRY(launch_attention1(d->enc_q, d->enc_k, d->enc_v, d->log_mask[0], M, c.heads, dm / c.heads, src, batch, 2, a, sa, s));
     MI8D_TRY(quantize_act(d, a, M, dm, sa, d->enc_aq, s));
     MI8D_TRY(gemm_act(d, d->enc_aq, M, w.o, false, d->enc_q, s));
-    MI8D_TRY(add_ln(d, d->enc_q, x, w.ln_att, M, a, nullptr, s1, s));                       // x1 = LN(Wo(a) + x)
-    MI8D_TRY(quantize_act(d, a, M, dm, s1, d->enc_aq, s));
+    if(lq) {                                                                                  // x1 = LN(Wo(a) + x)
+      MI8D_TRY(add_ln_quant(d, d->enc_q, x, w.ln_att, M, a, d->enc_aq, s));
+    } else {
+      MI8D_TRY(add_ln(d, d->enc_q, x, w.ln_att, M, a, nullptr, s1, s));
+      MI8D_TRY(quantize_act(d, a, M, dm, s1, d->enc_aq, s));
+    }
     MI8D_TRY(gemm_act(d, d->enc_aq, M, w.w1, true, d->enc_h, s, s3));                        // ReLU (and max|h|) in the write-back
     MI8D_TRY(quantize_act(d, d->enc_h, M, c.dim_ffn, s3, d->enc_aq, s));
     MI8D_TRY(gemm_act(d, d->enc_aq, M, w.w2, false, d->enc_q, s));
     const bool last = l + 1 == c.enc_depth;
     float* nx = last ? d->context[0] : x;                                                     // the last layer writes the context
     x_slot = d->enc_slot(l, 3);
-    MI8D_TRY(add_ln(d, d->enc_q, a, w.ln_ffn, M, nx, nullptr, x_slot, s));
+    if(lq && !last)
+      MI8D_TRY(add_ln_quant(d, d->enc_q, a, w.ln_ffn, M, nx, d->enc_aq, s));
+    else
+      MI8D_TRY(add_ln(d, d->enc_q, a, w.ln_ffn, M, nx, nullptr, x_slot, s));
     x = nx;
   }
   if(c.ssru) {
@@ -1039,13 +1063,15 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
 
   const int cell_new = d->cell_cur ^ 1;
   float* aq_tail = reinterpret_cast<float*>(d->aq + n_d);
+  const bool lq = ln_quantises(d, R);
   for(int l = 0; l < c.dec_depth; ++l) {
     LayerBufs& L = d->layers[l];
     const DecLayerW& w = d->dec_w[l];
     unsigned* x_slot = d->input_slot(l);
     unsigned* s1 = d->layer_slot(l, kSlotSelfLn);
     if(c.ssru) {
-      MI8D_TRY(quantize_act(d, x, R, dm, x_slot, d->aq, s));
+      if(l == 0 || !lq)
+        MI8D_TRY(quantize_act(d, x, R, dm, x_slot, d->aq, s));
       if(d->opt_fuse && w.rnn.ready) {
         float* outs[2] = {d->qbuf, d->fbuf};
         MI8D_TRY(gemm_fused(d, d->aq, aq_tail, R, w.rnn, outs, s));            // dot(input, W) and affine(input, Wf, bf)
@@ -1053,8 +1079,13 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
         MI8D_TRY(gemm_act(d, d->aq, R, w.rnn_w, false, d->qbuf, s));
         MI8D_TRY(gemm_act(d, d->aq, R, w.rnn_wf, false, d->fbuf, s));
       }
-      MI8D_TRY(launch_ssru_cell(L.cell[d->cell_cur], t == 0 ? nullptr : hyp_idx, d->qbuf, d->fbuf, R, dm, L.cell[cell_new], d->abuf, s));
-      MI8D_TRY(add_ln(d, d->abuf, x, w.ln_self, R, d->x1, nullptr, s1, s));
+      if(lq) {
+        MI8D_TRY(launch_add_layernorm_quant(nullptr, x, w.ln_self.g, w.ln_self.b, 1e-6f, R, dm, d->x1, d->aq, aq_tail, s, L.cell[d->cell_cur],
+                                            t == 0 ? nullptr : hyp_idx, d->qbuf, d->fbuf, L.cell[cell_new]));
+      } else {
+        MI8D_TRY(launch_ssru_cell(L.cell[d->cell_cur], t == 0 ? nullptr : hyp_idx, d->qbuf, d->fbuf, R, dm, L.cell[cell_new], d->abuf, s));
+        MI8D_TRY(add_ln(d, d->abuf, x, w.ln_self, R, d->x1, nullptr, s1, s));
+      }
     } else if(d->p8) {
       // packed8avx512 quantises every ROW of an activation on its own, so the keys/values of earlier steps never change:
       // the newest slab is projected and stored, the rest is a plain key/value cache (what the reference recomputes from the
@@ -1066,7 +1097,7 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
       MI8D_TRY(gemm_act(d, d->aq, R, w.self_v, false, L.vslab + static_cast<size_t>(t) * slab_stride, s));
       MI8D_TRY(launch_attention1(d->qbuf, L.kslab, L.vslab, nullptr, R, c.heads, dm / c.heads, t + 1, batch, 0, d->abuf, sa, s, d->anc[anc_new],
                                  SR, SR));
-      MI8D_TRY(quant_gemm_ln(d, d->abuf, R, sa, w.self_o, x, w.ln_self, d->obuf, d->x1, nullptr, s1, s));
+      MI8D_TRY(quant_gemm_ln(d, d->abuf, R, sa, w.self_o, x, w.ln_self, d->obuf, d->x1, nullptr, s1, s, nullptr, lq));
     } else {
       unsigned* sh = d->layer_slot(l, kSlotHistory);
       unsigned* sa = d->layer_slot(l, kSlotSelfAtt);
@@ -1140,17 +1171,17 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
         MI8D_CUDA(cudaStreamWaitEvent(s, d->ev_join, 0));
       MI8D_TRY(launch_attention1(d->qbuf, L.kslab, L.vslab, nullptr, R, c.heads, dm / c.heads, steps, batch, 0, d->abuf, sa, s,
                                  d->anc[anc_new], SR, SR));
-      MI8D_TRY(quant_gemm_ln(d, d->abuf, R, sa, w.self_o, x, w.ln_self, d->obuf, d->x1, nullptr, s1, s));
+      MI8D_TRY(quant_gemm_ln(d, d->abuf, R, sa, w.self_o, x, w.ln_self, d->obuf, d->x1, nullptr, s1, s, nullptr, lq));
     }
     {
       unsigned* sa = d->layer_slot(l, kSlotCtxAtt);
       unsigned* s2 = d->layer_slot(l, kSlotCtxLn);
-      MI8D_TRY(quant_gemm(d, d->x1, R, s1, w.ctx_q, false, d->qbuf, s));
+      MI8D_TRY(quant_gemm(d, d->x1, R, s1, w.ctx_q, false, d->qbuf, s, nullptr, lq));
       MI8D_TRY(launch_attention1(d->qbuf, L.cross_k, L.cross_v, lmask, R, c.heads, dm / c.heads, S, batch, 1, d->abuf, sa, s));
-      MI8D_TRY(quant_gemm_ln(d, d->abuf, R, sa, w.ctx_o, d->x1, w.ln_ctx, d->obuf, d->x2, nullptr, s2, s));
+      MI8D_TRY(quant_gemm_ln(d, d->abuf, R, sa, w.ctx_o, d->x1, w.ln_ctx, d->obuf, d->x2, nullptr, s2, s, nullptr, lq));
 
       unsigned* s3 = d->layer_slot(l, kSlotRelu);
-      MI8D_TRY(quant_gemm(d, d->x2, R, s2, w.w1, true, d->hbuf, s, s3));   // ReLU and max|h| fused in the write-back
+      MI8D_TRY(quant_gemm(d, d->x2, R, s2, w.w1, true, d->hbuf, s, s3, lq));   // ReLU and max|h| fused in the write-back
 
       // the block's output is the next layer's input: write it straight into that layer's history slab, and its
       // maximum into that layer's history abs-max as well
@@ -1158,14 +1189,16 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
       float* nx = last ? d->x_final : (c.ssru ? d->x_in : d->layers[l + 1].slab + static_cast<size_t>(t) * slab_stride);
       float* nx_rowmax = (last || c.ssru) ? nullptr : d->layers[l + 1].rowmax + static_cast<size_t>(t) * SR;
       unsigned* nx_hist = (last || c.ssru) ? nullptr : d->layer_slot(l + 1, kSlotHistory);
-      MI8D_TRY(quant_gemm_ln(d, d->hbuf, R, s3, w.w2, d->x2, w.ln_ffn, d->obuf, nx, nx_rowmax, d->layer_slot(l, kSlotOut), s, nx_hist));
+      MI8D_TRY(quant_gemm_ln(d, d->hbuf, R, s3, w.w2, d->x2, w.ln_ffn, d->obuf, nx, nx_rowmax, d->layer_slot(l, kSlotOut), s, nx_hist,
+                             lq && (last || c.ssru)));
       x = nx;
     }
   }
 
   // tied output layer, then log-softmax + n-best per sentence over beam x vocabulary
   unsigned* x_slot = d->input_slot(c.dec_depth);
-  MI8D_TRY(quantize_act(d, x, R, dm, x_slot, d->aq, s));
+  if(!lq)
+    MI8D_TRY(quantize_act(d, x, R, dm, x_slot, d->aq, s));
   // The plain GEMM followed by the log-softmax / top-k kernel is the faster route at every row count since that kernel scans
   // without candidate lists (beam 6, 2 sentences of transformer-base: 16.2 ms a mini-batch with the reducing write-back, 15.2 ms
   // without; student, 16 sentences x beam 4: 7.3 and 7.0; 64 x 4 and 128 x 4 rows: level).  opt_fused_out_rows > 0 brings the other back.

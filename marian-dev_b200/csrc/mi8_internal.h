@@ -190,6 +190,12 @@ int launch_step_begin(const int* host_ctrl, int* ctrl, int n_ctrl, unsigned* slo
 // slot2 (optional): a second 4-byte slot that receives the same maximum (the self-attention history's abs-max)
 int launch_add_layernorm(const float* a, const float* resid, const float* gamma, const float* beta, float eps, int rows, int dim,
                          float* out, float* rowmax, unsigned* slot, cudaStream_t s, unsigned* slot2 = nullptr);
+// the same for few rows with the quantisation of the result (q, d_qm) in the same launch; cell_old != nullptr: the SSRU cell's output
+// in the place of `a` (see launch_ssru_cell)
+bool add_layernorm_quant_supported(int rows, int dim);
+int launch_add_layernorm_quant(const float* a, const float* resid, const float* gamma, const float* beta, float eps, int rows, int dim, float* out,
+                               int8_t* q, float* d_qm, cudaStream_t s, const float* cell_old = nullptr, const int* hyp = nullptr,
+                               const float* xw = nullptr, const float* f = nullptr, float* cell_new = nullptr);
 int launch_quantize_slot(const float* x, size_t n, const unsigned* slot, int8_t* q, float* d_qm, cudaStream_t s);
 // the embedding of a step (slot2: the history's abs-max of layer 0) and the ancestor table; hist_layers > 0: also reduces, per layer, the
 // maximum of rowmax over the earlier slabs' ancestor rows into hist_slot[l]
