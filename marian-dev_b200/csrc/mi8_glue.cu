@@ -1017,8 +1017,10 @@ __device__ __forceinline__ void finish_step(const StepEnd& e, int r, int k, int 
 
 // Combines the per-block pairs (m_b, s_b) of one row, held in shared memory, into the row's log-sum-exp:
 // M = max_b m_b;  S = sum over b ascending of s_b * exp(m_b - M), product and sum rounded separately;
-// lse = M + log(S).  bm/bs: nb entries each; red: 33 floats.  Every thread returns the same value.
-__device__ __forceinline__ float lse_from_blocks(float* bm, float* bs, int nb, float* red) {
+// lse = M + log(S).  bm/bs: nb entries each; red: 33 floats.  Every thread returns the same value.  `beside` is called by all threads
+// while warp 0 walks the chain of additions (it may read bm).
+template <typename F>
+__device__ __forceinline__ float lse_from_blocks(const float* bm, float* bs, int nb, float* red, F&& beside) {
   float mx = -FLT_MAX;
   for(int b = threadIdx.x; b < nb; b += blockDim.x)
     mx = fmaxf(mx, bm[b]);
@@ -1041,6 +1043,7 @@ __device__ __forceinline__ float lse_from_blocks(float* bm, float* bs, int nb, f
       total = __fadd_rn(total, bs[b]);
     red[32] = __fadd_rn(mx, det_logf(total));
   }
+  beside();
   __syncthreads();
   return red[32];
 }
@@ -1059,10 +1062,12 @@ __device__ __forceinline__ float lse_from_blocks(float* bm, float* bs, int nb, f
 //     from the block maxima, their entries that reach the k-th maximum are collected, and an entry's place in the
 //     output is the number of collected entries before it.
 // 512 rows of 32000 logits with a list of k per thread and a block of 128 per lane: 55.6 us back to back and 42.6 us inside a
-// decoder step (logits in L2); now 34.0 and 24.7 us.
-// kThreads: 1024 (one pass over 32000 logits) while there is at most a block per half SM, 256 otherwise.
+// decoder step (logits in L2); 34.0 and 24.7 us as described, 26.9 back to back with the block sizes below.
+// kThreads: 1024 (one pass over 32000 logits, one block per SM) while every row has an SM to itself, 512 (two blocks per SM) up to two
+// rows per SM, 256 (four) beyond, registers held to 64 so that they fit: 148 rows 14.9 us with the picks after the sum, 13.4 now; 256
+// rows 29.1 us with 256 threads, 18.0 now; 512 rows 33.8 us, 26.9 now.
 template <int kThreads>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads)
 lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float* __restrict__ prev_scores, float* cand_score, int* cand_word,
                 const StepEnd end) {
   pdl_launch_dependents();
@@ -1133,17 +1138,19 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
     }
   }
   __syncthreads();
-  // the k blocks with the best maxima (warp 0): k rounds, each picks the best block that follows the last pick
-  if(warp == 0) {
+  // While warp 0 sums the blocks: the k blocks with the best maxima (warp 1), k rounds, each picks the best block that follows the
+  // last pick.
+  auto pick_blocks = [&]() {
+    if(warp != 1)
+      return;
     float last_v = FLT_MAX;
     int last_i = -1;
-    bool first = true;
     for(int j = 0; j < k; ++j) {
       float v = -FLT_MAX;
       int i = 0x7fffffff;
       for(int b = lane; b < nb; b += 32) {
         const float bv = bm[b];
-        if((first || better(last_v, last_i, bv, b)) && better(bv, b, v, i)) {
+        if((j == 0 || better(last_v, last_i, bv, b)) && better(bv, b, v, i)) {
           v = bv;
           i = b;
         }
@@ -1159,14 +1166,13 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
       }
       last_v = v;
       last_i = i;
-      first = false;
       if(lane == 0)
         pick[j] = i;   // 0x7fffffff: there are fewer than k blocks
     }
     if(lane == 0)
       s_floor = last_v;
-  }
-  __syncthreads();
+  };
+  const float lse = lse_from_blocks(bm, bs, nb, red, pick_blocks);
   const float floor_v = s_floor;
   // Without k maxima above the lowest finite value the argument above does not hold (a block without a single number shares that
   // maximum): then the k best are searched for one by one.
@@ -1187,7 +1193,7 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
       }
     }
   }
-  const float lse = lse_from_blocks(bm, bs, nb, red);   // (its barriers also order the collection above)
+  __syncthreads();
   const float ps = prev_scores ? prev_scores[r] : 0.f;
   if(by_pick) {
     const int n = n_cand;
@@ -1284,7 +1290,7 @@ lse_merge_kernel(const float* __restrict__ blk_max, const float* __restrict__ bl
     s_i[threadIdx.x * KT + j] = t.i[j];
   }
   __syncthreads();
-  const float lse = lse_from_blocks(bm, bs, nb, red);
+  const float lse = lse_from_blocks(bm, bs, nb, red, []() {});
   topk_block_merge<KT>(s_v, s_i);
   if(threadIdx.x < k) {
     const float ps = prev_scores ? prev_scores[r] : 0.f;
@@ -1595,9 +1601,10 @@ int launch_lse_topk(const float* logits, int rows, int vocab, int k, const float
   const size_t smem = 2 * static_cast<size_t>((vocab + 127) / 128) * sizeof(float);
   if(smem > 32 * 1024)
     return MI8_ERR_UNSUPPORTED;
-  // Few rows: 1024 threads each, so that a row of 32000 takes one pass. 
-  if(rows <= 2 * sm_count())
+  if(rows <= sm_count())
     launch_kernel(lse_topk_kernel<1024>, dim3(rows), dim3(1024), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word, end);
+  else if(rows <= 2 * sm_count())
+    launch_kernel(lse_topk_kernel<512>, dim3(rows), dim3(512), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word, end);
   else
     launch_kernel(lse_topk_kernel<256>, dim3(rows), dim3(256), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word, end);
   count_launch();

@@ -132,7 +132,7 @@ def test_cross_attention_rows_of_a_sentence_together(cuda_device, oracle, rows, 
         assert slot.view(torch.float32).item() == np.abs(want).max()
 
 
-@pytest.mark.parametrize("rows", [3, 400])                     # 1024 and 256 threads per row
+@pytest.mark.parametrize("rows", [3, 200, 400])                # 1024, 512 and 256 threads per row
 @pytest.mark.parametrize("vocab,k", [(128, 1), (129, 2), (1000, 8), (1027, 8), (4096, 4), (32000, 4)])
 def test_lse_topk_awkward_rows(cuda_device, oracle, rows, vocab, k):
     """Masked entries (lowest finite value, -inf), whole blocks of them, fewer usable entries than k, equal values everywhere."""
