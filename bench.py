@@ -579,7 +579,7 @@ def pick_workers(requested, n_batches):
 
 TRACE_KERNELS = {1: "mi8_gemm_kernel", 2: "mi8_gemm_pair_kernel", 3: "quantize_slot_kernel", 4: "quantize_dual_kernel", 5: "add_layernorm_kernel",
                  6: "attention1_kernel", 7: "attention_enc_kernel", 8: "lse_topk_kernel", 9: "lse_merge_kernel", 10: "nbest_merge_kernel",
-                 11: "embed_kernel", 12: "ancestors_update_kernel", 13: "history_commit_kernel", 14: "gather_rows_kernel", 15: "ssru_cell_kernel",
+                 11: "embed_kernel", 14: "gather_rows_kernel", 15: "ssru_cell_kernel",
                  16: "mi8_absmax_kernel", 17: "mi8_quantize_kernel", 18: "mi8_gemm_kernel (output layer, reducing write-back)",
                  19: "mi8_gemm_kernel (quantising its activation)", 20: "mi8_gemm_cq_kernel"}
 
