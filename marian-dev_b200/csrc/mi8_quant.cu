@@ -214,28 +214,47 @@ constexpr int kPrepareCtas = 8;
 constexpr size_t kOneCtaMaxN = 512 * 16, kClusterMinN = 2 * 1024 * 16;
 constexpr size_t kClusterMaxN = static_cast<size_t>(kPrepareCtas) * 1024 * 16 * 2;
 
-// W fp32 [K,N] row-major -> Bt int8 [N,K] row-major.  A block moves a 32(k) x 32(n) tile through
-// shared memory so that both the fp32 reads (along n) and the int8 writes (along k) are contiguous.
+// W fp32 [K,N] row-major -> Bt int8 [N,K] row-major.  A block moves a 128(k) x 32(n) tile: a thread reads four values of one column
+// (a warp 128 bytes of a row each time, sixteen loads in flight per thread), packs them into a word and parks it in shared memory, and a
+// warp stores 128 consecutive bytes of a row of Bt.  Bound by the read of W (from L2 behind the abs-max while W fits there).
+// Conversion of 4096 x 8192: 81 us with 32 x 32 tiles and a byte per store, 53 us now (up to about 1024 x 4096 it is bound by the call).
 __global__ void __launch_bounds__(256)
 mi8_transpose_quantize_kernel(const float* __restrict__ w, int K, int N, const float* __restrict__ d_quant_mult,
-                              int8_t* __restrict__ bt) {
+                              int8_t* __restrict__ bt, int words) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float tile[32][33];
+  __shared__ unsigned tile[32][33];   // [n][k / 4]
   const float qm = *d_quant_mult;
-  const int n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+  const int n0 = blockIdx.x * 32, k0 = blockIdx.y * 128;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n = n0 + lane;
+  float4 v[4];
 #pragma unroll
-  for(int r = 0; r < 32; r += 8) {
-    const int k = k0 + ty + r, n = n0 + tx;
-    tile[ty + r][tx] = (k < K && n < N) ? w[static_cast<size_t>(k) * N + n] : 0.0f;
+  for(int i = 0; i < 4; ++i) {
+    const int k = k0 + 4 * (warp + 8 * i);
+    const float* src = w + static_cast<size_t>(k) * N + n;
+    v[i].x = (k < K && n < N) ? __ldg(src) : 0.0f;
+    v[i].y = (k + 1 < K && n < N) ? __ldg(src + N) : 0.0f;
+    v[i].z = (k + 2 < K && n < N) ? __ldg(src + 2 * static_cast<size_t>(N)) : 0.0f;
+    v[i].w = (k + 3 < K && n < N) ? __ldg(src + 3 * static_cast<size_t>(N)) : 0.0f;
   }
+#pragma unroll
+  for(int i = 0; i < 4; ++i)
+    tile[lane][warp + 8 * i] = pack4(v[i], qm);
   __syncthreads();
 #pragma unroll
-  for(int r = 0; r < 32; r += 8) {
-    const int n = n0 + ty + r, k = k0 + tx;
-    if(n < N && k < K)
-      bt[static_cast<size_t>(n) * K + k] = static_cast<int8_t>(quantize_one(tile[tx][ty + r], qm));
+  for(int i = 0; i < 4; ++i) {
+    const int r = warp + 8 * i, k = k0 + 4 * lane;
+    if(n0 + r < N && k < K) {
+      int8_t* dst = bt + static_cast<size_t>(n0 + r) * K + k;
+      const unsigned o = tile[r][lane];
+      if(words) {   // K is a multiple of four and Bt 4-byte aligned
+        *reinterpret_cast<unsigned*>(dst) = o;
+      } else {
+        for(int e = 0; e < 4 && k + e < K; ++e)
+          dst[e] = static_cast<int8_t>(o >> (8 * e));
+      }
+    }
   }
 }
 
@@ -350,10 +369,10 @@ int launch_prepare(const float* x, size_t n, float* d_quant_mult, int8_t* q, voi
 int launch_transpose_quantize(const float* w, int K, int N, const float* d_quant_mult, int8_t* bt, cudaStream_t stream) {
   if(w == nullptr || bt == nullptr || d_quant_mult == nullptr || K <= 0 || N <= 0)
     return MI8_ERR_BAD_ARG;
-  dim3 grid((N + 31) / 32, (K + 31) / 32);
-  if(grid.y > 65535)
+  if((K + 31) / 32 > 65535)
     return MI8_ERR_UNSUPPORTED;
-  launch_kernel(mi8_transpose_quantize_kernel, dim3(grid), dim3(256), 0, stream, w, K, N, d_quant_mult, bt);
+  const int words = K % 4 == 0 && (reinterpret_cast<uintptr_t>(bt) & 3u) == 0 ? 1 : 0;
+  launch_kernel(mi8_transpose_quantize_kernel, dim3((N + 31) / 32, (K + 127) / 128), dim3(256), 0, stream, w, K, N, d_quant_mult, bt, words);
   count_launch();
   return check_launch();
 }

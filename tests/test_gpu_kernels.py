@@ -169,6 +169,26 @@ def test_cta_pair_kernel_many_tiles(cuda_device, oracle):
     _run_affine(cuda_device, oracle, 2100, 1024, 1000, True, False, 13, out_dtype=torch.float16, tile_m=512)
 
 
+@pytest.mark.parametrize("k,n,offset", [(16, 1, 0), (112, 31, 0), (128, 32, 0), (144, 33, 0), (1024, 100, 0), (30, 65, 0), (127, 33, 0), (131, 40, 0), (128, 33, 2)])
+def test_conversion_tile_edges(cuda_device, k, n, offset):
+    """W [K,N] -> Bt [N,K]: tiles that end inside K or N, inner dimensions that are not whole words and an output off a word boundary."""
+    from marian_dev_b200.binding import check, lib
+    L = lib()
+    w = np.random.default_rng(k + n).standard_normal((k, n)).astype(np.float32)
+    wd = torch.from_numpy(w).to(cuda_device)
+    out = torch.full((n * k + offset + 16,), 99, dtype=torch.int8, device=cuda_device)
+    qm = torch.zeros(1, device=cuda_device)
+    ws = torch.zeros(1 << 20, dtype=torch.uint8, device=cuda_device)
+    check(L.mi8_prepare_b_f32(wd.data_ptr(), k, n, 0, out[offset:].data_ptr(), qm.data_ptr(), ws.data_ptr(), ws.numel(),
+                              torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    want_qm = np.float32(127) / np.abs(w).max()
+    got = out.cpu().numpy()
+    assert np.float32(qm.item()) == want_qm
+    assert np.array_equal(got[offset:offset + n * k].reshape(n, k), np.rint(w * want_qm).astype(np.int8).T)
+    assert (got[:offset] == 99).all() and (got[offset + n * k:] == 99).all()
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 16), (3, 16), (1, 8176), (2, 4096), (1, 8208), (2, 16368), (2, 16384), (1, 32784), (128, 1024), (1, 131088),
                                        (256, 1024), (1, 262160)])
 @pytest.mark.parametrize("where", ["first", "last", "zero"])
