@@ -327,7 +327,10 @@ int launch_quantize(const float* x, size_t n, const float* d_quant_mult, int8_t*
     return MI8_ERR_BAD_ARG;
   if((reinterpret_cast<uintptr_t>(x) & 15u) || (reinterpret_cast<uintptr_t>(q) & 15u))
     return MI8_ERR_MISALIGNED;
-  const int grid = stream_grid(n / 16 + 1);
+  // A chunk of 16 floats per thread until the SMs are full: with four in turn, 4 M floats were 246 blocks, 13 warps per SM
+  // (affine 3937 x 1024 x 4096 41.3 -> 34.3 us, 2000 x 4096 x 1024 35.2 -> 30.0, 4096 x 1024 x 32000 134.8 -> 130.6).
+  const size_t want = (n / 16 + kBlock) / kBlock, cap = static_cast<size_t>(sm_count()) * 8;
+  const int grid = static_cast<int>(want < cap ? want : cap);
   launch_kernel(mi8_quantize_kernel, dim3(grid), dim3(kBlock), 0, stream, x, n, d_quant_mult, q);
   count_launch();
   return check_launch();
