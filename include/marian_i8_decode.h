@@ -155,6 +155,11 @@ int mi8g_output_topk(const int8_t* aq, const float* d_qa, const int8_t* wq, cons
 /* Per sentence: the k best of its beam x k row candidates, sorted; ties to the smaller (beam, word) key. */
 int mi8g_nbest_merge(const float* cand_score, const int* cand_word, int beam, int batch, int vocab, int k,
                      float* out_score, int* out_beam, int* out_word, void* stream);
+/* mi8g_lse_topk over the rows of `beam` hypotheses of `batch` sentences (row = hypothesis * batch + sentence) and mi8g_nbest_merge in one
+ * launch, as a decoder step ends: whichever row of a sentence is done last merges the sentence.  arrivals [batch]: zeroed by the
+ * caller before every call.  beam * k <= 1024 (MI8_ERR_UNSUPPORTED otherwise; mi8d_step then launches mi8g_nbest_merge's kernel). */
+int mi8g_lse_topk_nbest(const float* logits, int beam, int batch, int vocab, int k, const float* prev_scores, float* cand_score,
+                        int* cand_word, unsigned* arrivals, float* out_score, int* out_beam, int* out_word, void* stream);
 
 /* How often the stored self-attention keys/values could be kept: out[0] = (layer, step) pairs whose
  * history abs-max was bit-identical to the previous step's, out[1] = all pairs; reset != 0 clears the

@@ -865,6 +865,20 @@ int mi8g_nbest_merge(const float* cand_score, const int* cand_word, int beam, in
     return MI8_ERR_BAD_ARG;
   return launch_nbest_merge(cand_score, cand_word, beam, batch, vocab, k, out_score, out_beam, out_word, as_stream(stream));
 }
+int mi8g_lse_topk_nbest(const float* logits, int beam, int batch, int vocab, int k, const float* prev_scores, float* cand_score,
+                        int* cand_word, unsigned* arrivals, float* out_score, int* out_beam, int* out_word, void* stream) {
+  if(logits == nullptr || cand_score == nullptr || cand_word == nullptr || arrivals == nullptr || out_score == nullptr || out_beam == nullptr ||
+     out_word == nullptr || beam < 1 || batch < 1 || beam > INT32_MAX / batch)
+    return MI8_ERR_BAD_ARG;
+  StepEnd end;
+  end.beam = beam;
+  end.batch = batch;
+  end.arrivals = arrivals;
+  end.out_score = out_score;
+  end.out_beam = out_beam;
+  end.out_word = out_word;
+  return launch_lse_topk(logits, beam * batch, vocab, k, prev_scores, cand_score, cand_word, as_stream(stream), end);
+}
 
 int mi8d_start(mi8d_decoder* d, const float* context, const float* log_mask, int batch, int src, void* stream) {
   if(d == nullptr || context == nullptr || log_mask == nullptr || batch <= 0 || src <= 0)
@@ -1203,10 +1217,11 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
   // without candidate lists (beam 6, 2 sentences of transformer-base: 16.2 ms a mini-batch with the reducing write-back, 15.2 ms
   // without; student, 16 sentences x beam 4: 7.3 and 7.0; 64 x 4 and 128 x 4 rows: level).  opt_fused_out_rows > 0 brings the other back.
   const bool fused_output = !d->p8 && !d->keep_logits && R <= d->opt_fused_out_rows && n_best >= 2;
+  const bool merge_apart = !step_end_fits(beam, n_best);
   StepEnd end;
   end.beam = beam;
   end.batch = batch;
-  end.arrivals = d->arrivals();
+  end.arrivals = merge_apart ? nullptr : d->arrivals();
   end.out_score = out_score;
   end.out_beam = out_beam;
   end.out_word = out_word;
@@ -1229,6 +1244,8 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
     MI8D_TRY(launch_lse_merge(d->blk_max, d->blk_sum, d->blk_topv, d->blk_topi, R, c.vocab, k_top, n_best, prev_scores, d->cand_score,
                               d->cand_word, s, end));
   }
+  if(merge_apart)
+    MI8D_TRY(launch_nbest_merge(d->cand_score, d->cand_word, beam, batch, c.vocab, n_best, out_score, out_beam, out_word, s));
   d->anc_cur = anc_new;
   d->cell_cur = cell_new;
   d->t = t + 1;

@@ -958,6 +958,8 @@ __device__ __forceinline__ void topk_block_merge(float* s_v, int* s_i) {
 // candidates before it; places that stay empty get score -inf, beam 0, word 0.  Block 0 also remembers, per layer, the history
 // abs-max the stored keys/values now belong to (prev_bits[l] = slots[first + l * stride]; stats: pairs unchanged, all pairs).
 // In place of two launches, each of a launch's hand-over (6 us together in a transformer-base step).
+// The sentence's candidates lie in c_v / c_i: beam * k <= kStepEndCandidates (both launchers refuse more; mi8d_step then merges the
+// n-best lists with nbest_merge_kernel, which has no such limit).
 __device__ __forceinline__ void finish_step(const StepEnd& e, int r, int k, int vocab, const float* cand_score, const int* cand_word, float* c_v,
                                             int* c_i, int* s_last) {
   if(blockIdx.x == 0 && static_cast<int>(threadIdx.x) < e.layers) {
@@ -979,7 +981,7 @@ __device__ __forceinline__ void finish_step(const StepEnd& e, int r, int k, int 
   __syncthreads();
   if(!*s_last || threadIdx.x >= 32)
     return;
-  const int n = e.beam * k;   // at most kMaxK * kMaxK
+  const int n = e.beam * k;
   int valid = 0;
   for(int c0 = 0; c0 < n; c0 += 32) {
     const int c = c0 + threadIdx.x;
@@ -1076,6 +1078,7 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
   pdl_wait();
   trace_stamp_start(th, kTrLseTopk);
   extern __shared__ float lse_blocks[];   // [nb] block maxima, [nb] block sums
+  static_assert(kStepEndCandidates <= kMaxK * 128, "finish_step reuses these arrays");
   __shared__ float c_v[kMaxK * 128];      // collected candidates
   __shared__ int c_i[kMaxK * 128];
   __shared__ float red[33];
@@ -1262,6 +1265,7 @@ lse_merge_kernel(const float* __restrict__ blk_max, const float* __restrict__ bl
   unsigned long long* const tb = th.first;
   pdl_wait();
   trace_stamp_start(th, kTrLseMerge);
+  static_assert(kStepEndCandidates <= 256 * KT, "finish_step reuses these arrays");
   extern __shared__ float lse_blocks[];
   __shared__ float s_v[256 * KT];
   __shared__ int s_i[256 * KT];
@@ -1598,6 +1602,8 @@ int launch_lse_topk(const float* logits, int rows, int vocab, int k, const float
                     cudaStream_t s, const StepEnd& end) {
   if(rows <= 0 || vocab <= 0 || k < 1 || k > kMaxK)
     return MI8_ERR_BAD_ARG;
+  if(end.arrivals != nullptr && !step_end_fits(end.beam, k))
+    return MI8_ERR_UNSUPPORTED;
   const size_t smem = 2 * static_cast<size_t>((vocab + 127) / 128) * sizeof(float);
   if(smem > 32 * 1024)
     return MI8_ERR_UNSUPPORTED;
@@ -1615,6 +1621,8 @@ int launch_lse_merge(const float* blk_max, const float* blk_sum, const float* bl
                      int k_top, int k, const float* prev_scores, float* cand_score, int* cand_word, cudaStream_t s, const StepEnd& end) {
   if(rows <= 0 || vocab <= 0 || k < 1 || k > k_top || (k_top != 4 && k_top != 8))
     return MI8_ERR_BAD_ARG;
+  if(end.arrivals != nullptr && !step_end_fits(end.beam, k))
+    return MI8_ERR_UNSUPPORTED;
   const int nb = (vocab + 127) / 128;
   const size_t smem = 2 * static_cast<size_t>(nb) * sizeof(float);
   if(smem > 32 * 1024)

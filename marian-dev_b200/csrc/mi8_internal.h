@@ -172,6 +172,9 @@ struct StepEnd {
   unsigned* prev_bits = nullptr;
   unsigned* stats = nullptr;
 };
+// Candidates of one sentence (beam x k) that the row kernels' shared memory holds; wider beams end with launch_nbest_merge.
+constexpr int kStepEndCandidates = 1024;
+constexpr bool step_end_fits(int beam, int k) { return beam <= kStepEndCandidates / k; }
 
 // Output layer: GEMM whose write-back reduces every (row, block of 128 vocabulary entries) to its maximum, its sum
 // of exponentials and its k_top (4 or 8) best entries (blk_* arrays: [rows][ceil(vocab/128)] (x k_top)); then

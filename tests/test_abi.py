@@ -145,3 +145,11 @@ def test_new_entry_points_reject_bad_arguments_before_any_launch():
     assert L.mi8g_output_scratch_bytes(512, 32000) == 512 * 250 * 18 * 4
     assert L.mi8g_output_topk(16, 32, 48, 64, 8, 256, 64, 80, 4, None, 96, 16, None, 112, 128, None) == 4
     assert L.mi8g_output_topk(16, 32, 48, 64, 8, 256, 64, 80, 9, None, 96, 1 << 20, None, 112, 128, None) == 1
+
+
+@pytest.mark.parametrize("beam,k", [(129, 8), (257, 4), (1025, 1), (2 ** 31 - 1, 1)])
+def test_end_of_a_step_refuses_more_candidates_than_it_holds(beam, k):
+    """A sentence's beam x k candidates are merged in 1024 entries of shared memory; more are refused before any launch."""
+    from marian_dev_b200.binding import lib
+    p = ctypes.c_void_p(4096)                                        # never dereferenced
+    assert lib().mi8g_lse_topk_nbest(p, beam, 1, 1000, k, None, p, p, p, p, p, p, None) == 3

@@ -190,6 +190,53 @@ def test_lse_topk_and_merge_bit_exact(cuda_device, oracle, rows, vocab, k):
         assert ob[n].item() == cands[n][1] // vocab and ow[n].item() == cands[n][1] % vocab
 
 
+def _nbest_of(cs, cw, beam, batch, vocab, k):
+    """The k best of a sentence's candidates by (score, then smaller flattened key), empty places -inf / 0 / 0."""
+    score, hyp, word = np.full((batch, k), -np.inf, np.float32), np.zeros((batch, k), np.int32), np.zeros((batch, k), np.int32)
+    for b in range(batch):
+        rows = [j * batch + b for j in range(beam)]
+        cands = sorted((-float(cs[r, c]), j * vocab + int(cw[r, c])) for j, r in enumerate(rows) for c in range(k) if cs[r, c] > np.finfo(np.float32).min)
+        for n, (s, key) in enumerate(cands[:k]):
+            score[b, n], hyp[b, n], word[b, n] = -s, key // vocab, key % vocab
+    return score, hyp, word
+
+
+@pytest.mark.parametrize("beam,batch,vocab,k", [(1, 1, 130, 1), (1, 3, 5, 8), (3, 5, 130, 3), (8, 2, 1000, 8), (6, 40, 300, 6), (4, 129, 140, 4), (128, 2, 130, 8),
+                                                (341, 1, 129, 3), (1024, 1, 64, 1)])
+def test_end_of_a_step_merges_the_sentences(cuda_device, oracle, beam, batch, vocab, k):
+    """Log-softmax, row candidates and n-best lists in one launch: ties across hypotheses, dummy hypotheses, sentences with fewer
+    candidates than k and with none, up to the 1024 candidates a sentence may have; the separate merge agrees."""
+    L, check = _lib()
+    rng = np.random.default_rng(beam * k + vocab)
+    rows = beam * batch
+    logits = rng.integers(-3, 4, (rows, vocab)).astype(np.float32)                # coarse values: many ties within a row
+    prev = rng.integers(-2, 3, rows).astype(np.float32)
+    if beam > 1:                                                                  # hypotheses 0 and 1 of a sentence are the same row
+        logits[batch:2 * batch] = logits[:batch]
+        prev[batch:2 * batch] = prev[:batch]
+    prev[rng.random(rows) < 0.2] = -np.inf                                        # dummy hypotheses
+    if batch > 1:
+        prev[batch - 1::batch] = -np.inf                                          # the last sentence has no other
+        prev[0::batch] = -np.inf                                                  # the first has one, with two words above the lowest value
+        prev[0] = 0.5
+        logits[0] = np.finfo(np.float32).min
+        logits[0, [1, vocab - 1]] = 1.0
+    cs_w, cw_w = oracle.lse_topk(logits, k, prev)
+    ld, pd = _dev(logits, cuda_device), _dev(prev, cuda_device)
+    cs = torch.empty(rows, k, device=cuda_device)
+    cw = torch.empty(rows, k, dtype=torch.int32, device=cuda_device)
+    arrivals = torch.zeros(batch, dtype=torch.int32, device=cuda_device)
+    outs = [torch.full((batch, k), 7, dtype=t, device=cuda_device) for t in (torch.float32, torch.int32, torch.int32) * 2]
+    check(L.mi8g_lse_topk_nbest(ld.data_ptr(), beam, batch, vocab, k, pd.data_ptr(), cs.data_ptr(), cw.data_ptr(), arrivals.data_ptr(),
+                                *[o.data_ptr() for o in outs[:3]], _stream()))
+    check(L.mi8g_nbest_merge(cs.data_ptr(), cw.data_ptr(), beam, batch, vocab, k, *[o.data_ptr() for o in outs[3:]], _stream()))
+    torch.cuda.synchronize()
+    assert np.array_equal(cs.cpu().numpy(), cs_w) and np.array_equal(cw.cpu().numpy(), cw_w)
+    for got, apart, want in zip(outs[:3], outs[3:], _nbest_of(cs_w, cw_w, beam, batch, vocab, k)):
+        assert np.array_equal(got.cpu().numpy(), want)
+        assert np.array_equal(apart.cpu().numpy(), want)
+
+
 def test_embed_and_quantize_slot(cuda_device, oracle):
     L, check = _lib()
     rng = np.random.default_rng(4)

@@ -45,3 +45,43 @@ def test_merged_launches_give_the_same_bits(cuda_device, dim, rnn, batch, beam):
         for a, b in zip(got, want):
             assert [list(t) for t, _ in a] == [list(t) for t, _ in b], options
             assert [np.float32(s) for _, s in a] == [np.float32(s) for _, s in b], options
+
+
+@pytest.mark.parametrize("beam,n_best", [(128, 8), (129, 8), (160, 8), (257, 4)])
+@pytest.mark.parametrize("fused_output", [0, 512])
+def test_step_of_a_wide_beam(cuda_device, beam, n_best, fused_output):
+    """mi8d_step takes as many hypotheses per sentence as the driver has rows: up to 1024 candidates the n-best lists are merged by the
+    step's last kernel, beyond by a launch of their own."""
+    import ctypes
+    from marian_dev_b200 import decoder, model, ops
+    cfg = model.CONFIGS["tiny-ssru"]
+    net = decoder.Int8Transformer(cfg, model.random_init(cfg, 3), cuda_device)
+    stepper = decoder.NativeStepper(net, max_batch=1, beam=beam, max_src=6, max_steps=8)
+    stepper.set_option("fused_output_max_rows", fused_output)
+    rng = np.random.default_rng(beam)
+    ids = torch.from_numpy(rng.integers(4, cfg.vocab, (1, 5))).to(cuda_device)
+    stepper.encode(ids, torch.ones(1, 5, device=cuda_device))
+    stepper.step(None, None, None, None, 1, 1, n_best)
+    words = rng.integers(4, cfg.vocab, beam)
+    words[beam // 2:] = words[:beam - beam // 2]                     # equal hypotheses with equal scores: ties across the beam
+    prev = rng.integers(-3, 1, beam).astype(np.float32)
+    prev[beam // 2:] = prev[:beam - beam // 2]
+    prev[0] = -np.inf                                                # a dummy hypothesis
+    score, hyp, word, *_ = stepper.step(np.zeros(beam, np.int64), words, np.zeros(1, np.int64), prev, beam, 1, n_best)
+    assert ops.poll_status() == 0
+    # the same step again on a second driver that keeps its logits; candidates and lists through the separate kernels
+    ref = decoder.NativeStepper(net, max_batch=1, beam=beam, max_src=6, max_steps=8)
+    ref.check(ref.L.mi8d_keep_logits(ref.h, 1))
+    ref.encode(ids, torch.ones(1, 5, device=cuda_device))
+    ref.step(None, None, None, None, 1, 1, n_best)
+    ref.step(np.zeros(beam, np.int64), words, np.zeros(1, np.int64), prev, beam, 1, 1)
+    cs = torch.empty(beam, n_best, device=cuda_device)
+    cw = torch.empty(beam, n_best, dtype=torch.int32, device=cuda_device)
+    out = [torch.empty(n_best, dtype=t, device=cuda_device) for t in (torch.float32, torch.int32, torch.int32)]
+    pd = torch.from_numpy(prev).to(cuda_device)
+    stream = torch.cuda.current_stream().cuda_stream
+    ref.check(ref.L.mi8g_lse_topk(ctypes.c_void_p(ref.L.mi8d_last_logits(ref.h)), beam, cfg.vocab, n_best, pd.data_ptr(), cs.data_ptr(), cw.data_ptr(), stream))
+    ref.check(ref.L.mi8g_nbest_merge(cs.data_ptr(), cw.data_ptr(), beam, 1, cfg.vocab, n_best, *[o.data_ptr() for o in out], stream))
+    torch.cuda.synchronize()
+    assert np.array_equal(score[0], out[0].cpu().numpy())
+    assert np.array_equal(hyp[0], out[1].cpu().numpy()) and np.array_equal(word[0], out[2].cpu().numpy())
