@@ -1040,7 +1040,8 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       const int cols_valid = min(T::kTM, p.M - m0);
       int seg = 0, n_loc = n;
       if(!kP8 && p.nseg > 1) {
-        seg = ((2 * wi.n_tile + static_cast<int>(rank)) * kTileN) / p.seg_n;
+        // (an odd number of 128-row weight tiles: the second CTA of the last pair has none, and stores nothing (n_ok))
+        seg = min(((2 * wi.n_tile + static_cast<int>(rank)) * kTileN) / p.seg_n, p.nseg - 1);
         n_loc = n - seg * p.seg_n;
         unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(*p.seg_qa[seg], *p.seg_qb[seg])), p.scale);
       }

@@ -58,6 +58,16 @@ def test_multi_weight_decoder_shapes(cuda_device, oracle, m, k, n_each, count):
     _run(cuda_device, oracle, m, k, n_each, count, with_bias="all" if count == 3 else True)
 
 
+@pytest.mark.parametrize("m,k,n_each", [(4100, 1024, 384), (12700, 912, 128), (1500, 1024, 1152)])
+@pytest.mark.parametrize("with_bias", [False, "all"])
+def test_multi_weight_pair_kernel_odd_tiles(cuda_device, oracle, m, k, n_each, with_bias):
+    """Three matrices of an odd number of 128-row weight tiles each in the two-CTA kernel: the last pair's second CTA has no tile."""
+    from marian_dev_b200 import multiply_plan
+    assert multiply_plan(m, 3 * n_each, k)["tile_m"] == 512 and 3 * n_each // 128 % 2 == 1
+    _run(cuda_device, oracle, m, k, n_each, 3, with_bias=with_bias)
+    _run(cuda_device, oracle, m, k, n_each, 3, with_bias=with_bias, out_dtype=torch.float16)
+
+
 def test_multi_weight_fp16_relu(cuda_device, oracle):
     _run(cuda_device, oracle, 96, 256, 256, 2, with_bias="all", relu=True, out_dtype=torch.float16)
 
