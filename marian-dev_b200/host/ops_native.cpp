@@ -4,8 +4,9 @@
 // Python route took 40 us of host time per affine (measured, 4 x 256 x 1536), so the GPU idled between calls.  Here one call
 // checks its arguments, takes output and scratch from torch's caching allocator and calls the C ABI: about 5 us.
 //
-// Every function returns None for arguments it does not take (another device, type or layout; wrong sizes): the caller then
-// goes through the general Python route, which handles or rejects them.  A non-zero library status is returned as an int.
+// Every function returns None for arguments it does not take (another device, type or layout; wrong sizes; tensors without memory
+// of their own, such as fake or vmapped ones): the caller then goes through the general Python route, which handles or rejects
+// them.  A non-zero library status is returned as an int.  C++ exceptions (an allocation that fails) become torch's Python ones.
 #include <Python.h>
 #include <dlfcn.h>
 
@@ -13,8 +14,11 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <vector>
 
@@ -76,14 +80,30 @@ bool workspace(const at::Tensor& like, PyObject* like_obj, cudaStream_t stream, 
   return ok;
 }
 
-// A CUDA tensor of the current device, contiguous and of the given type, or null.
-const at::Tensor* device_tensor(PyObject* o, at::ScalarType type) {
+// A CUDA tensor of the current device, contiguous and of the given type, with its address; or nothing.
+struct DeviceTensor {
+  const at::Tensor* t = nullptr;
+  void* ptr = nullptr;
+  explicit operator bool() const { return t != nullptr; }
+  const at::Tensor* operator->() const { return t; }
+  template <typename T>
+  T* as() const {
+    return static_cast<T*>(ptr);
+  }
+};
+DeviceTensor device_tensor(PyObject* o, at::ScalarType type) {
   if(!THPVariable_Check(o))
-    return nullptr;
+    return {};
   const at::Tensor& t = THPVariable_Unpack(o);
-  if(!t.is_cuda() || t.scalar_type() != type || !t.is_contiguous() || t.device().index() != c10::cuda::current_device())
-    return nullptr;
-  return &t;
+  try {
+    if(!t.is_cuda() || t.scalar_type() != type || !t.is_contiguous() || t.device().index() != c10::cuda::current_device())
+      return {};
+    void* ptr = t.data_ptr();   // (throws, or is null, for a tensor without memory of its own)
+    return ptr != nullptr || t.numel() == 0 ? DeviceTensor{&t, ptr} : DeviceTensor{};
+  } catch(const std::exception&) {
+    PyErr_Clear();
+    return {};
+  }
 }
 
 at::Tensor new_tensor(c10::IntArrayRef sizes, at::ScalarType type, c10::Device device) {
@@ -107,10 +127,11 @@ PyObject* status(int rc) { return PyLong_FromLong(rc); }
 // The library's calls run without the GIL: a launch waits when the device's queue is full.
 template <typename F>
 int without_gil(F&& f) {
-  PyThreadState* st = PyEval_SaveThread();
-  const int rc = f();
-  PyEval_RestoreThread(st);
-  return rc;
+  struct Release {
+    PyThreadState* st = PyEval_SaveThread();
+    ~Release() { PyEval_RestoreThread(st); }
+  } release;
+  return f();
 }
 
 // Output sizes: the activation's leading dimensions and the weight's width.
@@ -121,22 +142,22 @@ void out_sizes(const at::Tensor& a, int64_t n, c10::SmallVector<int64_t, 6>& siz
 
 // affine(a, weight storage, K, N, bias or None, scale, relu, half) -> tensor [..., N]
 PyObject* py_affine(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
   if(nargs != 8)
     Py_RETURN_NONE;
-  const at::Tensor* a = device_tensor(args[0], at::kFloat);
-  const at::Tensor* w = device_tensor(args[1], at::kByte);
+  const DeviceTensor a = device_tensor(args[0], at::kFloat), w = device_tensor(args[1], at::kByte);
   const int64_t K = PyLong_AsLongLong(args[2]), N = PyLong_AsLongLong(args[3]);
   const double scale = PyFloat_AsDouble(args[5]);
   if(PyErr_Occurred())
     return nullptr;
-  if(a == nullptr || w == nullptr || K <= 0 || N <= 0 || a->dim() < 1 || a->size(-1) != K || a->numel() == 0 || w->numel() < N * K + 4)
+  if(!a || !w || K <= 0 || N <= 0 || a->dim() < 1 || a->size(-1) != K || a->numel() == 0 || w->numel() < N * K + 4)
     Py_RETURN_NONE;
   const float* bias = nullptr;
   if(args[4] != Py_None) {
-    const at::Tensor* b = device_tensor(args[4], at::kFloat);
-    if(b == nullptr || b->numel() != N)
+    const DeviceTensor b = device_tensor(args[4], at::kFloat);
+    if(!b || b->numel() != N)
       Py_RETURN_NONE;
-    bias = static_cast<const float*>(b->data_ptr());
+    bias = b.as<float>();
   }
   const int64_t M = a->numel() / K;
   if(M > INT32_MAX || N > INT32_MAX || K > INT32_MAX)
@@ -145,54 +166,52 @@ PyObject* py_affine(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
   void* ws = nullptr;
   size_t ws_bytes = 0;
-  if(!workspace(*a, args[0], stream, &ws, &ws_bytes))
+  if(!workspace(*a.t, args[0], stream, &ws, &ws_bytes))
     return nullptr;
-  try {
-    c10::SmallVector<int64_t, 6> sizes;
-    out_sizes(*a, N, sizes);
-    at::Tensor out = new_tensor(sizes, half ? at::kHalf : at::kFloat, a->device());
-    const int64_t scratch_bytes = static_cast<int64_t>(round256(static_cast<size_t>(M) * K + 4));
-    at::Tensor scratch = new_tensor({scratch_bytes}, at::kByte, a->device());
-    const int8_t* bt = static_cast<const int8_t*>(w->data_ptr());
-    const int rc = without_gil([&] { return g_lib.affine(static_cast<const float*>(a->data_ptr()), static_cast<int>(M), static_cast<int>(K), bt,
-                                reinterpret_cast<const float*>(bt + N * K), static_cast<int>(N), bias, static_cast<float>(scale), args[6] == Py_True,
-                                out.data_ptr(), half ? MI8_F16 : MI8_F32, static_cast<int8_t*>(scratch.data_ptr()), ws, ws_bytes, stream); });
-    return rc == MI8_OK ? THPVariable_Wrap(std::move(out)) : status(rc);
-  } catch(const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  c10::SmallVector<int64_t, 6> sizes;
+  out_sizes(*a.t, N, sizes);
+  at::Tensor out = new_tensor(sizes, half ? at::kHalf : at::kFloat, a->device());
+  const int64_t scratch_bytes = static_cast<int64_t>(round256(static_cast<size_t>(M) * K + 4));
+  at::Tensor scratch = new_tensor({scratch_bytes}, at::kByte, a->device());
+  const int8_t* bt = w.as<int8_t>();
+  void* c = out.data_ptr();
+  int8_t* aq = static_cast<int8_t*>(scratch.data_ptr());
+  const int rc = without_gil([&] {
+    return g_lib.affine(a.as<float>(), static_cast<int>(M), static_cast<int>(K), bt, reinterpret_cast<const float*>(bt + N * K), static_cast<int>(N), bias,
+                        static_cast<float>(scale), args[6] == Py_True, c, half ? MI8_F16 : MI8_F32, aq, ws, ws_bytes, stream);
+  });
+  return rc == MI8_OK ? THPVariable_Wrap(std::move(out)) : status(rc);
+  END_HANDLE_TH_ERRORS
 }
 
 // prepare_b(w, K, N, w_is_nk) -> uint8 storage: int8 [N, K], its multiplier behind it
 PyObject* py_prepare_b(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
   if(nargs != 4)
     Py_RETURN_NONE;
-  const at::Tensor* w = device_tensor(args[0], at::kFloat);
+  const DeviceTensor w = device_tensor(args[0], at::kFloat);
   const int64_t K = PyLong_AsLongLong(args[1]), N = PyLong_AsLongLong(args[2]);
   if(PyErr_Occurred())
     return nullptr;
-  if(w == nullptr || K <= 0 || N <= 0 || K > INT32_MAX || N > INT32_MAX || (K * N) % 4 != 0 || w->numel() != K * N)
+  if(!w || K <= 0 || N <= 0 || K > INT32_MAX || N > INT32_MAX || (K * N) % 4 != 0 || w->numel() != K * N)
     Py_RETURN_NONE;
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
   void* ws = nullptr;
   size_t ws_bytes = 0;
-  if(!workspace(*w, args[0], stream, &ws, &ws_bytes))
+  if(!workspace(*w.t, args[0], stream, &ws, &ws_bytes))
     return nullptr;
-  try {
-    at::Tensor out = new_tensor({static_cast<int64_t>(round256(static_cast<size_t>(K) * N + 4))}, at::kByte, w->device());
-    int8_t* bt = static_cast<int8_t*>(out.data_ptr());
-    const int rc = without_gil([&] { return g_lib.prepare_b(static_cast<const float*>(w->data_ptr()), static_cast<int>(K), static_cast<int>(N), args[3] == Py_True, bt,
-                                   reinterpret_cast<float*>(bt + K * N), ws, ws_bytes, stream); });
-    return rc == MI8_OK ? THPVariable_Wrap(std::move(out)) : status(rc);
-  } catch(const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  at::Tensor out = new_tensor({static_cast<int64_t>(round256(static_cast<size_t>(K) * N + 4))}, at::kByte, w->device());
+  int8_t* bt = static_cast<int8_t*>(out.data_ptr());
+  const int rc = without_gil([&] {
+    return g_lib.prepare_b(w.as<float>(), static_cast<int>(K), static_cast<int>(N), args[3] == Py_True, bt, reinterpret_cast<float*>(bt + K * N), ws, ws_bytes, stream);
+  });
+  return rc == MI8_OK ? THPVariable_Wrap(std::move(out)) : status(rc);
+  END_HANDLE_TH_ERRORS
 }
 
 // intgemm_views(storage, rows, cols) -> (int8 [rows, cols], float32 [1] behind it)
 PyObject* py_intgemm_views(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
   if(nargs != 3 || !THPVariable_Check(args[0])) {
     PyErr_SetString(PyExc_TypeError, "intgemm_views(storage, rows, cols)");
     return nullptr;
@@ -204,86 +223,77 @@ PyObject* py_intgemm_views(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const size_t first = static_cast<size_t>(s.storage_offset()) * s.element_size();
   if(s.scalar_type() != at::kByte || !s.is_contiguous() || s.numel() < rows * cols + 4 || (first + static_cast<size_t>(rows) * cols) % 4 != 0)
     Py_RETURN_NONE;   // (an unusual storage: the caller takes views the general way, which says what is wrong)
-  try {
-    PyObject* data = THPVariable_Wrap(view_bytes(s, 0, {rows, cols}, at::kChar));
-    PyObject* mult = THPVariable_Wrap(view_bytes(s, static_cast<size_t>(rows) * cols, {1}, at::kFloat));
-    return Py_BuildValue("(NN)", data, mult);
-  } catch(const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  const THPObjectPtr data(THPVariable_Wrap(view_bytes(s, 0, {rows, cols}, at::kChar)));
+  const THPObjectPtr mult(THPVariable_Wrap(view_bytes(s, static_cast<size_t>(rows) * cols, {1}, at::kFloat)));
+  return data && mult ? PyTuple_Pack(2, data.get(), mult.get()) : nullptr;
+  END_HANDLE_TH_ERRORS
 }
 
 // p8_prepare_b(w [K, N]) -> (item, bt, scale_b, zp_b, off_b): the packed8avx512 item, its row-major copy and its tail
 PyObject* py_p8_prepare_b(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-  const at::Tensor* w = nargs == 1 ? device_tensor(args[0], at::kFloat) : nullptr;
-  if(w == nullptr || w->dim() != 2 || w->numel() == 0 || w->size(0) > INT32_MAX || w->size(1) > INT32_MAX)
+  HANDLE_TH_ERRORS
+  const DeviceTensor w = nargs == 1 ? device_tensor(args[0], at::kFloat) : DeviceTensor{};
+  if(!w || w->dim() != 2 || w->numel() == 0 || w->size(0) > INT32_MAX || w->size(1) > INT32_MAX)
     Py_RETURN_NONE;
   const int64_t K = w->size(0), N = w->size(1);
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
-  try {
-    at::Tensor item = new_tensor({static_cast<int64_t>(g_lib.packed_bytes(static_cast<int>(K), static_cast<int>(N)))}, at::kChar, w->device());
-    int8_t* p = static_cast<int8_t*>(item.data_ptr());
-    int rc = without_gil([&] { return g_lib.p8_prepare_b(static_cast<const float*>(w->data_ptr()), static_cast<int>(K), static_cast<int>(N), p, stream); });
-    if(rc != MI8_OK)
-      return status(rc);
-    at::Tensor bt = new_tensor({N, K}, at::kChar, w->device());
-    rc = without_gil([&] { return g_lib.p8_unpack_b(p, static_cast<int>(K), static_cast<int>(N), static_cast<int8_t*>(bt.data_ptr()), stream); });
-    if(rc != MI8_OK)
-      return status(rc);
-    const size_t tail = static_cast<size_t>(K) * N;
-    PyObject* scale = THPVariable_Wrap(view_bytes(item, tail, {N}, at::kFloat));
-    PyObject* zp = THPVariable_Wrap(view_bytes(item, tail + 4 * N, {N}, at::kInt));
-    PyObject* off = THPVariable_Wrap(view_bytes(item, tail + 8 * N, {N}, at::kInt));
-    return Py_BuildValue("(NNNNN)", THPVariable_Wrap(std::move(item)), THPVariable_Wrap(std::move(bt)), scale, zp, off);
-  } catch(const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  at::Tensor item = new_tensor({static_cast<int64_t>(g_lib.packed_bytes(static_cast<int>(K), static_cast<int>(N)))}, at::kChar, w->device());
+  int8_t* p = static_cast<int8_t*>(item.data_ptr());
+  int rc = without_gil([&] { return g_lib.p8_prepare_b(w.as<float>(), static_cast<int>(K), static_cast<int>(N), p, stream); });
+  if(rc != MI8_OK)
+    return status(rc);
+  at::Tensor bt = new_tensor({N, K}, at::kChar, w->device());
+  int8_t* pt = static_cast<int8_t*>(bt.data_ptr());
+  rc = without_gil([&] { return g_lib.p8_unpack_b(p, static_cast<int>(K), static_cast<int>(N), pt, stream); });
+  if(rc != MI8_OK)
+    return status(rc);
+  const size_t tail = static_cast<size_t>(K) * N;   // (K a multiple of 256, N of 32: the library takes no others)
+  const THPObjectPtr scale(THPVariable_Wrap(view_bytes(item, tail, {N}, at::kFloat)));
+  const THPObjectPtr zp(THPVariable_Wrap(view_bytes(item, tail + 4 * N, {N}, at::kInt)));
+  const THPObjectPtr off(THPVariable_Wrap(view_bytes(item, tail + 8 * N, {N}, at::kInt)));
+  const THPObjectPtr item_obj(THPVariable_Wrap(std::move(item))), bt_obj(THPVariable_Wrap(std::move(bt)));
+  return scale && zp && off && item_obj && bt_obj ? PyTuple_Pack(5, item_obj.get(), bt_obj.get(), scale.get(), zp.get(), off.get()) : nullptr;
+  END_HANDLE_TH_ERRORS
 }
 
 // p8_gemm(a, bt, scale_b, zp_b, off_b, bias or None) -> tensor [..., N]
 PyObject* py_p8_gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
   if(nargs != 6)
     Py_RETURN_NONE;
-  const at::Tensor* a = device_tensor(args[0], at::kFloat);
-  const at::Tensor* bt = device_tensor(args[1], at::kChar);
-  const at::Tensor* sb = device_tensor(args[2], at::kFloat);
-  const at::Tensor* zb = device_tensor(args[3], at::kInt);
-  const at::Tensor* ob = device_tensor(args[4], at::kInt);
-  if(a == nullptr || bt == nullptr || sb == nullptr || zb == nullptr || ob == nullptr || bt->dim() != 2)
+  const DeviceTensor a = device_tensor(args[0], at::kFloat), bt = device_tensor(args[1], at::kChar), sb = device_tensor(args[2], at::kFloat);
+  const DeviceTensor zb = device_tensor(args[3], at::kInt), ob = device_tensor(args[4], at::kInt);
+  if(!a || !bt || !sb || !zb || !ob || bt->dim() != 2)
     Py_RETURN_NONE;
   const int64_t N = bt->size(0), K = bt->size(1);
   if(a->dim() < 1 || a->numel() == 0 || a->size(-1) != K || sb->numel() != N || zb->numel() != N || ob->numel() != N || a->numel() / K > INT32_MAX)
     Py_RETURN_NONE;
   const float* bias = nullptr;
   if(args[5] != Py_None) {
-    const at::Tensor* b = device_tensor(args[5], at::kFloat);
-    if(b == nullptr || b->numel() != N)
+    const DeviceTensor b = device_tensor(args[5], at::kFloat);
+    if(!b || b->numel() != N)
       Py_RETURN_NONE;
-    bias = static_cast<const float*>(b->data_ptr());
+    bias = b.as<float>();
   }
   const int M = static_cast<int>(a->numel() / K);
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
   void* ws = nullptr;
   size_t ws_bytes = 0;
-  if(!workspace(*a, args[0], stream, &ws, &ws_bytes))
+  if(!workspace(*a.t, args[0], stream, &ws, &ws_bytes))
     return nullptr;
-  try {
-    c10::SmallVector<int64_t, 6> sizes;
-    out_sizes(*a, N, sizes);
-    at::Tensor out = new_tensor(sizes, at::kFloat, a->device());
-    const size_t need = g_lib.p8_scratch_bytes(M, static_cast<int>(K));
-    at::Tensor scratch = new_tensor({static_cast<int64_t>(need > 256 ? need : 256)}, at::kByte, a->device());
-    const int rc = without_gil([&] { return g_lib.p8_gemm(static_cast<const float*>(a->data_ptr()), static_cast<const int8_t*>(bt->data_ptr()),
-                                 static_cast<const float*>(sb->data_ptr()), static_cast<const int32_t*>(zb->data_ptr()),
-                                 static_cast<const int32_t*>(ob->data_ptr()), bias, static_cast<float*>(out.data_ptr()), M, static_cast<int>(N),
-                                 static_cast<int>(K), scratch.data_ptr(), static_cast<size_t>(scratch.numel()), ws, ws_bytes, stream); });
-    return rc == MI8_OK ? THPVariable_Wrap(std::move(out)) : status(rc);
-  } catch(const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  c10::SmallVector<int64_t, 6> sizes;
+  out_sizes(*a.t, N, sizes);
+  at::Tensor out = new_tensor(sizes, at::kFloat, a->device());
+  const size_t need = std::max<size_t>(g_lib.p8_scratch_bytes(M, static_cast<int>(K)), 256);
+  at::Tensor scratch = new_tensor({static_cast<int64_t>(need)}, at::kByte, a->device());
+  float* c = static_cast<float*>(out.data_ptr());
+  void* scratch_ptr = scratch.data_ptr();
+  const int rc = without_gil([&] {
+    return g_lib.p8_gemm(a.as<float>(), bt.as<int8_t>(), sb.as<float>(), zb.as<int32_t>(), ob.as<int32_t>(), bias, c, M, static_cast<int>(N),
+                         static_cast<int>(K), scratch_ptr, need, ws, ws_bytes, stream);
+  });
+  return rc == MI8_OK ? THPVariable_Wrap(std::move(out)) : status(rc);
+  END_HANDLE_TH_ERRORS
 }
 
 template <typename F>

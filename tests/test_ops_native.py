@@ -1,0 +1,83 @@
+"""The native per-call host path (host/ops_native.cpp): what it declines goes through the general Python route with that route's results and
+errors, and no argument ends the process."""
+import os
+import subprocess
+import sys
+
+import pytest
+import torch
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+_DECLINED = """
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+from marian_dev_b200 import ops
+n = ops.native()
+with FakeTensorMode():                                     # CUDA tensors without memory (and here without a GPU)
+    a, w, f, i = (torch.empty(s, dtype=t, device="cuda") for s, t in (((4, 256), torch.float32), (32 * 256 + 256, torch.uint8), (32, torch.float32),
+                                                                     (32, torch.int32)))
+    bt = torch.empty(32, 256, dtype=torch.int8, device="cuda")
+for a, w, f, i, bt in ((a, w, f, i, bt), [torch.empty(x.shape, dtype=x.dtype) for x in (a, w, f, i, bt)], ["a", None, 3, 4.0, []]):
+    assert n.affine(a, w, 256, 32, f, 1.0, False, False) is None
+    assert n.prepare_b(a, 4, 256, False) is None
+    assert n.p8_prepare_b(a) is None
+    assert n.p8_gemm(a, bt, f, i, i, f) is None
+print("declined")
+"""
+
+
+def test_tensors_without_device_memory_are_declined():
+    """In a process of its own: an exception that leaves the extension ends the process."""
+    r = subprocess.run([sys.executable, "-c", _DECLINED], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip() == "declined", r.stderr[-2000:]
+
+
+def _operands(device, m=6, k=64, n=40):
+    from marian_dev_b200 import ops
+    g = torch.Generator(device=device).manual_seed(m * k + n)
+    x = torch.randn(m, k, generator=g, device=device)
+    return x, ops.prepareB(torch.randn(k, n, generator=g, device=device) * 0.05), torch.randn(n, generator=g, device=device)
+
+
+@pytest.mark.gpu
+def test_vmapped_operands_raise(cuda_device):
+    from marian_dev_b200 import ops, packed8
+    x, w, b = _operands(cuda_device)
+    w8 = packed8.prepareB(torch.randn(256, 32, device=cuda_device))
+    x8, b8 = torch.randn(6, 256, device=cuda_device), torch.randn(32, device=cuda_device)
+    for f, arg in ((lambda t: ops.affine(x, w, t), b), (lambda t: ops.affine(t, w, b), x), (lambda t: ops.prepareB(t).storage, x),
+                   (lambda t: packed8.gemmInt8Packed(x8, w8, t), b8), (lambda t: packed8.gemmInt8Packed(t, w8, b8), x8),
+                   (lambda t: packed8.prepareB(t).item, torch.randn(256, 32, device=cuda_device))):
+        with pytest.raises(RuntimeError):
+            torch.func.vmap(f)(torch.stack([arg, arg]))
+    torch.cuda.synchronize()
+    assert ops.affine(x, w, b).shape == (6, 40) and ops.poll_status() == 0
+
+
+@pytest.mark.gpu
+def test_declined_operands_take_the_general_route(cuda_device):
+    """Layouts that the native route leaves alone give the bits of the contiguous operands; refused ones raise as they do with an explicit
+    workspace, which always takes the general route."""
+    from marian_dev_b200 import ops
+    x, w, b = _operands(cuda_device)
+    want = ops.affine(x, w, b)
+    assert torch.equal(ops.affine(x, w, b, ws=ops.default_workspace(cuda_device)), want)
+    assert torch.equal(ops.affine(x.t().contiguous().t(), w, b), want)
+    assert torch.equal(ops.affine(x, w, torch.stack([b, b], 1)[:, 0]), want)
+    assert torch.equal(ops.affine(x.t().contiguous(), w, b, transA=True), want)
+    assert ops.affine(x.reshape(2, 3, 64), w, b).shape == (2, 3, 40) and ops.affine(x[0], w, b).shape == (40,)
+    for args in ((x.half(), w, b), (x[:, :32].contiguous(), w, b), (x, w, b[:39]), (x, w, b.half()), (x.cpu(), w, b), (x, w, b.cpu()), (x, w.data, b)):
+        for kw in ({}, {"ws": ops.default_workspace(cuda_device)}):
+            with pytest.raises(ops.Mi8Error):
+                ops.affine(*args, **kw)
+    assert ops.poll_status() == 0
+
+
+@pytest.mark.gpu
+def test_failed_allocation_raises_torchs_error(cuda_device):
+    from marian_dev_b200 import ops
+    n = 1 << 24
+    w = ops.prepareB(torch.zeros(16, n, device=cuda_device))
+    with pytest.raises(torch.OutOfMemoryError):          # 4 TB of output
+        ops.affine(torch.zeros(1 << 16, 16, device=cuda_device), w, None)
