@@ -7,7 +7,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from .binding import check, lib
+from .binding import Mi8Error, check, lib
 from .ops import Workspace, _require_cuda, _stream_ptr, default_workspace, native
 
 
@@ -49,9 +49,26 @@ def prepareB(w: torch.Tensor) -> Packed8Weight:
     return Packed8Weight(item, K, N, device=w.device)
 
 
+def _require_float(t: torch.Tensor, what: str) -> None:
+    _require_cuda(t, what)
+    if t.dtype != torch.float32:
+        raise Mi8Error(1, f"{what} must be float32 not {t.dtype}")
+
+
+def _bias_ptr(bias, n: int):
+    """(the bias kept contiguous, its address) or (None, None); raises for one that does not have a float32 value per column."""
+    if bias is None:
+        return None, None
+    _require_float(bias, "bias")
+    if bias.numel() != n:
+        raise Mi8Error(1, f"bias has {bias.numel()} values for {n} output columns")
+    bias = bias.contiguous()
+    return bias, bias.data_ptr()
+
+
 def quantize_rows(a: torch.Tensor):
     """computeQuantizationParams + quantize per row (mjdgemm_avx512.cpp:195-276): (aq uint8, scaleA, zeroPointA, sumA)."""
-    _require_cuda(a, "A")
+    _require_float(a, "A")
     a2 = a.reshape(-1, a.shape[-1]).contiguous()
     M, K = a2.shape
     aq = torch.empty((M, K), dtype=torch.uint8, device=a.device)
@@ -68,12 +85,13 @@ def multiply(aq, scale_a, zp_a, sum_a, w: Packed8Weight, bias=None, relu: bool =
     M, K = aq.shape
     if K != w.K:
         raise ValueError("inner dimensions differ")
+    bias, bias_ptr = _bias_ptr(bias, w.N)
     ws = ws or default_workspace(aq.device)
     c = torch.empty((M, w.N), dtype=torch.float32, device=aq.device)
     acc = torch.empty((M, w.N), dtype=torch.int32, device=aq.device) if want_acc else None
     check(lib().mi8p_multiply(aq.data_ptr(), scale_a.data_ptr(), zp_a.data_ptr(), sum_a.data_ptr(), w.bt.data_ptr(),
                               w.scale_b.data_ptr(), w.zp_b.data_ptr(), w.off_b.data_ptr(), M, w.N, K,
-                              bias.data_ptr() if bias is not None else None, int(relu), c.data_ptr(),
+                              bias_ptr, int(relu), c.data_ptr(),
                               acc.data_ptr() if acc is not None else None, ws.ptr, ws.nbytes, _stream_ptr(), tile_m, splits))
     return (c, acc) if want_acc else c
 
@@ -86,8 +104,18 @@ def gemmInt8Packed(a: torch.Tensor, w: Packed8Weight, bias: torch.Tensor | None 
         c = native().p8_gemm(a, w.bt, w.scale_b, w.zp_b, w.off_b, bias)
         if isinstance(c, torch.Tensor):
             return c
-        check(c or 0)        # (None: arguments for the general route)
-    a2 = a.reshape(-1, a.shape[-1]).contiguous()
+        check(c or 0)        # (None: arguments for the general route, which handles or rejects them)
+    _require_float(a, "A")
+    if a.dim() < 1 or a.shape[-1] != w.K:
+        raise Mi8Error(1, f"inner dimensions differ: A is {tuple(a.shape)}, B has {w.K} rows")
+    if out is not None:
+        _require_float(out, "output")
+        if out.numel() != a.numel() // w.K * w.N or not out.is_contiguous():
+            raise Mi8Error(1, "output tensor has the wrong size or layout")
+    if scratch is not None:
+        _require_cuda(scratch, "scratch")
+    bias, bias_ptr = _bias_ptr(bias, w.N)
+    a2 = a.reshape(-1, w.K).contiguous()
     M, K = a2.shape
     L = lib()
     need = int(L.mi8p_scratch_bytes(M, K))
@@ -96,6 +124,6 @@ def gemmInt8Packed(a: torch.Tensor, w: Packed8Weight, bias: torch.Tensor | None 
     ws = ws or default_workspace(a.device)
     c = out if out is not None else torch.empty((M, w.N), dtype=torch.float32, device=a.device)
     check(L.mi8p_gemm_int8_packed(a2.data_ptr(), w.bt.data_ptr(), w.scale_b.data_ptr(), w.zp_b.data_ptr(), w.off_b.data_ptr(),
-                                  bias.data_ptr() if bias is not None else None, c.data_ptr(), M, w.N, K, scratch.data_ptr(),
+                                  bias_ptr, c.data_ptr(), M, w.N, K, scratch.data_ptr(),
                                   scratch.numel(), ws.ptr, ws.nbytes, _stream_ptr()))
     return c.reshape(tuple(a.shape[:-1]) + (w.N,))

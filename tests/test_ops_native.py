@@ -33,6 +33,34 @@ def test_tensors_without_device_memory_are_declined():
     assert r.returncode == 0 and r.stdout.strip() == "declined", r.stderr[-2000:]
 
 
+def test_packed8_general_route_rejects_bad_operands():
+    """What the native route declines is checked again before any address is taken: fake CUDA tensors have none."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from marian_dev_b200 import ops, packed8
+    with FakeTensorMode():
+        new = lambda *s, dtype=torch.float32, device="cuda": torch.empty(s, dtype=dtype, device=device)
+        w = packed8.Packed8Weight.__new__(packed8.Packed8Weight)
+        w.K, w.N, w.item = 256, 32, new(256 * 32 + 384, dtype=torch.int8)
+        w.bt, w.scale_b, w.zp_b, w.off_b = new(32, 256, dtype=torch.int8), new(32), new(32, dtype=torch.int32), new(32, dtype=torch.int32)
+        bad = [(new(4, 128), None), (new(4, 512), None), (new(), None), (new(4, 256, dtype=torch.float16), None), (new(4, 256, dtype=torch.float64), None),
+               (new(4, 256, device="cpu"), None), (new(4, 256), new(31)), (new(4, 256), new(33)), (new(4, 256), new(32, dtype=torch.float16)),
+               (new(4, 256), new(32, dtype=torch.int32)), (new(4, 256), new(32, device="cpu"))]
+        outs = [new(4, 31), new(4, 32, dtype=torch.float16), new(32, 4).t(), new(4, 32, device="cpu")]
+    for a, bias in bad:
+        with pytest.raises(ops.Mi8Error):
+            packed8.gemmInt8Packed(a, w, bias)
+    for out in outs:
+        with pytest.raises(ops.Mi8Error):
+            packed8.gemmInt8Packed(bad[6][0], w, None, out=out)
+    for a in (bad[3][0], bad[4][0]):
+        with pytest.raises(ops.Mi8Error):
+            packed8.quantize_rows(a)
+    aq, f, i = w.bt.view(torch.uint8)[:4], w.scale_b, w.zp_b
+    for bias in (b for _, b in bad if b is not None):
+        with pytest.raises(ops.Mi8Error):
+            packed8.multiply(aq, f, i, i, w, bias)
+
+
 def _operands(device, m=6, k=64, n=40):
     from marian_dev_b200 import ops
     g = torch.Generator(device=device).manual_seed(m * k + n)
@@ -71,6 +99,23 @@ def test_declined_operands_take_the_general_route(cuda_device):
         for kw in ({}, {"ws": ops.default_workspace(cuda_device)}):
             with pytest.raises(ops.Mi8Error):
                 ops.affine(*args, **kw)
+    assert ops.poll_status() == 0
+
+
+@pytest.mark.gpu
+def test_packed8_general_route_gives_the_same_bits(cuda_device):
+    from marian_dev_b200 import ops, packed8
+    g = torch.Generator(device=cuda_device).manual_seed(5)
+    x, b = torch.randn(6, 256, generator=g, device=cuda_device), torch.randn(32, generator=g, device=cuda_device)
+    w = packed8.prepareB(torch.randn(256, 32, generator=g, device=cuda_device))
+    want = packed8.gemmInt8Packed(x, w, b)
+    out = torch.empty(6, 32, device=cuda_device)
+    assert torch.equal(packed8.gemmInt8Packed(x, w, b, out=out), want) and torch.equal(out, want)
+    assert torch.equal(packed8.gemmInt8Packed(x.t().contiguous().t(), w, torch.stack([b, b], 1)[:, 0]), want)
+    assert torch.equal(packed8.gemmInt8Packed(x, w, b, ws=ops.default_workspace(cuda_device)), want)
+    assert packed8.gemmInt8Packed(x.reshape(2, 3, 256), w).shape == (2, 3, 32) and packed8.gemmInt8Packed(x[0], w).shape == (32,)
+    assert packed8.gemmInt8Packed(x[:0], w, b).shape == (0, 32)
+    assert torch.equal(packed8.multiply(*packed8.quantize_rows(x), w, torch.stack([b, b], 1)[:, 0]), want)
     assert ops.poll_status() == 0
 
 
