@@ -1,6 +1,6 @@
 """ctypes binding of libmarian_i8.so (the C ABI declared in include/marian_i8.h).
 
-The shared object is built in-tree by ``csrc/Makefile``.  Nothing here falls back to another
+The shared object and the operators' native host path are built in-tree by ``csrc/Makefile``.  Nothing here falls back to another
 implementation: if the library is missing the import raises, and every non-zero status raises
 ``Mi8Error`` the way Marian's host code turns an error into ABORT (src/common/logging.h:100-140).
 """
@@ -12,6 +12,8 @@ import subprocess
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("MARIAN_I8_LIBRARY") or os.path.join(_HERE, "libmarian_i8.so")   # (the variable selects another build of the same ABI)
+
+HOST_DIR = os.path.join(_HERE, "host")
 
 MI8_F32, MI8_F16 = 0, 1
 
@@ -69,13 +71,14 @@ class Mi8Error(RuntimeError):
 
 
 def build_library(verbose: bool = False) -> str:
-    """Compile every CUDA source for sm_100a into libmarian_i8.so (nvcc cross-compiles without a GPU)."""
+    """Compile every CUDA source for sm_100a into libmarian_i8.so (nvcc cross-compiles without a GPU) and, against the installed
+    torch, the operators' native host path _ops_native.so."""
     out = subprocess.run(["make", "-C", os.path.join(_HERE, "csrc"), "-B"], capture_output=True, text=True)
     if verbose or out.returncode != 0:
         print(out.stdout[-4000:])
         print(out.stderr[-8000:])
     if out.returncode != 0:
-        raise RuntimeError("building libmarian_i8.so failed")
+        raise RuntimeError("building libmarian_i8.so and _ops_native.so failed")
     return LIB_PATH
 
 

@@ -17,9 +17,11 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/object_ptr.h>
+#include <torch/version.h>
 
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
 #include <vector>
 
 #include "../../include/marian_i8.h"
@@ -304,12 +306,17 @@ bool resolve(void* handle, const char* name, F& fn) {
   return fn != nullptr;
 }
 
-// init(library path, default_workspace): must be called once before anything else
+// init(library path, default_workspace, torch's version): must be called once before anything else
 PyObject* py_init(PyObject*, PyObject* args) {
-  const char* path = nullptr;
+  const char *path = nullptr, *torch_version = nullptr;
   PyObject* fn = nullptr;
-  if(!PyArg_ParseTuple(args, "sO", &path, &fn))
+  if(!PyArg_ParseTuple(args, "sOs", &path, &fn, &torch_version))
     return nullptr;
+  const size_t n = std::strlen(TORCH_VERSION);   // "2.11.0", where the module says "2.11.0", "2.11.0+cu128" or "2.11.0a0+git..."
+  if(std::strncmp(torch_version, TORCH_VERSION, n) != 0 || (torch_version[n] >= '0' && torch_version[n] <= '9')) {
+    PyErr_Format(PyExc_ImportError, "_ops_native.so was built for torch %s, not %s", TORCH_VERSION, torch_version);
+    return nullptr;
+  }
   void* h = dlopen(path, RTLD_NOW);   // already loaded by the ctypes binding: the same handle
   if(h == nullptr) {
     PyErr_Format(PyExc_ImportError, "%s", dlerror());
@@ -328,7 +335,7 @@ PyObject* py_init(PyObject*, PyObject* args) {
 PyCFunction fast(PyObject* (*f)(PyObject*, PyObject* const*, Py_ssize_t)) { return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)); }
 
 PyMethodDef methods[] = {
-    {"init", py_init, METH_VARARGS, "init(library path, default_workspace)"},
+    {"init", py_init, METH_VARARGS, "init(library path, default_workspace, torch version)"},
     {"affine", fast(py_affine), METH_FASTCALL, "affine(a, weight storage, K, N, bias, scale, relu, half)"},
     {"prepare_b", fast(py_prepare_b), METH_FASTCALL, "prepare_b(w, K, N, w_is_nk)"},
     {"intgemm_views", fast(py_intgemm_views), METH_FASTCALL, "intgemm_views(storage, rows, cols)"},

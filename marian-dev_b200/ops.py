@@ -66,8 +66,11 @@ def native():
     global _native_ext
     if _native_ext is None:
         lib()
-        from . import _ops_native
-        _ops_native.init(binding.LIB_PATH, default_workspace)
+        try:
+            from . import _ops_native
+            _ops_native.init(binding.LIB_PATH, default_workspace, torch.__version__)
+        except ImportError as e:
+            raise ImportError(f"{e}: build _ops_native.so for this Python and torch with `make -C {binding.HOST_DIR} ops`") from e
         _native_ext = _ops_native
     return _native_ext
 

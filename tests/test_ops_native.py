@@ -126,3 +126,24 @@ def test_failed_allocation_raises_torchs_error(cuda_device):
     w = ops.prepareB(torch.zeros(16, n, device=cuda_device))
     with pytest.raises(torch.OutOfMemoryError):          # 4 TB of output
         ops.affine(torch.zeros(1 << 16, 16, device=cuda_device), w, None)
+
+
+def test_documented_build_makes_the_extension():
+    """`make -C marian-dev_b200/csrc` and build_library() are the documented builds of all that the Python operators need."""
+    out = subprocess.run(["make", "-n", "-B", "-C", os.path.join(ROOT, "marian-dev_b200", "csrc")], capture_output=True, text=True, check=True).stdout
+    assert "-o ../libmarian_i8.so" in out and "-o ../_ops_native.so" in out and "-D_GLIBCXX_USE_CXX11_ABI=" in out
+
+
+def test_missing_or_foreign_extension_names_the_build(monkeypatch):
+    from marian_dev_b200 import ops
+    ops.native()
+    monkeypatch.setattr(ops, "_native_ext", None)
+    with monkeypatch.context() as m, pytest.raises(ImportError, match="built for torch .*make -C .*host ops"):
+        m.setattr(torch, "__version__", "1.0.0")
+        ops.native()
+    pkg = sys.modules[ops.__name__.rpartition(".")[0]]
+    with monkeypatch.context() as m, pytest.raises(ImportError, match="make -C .*host ops"):
+        m.setitem(sys.modules, pkg.__name__ + "._ops_native", None)
+        m.delattr(pkg, "_ops_native")
+        ops.native()
+    assert ops.native().affine
