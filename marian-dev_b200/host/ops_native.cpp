@@ -223,7 +223,7 @@ PyObject* py_intgemm_views(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if(PyErr_Occurred())
     return nullptr;
   const size_t first = static_cast<size_t>(s.storage_offset()) * s.element_size();
-  if(s.scalar_type() != at::kByte || !s.is_contiguous() || s.numel() < rows * cols + 4 || (first + static_cast<size_t>(rows) * cols) % 4 != 0)
+  if(s.scalar_type() != at::kByte || s.dim() != 1 || !s.is_contiguous() || s.numel() < rows * cols + 4 || (first + static_cast<size_t>(rows) * cols) % 4 != 0)
     Py_RETURN_NONE;   // (an unusual storage: the caller takes views the general way, which says what is wrong)
   const THPObjectPtr data(THPVariable_Wrap(view_bytes(s, 0, {rows, cols}, at::kChar)));
   const THPObjectPtr mult(THPVariable_Wrap(view_bytes(s, static_cast<size_t>(rows) * cols, {1}, at::kFloat)));

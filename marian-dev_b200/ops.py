@@ -105,7 +105,8 @@ class IntgemmTensor:
         if n % 4 != 0:
             raise Mi8Error(2, "intgemm8 tensors need a multiple of 4 elements so the multiplier is aligned")
         need = ((n + 4 + 255) // 256) * 256
-        if storage is None:
+        given = storage is not None
+        if not given:
             storage = torch.empty(need, dtype=torch.uint8, device=device)
         elif storage.numel() < n + 4:
             raise Mi8Error(4, "storage too small for an intgemm8 tensor")
@@ -113,6 +114,8 @@ class IntgemmTensor:
         self.rows, self.cols = rows, cols
         self._views = None
         self.shape = tuple(logical_shape) if logical_shape is not None else (rows, cols)
+        if given:
+            self._get_views()      # raises for a storage that cannot be viewed this way
 
     # The views are made when first asked for: an affine needs the storage's address only.
     def _get_views(self):
@@ -295,7 +298,7 @@ def _affine_or_dot(a: torch.Tensor, b: IntgemmTensor, bias, transA: bool, transB
                    out_dtype=torch.float32, ws: Workspace | None = None, aq: IntgemmTensor | None = None) -> torch.Tensor:
     if not isinstance(b, IntgemmTensor):
         raise Mi8Error(1, f"Intgemm expects type of B to be a variant of intgemm not {type(b).__name__}")
-    if aq is None and ws is None and not transA and (out_dtype is torch.float32 or out_dtype is torch.float16):
+    if aq is None and ws is None and not transA and b.shape[-1] == b.rows and (out_dtype is torch.float32 or out_dtype is torch.float16):
         out = native().affine(a, b.storage, b.cols, b.rows, bias, scale, relu, out_dtype is torch.float16)
         if isinstance(out, torch.Tensor):
             return out

@@ -147,3 +147,24 @@ def test_missing_or_foreign_extension_names_the_build(monkeypatch):
         m.delattr(pkg, "_ops_native")
         ops.native()
     assert ops.native().affine
+
+
+@pytest.mark.parametrize("storage", [torch.zeros(300, dtype=torch.uint8)[1:], torch.zeros(600, dtype=torch.uint8)[::2], torch.zeros(300), torch.zeros(20, 16, dtype=torch.uint8)],
+                         ids=["off a word boundary", "strided", "float", "matrix"])
+def test_given_storage_that_cannot_be_viewed_is_refused(storage):
+    from marian_dev_b200 import ops
+    with pytest.raises(RuntimeError):
+        ops.IntgemmTensor(16, 16, "cpu", storage=storage)
+    ok = ops.IntgemmTensor(16, 16, "cpu", storage=torch.arange(260, dtype=torch.uint8))
+    assert ok.data.shape == (16, 16) and ok.data.dtype == torch.int8 and int(ok.data[1, 2]) == 18
+    assert ok.quant_mult.shape == (1,) and torch.equal(ok.quant_mult.view(torch.uint8), ok.storage[256:260])
+
+
+@pytest.mark.gpu
+def test_weight_whose_shape_is_not_its_width_is_refused(cuda_device):
+    from marian_dev_b200 import ops
+    x, w, b = _operands(cuda_device)
+    other = ops.IntgemmTensor(w.rows, w.cols, cuda_device, storage=w.storage)      # shape [N,K]: not a weight's
+    for kw in ({}, {"ws": ops.default_workspace(cuda_device)}):
+        with pytest.raises(RuntimeError):
+            ops.affine(x, other, b, **kw)
