@@ -211,7 +211,7 @@ mi8_prepare_cluster_kernel(const float* __restrict__ x, int n16, float* d_quant_
   trace_stamp(th.last, kTrQuantize, 3);
 }
 constexpr int kPrepareCtas = 8;
-constexpr size_t kOneCtaMaxN = 512 * 16, kClusterMinN = 2 * 1024 * 16;
+constexpr size_t kOneCtaMaxN = 512 * 16;
 constexpr size_t kClusterMaxN = static_cast<size_t>(kPrepareCtas) * 1024 * 16 * 2;
 
 // W fp32 [K,N] row-major -> Bt int8 [N,K] row-major.  A block moves a 128(k) x 32(n) tile: a thread reads four values of one column
@@ -337,10 +337,10 @@ int launch_quantize(const float* x, size_t n, const float* d_quant_mult, int8_t*
 }
 
 int launch_prepare(const float* x, size_t n, float* d_quant_mult, int8_t* q, void* ws, size_t ws_bytes, cudaStream_t stream) {
-  // Up to kOneCtaMaxN floats one CTA, from kClusterMinN to kClusterMaxN the cluster (beyond, eight SMs read for longer than the other
-  // launch costs).  The range between keeps the two kernels: the cluster would gain there as well (16384 floats: 7.4 -> 5.4 us),
-  // but a small affine is accounted for as three launches (mi8_kernel_times_begin), 64 x 256 floats among them.
-  if(n == 0 || n % 16 != 0 || n > kClusterMaxN || (n > kOneCtaMaxN && n < kClusterMinN)) {
+  // Up to kOneCtaMaxN floats one CTA, up to kClusterMaxN the cluster (beyond, eight SMs read for longer than the other launch costs).
+  // Launches back to back, in us: one CTA 1.61 at 4096 floats, 2.08 at 8192; cluster 1.82 at 8208, 1.90 at 16384, 2.11 at 32752, 5.39 at
+  // 262144; the two kernels 5.25, 5.23 and 5.60 at 8208, 16384 and 32752 floats, 5.75 at 262160.
+  if(n == 0 || n % 16 != 0 || n > kClusterMaxN) {
     const int rc = launch_max_absolute(x, n, nullptr, d_quant_mult, ws, ws_bytes, stream);
     return rc != MI8_OK ? rc : launch_quantize(x, n, d_quant_mult, q, stream);
   }

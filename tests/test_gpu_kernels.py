@@ -371,13 +371,16 @@ def test_against_committed_golden_vectors(cuda_device):
     _assert_healthy()
 
 
-def test_kernel_times_facility(cuda_device):
-    """mi8_kernel_times_begin / _end attribute device time to the kernels launched in between."""
+@pytest.mark.parametrize("rows,quant", [(8, {"mi8_prepare_cluster_kernel": 3}), (64, {"mi8_prepare_cluster_kernel": 3}),
+                                        (2048, {"mi8_absmax_kernel": 3, "mi8_quantize_kernel": 3})])
+def test_kernel_times_facility(cuda_device, rows, quant):
+    """mi8_kernel_times_begin / _end attribute launches and device time to the kernels launched in between: the GEMM of each affine and
+    what quantises its activation at this size (one CTA, a cluster, two kernels)."""
     import ctypes
     from marian_dev_b200.binding import Mi8KernelTime, check, lib
     ops = _ops()
     L = lib()
-    a = torch.randn(64, 256, device=cuda_device)
+    a = torch.randn(rows, 256, device=cuda_device)
     b = ops.prepareB(torch.randn(256, 128, device=cuda_device) * 0.02)
     check(L.mi8_kernel_times_begin())
     for _ in range(3):
@@ -386,9 +389,10 @@ def test_kernel_times_facility(cuda_device):
     n = ctypes.c_int(0)
     check(L.mi8_kernel_times_end(buf, 16, ctypes.byref(n)))
     got = {r.name.decode(): (r.launches, r.total_us) for r in buf[:n.value]}
-    gemm = [v for k, v in got.items() if "mi8_gemm_kernel" in k]
-    assert gemm and gemm[0][0] == 3 and gemm[0][1] > 0
-    assert sum(v[0] for v in got.values()) == 9          # abs-max, quantise, GEMM per affine
+    for name, launches in {"mi8_gemm_kernel": 3, **quant}.items():
+        of_name = [v for k, v in got.items() if name in k]
+        assert len(of_name) == 1 and of_name[0][0] == launches and of_name[0][1] > 0
+    assert len(got) == 1 + len(quant)
     # off again: nothing is recorded
     ops.affine(a, b, None)
     check(L.mi8_kernel_times_begin())
