@@ -34,10 +34,10 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
-KERNEL_NAMES = ["mi8_gemm_pair_kernel", "mi8_gemm_kernel", "quantize_slot_kernel", "attention1_kernel", "attention_enc_kernel",
-                "add_layernorm_kernel", "quantize_dual_kernel", "lse_topk_kernel",
+KERNEL_NAMES = ["mi8_gemm_pair_kernel", "mi8_gemm_kernel", "quantize_slot_kernel", "attention1_kernel", "attention_cross_kernel", "attention_enc_kernel",
+                "add_layernorm_kernel", "add_layernorm_quant_kernel", "quantize_dual_kernel", "lse_topk_kernel",
                 "lse_merge_kernel", "nbest_merge_kernel", "step_begin_kernel", "embed_ancestors_kernel", "embed_kernel", "gather_rows_kernel",
-                "ssru_cell_kernel", "mi8_absmax_kernel", "mi8_quantize_kernel", "mi8_transpose_quantize_kernel"]
+                "ssru_cell_kernel", "mi8_absmax_kernel", "mi8_quantize_kernel", "mi8_prepare_cluster_kernel", "mi8_transpose_quantize_kernel"]
 METRIC = "int8_decode_tgt_tokens_per_sec"
 UNIT = "tokens/s"
 WORKLOAD = "transformer-big decode (6+6 layers, d=1024, ffn=4096, 16 heads, tied 32000 vocab, all affines int8), beam 4, mini-batch 128, lengths clip(N(30,12),4,128), max length 1.5x source"
@@ -579,9 +579,9 @@ def pick_workers(requested, n_batches):
 
 TRACE_KERNELS = {1: "mi8_gemm_kernel", 2: "mi8_gemm_pair_kernel", 3: "quantize_slot_kernel", 4: "quantize_dual_kernel", 5: "add_layernorm_kernel",
                  6: "attention1_kernel", 7: "attention_enc_kernel", 8: "lse_topk_kernel", 9: "lse_merge_kernel", 10: "nbest_merge_kernel",
-                 11: "embed_kernel", 14: "gather_rows_kernel", 15: "ssru_cell_kernel",
-                 16: "mi8_absmax_kernel", 17: "mi8_quantize_kernel", 18: "mi8_gemm_kernel (output layer, reducing write-back)",
-                 19: "mi8_gemm_kernel (quantising its activation)", 20: "mi8_gemm_cq_kernel"}
+                 11: "embed_kernel, embed_ancestors_kernel", 12: "step_begin_kernel", 13: "add_layernorm_quant_kernel", 14: "gather_rows_kernel", 15: "ssru_cell_kernel",
+                 16: "mi8_absmax_kernel", 17: "mi8_quantize_kernel, mi8_prepare_cluster_kernel", 18: "mi8_gemm_kernel (output layer, reducing write-back)",
+                 19: "mi8_gemm_kernel (quantising its activation)", 20: "mi8_gemm_cq_kernel", 21: "attention_cross_kernel"}
 
 
 def run_trace(args):

@@ -210,8 +210,8 @@ enum mi8d_option {
 };
 int mi8d_set_option(mi8d_decoder* d, int option, int value);   /* d may be NULL for the process-wide switches */
 
-/* keep != 0: every step also writes its logits [beam*batch, vocab] (the output layer then runs unfused);
- * mi8d_last_logits returns them.  Off by default: the fused output layer never materialises them. */
+/* keep != 0: every step writes its logits [beam*batch, vocab], also where MI8D_OPT_FUSED_OUTPUT_MAX_ROWS would have the output layer
+ * reduce them in its write-back; mi8d_last_logits returns them. */
 int mi8d_keep_logits(mi8d_decoder* d, int keep);
 /* Pointer to the last step's logits [beam*batch, vocab] (device); meaningful only with mi8d_keep_logits. */
 const float* mi8d_last_logits(const mi8d_decoder* d);

@@ -58,9 +58,9 @@ void mi8_launch_count_reset(void);
  * running decoder step.  device_buf: caller-owned device memory of 2 + 2 * capacity 64-bit words; on return from
  * mi8_trace_end word 0 holds the number of stamps taken (those beyond `capacity` are dropped), followed by pairs
  * (time in ns, extra << 16 | kernel << 8 | phase) in arrival order.  kernel: 1 GEMM, 2 CTA-pair GEMM, 3 quantize_slot,
- * 4 quantize_dual, 5 add_layernorm (also the quantising one), 6 attention1 (and cross-attention), 7 attention_enc, 8 lse_topk, 9 lse_merge, 10 nbest_merge, 11 embed,
- * (embed_ancestors too), 14 gather_rows, 15 ssru_cell, 16 absmax, 17 quantize, 18 output-layer GEMM,
- * 19 quantising GEMM; the GEMMs put N | K << 20 into `extra`.  Both calls synchronise the device.
+ * 4 quantize_dual, 5 add_layernorm, 6 attention1, 7 attention_enc, 8 lse_topk, 9 lse_merge, 10 nbest_merge, 11 embed (and embed_ancestors),
+ * 12 step_begin, 13 add_layernorm_quant, 14 gather_rows, 15 ssru_cell, 16 absmax, 17 quantize (and prepare_cluster), 18 output-layer GEMM,
+ * 19 quantising GEMM, 20 cluster GEMM, 21 attention_cross; the GEMMs put N | K << 20 into `extra`.  Both calls synchronise the device.
  * The stamps cost about 2 % of a decode even while no buffer is installed, so the product library is built without them
  * (mi8_trace_begin then returns MI8_ERR_UNSUPPORTED); libmarian_i8_trace.so, built from the same sources, carries them. */
 int mi8_trace_begin(unsigned long long* device_buf, int capacity);

@@ -92,12 +92,18 @@ embed_kernel(const float* __restrict__ wemb, const int* __restrict__ words, cons
 __global__ void __launch_bounds__(1024)
 step_begin_kernel(const int* host_ctrl, int* __restrict__ ctrl, int n_ctrl, unsigned* __restrict__ slots, int n_slots) {
   pdl_launch_dependents();
+  const TraceHandles th = trace_open_all();
   pdl_wait();
+  trace_stamp_start(th, kTrStepBegin);
   for(int i = threadIdx.x; i < n_slots; i += blockDim.x)
     slots[i] = 0u;
   const int4* src = reinterpret_cast<const int4*>(host_ctrl);   // (both arrays are 16-byte aligned and padded to whole vectors)
   for(int i = threadIdx.x; i < (n_ctrl + 3) / 4; i += blockDim.x)
     reinterpret_cast<int4*>(ctrl)[i] = __ldcv(src + i);
+#ifndef MI8_NO_TRACE
+  __syncthreads();   // (all stores are issued, so all words have arrived: the stamp counts their way over PCIe)
+#endif
+  trace_stamp(th.first, kTrStepBegin, 2);
 }
 
 // out = LayerNorm(a + resid) * gamma + beta, one block of 256 threads per row; biased variance
@@ -261,7 +267,7 @@ add_layernorm_quant_kernel(const float* __restrict__ a, const SsruArgs cell, con
   if(kCtas > 1)
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (this CTA runs: the others may write to cta_max)
   pdl_wait();
-  trace_stamp_start(th, kTrAddLn);
+  trace_stamp_start(th, kTrAddLnQuant);
   const int rank = kCtas > 1 ? static_cast<int>(blockIdx.x) : 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = static_cast<int>(blockDim.x) >> 5;
   const int groups = warps / group_warps, group = warp / group_warps;
@@ -339,8 +345,8 @@ add_layernorm_quant_kernel(const float* __restrict__ a, const SsruArgs cell, con
   }
   if(live)
     reinterpret_cast<unsigned*>(q)[o] = pack4(x, qm);
-  trace_stamp(tb, kTrAddLn, 2);
-  trace_stamp(th.last, kTrAddLn, 3);
+  trace_stamp(tb, kTrAddLnQuant, 2);
+  trace_stamp(th.last, kTrAddLnQuant, 3);
 }
 
 // Two quantisations in one launch, for the start of a decoder self-attention block: blocks [0, blocks_x)
@@ -708,7 +714,7 @@ attention_cross_kernel(const float* __restrict__ q, const float* __restrict__ k,
       prefetch_l2((i < len ? k : v) + (static_cast<size_t>(b) * len + (i < len ? i : i - len)) * dim + blockIdx.y * 128, bytes);
   }
   pdl_wait();
-  trace_stamp_start(th, kTrAttention1);
+  trace_stamp_start(th, kTrAttentionCross);
 #pragma unroll
   for(int i = 0; i < kCrossStages - 1; ++i)
     fetch(i);
@@ -804,8 +810,8 @@ attention_cross_kernel(const float* __restrict__ q, const float* __restrict__ k,
         atomicMax(absmax_slot, m_abs);
     }
   }
-  trace_stamp(tb, kTrAttention1, 2);
-  trace_stamp(th.last, kTrAttention1, 3);
+  trace_stamp(tb, kTrAttentionCross, 2);
+  trace_stamp(th.last, kTrAttentionCross, 3);
 }
 
 // Encoder self-attention (mode 2) with the keys and values of one (sentence, head) staged in shared memory: block
