@@ -963,7 +963,9 @@ def time_affine(m, k, n, iters=40):
         ops.multiply(aq[j], ws[j], bias, 1.0, True, out=outs[j], ws=wsp)
 
     for i in range(5):
+        launched = ops.launch_count()
         run(i)
+        launched = ops.launch_count() - launched
     torch.cuda.synchronize()
     g = torch.cuda.CUDAGraph()
     s = torch.cuda.Stream()
@@ -981,7 +983,7 @@ def time_affine(m, k, n, iters=40):
     us = e0.elapsed_time(e1) * 1000.0 / iters
     by = 4 * m * k + k * n + 4 * n + 4 * m * n + 8
     return {"M": m, "K": k, "N": n, "us_per_affine": round(us, 2), "GBps": round(by / us / 1e3, 1), "TOPS": round(2.0 * m * n * k / us / 1e6, 2),
-            "algorithmic_bytes": by, "launches_per_affine": 3, "operand_sets": copies}
+            "algorithmic_bytes": by, "launches_per_affine": launched, "operand_sets": copies}
 
 
 def time_affine_sharded(m, k, n, rank, world, iters=40):

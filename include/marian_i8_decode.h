@@ -167,8 +167,9 @@ int mi8g_lse_topk_nbest(const float* logits, int beam, int batch, int vocab, int
 int mi8d_history_reuse(mi8d_decoder* d, unsigned out[2], int reset);
 
 /* Tuning switches of the step driver; every setting computes the same values, bit for bit.
- *   MI8D_OPT_FUSE_WEIGHTS (default 1): matrices that multiply the same activation (Wk|Wv of an attention block,
- *     Wq|Wk|Wv of an encoder layer, the SSRU's W|Wf) run as ONE GEMM launch over copies stored one behind the other;
+ *   MI8D_OPT_FUSE_WEIGHTS (default 1): matrices that multiply the same activation (Wk|Wv of a context attention, Wq|Wk|Wv of
+ *     an encoder layer, the SSRU's W|Wf) run as ONE GEMM launch over copies stored one behind the other, and so do Wq|Wk|Wv of the
+ *     decoder's self-attention, whose query takes its own quantisation of the layer input;
  *   MI8D_OPT_QUANT_IN_GEMM (default 0): affines with K <= 1024 whose tiles fit one wave of CTAs quantise their
  *     activation while loading it (mi8_multiply_f32_slot) instead of through a quantisation launch;
  *   MI8D_OPT_FUSED_OUTPUT_MAX_ROWS (default 0): up to this many rows the output layer reduces its logits inside
@@ -176,10 +177,11 @@ int mi8d_history_reuse(mi8d_decoder* d, unsigned out[2], int reset);
  *   MI8D_OPT_SIDE_STREAM (default 1): the re-projection of the earlier history slabs runs on an internal stream;
  *   MI8D_OPT_ATTENTION_UNROLL (8 or 16, default 8; process-wide): key/value rows a thread keeps in flight;
  *   MI8D_OPT_ATTENTION_BLOCK_HEADS (default 8, 0 = all; process-wide): heads one block of the decoder attention serves;
- *     a divisor of the head count splits every query row over several smaller blocks;
+ *     a divisor of the head count splits every query row over several smaller blocks.  (Both: self-attention, and the
+ *     cross-attention of sentences too long for the kernel that serves a sentence's hypotheses together;)
  *   MI8D_OPT_CLUSTER_AFFINE (default 0): affines whose activation comes with an abs-max slot run as ONE launch of the
  *     cluster GEMM (mi8g_affine_slot) instead of a quantisation launch and a GEMM launch.  Off by default: 74 to 98
- *     instead of 122 launches per step of the transformer-big decoder, but 5 to 20 % fewer tokens per second (the
+ *     launches per step of the transformer-big decoder, which then had 122 (113 now), but 5 to 20 % fewer tokens per second (the
  *     stores into the other CTAs' shared memory and the placement of whole clusters cost more than the launches saved);
  *   MI8D_OPT_FUSED_LAYERNORM (default 1; has an effect only with the above): the last affine of a sub-layer also applies the residual add and
  *     the LayerNorm that follow it (mi8g_affine_slot_add_layernorm) when the model width is at most 1024;
