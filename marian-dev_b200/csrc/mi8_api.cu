@@ -311,7 +311,8 @@ int mi8_trace_begin(unsigned long long* device_buf, int capacity) {
     set_last_cuda_error(e);
     return MI8_ERR_LAUNCH;
   }
-  if(trace_set_glue(device_buf) != 0 || trace_set_gemm(device_buf) != 0 || trace_set_quant(device_buf) != 0) {
+  if(trace_set_glue(device_buf) != 0 || trace_set_gemm(device_buf) != 0 || trace_set_quant(device_buf) != 0 ||
+     trace_set_rows(device_buf) != 0) {
     set_last_cuda_error(cudaGetLastError());
     return MI8_ERR_LAUNCH;
   }
@@ -320,7 +321,7 @@ int mi8_trace_begin(unsigned long long* device_buf, int capacity) {
 
 int mi8_trace_end(void) {
   cudaError_t e = cudaDeviceSynchronize();
-  const int rc = trace_set_glue(nullptr) | trace_set_gemm(nullptr) | trace_set_quant(nullptr);
+  const int rc = trace_set_glue(nullptr) | trace_set_gemm(nullptr) | trace_set_quant(nullptr) | trace_set_rows(nullptr);
   if(e != cudaSuccess || rc != 0) {
     set_last_cuda_error(e != cudaSuccess ? e : cudaGetLastError());
     return MI8_ERR_LAUNCH;

@@ -123,6 +123,9 @@ struct mi8d_decoder {
   const float* out_bias = nullptr;
   Aff out_w;
   std::vector<int8_t*> fused_enc, fused_self, fused_ctx;   // arena storage of the fused matrices
+  DecoderRowsParams rows;             // for launch_decoder_rows: what does not change from step to step is filled in by resolve()
+  float* rows_pack = nullptr;
+  bool rows_ready = false;
 
   std::vector<LayerBufs> layers;
   float* x_in = nullptr;                 // layer-0 input when there are no slabs (SSRU) and the final layer output
@@ -253,6 +256,8 @@ struct mi8d_decoder {
       for(auto& p : fused_ctx)
         p = arena.take<int8_t>(2 * d * d);
     }
+    const size_t n_pack = c.ssru && can_fuse ? decoder_rows_pack_floats(c.dim_emb, c.dim_ffn, c.heads, c.dec_depth) : 0;
+    rows_pack = n_pack != 0 ? arena.take<float>(n_pack) : nullptr;
   }
 
   unsigned* layer_slot(int l, int which) const { return slots + 1 + kSlotsPerLayer * l + which; }
@@ -329,6 +334,32 @@ struct mi8d_decoder {
     return true;
   }
 
+  // What launch_decoder_rows needs of the layers, where all of them have it (an SSRU decoder whose W and Wf lie one behind the other).
+  bool resolve_rows(cudaStream_t s) {
+    const mi8d_config& c = cfg;
+    rows_ready = false;
+    if(rows_pack == nullptr || p8)
+      return true;
+    DecoderRowsVectors v[kDecoderRowsLayers];
+    const int dm = c.dim_emb, f = c.dim_ffn;
+    for(int l = 0; l < c.dec_depth; ++l) {
+      const DecLayerW& w = dec_w[l];
+      auto shape = [](const Aff& a, int K, int N) { return a.K == K && a.N == N && a.bias != nullptr; };
+      if(!w.rnn.ready || w.rnn.n != dm || w.rnn.K != dm || w.rnn.bias[0] != nullptr || w.rnn.bias[1] == nullptr || !shape(w.ctx_q, dm, dm) ||
+         !shape(w.ctx_o, dm, dm) || !shape(w.w1, dm, f) || !shape(w.w2, f, dm))
+        return true;
+      CUtensorMap* m = rows.map[l];
+      if(rows_weight_map(m, w.rnn.bt, 2 * dm, dm) != MI8_OK || rows_weight_map(m + 1, w.ctx_q.bt, dm, dm) != MI8_OK ||
+         rows_weight_map(m + 2, w.ctx_o.bt, dm, dm) != MI8_OK || rows_weight_map(m + 3, w.w1.bt, f, dm) != MI8_OK ||
+         rows_weight_map(m + 4, w.w2.bt, dm, f) != MI8_OK)
+        return true;
+      v[l] = DecoderRowsVectors{{w.rnn.qm[0], w.rnn.qm[1], w.ctx_q.qm, w.ctx_o.qm, w.w1.qm, w.w2.qm}, w.rnn.bias[1], w.ctx_q.bias, w.ctx_o.bias,
+                                w.w1.bias, w.w2.bias, {w.ln_self.g, w.ln_self.b, w.ln_ctx.g, w.ln_ctx.b, w.ln_ffn.g, w.ln_ffn.b}};
+    }
+    rows_ready = launch_decoder_rows_pack(v, dm, f, c.heads, c.dec_depth, rows_pack, s) == MI8_OK;
+    return rows_ready;
+  }
+
   // Looks every parameter up once and builds the fused matrices.  MI8_ERR_BAD_ARG names a missing parameter.
   int resolve(cudaStream_t s) {
     const mi8d_config& c = cfg;
@@ -366,6 +397,8 @@ struct mi8d_decoder {
       if(ok)
         copies = copies && fuse(w.ctx_kv, fused_ctx[l], {&w.ctx_k, &w.ctx_v}, s);
     }
+    if(ok)
+      copies = copies && resolve_rows(s);
     wemb = P("Wemb");
     ok = ok && wemb != nullptr && aff(out_w, p8 ? "Wemb_packed8" : "Wemb_intgemm8", "decoder_ff_logit_out_b");
     out_bias = out_w.bias;
@@ -512,6 +545,12 @@ int add_ln(mi8d_decoder* d, const float* a, const float* resid, const Norm& n, i
 // Whether a LayerNorm of `rows` rows whose result only feeds affines of its own multiplier also quantises it (into d->aq / enc_aq).
 bool ln_quantises(const mi8d_decoder* d, int rows) {
   return !d->p8 && !d->opt_cluster && !d->opt_quant_in_gemm && add_layernorm_quant_supported(rows, d->cfg.dim_emb);
+}
+// Whether launch_decoder_rows runs the layers of a step of `rows` rows.
+bool decoder_rows_apply(const mi8d_decoder* d, int rows) {
+  const mi8d_config& c = d->cfg;
+  return d->rows_ready && d->opt_fuse && !d->opt_cluster && !d->opt_quant_in_gemm &&
+         decoder_rows_supported(rows, c.dim_emb, c.dim_ffn, c.heads, c.dec_depth, d->src);
 }
 int add_ln_quant(mi8d_decoder* d, const float* a, const float* resid, const Norm& n, int rows, float* out, int8_t* q, cudaStream_t s) {
   return launch_add_layernorm_quant(a, resid, n.g, n.b, 1e-6f, rows, d->cfg.dim_emb, out, q,
@@ -1016,7 +1055,12 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
   const size_t slab_stride = static_cast<size_t>(SR) * dm;
   const size_t n_d = static_cast<size_t>(R) * dm;
 
-  MI8D_TRY(launch_step_begin(d->step_ctrl, d->s_ctrl, d->n_step_ctrl, d->slots, d->n_slots, s));
+  // Few rows of an SSRU decoder: all layers in one launch, which also brings the control words to the device unless the batch
+  // changed (the gather below reads them).
+  const bool rows_path = decoder_rows_apply(d, R);
+  const bool begin_apart = !rows_path || batch != d->batch;
+  if(begin_apart)
+    MI8D_TRY(launch_step_begin(d->step_ctrl, d->s_ctrl, d->n_step_ctrl, d->slots, d->n_slots, s));
 
   // sentences that finished leave the batch: compact the encoder context, recompute cross K/V
   if(batch != d->batch) {
@@ -1061,7 +1105,38 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
   const int* words = t == 0 ? nullptr : prev_words;
   const float* pos = d->positions + static_cast<size_t>(t) * dm;
   const float emb_scale = sqrtf(static_cast<float>(dm));
-  if(c.ssru) {
+  const int cell_new = d->cell_cur ^ 1;
+  float* aq_tail = reinterpret_cast<float*>(d->aq + n_d);
+  if(rows_path) {
+    DecoderRowsParams& p = d->rows;
+    p.rows = R;
+    p.ffn = c.dim_ffn;
+    p.layers = c.dec_depth;
+    p.src = S;
+    p.batch = batch;
+    p.emb_scale = emb_scale;
+    p.att_scale = 1.0f / sqrtf(static_cast<float>(dm / c.heads));
+    p.wemb = d->wemb;
+    p.pos = pos;
+    p.log_mask = lmask;
+    p.words = words;
+    p.hyp = t == 0 ? nullptr : hyp_idx;
+    p.ctrl = d->s_ctrl;
+    p.n_ctrl = begin_apart ? 0 : d->n_step_ctrl;
+    std::copy(d->step_ctrl, d->step_ctrl + p.n_ctrl, p.ctrl_words);   // (3 R + batch words, batch <= R <= kDecoderRowsMax)
+    p.slots = d->slots;
+    p.n_slots = begin_apart ? 0 : d->n_slots;
+    p.out_q = d->aq;
+    p.out_qm = aq_tail;
+    const LayerBufs &first = d->layers[0], &next = d->layers[c.dec_depth > 1 ? 1 : 0];   // (every layer's buffers are laid out alike)
+    p.pack = d->rows_pack;
+    p.cross_k = first.cross_k;
+    p.cross_v = first.cross_v;
+    p.cell_old = first.cell[d->cell_cur];
+    p.cell_new = first.cell[cell_new];
+    p.layer_stride = static_cast<size_t>(next.cross_k - first.cross_k);
+    MI8D_TRY(launch_decoder_rows(p, dm, c.heads, s));
+  } else if(c.ssru) {
     MI8D_TRY(launch_embed(d->wemb, words, pos, 0, emb_scale, R, dm, x, nullptr, d->input_slot(0), s));
   } else {
     const float* rowmax[16];
@@ -1075,10 +1150,8 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
                                     d->p8 ? 0 : c.dec_depth, rowmax, hslot));
   }
 
-  const int cell_new = d->cell_cur ^ 1;
-  float* aq_tail = reinterpret_cast<float*>(d->aq + n_d);
-  const bool lq = ln_quantises(d, R);
-  for(int l = 0; l < c.dec_depth; ++l) {
+  const bool lq = rows_path || ln_quantises(d, R);
+  for(int l = 0; l < c.dec_depth && !rows_path; ++l) {
     LayerBufs& L = d->layers[l];
     const DecLayerW& w = d->dec_w[l];
     unsigned* x_slot = d->input_slot(l);

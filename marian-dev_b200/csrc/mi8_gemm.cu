@@ -1823,6 +1823,8 @@ int launch_pair(const CUtensorMap& tw, const CUtensorMap& ta, const GemmParams& 
 
 MI8_DEFINE_TRACE_SETTER(trace_set_gemm)
 
+int rows_weight_map(CUtensorMap* map, const int8_t* bt, int N, int K) { return encode_kmajor_map(map, bt, N, K, 16); }
+
 void test_wait_fault(int withhold_item, unsigned spin_limit) {
   g_test_withhold_item = withhold_item;
   g_test_spin_limit = spin_limit;

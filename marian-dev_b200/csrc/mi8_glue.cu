@@ -245,14 +245,6 @@ struct SsruArgs {
   const float* f = nullptr;
   float* cell_new = nullptr;
 };
-__device__ __forceinline__ float ssru_cell(float c, float x, float f, float* h) {
-  // sigmoid and highway with every rounding explicit: sig = 1 / (1 + det_expf(-f)); c' = fma(x, 1 - sig, c * sig); h = relu(c')
-  const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, det_expf(-f)));
-  const float cn = __fmaf_rn(x, __fadd_rn(1.0f, -sig), __fmul_rn(c, sig));
-  *h = cn > 0.f ? cn : 0.f;
-  return cn;
-}
-
 template <int kCtas>
 __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(1024)
 add_layernorm_quant_kernel(const float* __restrict__ a, const SsruArgs cell, const float* __restrict__ resid, const float* __restrict__ gamma,

@@ -56,6 +56,15 @@ __device__ __forceinline__ float det_logf(float x) {
   return __fmaf_rn(static_cast<float>(e), 0.693147182f, lm);
 }
 
+// SSRU cell: returns the new state, *h its output.
+__device__ __forceinline__ float ssru_cell(float c, float x, float f, float* h) {
+  // sigmoid and highway with every rounding explicit: sig = 1 / (1 + det_expf(-f)); c' = fma(x, 1 - sig, c * sig); h = relu(c')
+  const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, det_expf(-f)));
+  const float cn = __fmaf_rn(x, __fadd_rn(1.0f, -sig), __fmul_rn(c, sig));
+  *h = cn > 0.f ? cn : 0.f;
+  return cn;
+}
+
 // Butterfly all-reduce over the 32 lanes of a warp: v <- v + v[lane ^ o] for o = 16, 8, 4, 2, 1.
 // Floating-point addition is commutative, so every lane ends with the same bits.
 __device__ __forceinline__ float warp_sum_det(float v) {
