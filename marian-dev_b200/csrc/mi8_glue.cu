@@ -245,6 +245,7 @@ struct SsruArgs {
   const float* f = nullptr;
   float* cell_new = nullptr;
 };
+
 template <int kCtas>
 __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(1024)
 add_layernorm_quant_kernel(const float* __restrict__ a, const SsruArgs cell, const float* __restrict__ resid, const float* __restrict__ gamma,
@@ -971,13 +972,17 @@ __device__ __forceinline__ void finish_step(const StepEnd& e, int r, int k, int 
     return;
   const int b = r % e.batch;
   __syncthreads();   // the row's candidates are written
-  if(threadIdx.x == 0) {
-    __threadfence();
-    *s_last = atomicAdd(e.arrivals + b, 1u) == static_cast<unsigned>(e.beam - 1) ? 1 : 0;
-    __threadfence();
+  if(e.beam > 1) {   // (a sentence's only row is its last)
+    if(threadIdx.x == 0) {
+      __threadfence();
+      *s_last = atomicAdd(e.arrivals + b, 1u) == static_cast<unsigned>(e.beam - 1) ? 1 : 0;
+      __threadfence();
+    }
+    __syncthreads();
+    if(!*s_last)
+      return;
   }
-  __syncthreads();
-  if(!*s_last || threadIdx.x >= 32)
+  if(threadIdx.x >= 32)
     return;
   const int n = e.beam * k;
   int valid = 0;
@@ -1066,10 +1071,11 @@ __device__ __forceinline__ float lse_from_blocks(const float* bm, float* bs, int
 // kThreads: 1024 (one pass over 32000 logits, one block per SM) while every row has an SM to itself, 512 (two blocks per SM) up to two
 // rows per SM, 256 (four) beyond, registers held to 64 so that they fit: 148 rows 14.9 us with the picks after the sum, 13.4 now; 256
 // rows 29.1 us with 256 threads, 18.0 now; 512 rows 33.8 us, 26.9 now.
-template <int kThreads>
+// kFromBlocks: the blocks' maxima and sums were left by the output layer's write-back (few rows); no scan.
+template <int kThreads, bool kFromBlocks = false>
 __global__ void __launch_bounds__(kThreads, 1024 / kThreads)
 lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float* __restrict__ prev_scores, float* cand_score, int* cand_word,
-                const StepEnd end) {
+                const StepEnd end, const float* __restrict__ block_max, const float* __restrict__ block_sum) {
   pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
@@ -1093,7 +1099,13 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
   const bool vec = (vocab & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15u) == 0;
   if(threadIdx.x == 0)
     n_cand = 0;
-  for(int b0 = warp * 8; b0 < nb; b0 += kThreads / 4) {
+  if(kFromBlocks) {
+    for(int b = threadIdx.x; b < nb; b += kThreads) {
+      bm[b] = __ldg(block_max + static_cast<size_t>(r) * nb + b);
+      bs[b] = __ldg(block_sum + static_cast<size_t>(r) * nb + b);
+    }
+  }
+  for(int b0 = warp * 8; !kFromBlocks && b0 < nb; b0 += kThreads / 4) {
     const int b = b0 + (lane >> 2);
     const int lo = b * 128 + (lane & 3) * 32;
     const int cnt = b < nb ? max(0, min(32, vocab - lo)) : 0;   // this lane's entries that exist
@@ -1597,7 +1609,7 @@ int launch_attention1(const float* q, const float* k, const float* v, const floa
 }
 
 int launch_lse_topk(const float* logits, int rows, int vocab, int k, const float* prev_scores, float* cand_score, int* cand_word,
-                    cudaStream_t s, const StepEnd& end) {
+                    cudaStream_t s, const StepEnd& end, const float* block_max, const float* block_sum) {
   if(rows <= 0 || vocab <= 0 || k < 1 || k > kMaxK)
     return MI8_ERR_BAD_ARG;
   if(end.arrivals != nullptr && !step_end_fits(end.beam, k))
@@ -1605,12 +1617,14 @@ int launch_lse_topk(const float* logits, int rows, int vocab, int k, const float
   const size_t smem = 2 * static_cast<size_t>((vocab + 127) / 128) * sizeof(float);
   if(smem > 32 * 1024)
     return MI8_ERR_UNSUPPORTED;
-  if(rows <= sm_count())
-    launch_kernel(lse_topk_kernel<1024>, dim3(rows), dim3(1024), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word, end);
+  if(block_max != nullptr)
+    launch_kernel(lse_topk_kernel<256, true>, dim3(rows), dim3(256), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word, end, block_max, block_sum);
+  else if(rows <= sm_count())
+    launch_kernel(lse_topk_kernel<1024>, dim3(rows), dim3(1024), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word, end, block_max, block_sum);
   else if(rows <= 2 * sm_count())
-    launch_kernel(lse_topk_kernel<512>, dim3(rows), dim3(512), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word, end);
+    launch_kernel(lse_topk_kernel<512>, dim3(rows), dim3(512), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word, end, block_max, block_sum);
   else
-    launch_kernel(lse_topk_kernel<256>, dim3(rows), dim3(256), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word, end);
+    launch_kernel(lse_topk_kernel<256>, dim3(rows), dim3(256), smem, s, logits, vocab, k, prev_scores, cand_score, cand_word, end, block_max, block_sum);
   count_launch();
   return check_launch();
 }

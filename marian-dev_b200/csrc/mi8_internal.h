@@ -76,6 +76,7 @@ int launch_gemm(const int8_t* aq, const int8_t* bt, int M, int N, int K, const f
 
 // The general form: one activation against up to three weight matrices of the same shape stored one behind the
 // other (N = nseg * rows of one of them), each with its own multiplier, bias and output matrix [M, N / nseg].
+constexpr int kBlockRows = 32;
 struct GemmCall {
   const int8_t* aq = nullptr;
   const int8_t* bt = nullptr;
@@ -97,6 +98,9 @@ struct GemmCall {
   const unsigned* skip_a = nullptr;
   const unsigned* skip_b = nullptr;
   int skip_rows_below = 0;
+  // optional, up to kBlockRows rows of one fp32 result: per (row, block of 128 columns) the maximum and the sum of exponentials [M][ceil(N / 128)]
+  float* block_max = nullptr;
+  float* block_sum = nullptr;
   int a_rows_cap = 0;   // rows the activation buffer holds (extent of its tensor map); 0 = M
   int a_row0 = 0;       // the M rows start at this row of the buffer `aq` points to (needs a_rows_cap >= a_row0 + M)
   // per segment, where it differs: the first of its M activation rows (-1: a_row0) and their multiplier (null: d_qa)
@@ -218,8 +222,9 @@ int trace_set_quant(unsigned long long* buf);
 int launch_attention1(const float* q, const float* k, const float* v, const float* log_mask, int rows, int heads, int dim_head,
                       int len, int batch, int mode, float* out, unsigned* slot, cudaStream_t s, const int* anc = nullptr,
                       int anc_stride = 0, int kv_rows = 0);
+// block_max / block_sum (optional, both): what GemmCall's write-back left of the rows' blocks, in the place of a scan of the logits
 int launch_lse_topk(const float* logits, int rows, int vocab, int k, const float* prev_scores, float* cand_score, int* cand_word,
-                    cudaStream_t s, const StepEnd& end = StepEnd());
+                    cudaStream_t s, const StepEnd& end = StepEnd(), const float* block_max = nullptr, const float* block_sum = nullptr);
 int launch_nbest_merge(const float* cand_score, const int* cand_word, int beam, int batch, int vocab, int k, float* out_score,
                        int* out_beam, int* out_word, cudaStream_t s);
 int launch_gather_rows(const float* in, const int* idx, int rows, int dim, float* out, cudaStream_t s);
