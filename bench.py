@@ -582,7 +582,7 @@ TRACE_KERNELS = {1: "mi8_gemm_kernel", 2: "mi8_gemm_pair_kernel", 3: "quantize_s
                  11: "embed_kernel, embed_ancestors_kernel", 12: "step_begin_kernel", 13: "add_layernorm_quant_kernel", 14: "gather_rows_kernel", 15: "ssru_cell_kernel",
                  16: "mi8_absmax_kernel", 17: "mi8_quantize_kernel, mi8_prepare_cluster_kernel", 18: "mi8_gemm_kernel (output layer, reducing write-back)",
                  19: "mi8_gemm_kernel (quantising its activation)", 20: "mi8_gemm_cq_kernel", 21: "attention_cross_kernel",
-                 22: "decoder_rows_kernel"}
+                 22: "decoder_rows_kernel", 23: "attention_hist_kernel"}
 
 
 def run_trace(args):

@@ -60,7 +60,7 @@ void mi8_launch_count_reset(void);
  * (time in ns, extra << 16 | kernel << 8 | phase) in arrival order.  kernel: 1 GEMM, 2 CTA-pair GEMM, 3 quantize_slot,
  * 4 quantize_dual, 5 add_layernorm, 6 attention1, 7 attention_enc, 8 lse_topk, 9 lse_merge, 10 nbest_merge, 11 embed (and embed_ancestors),
  * 12 step_begin, 13 add_layernorm_quant, 14 gather_rows, 15 ssru_cell, 16 absmax, 17 quantize (and prepare_cluster), 18 output-layer GEMM,
- * 19 quantising GEMM, 20 cluster GEMM, 21 attention_cross, 22 decoder_rows; the GEMMs put N | K << 20 into `extra`.  Both calls synchronise the device.
+ * 19 quantising GEMM, 20 cluster GEMM, 21 attention_cross, 22 decoder_rows, 23 attention_hist; the GEMMs put N | K << 20 into `extra`.  Both calls synchronise the device.
  * The stamps cost about 2 % of a decode even while no buffer is installed, so the product library is built without them
  * (mi8_trace_begin then returns MI8_ERR_UNSUPPORTED); libmarian_i8_trace.so, built from the same sources, carries them. */
 int mi8_trace_begin(unsigned long long* device_buf, int capacity);

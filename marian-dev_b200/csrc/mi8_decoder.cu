@@ -133,6 +133,7 @@ struct mi8d_decoder {
   float *x1 = nullptr, *x2 = nullptr;    // after self / cross blocks
   float *qbuf = nullptr, *abuf = nullptr, *obuf = nullptr, *hbuf = nullptr, *fbuf = nullptr;
   int8_t *aq = nullptr, *cq = nullptr;
+  HistLists lists;                 // of the running step; `batch` is set where they are used
   unsigned* prev_bits = nullptr;   // per layer: history abs-max (bit pattern) the stored keys/values were computed with
   unsigned* reuse_stats = nullptr; // [0] (layer, step) pairs that reused stored keys/values, [1] all pairs
   int slab_rows = 0;               // rows reserved per history slab for the current mini-batch
@@ -210,6 +211,9 @@ struct mi8d_decoder {
     if(!c.ssru) {
       anc[0] = arena.take<int>(T * R);
       anc[1] = arena.take<int>(T * R);
+      lists.list = arena.take<int>(T * R);
+      lists.which = arena.take<int>(T * R);
+      lists.count = arena.take<int>(B);
       prev_bits = arena.take<unsigned>(c.dec_depth);
       reuse_stats = arena.take<unsigned>(2);
     }
@@ -1101,6 +1105,14 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
   // launch, the ancestor table of this step and every layer's history abs-max over the earlier slabs; the producer of a
   // layer's newest slab (this embedding / the previous layer's last LayerNorm) adds that slab's maximum.
   const int anc_new = d->anc_cur ^ 1;
+  HistLists lists = d->lists;
+  lists.batch = 0;
+  // single-query attention over the stored keys/values of steps 0 .. t
+  auto self_attention = [&](const LayerBufs& L, unsigned* sa) {
+    if(lists.batch > 0)
+      return launch_attention_hist(d->qbuf, L.kslab, L.vslab, R, c.heads, dm / c.heads, t + 1, d->abuf, sa, s, lists);
+    return launch_attention1(d->qbuf, L.kslab, L.vslab, nullptr, R, c.heads, dm / c.heads, t + 1, batch, 0, d->abuf, sa, s, d->anc[anc_new], SR, SR);
+  };
   float* x = c.ssru ? d->x_in : d->layers[0].slab + static_cast<size_t>(t) * slab_stride;
   const int* words = t == 0 ? nullptr : prev_words;
   const float* pos = d->positions + static_cast<size_t>(t) * dm;
@@ -1145,9 +1157,10 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
       rowmax[l] = d->layers[l].rowmax;
       hslot[l] = d->layer_slot(l, kSlotHistory);
     }
+    lists.batch = attention_hist_supported(beam, dm / c.heads, t + 1) ? batch : 0;
     MI8D_TRY(launch_embed_ancestors(d->wemb, words, pos, emb_scale, dm, x, d->layers[0].rowmax + static_cast<size_t>(t) * SR, d->input_slot(0),
                                     d->layer_slot(0, kSlotHistory), d->anc[d->anc_cur], d->anc[anc_new], hyp_idx, t, R, SR, s,
-                                    d->p8 ? 0 : c.dec_depth, rowmax, hslot));
+                                    d->p8 ? 0 : c.dec_depth, rowmax, hslot, lists));
   }
 
   const bool lq = rows_path || ln_quantises(d, R);
@@ -1182,8 +1195,7 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
       MI8D_TRY(gemm_act(d, d->aq, R, w.self_q, false, d->qbuf, s));
       MI8D_TRY(gemm_act(d, d->aq, R, w.self_k, false, L.kslab + static_cast<size_t>(t) * slab_stride, s));
       MI8D_TRY(gemm_act(d, d->aq, R, w.self_v, false, L.vslab + static_cast<size_t>(t) * slab_stride, s));
-      MI8D_TRY(launch_attention1(d->qbuf, L.kslab, L.vslab, nullptr, R, c.heads, dm / c.heads, t + 1, batch, 0, d->abuf, sa, s, d->anc[anc_new],
-                                 SR, SR));
+      MI8D_TRY(self_attention(L, sa));
       MI8D_TRY(quant_gemm_ln(d, d->abuf, R, sa, w.self_o, x, w.ln_self, d->obuf, d->x1, nullptr, s1, s, nullptr, lq));
     } else {
       unsigned* sh = d->layer_slot(l, kSlotHistory);
@@ -1256,8 +1268,7 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
       }
       if(side)
         MI8D_CUDA(cudaStreamWaitEvent(s, d->ev_join, 0));
-      MI8D_TRY(launch_attention1(d->qbuf, L.kslab, L.vslab, nullptr, R, c.heads, dm / c.heads, steps, batch, 0, d->abuf, sa, s,
-                                 d->anc[anc_new], SR, SR));
+      MI8D_TRY(self_attention(L, sa));
       MI8D_TRY(quant_gemm_ln(d, d->abuf, R, sa, w.self_o, x, w.ln_self, d->obuf, d->x1, nullptr, s1, s, nullptr, lq));
     }
     {

@@ -204,11 +204,20 @@ int launch_add_layernorm_quant(const float* a, const float* resid, const float* 
                                int8_t* q, float* d_qm, cudaStream_t s, const float* cell_old = nullptr, const int* hyp = nullptr,
                                const float* xw = nullptr, const float* f = nullptr, float* cell_new = nullptr);
 int launch_quantize_slot(const float* x, size_t n, const unsigned* slot, int8_t* q, float* d_qm, cudaStream_t s);
-// the embedding of a step (slot2: the history's abs-max of layer 0) and the ancestor table; hist_layers > 0: also reduces, per layer, the
+// Per sentence the distinct slab rows its hypotheses descend from (mi8_glue.cu, history_list); batch == 0: none.
+struct HistLists {
+  int batch = 0;
+  int *list = nullptr, *which = nullptr, *count = nullptr;
+};
+// the embedding of a step (slot2: the history's abs-max of layer 0) and the ancestor table (and, optionally, the history lists); hist_layers > 0: also reduces, per layer, the
 // maximum of rowmax over the earlier slabs' ancestor rows into hist_slot[l]
 int launch_embed_ancestors(const float* wemb, const int* words, const float* pos, float scale, int dim, float* out, float* rowmax, unsigned* slot,
                            unsigned* slot2, const int* anc_old, int* anc_new, const int* hyp, int t, int rows, int stride, cudaStream_t s,
-                           int hist_layers, const float* const* hist_rowmax, unsigned* const* hist_slot);
+                           int hist_layers, const float* const* hist_rowmax, unsigned* const* hist_slot, const HistLists& lists = HistLists());
+// decoder self-attention (mode 0 with an ancestor table) for all hypotheses of a sentence together, from the lists of this step
+bool attention_hist_supported(int beams, int dim_head, int len);
+int launch_attention_hist(const float* q, const float* k, const float* v, int rows, int heads, int dim_head, int len, float* out, unsigned* slot,
+                          cudaStream_t s, const HistLists& lists);
 // layer input x and the self-attention history quantised by one launch (see quantize_dual_kernel)
 int launch_quantize_dual(const float* x, size_t n, const unsigned* slot_x, int8_t* q, float* qm_x, const float* slabs, int slab_rows,
                          int steps, int rows_new, int dim, const unsigned* slot_h, const unsigned* prev_bits, int8_t* hq, float* qm_h,

@@ -42,7 +42,7 @@ static __device__ unsigned long long* s_trace_buf = nullptr;
 enum TraceKernel : int {
   kTrGemm = 1, kTrGemmPair, kTrQuantSlot, kTrQuantDual, kTrAddLn, kTrAttention1, kTrAttentionEnc, kTrLseTopk, kTrLseMerge,
   kTrNbest, kTrEmbed, kTrStepBegin, kTrAddLnQuant, kTrGather, kTrSsru, kTrAbsmax, kTrQuantize, kTrGemmLogits, kTrGemmQuantA, kTrGemmCq,
-  kTrAttentionCross, kTrDecoderRows
+  kTrAttentionCross, kTrDecoderRows, kTrAttentionHist
 };
 // Every kernel reads the pointer ONCE, at its entry (before its wait for the preceding kernel, so the load overlaps that
 // kernel's tail), in the two threads that stamp: the last thread of block 0 and the last thread of the last block.  All other
