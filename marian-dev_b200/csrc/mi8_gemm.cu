@@ -263,28 +263,27 @@ __device__ __forceinline__ float p8_value(int acc, int zp_a, int sum_a, float sc
 // (m_first is a multiple of 16 and the arrays are 16-byte aligned; a warp reads the same address, so each
 // load is one broadcast transaction); the ragged last chunk of a tile takes the element-wise path.
 template <int CH>
-__device__ __forceinline__ void write_back_chunk_p8(const GemmParams& p, const int32_t (&v)[CH], size_t base, int valid, int m_first, float scale_b,
+__device__ __forceinline__ void write_back_chunk_p8(const GemmParams& p, const int32_t (&v)[CH], size_t base, int valid, int m_first, float* c, int ldc, bool has_bias, float scale_b,
                                                     int zp_b, int off_b, float bias_n) {
-  float* dst = reinterpret_cast<float*>(p.c) + base;
-  int32_t* acc_dst = p.acc_out != nullptr ? p.acc_out + base : nullptr;
-  const bool has_bias = p.bias != nullptr;
+  float* dst = c + base;
+  int32_t* acc_dst = p.acc_out != nullptr ? p.acc_out + base : nullptr;   // (single-segment launches only: ldc == N)
   if(valid >= CH) {
 #pragma unroll
     for(int j = 0; j < CH; j += 4) {
       const int4 za = __ldg(reinterpret_cast<const int4*>(p.p8_zp_a + m_first + j));
       const int4 su = __ldg(reinterpret_cast<const int4*>(p.p8_sum_a + m_first + j));
       const float4 sa = __ldg(reinterpret_cast<const float4*>(p.p8_scale_a + m_first + j));
-      dst[static_cast<size_t>(j + 0) * p.N] = p8_value(v[j + 0], za.x, su.x, sa.x, scale_b, zp_b, off_b, has_bias, bias_n, p.relu);
-      dst[static_cast<size_t>(j + 1) * p.N] = p8_value(v[j + 1], za.y, su.y, sa.y, scale_b, zp_b, off_b, has_bias, bias_n, p.relu);
-      dst[static_cast<size_t>(j + 2) * p.N] = p8_value(v[j + 2], za.z, su.z, sa.z, scale_b, zp_b, off_b, has_bias, bias_n, p.relu);
-      dst[static_cast<size_t>(j + 3) * p.N] = p8_value(v[j + 3], za.w, su.w, sa.w, scale_b, zp_b, off_b, has_bias, bias_n, p.relu);
+      dst[static_cast<size_t>(j + 0) * ldc] = p8_value(v[j + 0], za.x, su.x, sa.x, scale_b, zp_b, off_b, has_bias, bias_n, p.relu);
+      dst[static_cast<size_t>(j + 1) * ldc] = p8_value(v[j + 1], za.y, su.y, sa.y, scale_b, zp_b, off_b, has_bias, bias_n, p.relu);
+      dst[static_cast<size_t>(j + 2) * ldc] = p8_value(v[j + 2], za.z, su.z, sa.z, scale_b, zp_b, off_b, has_bias, bias_n, p.relu);
+      dst[static_cast<size_t>(j + 3) * ldc] = p8_value(v[j + 3], za.w, su.w, sa.w, scale_b, zp_b, off_b, has_bias, bias_n, p.relu);
     }
   } else {
 #pragma unroll
     for(int j = 0; j < CH; ++j)
       if(j < valid) {
         const int m = m_first + j;
-        dst[static_cast<size_t>(j) * p.N] = p8_value(v[j], __ldg(p.p8_zp_a + m), __ldg(p.p8_sum_a + m), __ldg(p.p8_scale_a + m), scale_b, zp_b,
+        dst[static_cast<size_t>(j) * ldc] = p8_value(v[j], __ldg(p.p8_zp_a + m), __ldg(p.p8_sum_a + m), __ldg(p.p8_scale_a + m), scale_b, zp_b,
                                                      off_b, has_bias, bias_n, p.relu);
       }
   }
@@ -292,7 +291,7 @@ __device__ __forceinline__ void write_back_chunk_p8(const GemmParams& p, const i
 #pragma unroll
     for(int j = 0; j < CH; ++j)
       if(j < valid)
-        acc_dst[static_cast<size_t>(j) * p.N] = v[j];
+        acc_dst[static_cast<size_t>(j) * ldc] = v[j];
   }
 }
 
@@ -585,10 +584,11 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       const int cols_valid = min(TM, p.M - m0);  // activation rows of this tile that exist
       // the weight segment this tile belongs to: its multiplier, bias, output matrix and the column inside it
       int seg = 0, n_loc = n;
-      if(!kP8 && kTopK == 0 && p.nseg > 1) {
+      if(kTopK == 0 && p.nseg > 1) {
         seg = (wi.n_tile * kTileN) / p.seg_n;
         n_loc = n - seg * p.seg_n;
-        unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(*p.seg_qa[seg], *p.seg_qb[seg])), p.scale);
+        if(!kP8)
+          unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(*p.seg_qa[seg], *p.seg_qb[seg])), p.scale);
       }
       const float* seg_bias = p.seg_bias[seg];
       void* seg_c = p.seg_c[seg];
@@ -828,7 +828,8 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
           }
           if constexpr(kP8) {
             if(n_ok)
-              write_back_chunk_p8<T::kChunk>(p, v, static_cast<size_t>(m0 + col0) * p.N + n, cols_valid - col0, m0 + col0, p8_scale_b, p8_zp_b,
+              write_back_chunk_p8<T::kChunk>(p, v, static_cast<size_t>(m0 + col0) * ldc + n_loc, cols_valid - col0, m0 + col0, static_cast<float*>(seg_c),
+                                             ldc, seg_bias != nullptr, p8_scale_b, p8_zp_b,
                                              p8_off_b, bias_n);
           } else if(n_ok)
             out_max = write_back_chunk<T::kChunk>(p, v, static_cast<size_t>(m0 + col0) * ldc + n_loc, cols_valid - col0, unquant, bias_n,
@@ -1104,11 +1105,12 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       const int m0 = wi.m_tile * T::kTM;
       const int cols_valid = min(T::kTM, p.M - m0);
       int seg = 0, n_loc = n;
-      if(!kP8 && p.nseg > 1) {
+      if(p.nseg > 1) {
         // (an odd number of 128-row weight tiles: the second CTA of the last pair has none, and stores nothing (n_ok))
         seg = min(((2 * wi.n_tile + static_cast<int>(rank)) * kTileN) / p.seg_n, p.nseg - 1);
         n_loc = n - seg * p.seg_n;
-        unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(*p.seg_qa[seg], *p.seg_qb[seg])), p.scale);
+        if(!kP8)
+          unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(*p.seg_qa[seg], *p.seg_qb[seg])), p.scale);
       }
       const float* seg_bias = p.seg_bias[seg];
       void* seg_c = p.seg_c[seg];
@@ -1135,7 +1137,8 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         tc_wait_ld();
         if constexpr(kP8) {
           if(n_ok)
-            write_back_chunk_p8<T::kChunk>(p, v, static_cast<size_t>(m0 + col0) * p.N + n, cols_valid - col0, m0 + col0, p8_scale_b, p8_zp_b,
+            write_back_chunk_p8<T::kChunk>(p, v, static_cast<size_t>(m0 + col0) * ldc + n_loc, cols_valid - col0, m0 + col0, static_cast<float*>(seg_c),
+                                           ldc, seg_bias != nullptr, p8_scale_b, p8_zp_b,
                                            p8_off_b, bias_n);
         } else if(n_ok)
           out_max = write_back_chunk<T::kChunk>(p, v, static_cast<size_t>(m0 + col0) * ldc + n_loc, cols_valid - col0, unquant, bias_n, out_max,
@@ -2358,7 +2361,12 @@ int launch_gemm_cq(const CqCall& g) {
 // split-K machinery are the same, only the operand signedness and the write-back differ.
 int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a, const int32_t* sum_a, const int8_t* bt,
                    const float* scale_b, const int32_t* zp_b, const int32_t* off_b, int M, int N, int K, const float* bias, int relu,
-                   float* c, int32_t* acc_out, void* ws, size_t ws_bytes, cudaStream_t stream, int force_tile_m, int force_splits) {
+                   float* c, int32_t* acc_out, void* ws, size_t ws_bytes, cudaStream_t stream, int force_tile_m, int force_splits, int nseg,
+                   float* const* seg_c, const float* const* seg_bias) {
+  if(nseg < 1 || nseg > kMaxSegments || (nseg > 1 && (seg_c == nullptr || seg_bias == nullptr || N % nseg != 0 || (N / nseg) % kTileN != 0 || acc_out != nullptr)))
+    return MI8_ERR_BAD_ARG;
+  if(nseg > 1)
+    c = seg_c[0];
   if(M < 0 || N <= 0 || K <= 0 || force_tile_m < 0 || force_splits < 0)
     return MI8_ERR_BAD_ARG;
   if(M == 0)
@@ -2411,6 +2419,12 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
   if(p.status == nullptr)
     return MI8_ERR_LAUNCH;
   single_segment(p);
+  p.nseg = nseg;
+  p.seg_n = N / nseg;
+  for(int i = 0; i < nseg && nseg > 1; ++i) {
+    p.seg_bias[i] = seg_bias[i];
+    p.seg_c[i] = seg_c[i];
+  }
   finish_params(p);
   if(plan.pair)
     return launch_pair<true>(tw, ta, p, plan, stream);
