@@ -1200,9 +1200,12 @@ __device__ __forceinline__ void finish_step(const StepEnd& e, int r, int k, int 
     if(c < n) {
       const int row = (c / k) * e.batch + b;
       const float v = __ldcg(cand_score + row * k + c % k);
-      ok = v > -FLT_MAX;   // (not -inf: a dummy hypothesis; not the filler of a row with fewer than k entries)
-      c_v[c] = v;
-      c_i[c] = ok ? (c / k) * vocab + __ldcg(cand_word + row * k + c % k) : 0x7fffffff;
+      // not -inf: a dummy hypothesis; not a filler, neither of a row with fewer than k entries nor of one without a number (its
+      // log-sum-exp is one, and would lift the filler's score)
+      const int word = __ldcg(cand_word + row * k + c % k);
+      ok = v > -FLT_MAX && static_cast<unsigned>(word) < static_cast<unsigned>(vocab);
+      c_v[c] = ok ? v : -FLT_MAX;
+      c_i[c] = ok ? (c / k) * vocab + word : 0x7fffffff;
     }
     valid += __popc(__ballot_sync(0xffffffffu, ok));
   }
@@ -1552,7 +1555,10 @@ __global__ void nbest_merge_kernel(const float* __restrict__ cand_score, const i
     const int row = j * batch + b;
     for(int c = 0; c < K; ++c) {
       const float s = cand_score[row * K + c];
-      const int key = j * vocab + cand_word[row * K + c];  // the reference's flattened (beam, word) key
+      const int word = cand_word[row * K + c];
+      if(static_cast<unsigned>(word) >= static_cast<unsigned>(vocab))   // (a filler)
+        continue;
+      const int key = j * vocab + word;  // the reference's flattened (beam, word) key
       // -inf candidates (dummy hypotheses) must stay behind every real one but keep a defined order
       topk_insert<K>(t, s == -INFINITY ? -FLT_MAX : s, key);
     }
