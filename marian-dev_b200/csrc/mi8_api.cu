@@ -389,7 +389,7 @@ int mi8_multiply_plan(int M, int N, int K, int force_tile_m, int force_splits, i
   if(out == nullptr)
     return MI8_ERR_BAD_ARG;
   GemmPlan plan;
-  int rc = make_gemm_plan(M, N, K, force_tile_m, force_splits, &plan);
+  int rc = make_gemm_plan(M, N, K, force_tile_m, force_splits, &plan, true);
   if(rc != MI8_OK)
     return rc;
   out[0] = plan.pair ? 512 : plan.tile_m;

@@ -70,10 +70,11 @@ struct Control {
 constexpr int kLogitPitch = kTileN + 4;   // floats per row of a parked tile of logits (kBlocks), which lie this far behind the control block
 constexpr int kParkedOffset = 256;
 static_assert(sizeof(Control) <= kParkedOffset, "");
-template <int TM, bool kBlocks = false>
+constexpr int kDuoBytes = 32 * kTileN * static_cast<int>(sizeof(int32_t));   // the partial sums a CTA receives from its pair (kDuo)
+template <int TM, bool kBlocks = false, bool kDuo = false>
 constexpr int smem_bytes_for() {
   return TileCfg<TM>::kStages * TileCfg<TM>::kStageBytes + static_cast<int>(sizeof(Control)) + 1024 +
-         (kBlocks ? kParkedOffset + 2 * TM * kLogitPitch * static_cast<int>(sizeof(float)) : 0);
+         (kBlocks ? kParkedOffset + 2 * TM * kLogitPitch * static_cast<int>(sizeof(float)) : 0) + (kDuo ? kParkedOffset + kDuoBytes : 0);
 }
 
 struct GemmParams {
@@ -309,7 +310,9 @@ __device__ __forceinline__ void write_back_chunk_p8(const GemmParams& p, const i
 // numbers per block (lse_topk_kernel).  The reduction runs on the write-back warps beside the next tile's MMAs.
 // With it a row's log-softmax / top-k no longer scans 32000 logits on one SM (14 us at one row, 17 at 16): student, one sentence 2.82 -> 2.54 ms
 // a mini-batch, 16 sentences 3.94 -> 3.67.  Up to 32 rows (kBlockRows): a wider tile's values would not fit beside the ring.
-template <int TM, bool kQuantA, int kTopK = 0, bool kP8 = false, bool kBlocks = false>
+// kDuo (long inner dimensions of a few hundred rows): the two CTAs of a cluster take one half of K each for the same 64-row tile.  Each keeps 32 of the
+// tile's rows, gets their other partial sums from its pair through distributed shared memory and writes them back.  One tile per CTA.
+template <int TM, bool kQuantA, int kTopK = 0, bool kP8 = false, bool kBlocks = false, bool kDuo = false>
 __global__ void __launch_bounds__(kThreads, 1)
 mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
   using T = TileCfg<TM>;
@@ -354,6 +357,10 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&ctl->tmem_base);
+  if constexpr(kDuo)
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (this CTA runs: its pair may store into it)
+  const uint32_t duo_rank = kDuo ? blockIdx.x & 1u : 0u;
+  int32_t* const received = reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(ctl) + kParkedOffset);   // kDuo: [32 activation rows][128 weight rows]
 
   bool ok = true;
 
@@ -578,6 +585,24 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       tc_fence_after_sync();
 
       const uint32_t t_addr = tmem_base + as * T::kAccStride + (static_cast<uint32_t>(quarter * 32) << 16);
+      if constexpr(kDuo) {
+        static_assert(TM == 64 && !kBlocks && !kP8 && !kQuantA && kTopK == 0, "two chunks, one per CTA");
+        // the rows that the pair writes back: their partial sums go there
+        if(group != static_cast<int>(duo_rank)) {
+          int32_t v[T::kChunk];
+          tmem_ld_chunk<T::kChunk>(t_addr + group * T::kChunk, v);
+          tc_wait_ld();
+          asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+          const uint32_t dst = mapa_shared(smem_u32(received + row), duo_rank ^ 1u);
+#pragma unroll
+          for(int e = 0; e < T::kChunk; ++e)
+            st_cluster_u32(dst + e * kTileN * static_cast<uint32_t>(sizeof(int32_t)), static_cast<uint32_t>(v[e]));
+        } else {
+          asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        }
+        ++acc_it;
+        break;   // (the rest behind the cluster's barrier below)
+      }
       const int n = wi.n_tile * kTileN + row;
       const bool n_ok = n < p.N;
       const int m0 = wi.m_tile * TM;
@@ -850,6 +875,42 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       *abort_flag = 1;
       if(lane == 0)
         atomicMax(p.status, static_cast<int>(kDevTimeoutEpilogue));
+    }
+  }
+
+  if constexpr(kDuo) {
+    // every thread of both CTAs comes here, whatever happened before: the roles without a tile to hand over, or that gave up, wait for the first
+    // barrier now
+    __syncwarp();
+    if(warp < 2 || !ok)
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sync_all();
+    const int quarter = warp & 3, group = (warp - 2) >> 2, row = quarter * 32 + lane;
+    if(warp >= 2 && ok && group == static_cast<int>(duo_rank)) {
+      const WorkItem wi = decode_work(p, blockIdx.x);
+      tc_fence_after_sync();
+      int32_t v[T::kChunk];
+      tmem_ld_chunk<T::kChunk>(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + group * T::kChunk, v);
+      tc_wait_ld();
+#pragma unroll
+      for(int e = 0; e < T::kChunk; ++e)
+        v[e] += received[e * kTileN + row];
+      const int n = wi.n_tile * kTileN + row;
+      const bool n_ok = n < p.N;
+      const int seg = p.nseg > 1 ? (wi.n_tile * kTileN) / p.seg_n : 0, n_loc = n - seg * p.seg_n;
+      const float unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(*p.seg_qa[seg], *p.seg_qb[seg])), p.scale);
+      const float* seg_bias = p.seg_bias[seg];
+      const int ldc = p.seg_n, m0 = wi.m_tile * TM + group * T::kChunk;
+      const bool paired = p.out_f16 && (ldc & 1) == 0 && (reinterpret_cast<uintptr_t>(p.seg_c[seg]) & 3u) == 0 && __all_sync(0xffffffffu, n_ok);
+      unsigned out_max = 0u;
+      if(n_ok)
+        out_max = write_back_chunk<T::kChunk>(p, v, static_cast<size_t>(m0) * ldc + n_loc, p.M - m0, unquant, seg_bias != nullptr ? __ldg(seg_bias + n_loc) : 0.0f,
+                                              out_max, p.seg_c[seg], ldc, seg_bias != nullptr, paired);
+      if(p.absmax_out != nullptr) {
+        out_max = __reduce_max_sync(0xffffffffu, out_max);
+        if(lane == 0 && out_max != 0u)
+          atomicMax(p.absmax_out, out_max);
+      }
     }
   }
 
@@ -1815,6 +1876,59 @@ int launch_cfg(const CUtensorMap& tw, const CUtensorMap& ta, const GemmParams& p
   return check_launch();
 }
 
+// Launch of kDuo: clusters of two CTAs, one tile each.
+int launch_duo(const CUtensorMap& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
+  static bool attr_set[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  auto kernel = mi8_gemm_kernel<64, false, 0, false, false, true>;
+  constexpr int smem = smem_bytes_for<64, false, true>();
+  if(dev >= 0 && dev < 64 && !attr_set[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if(e != cudaSuccess) {
+      set_last_cuda_error(e);
+      return MI8_ERR_LAUNCH;
+    }
+    attr_set[dev] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(plan.grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  ProfileRecord rec{};
+  const bool profiled = t_profile.on && t_profile.records.size() < t_profile.capacity;
+  if(profiled) {
+    rec = ProfileRecord{p.M, p.N, p.K, p.out_f16 ? 2 : 4, t_profile.take(), t_profile.take()};
+    if(rec.start != nullptr && rec.stop != nullptr)
+      cudaEventRecord(rec.start, stream);
+  }
+  const bool timed = kernel_times_on();
+  cfg.numAttrs = pdl_enabled() && !timed ? 2 : 1;
+  if(timed)
+    kernel_times_before(reinterpret_cast<const void*>(kernel), stream);
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, tw, ta, p);
+  if(timed)
+    kernel_times_after(stream);
+  if(le != cudaSuccess) {
+    set_last_cuda_error(le);
+    return MI8_ERR_LAUNCH;
+  }
+  if(profiled && rec.start != nullptr && rec.stop != nullptr) {
+    cudaEventRecord(rec.stop, stream);
+    t_profile.records.push_back(rec);
+  }
+  count_launch();
+  return check_launch();
+}
+
 // Launch of the CTA-pair kernel: clusters of two CTAs, as many as can be resident at once.
 template <bool kP8 = false>
 int launch_pair(const CUtensorMap& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
@@ -1957,12 +2071,13 @@ int profile_end(mi8_gemm_record* out, int capacity, int* count) {
   return MI8_OK;
 }
 
-int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, GemmPlan* plan) {
+int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, GemmPlan* plan, bool allow_duo) {
   if(M <= 0 || N <= 0 || K <= 0)
     return MI8_ERR_BAD_ARG;
   const int sms = sm_count();
   int tm = force_tile_m;
   plan->pair = 0;
+  plan->duo = 0;
   if(tm == 0 && force_splits <= 1 && M > 64) {
     // Enough 128 x 256 tiles for every SM and at least eight K blocks per tile: the CTA-pair kernel
     // moves a third less operand data from L2 into shared memory per output and measured 10-20 % faster
@@ -1989,6 +2104,25 @@ int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, Gemm
     const long long pairs = pair_tiles < sms / 2 ? pair_tiles : sms / 2;
     plan->grid = static_cast<int>(2 * pairs);
     plan->smem_bytes = smem_bytes_pair();
+    plan->partial_bytes = 0;
+    return MI8_OK;
+  }
+  // Long inner dimensions: 64-row tiles, two CTAs each, where that is one wave of at least half of the SMs.  512 x 4096 x 1024 on 128 CTAs 11.5 us with
+  // 32-row tiles, 9.4 now, 200 x 4096 x 2000 11.6 and 9.5, 500 x 2048 x 1024 7.5 and 7.3 (transformer-big, 128 x beam 4, whose W2 this is: 43.3 ->
+  // 42.5 ms a mini-batch).  On fewer SMs the plan below is as good or better: 128 x 4096 x 1024 on 32 CTAs 8.4, 7.9 below, 256 x 2048 x 512 6.3 against
+  // 7.7 back to back, but transformer-base 35.3 against 35.15 ms.
+  const long long duo_tiles = static_cast<long long>((N + kTileN - 1) / kTileN) * ((M + 63) / 64);
+  if(allow_duo && tm == 0 && force_splits == 0 && M > 64 && (K + kTileKBytes - 1) / kTileKBytes >= 16 && 2 * duo_tiles <= sms && 4 * duo_tiles >= sms) {
+    plan->duo = 1;
+    plan->tile_m = 64;
+    plan->stages = TileCfg<64>::kStages;
+    plan->n_tiles = (N + kTileN - 1) / kTileN;
+    plan->m_tiles = (M + 63) / 64;
+    plan->kb_total = (K + kTileKBytes - 1) / kTileKBytes;
+    plan->kb_per_split = (plan->kb_total + 1) / 2;
+    plan->splits = 2;
+    plan->grid = static_cast<int>(2 * duo_tiles);
+    plan->smem_bytes = smem_bytes_for<64, false, true>();
     plan->partial_bytes = 0;
     return MI8_OK;
   }
@@ -2096,6 +2230,10 @@ int launch_gemm_call(const GemmCall& g) {
     if(g.ws == nullptr || g.ws_bytes < kWsHeaderBytes + plan.partial_bytes)
       return MI8_ERR_WORKSPACE;
   }
+  // (after the check above: a call without the workspace that the other plan needs stays refused)
+  GemmPlan duo;
+  if(!blocks && g.skip_a == nullptr && M > 64 && K > 15 * kTileKBytes && make_gemm_plan(M, N, K, g.force_tile_m, g.force_splits, &duo, true) == MI8_OK && duo.duo)
+    plan = duo;
   CUtensorMap tw, ta;
   rc = get_kmajor_map(&tw, g.bt, N, K, kTileN);
   if(rc != MI8_OK)
@@ -2157,6 +2295,8 @@ int launch_gemm_call(const GemmCall& g) {
 
   if(blocks)
     return plan.tile_m == 16 ? launch_cfg<16, false, 0, false, true>(tw, ta, p, plan, g.stream) : launch_cfg<32, false, 0, false, true>(tw, ta, p, plan, g.stream);
+  if(plan.duo)
+    return launch_duo(tw, ta, p, plan, g.stream);
   if(plan.pair)
     return launch_pair(tw, ta, p, plan, g.stream);
   switch(plan.tile_m) {

@@ -39,6 +39,7 @@ int check_launch();
 struct GemmPlan {
   int tile_m;        // activation rows per tile (MMA N): 16, 32, 64, 128 or 256
   int pair;          // 1: CTA-pair kernel (256 weight rows x 256 activation rows per cluster of two CTAs)
+  int duo;           // 1: two CTAs of a cluster share a 64-row tile's inner dimension (splits == 2, no workspace)
   int stages;        // shared-memory pipeline depth
   int splits;        // split-K factor
   int n_tiles;       // tiles of 128 weight rows
@@ -49,7 +50,7 @@ struct GemmPlan {
   int smem_bytes;
   size_t partial_bytes;
 };
-int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, GemmPlan* plan);
+int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, GemmPlan* plan, bool allow_duo = false);
 
 // mi8_peak.cu: TOPS of a loop of this library's int8 MMAs alone (k_blocks 128-byte K blocks per SM).
 int measure_int8_mma_peak(int k_blocks, float* tops_out, cudaStream_t stream);
