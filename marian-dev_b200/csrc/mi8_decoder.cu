@@ -1349,22 +1349,28 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
     end.prev_bits = d->prev_bits;
     end.stats = d->reuse_stats;
   }
-  if(!fused_output && !d->p8 && R <= kBlockRows) {
+  if(!fused_output && R <= kBlockRows) {
     // few rows: the write-back reduces the blocks of the log-softmax as well
-    GemmCall g;
-    g.aq = d->aq;
-    g.bt = d->out_w.bt;
-    g.M = R;
-    g.N = d->out_w.N;
-    g.K = d->out_w.K;
-    g.d_qa = aq_tail;
-    g.seg_qb[0] = d->out_w.qm;
-    g.seg_bias[0] = d->out_bias;
-    g.seg_c[0] = d->logits;
-    g.stream = s;
-    g.block_max = d->blk_max;
-    g.block_sum = d->blk_sum;
-    MI8D_TRY(launch_gemm_call(g));
+    if(d->p8) {
+      const Aff& w = d->out_w;
+      MI8D_TRY(launch_gemm_p8(reinterpret_cast<const uint8_t*>(d->aq), d->p8_scale_a, d->p8_zp_a, d->p8_sum_a, w.bt, w.scale_b, w.zp_b, w.off_b, R, w.N,
+                              w.K, w.bias, 0, d->logits, nullptr, d->ws, d->ws_bytes, s, 0, 0, 1, nullptr, nullptr, d->blk_max, d->blk_sum));
+    } else {
+      GemmCall g;
+      g.aq = d->aq;
+      g.bt = d->out_w.bt;
+      g.M = R;
+      g.N = d->out_w.N;
+      g.K = d->out_w.K;
+      g.d_qa = aq_tail;
+      g.seg_qb[0] = d->out_w.qm;
+      g.seg_bias[0] = d->out_bias;
+      g.seg_c[0] = d->logits;
+      g.stream = s;
+      g.block_max = d->blk_max;
+      g.block_sum = d->blk_sum;
+      MI8D_TRY(launch_gemm_call(g));
+    }
     MI8D_TRY(launch_lse_topk(d->logits, R, c.vocab, n_best, prev_scores, d->cand_score, d->cand_word, s, end, d->blk_max, d->blk_sum));
   } else if(!fused_output) {
     MI8D_TRY(gemm_act(d, d->aq, R, d->out_w, false, d->logits, s));

@@ -309,7 +309,7 @@ __device__ __forceinline__ void write_back_chunk_p8(const GemmParams& p, const i
 // of logits it stores, the block's maximum and its sum of exponentials in ascending order; what is left of the log-softmax reads two
 // numbers per block (lse_topk_kernel).  The reduction runs on the write-back warps beside the next tile's MMAs.
 // With it a row's log-softmax / top-k no longer scans 32000 logits on one SM (14 us at one row, 17 at 16): student, one sentence 2.82 -> 2.54 ms
-// a mini-batch, 16 sentences 3.94 -> 3.67.  Up to 32 rows (kBlockRows): a wider tile's values would not fit beside the ring.
+// a mini-batch, 16 sentences 3.94 -> 3.67; packed8avx512 (kP8): student 4.60 -> 4.45 and 5.38 -> 5.20, transformer-base, 4 x beam 4 14.86 -> 14.71.  Up to 32 rows (kBlockRows): a wider tile's values would not fit beside the ring.
 // kDuo (long inner dimensions of a few hundred rows): the two CTAs of a cluster take one half of K each for the same 64-row tile.  Each keeps 32 of the
 // tile's rows, gets their other partial sums from its pair through distributed shared memory and writes them back.  One tile per CTA.
 template <int TM, bool kQuantA, int kTopK = 0, bool kP8 = false, bool kBlocks = false, bool kDuo = false>
@@ -779,7 +779,7 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       }
 
       if constexpr(kBlocks) {
-        static_assert(TM <= 32 && !kP8 && !kQuantA, "one chunk per tile");
+        static_assert(TM <= 32 && !kQuantA, "one chunk per tile");
         // a place of its own for every second tile: this tile's sums may still be under way when the next one's values come
         float* parked = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ctl) + kParkedOffset) + (acc_it & 1u) * (TM * kLogitPitch);
         if(group == 0) {
@@ -789,9 +789,16 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
           float* dst = static_cast<float*>(seg_c) + static_cast<size_t>(m0) * ldc + n_loc;
 #pragma unroll
           for(int j = 0; j < T::kChunk; ++j) {
-            float x = __fmul_rn(__int2float_rn(v[j]), unquant);
-            if(seg_bias != nullptr)
-              x = __fadd_rn(x, bias_n);
+            float x;
+            if constexpr(kP8) {
+              const int m = m0 + min(j, cols_valid - 1);
+              x = p8_value(v[j], __ldg(p.p8_zp_a + m), __ldg(p.p8_sum_a + m), __ldg(p.p8_scale_a + m), p8_scale_b, p8_zp_b, p8_off_b, seg_bias != nullptr,
+                           bias_n, 0);
+            } else {
+              x = __fmul_rn(__int2float_rn(v[j]), unquant);
+              if(seg_bias != nullptr)
+                x = __fadd_rn(x, bias_n);
+            }
             if(j < cols_valid && n_ok)
               dst[static_cast<size_t>(j) * ldc] = x;
             parked[j * kLogitPitch + row] = n_ok ? x : -FLT_MAX;
@@ -2502,7 +2509,14 @@ int launch_gemm_cq(const CqCall& g) {
 int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a, const int32_t* sum_a, const int8_t* bt,
                    const float* scale_b, const int32_t* zp_b, const int32_t* off_b, int M, int N, int K, const float* bias, int relu,
                    float* c, int32_t* acc_out, void* ws, size_t ws_bytes, cudaStream_t stream, int force_tile_m, int force_splits, int nseg,
-                   float* const* seg_c, const float* const* seg_bias) {
+                   float* const* seg_c, const float* const* seg_bias, float* block_max, float* block_sum) {
+  const bool blocks = block_max != nullptr;
+  if(blocks && (M > kBlockRows || block_sum == nullptr || nseg != 1 || relu || acc_out != nullptr || force_tile_m != 0))
+    return MI8_ERR_UNSUPPORTED;
+  if(blocks) {
+    force_tile_m = M <= 16 ? 16 : 32;
+    force_splits = 1;
+  }
   if(nseg < 1 || nseg > kMaxSegments || (nseg > 1 && (seg_c == nullptr || seg_bias == nullptr || N % nseg != 0 || (N / nseg) % kTileN != 0 || acc_out != nullptr)))
     return MI8_ERR_BAD_ARG;
   if(nseg > 1)
@@ -2566,6 +2580,12 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
     p.seg_c[i] = seg_c[i];
   }
   finish_params(p);
+  if(blocks) {
+    p.lg_max = block_max;
+    p.lg_sum = block_sum;
+    p.lg_blocks = plan.n_tiles;
+    return plan.tile_m == 16 ? launch_cfg<16, false, 0, true, true>(tw, ta, p, plan, stream) : launch_cfg<32, false, 0, true, true>(tw, ta, p, plan, stream);
+  }
   if(plan.pair)
     return launch_pair<true>(tw, ta, p, plan, stream);
   switch(plan.tile_m) {
