@@ -128,7 +128,6 @@ struct mi8d_decoder {
   std::vector<int8_t*> fused_enc, fused_self, fused_ctx;   // arena storage of the fused matrices
   std::vector<float*> columns_enc, columns_self, columns_ctx;   // ... and of their columns' parameters (packed8avx512)
   DecoderRowsParams rows;             // for launch_decoder_rows: what does not change from step to step is filled in by resolve()
-  float* rows_pack = nullptr;
   bool rows_ready = false;
 
   std::vector<LayerBufs> layers;
@@ -273,8 +272,6 @@ struct mi8d_decoder {
       for(auto& p : fused_ctx)
         p = arena.take<int8_t>(2 * d * d);
     }
-    const size_t n_pack = c.ssru && can_fuse ? decoder_rows_pack_floats(c.dim_emb, c.dim_ffn, c.heads, c.dec_depth) : 0;
-    rows_pack = n_pack != 0 ? arena.take<float>(n_pack) : nullptr;
   }
 
   unsigned* layer_slot(int l, int which) const { return slots + 1 + kSlotsPerLayer * l + which; }
@@ -362,29 +359,32 @@ struct mi8d_decoder {
   }
 
   // What launch_decoder_rows needs of the layers, where all of them have it (an SSRU decoder whose W and Wf lie one behind the other).
-  bool resolve_rows(cudaStream_t s) {
+  void resolve_rows() {
     const mi8d_config& c = cfg;
     rows_ready = false;
-    if(rows_pack == nullptr || p8)
-      return true;
-    DecoderRowsVectors v[kDecoderRowsLayers];
+    if(!c.ssru || p8 || c.dec_depth > kDecoderRowsLayers)
+      return;
     const int dm = c.dim_emb, f = c.dim_ffn;
     for(int l = 0; l < c.dec_depth; ++l) {
       const DecLayerW& w = dec_w[l];
       auto shape = [](const Aff& a, int K, int N) { return a.K == K && a.N == N && a.bias != nullptr; };
       if(!w.rnn.ready || w.rnn.n != dm || w.rnn.K != dm || w.rnn.bias[0] != nullptr || w.rnn.bias[1] == nullptr || !shape(w.ctx_q, dm, dm) ||
          !shape(w.ctx_o, dm, dm) || !shape(w.w1, dm, f) || !shape(w.w2, f, dm))
-        return true;
+        return;
       CUtensorMap* m = rows.map[l];
       if(rows_weight_map(m, w.rnn.bt, 2 * dm, dm) != MI8_OK || rows_weight_map(m + 1, w.ctx_q.bt, dm, dm) != MI8_OK ||
          rows_weight_map(m + 2, w.ctx_o.bt, dm, dm) != MI8_OK || rows_weight_map(m + 3, w.w1.bt, f, dm) != MI8_OK ||
          rows_weight_map(m + 4, w.w2.bt, dm, f) != MI8_OK)
-        return true;
-      v[l] = DecoderRowsVectors{{w.rnn.qm[0], w.rnn.qm[1], w.ctx_q.qm, w.ctx_o.qm, w.w1.qm, w.w2.qm}, w.rnn.bias[1], w.ctx_q.bias, w.ctx_o.bias,
-                                w.w1.bias, w.w2.bias, {w.ln_self.g, w.ln_self.b, w.ln_ctx.g, w.ln_ctx.b, w.ln_ffn.g, w.ln_ffn.b}};
+        return;
+      DecoderRowsVectors& v = rows.vec[l];
+      v = DecoderRowsVectors{{w.rnn.qm[0], w.rnn.qm[1], w.ctx_q.qm, w.ctx_o.qm, w.w1.qm, w.w2.qm}, {w.rnn.bias[1], w.ctx_o.bias, w.w2.bias},
+                             w.ctx_q.bias, w.w1.bias, {w.ln_self.g, w.ln_self.b, w.ln_ctx.g, w.ln_ctx.b, w.ln_ffn.g, w.ln_ffn.b}};
+      const float* copied[] = {v.own[0], v.own[1], v.own[2], v.b_q, v.b_1, v.ln[0], v.ln[1], v.ln[2], v.ln[3], v.ln[4], v.ln[5]};
+      for(const float* x : copied)   // (the launch copies them 16 bytes at a time; the general route reads biases word by word)
+        if(reinterpret_cast<uintptr_t>(x) & 15u)
+          return;
     }
-    rows_ready = launch_decoder_rows_pack(v, dm, f, c.heads, c.dec_depth, rows_pack, s) == MI8_OK;
-    return rows_ready;
+    rows_ready = true;
   }
 
   // Looks every parameter up once and builds the fused matrices.  MI8_ERR_BAD_ARG names a missing parameter.
@@ -425,7 +425,7 @@ struct mi8d_decoder {
         copies = copies && fuse(w.ctx_kv, fused_ctx[l], columns_ctx[l], {&w.ctx_k, &w.ctx_v}, s);
     }
     if(ok)
-      copies = copies && resolve_rows(s);
+      resolve_rows();
     wemb = P("Wemb");
     ok = ok && wemb != nullptr && aff(out_w, p8 ? "Wemb_packed8" : "Wemb_intgemm8", "decoder_ff_logit_out_b");
     out_bias = out_w.bias;
@@ -1168,7 +1168,6 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
     p.out_q = d->aq;
     p.out_qm = aq_tail;
     const LayerBufs &first = d->layers[0], &next = d->layers[c.dec_depth > 1 ? 1 : 0];   // (every layer's buffers are laid out alike)
-    p.pack = d->rows_pack;
     p.cross_k = first.cross_k;
     p.cross_v = first.cross_v;
     p.cell_old = first.cell[d->cell_cur];

@@ -245,12 +245,18 @@ int launch_ssru_cell(const float* cell_old, const int* hyp, const float* xw, con
                      float* h_out, cudaStream_t s);
 
 // The layers of an SSRU decoder's step for few rows in one launch (mi8_rows.cu).
-constexpr int kDecoderRowsLayers = 4, kDecoderRowsMax = 32;
+constexpr int kDecoderRowsLayers = 4, kDecoderRowsMax = 32, kRowsMultipliers = 6;
+// A layer's parameters apart from the matrices, read from here by every launch; 16-byte aligned but for the multipliers.
+struct DecoderRowsVectors {
+  const float* qb[kRowsMultipliers];   // multipliers of W, Wf, Wq, Wo, W1, W2
+  const float* own[3];                 // biases of d columns that a CTA takes its share of: Wf's, Wo's, W2's
+  const float *b_q, *b_1;
+  const float* ln[6];                  // scale and bias behind the cell, the cross-attention, the feed-forward block
+};
 struct DecoderRowsParams {
   int rows = 0, ffn = 0, layers = 0, src = 0, batch = 0;
   float emb_scale = 0.f, att_scale = 0.f;
   const float *wemb = nullptr, *pos = nullptr, *log_mask = nullptr;
-  const float* pack = nullptr;                  // launch_decoder_rows_pack
   // layer 0's; layer l's lie l * layer_stride floats behind
   const float *cross_k = nullptr, *cross_v = nullptr, *cell_old = nullptr;
   float* cell_new = nullptr;
@@ -265,18 +271,12 @@ struct DecoderRowsParams {
   int ring = 0, inv_mt_ffn1 = 0, inv_nf4 = 0, inv_batch = 0, inv_rows = 0;   // set by the launcher (as `status`)
   // n_ctrl > 0: the control words (hypothesis rows, previous words, path scores, batch rows), used from here and brought to `ctrl`
   int ctrl_words[4 * kDecoderRowsMax];
+  DecoderRowsVectors vec[kDecoderRowsLayers];
   // per layer W above Wf, Wq, Wo, W1, W2: boxes of 16 rows x 128 bytes (rows_weight_map)
   CUtensorMap map[kDecoderRowsLayers][5];
 };
-// A layer's parameters apart from the matrices, as launch_decoder_rows reads them.
-struct DecoderRowsVectors {
-  const float* qb[6];   // multipliers of W, Wf, Wq, Wo, W1, W2
-  const float *b_wf, *b_q, *b_o, *b_1, *b_2;
-  const float* ln[6];   // scale and bias behind the cell, the cross-attention, the feed-forward block
-};
+static_assert(sizeof(DecoderRowsParams) <= 4096, "kernel parameters");
 int rows_weight_map(CUtensorMap* map, const int8_t* bt, int N, int K);
-size_t decoder_rows_pack_floats(int d, int f, int heads, int layers);   // 0: no kernel for these sizes
-int launch_decoder_rows_pack(const DecoderRowsVectors* v, int d, int f, int heads, int layers, float* pack, cudaStream_t stream);
 bool decoder_rows_supported(int rows, int d, int f, int heads, int layers, int src);
 int launch_decoder_rows(DecoderRowsParams& p, int d, int heads, cudaStream_t stream);
 int trace_set_rows(unsigned long long* buf);

@@ -86,11 +86,8 @@ __device__ __forceinline__ int div_small(int i, int inv) { return (i * inv) >> 1
 __device__ __forceinline__ void copy_async16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
 }
-// (both 16-byte aligned, a multiple of 16 bytes)
-__device__ __forceinline__ void bulk_load(void* smem, const void* gmem, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem)), "l"(gmem), "r"(bytes),
-               "r"(smem_u32(bar))
-               : "memory");
+__device__ __forceinline__ void copy_async4(void* smem, const void* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
@@ -133,7 +130,6 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
   constexpr int kNd = T::kNd, kNq = T::kNq, kNv = T::kKb;   // (a row is kNv float4 per lane of a warp)
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t full[kWarps][kMaxRing];
-  __shared__ uint64_t params_full;
   __shared__ unsigned redu[kWarps];
   __shared__ unsigned cta_max[kCtas];
   __shared__ int abort_word;
@@ -183,6 +179,26 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
       const int src = with_words ? p.ctrl_words[r] : (p.hyp ? p.hyp[r] : r);
       copy_async16(cell + (l * R + r) * kNd + c, p.cell_old + l * p.layer_stride + static_cast<size_t>(src) * kDim + rank * kNd + c);
     }
+  // The LayerNorms, this CTA's columns of the biases and the weights' multipliers, from where they were registered: a caller may rewrite
+  // them between steps.
+#pragma unroll 1
+  for(int l = 0; l < p.layers; ++l) {
+    const DecoderRowsVectors& v = p.vec[l];
+    float* own = prm + l * T::params(f);
+    constexpr int kLn = kDim / 4, kOwn = kNd / 4;   // 16-byte chunks
+#pragma unroll 1
+    for(int i = threadIdx.x; i < 6 * kLn + 3 * kOwn + (kNq + nf) / 4; i += kThreads) {
+      const int c = i - 6 * kLn, q = c - 3 * kOwn;
+      if(c < 0)
+        copy_async16(norms + l * T::kNorms + 4 * i, v.ln[i / kLn] + 4 * (i % kLn));
+      else if(q < 0)
+        copy_async16(own + 4 * c, v.own[c / kOwn] + rank * kNd + 4 * (c % kOwn));
+      else
+        copy_async16(own + 4 * c, q < kNq / 4 ? v.b_q + head0 * kDh + 4 * q : v.b_1 + rank * nf + 4 * q - kNq);
+    }
+    if(threadIdx.x < kRowsMultipliers)
+      copy_async4(own + 3 * kNd + kNq + nf + threadIdx.x, v.qb[threadIdx.x]);
+  }
   float4 pv[kNv];
 #pragma unroll
   for(int v = 0; v < kNv; ++v)
@@ -213,16 +229,6 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
         }
       }
     }
-  }
-  // biases, multipliers and LayerNorms: [layers][kCtas][params], then [layers][kNorms]
-  if(threadIdx.x == 0) {
-    mbar_init(&params_full, 1);
-    fence_mbar_init();
-    const uint32_t own = sizeof(float) * T::params(f), all = sizeof(float) * T::kNorms * p.layers;
-    mbar_arrive_expect_tx(&params_full, own * p.layers + all);
-    for(int l = 0; l < p.layers; ++l)
-      bulk_load(prm + l * T::params(f), p.pack + (l * kCtas + rank) * T::params(f), own, &params_full);
-    bulk_load(norms, p.pack + p.layers * kCtas * T::params(f), all, &params_full);
   }
   auto request = [&](int slot) {   // by the lane that knows the unit
     mbar_arrive_expect_tx(&full[warp][slot], kUnitBytes);
@@ -446,8 +452,6 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
 
   keep_residual();
   copy_async_wait();
-  if(!mbar_wait_bounded(&params_full, 0, abort_flag))
-    *abort_flag = 1;
   float qa = quantise();
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every CTA of the cluster runs
 
@@ -703,36 +707,6 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
   trace_stamp(th.last, kTrDecoderRows, 3);
 }
 
-// Lays the vectors of one layer out as the kernel above copies them: block c the share of CTA c, the last block the LayerNorms.
-template <int kDim, int kDh, int kCtas>
-__global__ void rows_pack_kernel(const DecoderRowsVectors v, int f, float* __restrict__ shares, float* __restrict__ norms) {
-  using T = Split<kDim, kDh, kCtas>;
-  const int c = blockIdx.x, nf = f / kCtas;
-  if(c == kCtas) {
-    for(int i = threadIdx.x; i < T::kNorms; i += blockDim.x)
-      norms[i] = v.ln[i / kDim][i % kDim];
-    return;
-  }
-  float* to = shares + static_cast<size_t>(c) * T::params(f);
-  for(int i = threadIdx.x; i < T::params(f); i += blockDim.x) {
-    int k = i;
-    float x = 0.f;
-    if(k < T::kNd)
-      x = v.b_wf[c * T::kNd + k];
-    else if((k -= T::kNd) < T::kNd)
-      x = v.b_o[c * T::kNd + k];
-    else if((k -= T::kNd) < T::kNd)
-      x = v.b_2[c * T::kNd + k];
-    else if((k -= T::kNd) < T::kNq)
-      x = v.b_q[c / T::kShare * T::kNq + k];
-    else if((k -= T::kNq) < nf)
-      x = v.b_1[c * nf + k];
-    else if((k -= nf) < 6)
-      x = *v.qb[k];
-    to[i] = x;
-  }
-}
-
 template <int kDim, int kDh, int kCtas, int kRw>
 struct RowsKernel {
   using T = Split<kDim, kDh, kCtas>;
@@ -769,16 +743,6 @@ struct RowsKernel {
     return rows * kDim <= kRw * kWarps * kDim && rows * T::kHeads <= kWarps * kCtas && f % (kUnitRows * kCtas) == 0 && f % 128 == 0 &&
            rows * (f / kCtas / 4) <= 2 * kThreads && rows * (f / kCtas / 4) * (f / kCtas / 4) < 65536 && layers * T::units(f) <= 32 * kWarps &&
            T::smem(rows, f, layers, src, 1) <= static_cast<size_t>(kMaxDynSmem) && available();
-  }
-  static size_t pack_floats(int f, int layers) { return f % (kUnitRows * kCtas) == 0 ? static_cast<size_t>(layers) * (kCtas * T::params(f) + T::kNorms) : 0; }
-  // (plain launches: parameters are read by the kernel above before its wait for the preceding one)
-  static int pack(const DecoderRowsVectors* v, int f, int layers, float* to, cudaStream_t stream) {
-    for(int l = 0; l < layers; ++l) {
-      rows_pack_kernel<kDim, kDh, kCtas><<<kCtas + 1, 256, 0, stream>>>(v[l], f, to + l * kCtas * T::params(f),
-                                                                      to + layers * kCtas * T::params(f) + l * T::kNorms);
-      count_launch();
-    }
-    return check_launch();
   }
   static int launch(DecoderRowsParams& p, cudaStream_t stream) {
     // as many units in flight per warp as fit, up to all of a warp's
@@ -833,17 +797,6 @@ bool decoder_rows_supported(int rows, int d, int f, int heads, int layers, int s
   if(d == 512 && heads == 8)
     return Rows512::supported(rows, f, layers, src);
   return false;
-}
-
-size_t decoder_rows_pack_floats(int d, int f, int heads, int layers) {
-  if(layers < 1 || layers > kDecoderRowsLayers || f < 1 || heads != 8)
-    return 0;
-  return d == 256 ? Rows256::pack_floats(f, layers) : d == 512 ? Rows512::pack_floats(f, layers) : 0;
-}
-int launch_decoder_rows_pack(const DecoderRowsVectors* v, int d, int f, int heads, int layers, float* pack, cudaStream_t stream) {
-  if(decoder_rows_pack_floats(d, f, heads, layers) == 0)
-    return MI8_ERR_UNSUPPORTED;
-  return d == 256 ? Rows256::pack(v, f, layers, pack, stream) : Rows512::pack(v, f, layers, pack, stream);
 }
 
 int launch_decoder_rows(DecoderRowsParams& p, int d, int heads, cudaStream_t stream) {
