@@ -47,15 +47,13 @@ struct P8Weight {
   int K = 0, N = 0;
 };
 // Several weights of the same shape multiplied with the same activation in one launch (Wk|Wv, Wq|Wk|Wv,
-// the SSRU's W|Wf): their int8 matrices copied one behind the other into the arena.
+// the SSRU's W|Wf): their int8 matrices copied one behind the other into the arena.  packed8avx512 matrices stay where they were registered.
 struct Fused {
-  int8_t* bt = nullptr;   // [nseg * n, K] in the arena
+  int8_t* bt = nullptr;   // intgemm8: [nseg * n, K] in the arena
   int nseg = 0, n = 0, K = 0;
   const float* qm[3] = {nullptr, nullptr, nullptr};
   const float* bias[3] = {nullptr, nullptr, nullptr};
-  // packed8avx512: the columns' scales, zero points and offsets of all matrices, copied likewise (in the arena, behind one another)
-  float* scale_b = nullptr;
-  int32_t *zp_b = nullptr, *off_b = nullptr;
+  P8Segments p8;          // packed8avx512; the outputs are the caller's
   bool ready = false;
 };
 struct Norm {
@@ -126,7 +124,6 @@ struct mi8d_decoder {
   const float* out_bias = nullptr;
   Aff out_w;
   std::vector<int8_t*> fused_enc, fused_self, fused_ctx;   // arena storage of the fused matrices
-  std::vector<float*> columns_enc, columns_self, columns_ctx;   // ... and of their columns' parameters (packed8avx512)
   DecoderRowsParams rows;             // for launch_decoder_rows: what does not change from step to step is filled in by resolve()
   bool rows_ready = false;
 
@@ -255,16 +252,7 @@ struct mi8d_decoder {
     fused_enc.assign(c.enc_depth, nullptr);
     fused_self.assign(c.dec_depth, nullptr);
     fused_ctx.assign(c.dec_depth, nullptr);
-    columns_enc.assign(c.enc_depth, nullptr);
-    columns_self.assign(c.dec_depth, nullptr);
-    columns_ctx.assign(c.dec_depth, nullptr);
     if(can_fuse) {
-      for(auto& p : columns_enc)
-        p = arena.take<float>(9 * d);
-      for(auto& p : columns_self)
-        p = arena.take<float>(9 * d);
-      for(auto& p : columns_ctx)
-        p = arena.take<float>(6 * d);
       for(auto& p : fused_enc)
         p = arena.take<int8_t>(3 * d * d);
       for(auto& p : fused_self)
@@ -322,8 +310,8 @@ struct mi8d_decoder {
     n.b = P(prefix + "_ln_bias");
     return n.g != nullptr && n.b != nullptr;
   }
-  // copies the matrices of `parts` one behind the other into `store` (stream-ordered on s)
-  bool fuse(Fused& f, int8_t* store, float* columns, std::initializer_list<const Aff*> parts, cudaStream_t s) {
+  // puts `parts` together; intgemm8: copies the matrices one behind the other into `store` (stream-ordered on s)
+  bool fuse(Fused& f, int8_t* store, std::initializer_list<const Aff*> parts, cudaStream_t s) {
     f = Fused();
     if(store == nullptr)
       return true;   // not fusable for this model: the step falls back to one launch per matrix
@@ -335,25 +323,22 @@ struct mi8d_decoder {
       } else if(a->N != f.n || a->K != f.K) {
         return true;
       }
-      if(cudaMemcpyAsync(store + static_cast<size_t>(i) * f.n * f.K, a->bt, static_cast<size_t>(f.n) * f.K, cudaMemcpyDeviceToDevice, s) !=
-         cudaSuccess)
-        return false;
       if(p8) {
-        const size_t total = parts.size() * static_cast<size_t>(f.n), bytes = sizeof(float) * f.n;
-        f.scale_b = columns;
-        f.zp_b = reinterpret_cast<int32_t*>(columns + total);
-        f.off_b = f.zp_b + total;
-        if(cudaMemcpyAsync(f.scale_b + static_cast<size_t>(i) * f.n, a->scale_b, bytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
-           cudaMemcpyAsync(f.zp_b + static_cast<size_t>(i) * f.n, a->zp_b, bytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
-           cudaMemcpyAsync(f.off_b + static_cast<size_t>(i) * f.n, a->off_b, bytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
-          return false;
+        f.p8.bt[i] = a->bt;
+        f.p8.scale_b[i] = a->scale_b;
+        f.p8.zp_b[i] = a->zp_b;
+        f.p8.off_b[i] = a->off_b;
+        f.p8.bias[i] = a->bias;
+      } else if(cudaMemcpyAsync(store + static_cast<size_t>(i) * f.n * f.K, a->bt, static_cast<size_t>(f.n) * f.K, cudaMemcpyDeviceToDevice, s) !=
+                cudaSuccess) {
+        return false;
       }
       f.qm[i] = a->qm;
       f.bias[i] = a->bias;
       ++i;
     }
     f.bt = store;
-    f.nseg = i;
+    f.nseg = f.p8.n = i;
     f.ready = f.n % 128 == 0;
     return true;
   }
@@ -400,7 +385,7 @@ struct mi8d_decoder {
            aff(e.o, pre + "_Wo", pre + "_bo") && aff(e.w1, ffn + "_W1", ffn + "_b1") && aff(e.w2, ffn + "_W2", ffn + "_b2") &&
            norm(e.ln_att, pre + "_Wo") && norm(e.ln_ffn, ffn + "_ffn");
       if(ok)
-        copies = copies && fuse(e.qkv, fused_enc[l], columns_enc[l], {&e.q, &e.k, &e.v}, s);
+        copies = copies && fuse(e.qkv, fused_enc[l], {&e.q, &e.k, &e.v}, s);
     }
     for(int l = 0; l < c.dec_depth && ok; ++l) {
       DecLayerW& w = dec_w[l];
@@ -409,20 +394,20 @@ struct mi8d_decoder {
         const std::string pre = li + "_rnn";
         ok = ok && aff(w.rnn_w, pre + "_W", "") && aff(w.rnn_wf, pre + "_Wf", pre + "_bf") && norm(w.ln_self, pre + "_ffn");
         if(ok)
-          copies = copies && fuse(w.rnn, fused_self[l], columns_self[l], {&w.rnn_w, &w.rnn_wf}, s);
+          copies = copies && fuse(w.rnn, fused_self[l], {&w.rnn_w, &w.rnn_wf}, s);
       } else {
         const std::string pre = li + "_self";
         ok = ok && aff(w.self_q, pre + "_Wq", pre + "_bq") && aff(w.self_k, pre + "_Wk", pre + "_bk") &&
              aff(w.self_v, pre + "_Wv", pre + "_bv") && aff(w.self_o, pre + "_Wo", pre + "_bo") && norm(w.ln_self, pre + "_Wo");
         if(ok)
-          copies = copies && fuse(w.self_qkv, fused_self[l], columns_self[l], {&w.self_q, &w.self_k, &w.self_v}, s);
+          copies = copies && fuse(w.self_qkv, fused_self[l], {&w.self_q, &w.self_k, &w.self_v}, s);
       }
       const std::string pre = li + "_context", ffn = li + "_ffn";
       ok = ok && aff(w.ctx_q, pre + "_Wq", pre + "_bq") && aff(w.ctx_k, pre + "_Wk", pre + "_bk") && aff(w.ctx_v, pre + "_Wv", pre + "_bv") &&
            aff(w.ctx_o, pre + "_Wo", pre + "_bo") && norm(w.ln_ctx, pre + "_Wo") && aff(w.w1, ffn + "_W1", ffn + "_b1") &&
            aff(w.w2, ffn + "_W2", ffn + "_b2") && norm(w.ln_ffn, ffn + "_ffn");
       if(ok)
-        copies = copies && fuse(w.ctx_kv, fused_ctx[l], columns_ctx[l], {&w.ctx_k, &w.ctx_v}, s);
+        copies = copies && fuse(w.ctx_kv, fused_ctx[l], {&w.ctx_k, &w.ctx_v}, s);
     }
     if(ok)
       resolve_rows();
@@ -507,9 +492,12 @@ GemmCall fused_call(mi8d_decoder* d, const int8_t* a, const Fused& f, int M, int
 // the same activation against all matrices of a fused group; outs[i] receives [M, f.n].  (packed8avx512, a launch per matrix before: transformer-base,
 // 16 sentences x beam 4 18.6 -> 16.7 ms a mini-batch, transformer-big, 8 x 4 20.1 -> 18.0, student, 4 x 4 5.6 -> 5.3.)
 int gemm_fused(mi8d_decoder* d, const int8_t* a, const float* qa, int M, const Fused& f, float* const* outs, cudaStream_t s) {
-  if(d->p8)
-    return launch_gemm_p8(reinterpret_cast<const uint8_t*>(a), d->p8_scale_a, d->p8_zp_a, d->p8_sum_a, f.bt, f.scale_b, f.zp_b, f.off_b, M, f.nseg * f.n,
-                          f.K, nullptr, 0, nullptr, nullptr, d->ws, d->ws_bytes, s, 0, 0, f.nseg, outs, f.bias);
+  if(d->p8) {
+    P8Segments segs = f.p8;
+    std::copy(outs, outs + f.nseg, segs.c);
+    return launch_gemm_p8(reinterpret_cast<const uint8_t*>(a), d->p8_scale_a, d->p8_zp_a, d->p8_sum_a, nullptr, nullptr, nullptr, nullptr, M,
+                          f.nseg * f.n, f.K, nullptr, 0, nullptr, nullptr, d->ws, d->ws_bytes, s, 0, 0, &segs);
+  }
   GemmCall g = fused_call(d, a, f, M, 0, f.nseg, 0, s);
   g.d_qa = qa;
   for(int i = 0; i < f.nseg; ++i)
@@ -1353,7 +1341,7 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
     if(d->p8) {
       const Aff& w = d->out_w;
       MI8D_TRY(launch_gemm_p8(reinterpret_cast<const uint8_t*>(d->aq), d->p8_scale_a, d->p8_zp_a, d->p8_sum_a, w.bt, w.scale_b, w.zp_b, w.off_b, R, w.N,
-                              w.K, w.bias, 0, d->logits, nullptr, d->ws, d->ws_bytes, s, 0, 0, 1, nullptr, nullptr, d->blk_max, d->blk_sum));
+                              w.K, w.bias, 0, d->logits, nullptr, d->ws, d->ws_bytes, s, 0, 0, nullptr, d->blk_max, d->blk_sum));
     } else {
       GemmCall g;
       g.aq = d->aq;

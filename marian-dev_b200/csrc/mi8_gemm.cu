@@ -43,7 +43,6 @@ constexpr int kThreads = 320;
 constexpr int kEpilogueThreads = 256;
 constexpr int kMaxStages = 8;
 constexpr int kPairTileCode = 512;  // force_tile_m value that selects the CTA-pair kernel
-constexpr int kMaxSegments = 3;
 
 template <int TM>
 struct TileCfg {
@@ -111,9 +110,9 @@ struct GemmParams {
   const float* p8_scale_a;
   const int32_t* p8_zp_a;
   const int32_t* p8_sum_a;
-  const float* p8_scale_b;
-  const int32_t* p8_zp_b;
-  const int32_t* p8_off_b;
+  const float* p8_scale_b[kMaxSegments];
+  const int32_t* p8_zp_b[kMaxSegments];
+  const int32_t* p8_off_b[kMaxSegments];
   int* status;
   // Several weight matrices of the same shape [seg_n, K] stored one behind the other and multiplied with the
   // same activation in one launch (Wk|Wv of an attention block, Wq|Wk|Wv of the encoder): segment s covers
@@ -121,6 +120,7 @@ struct GemmParams {
   // seg_n is a multiple of 128, so a tile never straddles two segments.  nseg == 1: the plain call
   // (seg_n = N, seg_qb[0] = d_qb, seg_bias[0] = bias, seg_c[0] = c).  A segment may also take its activation rows from another
   // place of the operand's buffer (seg_row0: their first row in the tensor map), quantised with a multiplier of its own (seg_qa).
+  // packed8avx512 matrices stay where they are: a tensor map for each (WeightMaps).
   int nseg, seg_n;
   int seg_row0[kMaxSegments];
   const float* seg_qa[kMaxSegments];
@@ -131,6 +131,21 @@ struct GemmParams {
   int withhold_item;        // test hook: the producer leaves out the loads of this pipeline item (-1 = none)
   uint32_t spin_limit;      // bound of every barrier wait of this launch
 };
+
+template <bool kP8>
+struct WeightMaps {
+  CUtensorMap map[kP8 ? kMaxSegments : 1];
+};
+// The weight rows from row n on: their matrix's map and the row in it (beyond the last matrix's rows: zeros).
+struct WeightRows {
+  const CUtensorMap* map;
+  int row;
+};
+template <bool kP8>
+__device__ __forceinline__ WeightRows weight_rows(const WeightMaps<kP8>& maps, int nseg, int seg_n, int n) {
+  const int seg = kP8 && nseg > 1 ? min(n / seg_n, nseg - 1) : 0;
+  return {&maps.map[seg], n - seg * seg_n};
+}
 
 struct WorkItem {
   int tile, split, n_tile, m_tile, kb_begin, kb_end;
@@ -314,7 +329,7 @@ __device__ __forceinline__ void write_back_chunk_p8(const GemmParams& p, const i
 // tile's rows, gets their other partial sums from its pair through distributed shared memory and writes them back.  One tile per CTA.
 template <int TM, bool kQuantA, int kTopK = 0, bool kP8 = false, bool kBlocks = false, bool kDuo = false>
 __global__ void __launch_bounds__(kThreads, 1)
-mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
+mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
   using T = TileCfg<TM>;
   constexpr int kConvWarps = kEpilogueThreads / 32;
   extern __shared__ uint8_t smem_raw[];
@@ -334,7 +349,7 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   const unsigned long long trace_extra = static_cast<unsigned long long>(p.N) | (static_cast<unsigned long long>(p.K) << 20) |
                                          (static_cast<unsigned long long>(p.M) << 40);
   if(threadIdx.x == 0) {
-    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(weight_rows(tmap_w, p.nseg, p.seg_n, decode_work(p, blockIdx.x).n_tile * kTileN).map);
     tma_prefetch_desc(&tmap_a);
     for(int s = 0; s < T::kStages; ++s) {
       mbar_init(&ctl->full[s], kQuantA ? 1 + kConvWarps : 1);   // producer (+ one arrival per quantising warp)
@@ -372,12 +387,13 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     uint32_t prefetched = 0;  // stages whose weight tile is already in flight
     if(p.skip_a == nullptr && kTopK == 0 && p.withhold_item < 0) {   // (output-layer variant: the M-side operand is the activation, nothing to prefetch)
       const WorkItem w0 = decode_work(p, blockIdx.x);
+      const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, w0.n_tile * kTileN);
       const int n_pre = min(T::kStages, w0.kb_end - w0.kb_begin);
       if(elect_one()) {
         for(int i = 0; i < n_pre; ++i) {
           uint8_t* st = tiles + i * T::kStageBytes;
           mbar_arrive_expect_tx(&ctl->full[i], kQuantA ? T::kWBytes : T::kStageBytes);
-          tma_load_2d(st, &tmap_w, (w0.kb_begin + i) * kTileKBytes, w0.n_tile * kTileN, &ctl->full[i]);
+          tma_load_2d(st, wr.map, (w0.kb_begin + i) * kTileKBytes, wr.row, &ctl->full[i]);
         }
       }
       __syncwarp();
@@ -391,6 +407,7 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       const WorkItem wi = decode_work(p, w);
       if(skip_on && (wi.m_tile + 1) * TM <= p.skip_rows_below)
         continue;
+      const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, wi.n_tile * kTileN);
       const int a_row0 = p.seg_row0[p.nseg > 1 ? (wi.n_tile * kTileN) / p.seg_n : 0];
       for(int kb = wi.kb_begin; kb < wi.kb_end; ++kb, ++it) {
         const uint32_t s = it % T::kStages;
@@ -406,7 +423,7 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
           uint8_t* st = tiles + s * T::kStageBytes;
           if(!pre) {
             mbar_arrive_expect_tx(&ctl->full[s], kQuantA ? T::kWBytes : T::kStageBytes);
-            tma_load_2d(st, &tmap_w, kb * kTileKBytes, wi.n_tile * kTileN, &ctl->full[s]);
+            tma_load_2d(st, wr.map, kb * kTileKBytes, wr.row, &ctl->full[s]);
           }
           if(!kQuantA)
             tma_load_2d(st + T::kWBytes, &tmap_a, kb * kTileKBytes, a_row0 + wi.m_tile * TM, &ctl->full[s]);
@@ -739,9 +756,9 @@ mi8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       int p8_zp_b = 0, p8_off_b = 0;
       if constexpr(kP8) {
         if(n_ok) {
-          p8_scale_b = __ldg(p.p8_scale_b + n);
-          p8_zp_b = __ldg(p.p8_zp_b + n);
-          p8_off_b = __ldg(p.p8_off_b + n);
+          p8_scale_b = __ldg(p.p8_scale_b[seg] + n_loc);
+          p8_zp_b = __ldg(p.p8_zp_b[seg] + n_loc);
+          p8_off_b = __ldg(p.p8_off_b[seg] + n_loc);
         }
       }
       // Split-K: every split adds its partial accumulators into one int32 buffer per tile with
@@ -973,7 +990,7 @@ constexpr int smem_bytes_pair() { return PairCfg::kStages * PairCfg::kStageBytes
 
 template <bool kP8>
 __global__ void __launch_bounds__(kThreads, 1)
-mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
+mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
   using T = PairCfg;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;  // same in both CTAs
@@ -995,7 +1012,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   const unsigned long long trace_extra = static_cast<unsigned long long>(p.N) | (static_cast<unsigned long long>(p.K) << 20) |
                                          (static_cast<unsigned long long>(p.M) << 40);
   if(threadIdx.x == 0) {
-    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(weight_rows(tmap_w, p.nseg, p.seg_n, (2 * decode_work(p, pair_id).n_tile + static_cast<int>(rank)) * kTileN).map);
     tma_prefetch_desc(&tmap_a);
     for(int s = 0; s < T::kStages; ++s) {
       mbar_init(&ctl->full[s], 1);
@@ -1030,13 +1047,14 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     if(p.skip_a == nullptr && pair_id < p.total_work && p.withhold_item < 0) {
       // weights do not depend on the previous kernel: request the first pipeline fill before waiting for it
       const WorkItem w0 = decode_work(p, pair_id);
+      const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, (2 * w0.n_tile + static_cast<int>(rank)) * kTileN);
       const int n_pre = min(T::kStages, w0.kb_end - w0.kb_begin);
       if(elect_one()) {
         for(int i = 0; i < n_pre; ++i) {
           uint8_t* st = tiles + i * T::kStageBytes;
           if(leader)
             mbar_arrive_expect_tx(&ctl->full[i], 2 * T::kStageBytes);
-          tma_load_2d_pair(st, &tmap_w, (w0.kb_begin + i) * kTileKBytes, (2 * w0.n_tile + static_cast<int>(rank)) * kTileN, full_addr(i));
+          tma_load_2d_pair(st, wr.map, (w0.kb_begin + i) * kTileKBytes, wr.row, full_addr(i));
         }
       }
       __syncwarp();
@@ -1051,6 +1069,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       if(skip_on && (wi.m_tile + 1) * T::kTM <= p.skip_rows_below)
         continue;
       // (both CTAs' weight rows lie in one segment, or all segments share the activation: launch_gemm_call sees to it)
+      const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, (2 * wi.n_tile + static_cast<int>(rank)) * kTileN);
       const int a_row0 = p.seg_row0[p.nseg > 1 ? (2 * wi.n_tile * kTileN) / p.seg_n : 0];
       for(int kb = wi.kb_begin; kb < wi.kb_end; ++kb, ++it) {
         const uint32_t s = it % T::kStages;
@@ -1066,7 +1085,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
           if(!pre) {
             if(leader)
               mbar_arrive_expect_tx(&ctl->full[s], 2 * T::kStageBytes);
-            tma_load_2d_pair(st, &tmap_w, kb * kTileKBytes, (2 * wi.n_tile + static_cast<int>(rank)) * kTileN, full_addr(s));
+            tma_load_2d_pair(st, wr.map, kb * kTileKBytes, wr.row, full_addr(s));
           }
           tma_load_2d_pair(st + T::kWBytes, &tmap_a, kb * kTileKBytes,
                            a_row0 + wi.m_tile * T::kTM + static_cast<int>(rank) * T::kHalfRows, full_addr(s));
@@ -1189,9 +1208,9 @@ mi8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       int p8_zp_b = 0, p8_off_b = 0;
       if constexpr(kP8) {
         if(n_ok) {
-          p8_scale_b = __ldg(p.p8_scale_b + n);
-          p8_zp_b = __ldg(p.p8_zp_b + n);
-          p8_off_b = __ldg(p.p8_off_b + n);
+          p8_scale_b = __ldg(p.p8_scale_b[seg] + n_loc);
+          p8_zp_b = __ldg(p.p8_zp_b[seg] + n_loc);
+          p8_off_b = __ldg(p.p8_off_b[seg] + n_loc);
         }
       }
       unsigned out_max = 0u;
@@ -1849,7 +1868,7 @@ void single_segment(GemmParams& p) {
 }
 
 template <int TM, bool kQuantA = false, int kTopK = 0, bool kP8 = false, bool kBlocks = false>
-int launch_cfg(const CUtensorMap& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
+int launch_cfg(const WeightMaps<kP8>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1884,7 +1903,7 @@ int launch_cfg(const CUtensorMap& tw, const CUtensorMap& ta, const GemmParams& p
 }
 
 // Launch of kDuo: clusters of two CTAs, one tile each.
-int launch_duo(const CUtensorMap& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
+int launch_duo(const WeightMaps<false>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1938,7 +1957,7 @@ int launch_duo(const CUtensorMap& tw, const CUtensorMap& ta, const GemmParams& p
 
 // Launch of the CTA-pair kernel: clusters of two CTAs, as many as can be resident at once.
 template <bool kP8 = false>
-int launch_pair(const CUtensorMap& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
+int launch_pair(const WeightMaps<kP8>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
   static bool attr_set[64] = {};
   static int max_clusters[64] = {};
   int dev = 0;
@@ -2241,8 +2260,9 @@ int launch_gemm_call(const GemmCall& g) {
   GemmPlan duo;
   if(!blocks && g.skip_a == nullptr && M > 64 && K > 15 * kTileKBytes && make_gemm_plan(M, N, K, g.force_tile_m, g.force_splits, &duo, true) == MI8_OK && duo.duo)
     plan = duo;
-  CUtensorMap tw, ta;
-  rc = get_kmajor_map(&tw, g.bt, N, K, kTileN);
+  WeightMaps<false> tw;
+  CUtensorMap ta;
+  rc = get_kmajor_map(&tw.map[0], g.bt, N, K, kTileN);
   if(rc != MI8_OK)
     return rc;
   rc = get_kmajor_map(&ta, g.aq, g.a_rows_cap > M ? g.a_rows_cap : M, K, plan.pair ? PairCfg::kHalfRows : plan.tile_m);
@@ -2283,8 +2303,8 @@ int launch_gemm_call(const GemmCall& g) {
   p.skip_a = g.skip_a;
   p.skip_b = g.skip_b;
   p.skip_rows_below = g.skip_rows_below;
-  p.p8_scale_a = p.p8_scale_b = nullptr;
-  p.p8_zp_a = p.p8_sum_a = p.p8_zp_b = p.p8_off_b = nullptr;
+  p.p8_scale_a = nullptr;
+  p.p8_zp_a = p.p8_sum_a = nullptr;
   p.status = device_status_ptr();
   if(p.status == nullptr)
     return MI8_ERR_LAUNCH;
@@ -2508,27 +2528,33 @@ int launch_gemm_cq(const CqCall& g) {
 // split-K machinery are the same, only the operand signedness and the write-back differ.
 int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a, const int32_t* sum_a, const int8_t* bt,
                    const float* scale_b, const int32_t* zp_b, const int32_t* off_b, int M, int N, int K, const float* bias, int relu,
-                   float* c, int32_t* acc_out, void* ws, size_t ws_bytes, cudaStream_t stream, int force_tile_m, int force_splits, int nseg,
-                   float* const* seg_c, const float* const* seg_bias, float* block_max, float* block_sum) {
+                   float* c, int32_t* acc_out, void* ws, size_t ws_bytes, cudaStream_t stream, int force_tile_m, int force_splits,
+                   const P8Segments* segs, float* block_max, float* block_sum) {
   const bool blocks = block_max != nullptr;
-  if(blocks && (M > kBlockRows || block_sum == nullptr || nseg != 1 || relu || acc_out != nullptr || force_tile_m != 0))
+  if(blocks && (M > kBlockRows || block_sum == nullptr || segs != nullptr || relu || acc_out != nullptr || force_tile_m != 0))
     return MI8_ERR_UNSUPPORTED;
   if(blocks) {
     force_tile_m = M <= 16 ? 16 : 32;
     force_splits = 1;
   }
-  if(nseg < 1 || nseg > kMaxSegments || (nseg > 1 && (seg_c == nullptr || seg_bias == nullptr || N % nseg != 0 || (N / nseg) % kTileN != 0 || acc_out != nullptr)))
+  const P8Segments one{1, {bt}, {scale_b}, {zp_b}, {off_b}, {bias}, {c}};
+  const P8Segments& sg = segs != nullptr ? *segs : one;
+  const int nseg = sg.n;
+  if(nseg < 1 || nseg > kMaxSegments || (nseg > 1 && (N % nseg != 0 || (N / nseg) % kTileN != 0 || acc_out != nullptr)))
     return MI8_ERR_BAD_ARG;
-  if(nseg > 1)
-    c = seg_c[0];
   if(M < 0 || N <= 0 || K <= 0 || force_tile_m < 0 || force_splits < 0)
     return MI8_ERR_BAD_ARG;
   if(M == 0)
     return MI8_OK;
-  if(aq == nullptr || bt == nullptr || c == nullptr || scale_a == nullptr || zp_a == nullptr || sum_a == nullptr || scale_b == nullptr
-     || zp_b == nullptr || off_b == nullptr)
+  if(aq == nullptr || scale_a == nullptr || zp_a == nullptr || sum_a == nullptr)
     return MI8_ERR_BAD_ARG;
-  if(K % 16 != 0 || (reinterpret_cast<uintptr_t>(aq) & 15u) || (reinterpret_cast<uintptr_t>(bt) & 15u))
+  uintptr_t addresses = reinterpret_cast<uintptr_t>(aq);
+  for(int i = 0; i < nseg; ++i) {
+    if(sg.bt[i] == nullptr || sg.c[i] == nullptr || sg.scale_b[i] == nullptr || sg.zp_b[i] == nullptr || sg.off_b[i] == nullptr)
+      return MI8_ERR_BAD_ARG;
+    addresses |= reinterpret_cast<uintptr_t>(sg.bt[i]);
+  }
+  if(K % 16 != 0 || (addresses & 15u))
     return MI8_ERR_MISALIGNED;
   if((reinterpret_cast<uintptr_t>(scale_a) & 15u) || (reinterpret_cast<uintptr_t>(zp_a) & 15u) || (reinterpret_cast<uintptr_t>(sum_a) & 15u))
     return MI8_ERR_MISALIGNED;   // the write-back reads the per-row arrays four rows at a time
@@ -2538,10 +2564,13 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
     return rc;
   if(plan.splits > 1 && (ws == nullptr || ws_bytes < kWsHeaderBytes + plan.partial_bytes))
     return MI8_ERR_WORKSPACE;
-  CUtensorMap tw, ta;
-  rc = get_kmajor_map(&tw, bt, N, K, kTileN);
-  if(rc != MI8_OK)
-    return rc;
+  WeightMaps<true> tw{};
+  CUtensorMap ta;
+  for(int i = 0; i < nseg; ++i) {
+    rc = get_kmajor_map(&tw.map[i], sg.bt[i], N / nseg, K, kTileN);
+    if(rc != MI8_OK)
+      return rc;
+  }
   rc = get_kmajor_map(&ta, reinterpret_cast<const int8_t*>(aq), M, K, plan.pair ? PairCfg::kHalfRows : plan.tile_m);
   if(rc != MI8_OK)
     return rc;
@@ -2556,9 +2585,9 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
   p.kb_per_split = plan.kb_per_split;
   p.total_work = plan.n_tiles * plan.m_tiles * plan.splits;
   p.scale = 1.0f;
-  p.bias = bias;
+  p.bias = sg.bias[0];
   p.relu = relu ? 1 : 0;
-  p.c = c;
+  p.c = sg.c[0];
   p.acc_out = acc_out;
   uint8_t* wsb = static_cast<uint8_t*>(ws);
   p.partials = wsb ? reinterpret_cast<int32_t*>(wsb + kWsOffPartials) : nullptr;
@@ -2566,18 +2595,18 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
   p.p8_scale_a = scale_a;
   p.p8_zp_a = zp_a;
   p.p8_sum_a = sum_a;
-  p.p8_scale_b = scale_b;
-  p.p8_zp_b = zp_b;
-  p.p8_off_b = off_b;
   p.status = device_status_ptr();
   if(p.status == nullptr)
     return MI8_ERR_LAUNCH;
   single_segment(p);
   p.nseg = nseg;
   p.seg_n = N / nseg;
-  for(int i = 0; i < nseg && nseg > 1; ++i) {
-    p.seg_bias[i] = seg_bias[i];
-    p.seg_c[i] = seg_c[i];
+  for(int i = 0; i < nseg; ++i) {
+    p.p8_scale_b[i] = sg.scale_b[i];
+    p.p8_zp_b[i] = sg.zp_b[i];
+    p.p8_off_b[i] = sg.off_b[i];
+    p.seg_bias[i] = sg.bias[i];
+    p.seg_c[i] = sg.c[i];
   }
   finish_params(p);
   if(blocks) {
@@ -2630,8 +2659,8 @@ int launch_gemm_quant_a(const float* a_f32, const unsigned* a_slot, float* qa_ou
   int rc = make_gemm_plan(M, N, K, tm, 1, &plan);
   if(rc != MI8_OK)
     return rc;
-  CUtensorMap tw;
-  rc = get_kmajor_map(&tw, bt, N, K, kTileN);
+  WeightMaps<false> tw;
+  rc = get_kmajor_map(&tw.map[0], bt, N, K, kTileN);
   if(rc != MI8_OK)
     return rc;
   GemmParams p;
@@ -2671,9 +2700,9 @@ int launch_gemm_quant_a(const float* a_f32, const unsigned* a_slot, float* qa_ou
   single_segment(p);
   finish_params(p);
   switch(tm) {   // the weight map stands in for the unused activation map
-    case 16: return launch_cfg<16, true>(tw, tw, p, plan, stream);
-    case 32: return launch_cfg<32, true>(tw, tw, p, plan, stream);
-    default: return launch_cfg<64, true>(tw, tw, p, plan, stream);
+    case 16: return launch_cfg<16, true>(tw, tw.map[0], p, plan, stream);
+    case 32: return launch_cfg<32, true>(tw, tw.map[0], p, plan, stream);
+    default: return launch_cfg<64, true>(tw, tw.map[0], p, plan, stream);
   }
 }
 
@@ -2699,8 +2728,9 @@ int launch_gemm_logits(const int8_t* aq, const float* d_qa, const int8_t* wq, co
   int rc = make_gemm_plan(vocab, rows, K, 256, 1, &plan);
   if(rc != MI8_OK)
     return rc;
-  CUtensorMap tw, ta;
-  rc = get_kmajor_map(&tw, aq, rows, K, kTileN);
+  WeightMaps<false> tw;
+  CUtensorMap ta;
+  rc = get_kmajor_map(&tw.map[0], aq, rows, K, kTileN);
   if(rc != MI8_OK)
     return rc;
   rc = get_kmajor_map(&ta, wq, vocab, K, 256);

@@ -156,16 +156,24 @@ bool gemm_cq_supported(int M, int N, int K, bool ln);
 int launch_gemm_cq(const CqCall& g);
 
 // packed8avx512 scheme (mi8_packed8.cu, mi8_gemm.cu): weight item back to Bt[N,K]; per-row uint8 quantisation of
-// the activation; uint8 x int8 GEMM whose write-back applies the zero points, the scales and the bias (nseg > 1: matrices of N / nseg
-// columns one behind the other, their columns' parameters too, each with an output and a bias of its own; block_max / block_sum: as
-// in GemmCall).
+// the activation; uint8 x int8 GEMM whose write-back applies the zero points, the scales and the bias.  `segs`: several matrices of N / n columns
+// each in the place of the one that the arguments name; block_max / block_sum: as in GemmCall.
+constexpr int kMaxSegments = 3;
+struct P8Segments {
+  int n = 0;
+  const int8_t* bt[kMaxSegments];
+  const float* scale_b[kMaxSegments];
+  const int32_t *zp_b[kMaxSegments], *off_b[kMaxSegments];
+  const float* bias[kMaxSegments];
+  float* c[kMaxSegments];
+};
 int launch_p8_prepare_b(const float* w, int K, int N, int8_t* packed, cudaStream_t stream);
 int launch_p8_unpack_bt(const int8_t* packed, int K, int N, int8_t* bt, cudaStream_t stream);
 int launch_p8_quantize_rows(const float* a, int M, int K, uint8_t* aq, float* scale_a, int32_t* zp_a, int32_t* sum_a, cudaStream_t stream);
 int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a, const int32_t* sum_a, const int8_t* bt,
                    const float* scale_b, const int32_t* zp_b, const int32_t* off_b, int M, int N, int K, const float* bias, int relu,
-                   float* c, int32_t* acc_out, void* ws, size_t ws_bytes, cudaStream_t stream, int force_tile_m, int force_splits, int nseg = 1,
-                   float* const* seg_c = nullptr, const float* const* seg_bias = nullptr, float* block_max = nullptr, float* block_sum = nullptr);
+                   float* c, int32_t* acc_out, void* ws, size_t ws_bytes, cudaStream_t stream, int force_tile_m, int force_splits,
+                   const P8Segments* segs = nullptr, float* block_max = nullptr, float* block_sum = nullptr);
 
 // What the last kernel of a decoder step does besides the rows' candidates: the n-best lists of the sentences (arrivals != nullptr; one
 // zeroed counter per sentence; the outputs may be pinned host memory) and the record of the history abs-max per layer (layers > 0).

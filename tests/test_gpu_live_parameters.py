@@ -32,7 +32,7 @@ def _search(net, stepper, beam, ids, mask):
 
 def _models(cuda_device, scheme, rnn, dim):
     from marian_dev_b200 import decoder, model
-    cfg = model.TransformerConfig(dim_emb=dim, dim_ffn=2 * dim, heads=8, enc_depth=1, dec_depth=2, vocab=1024,
+    cfg = model.TransformerConfig(dim_emb=dim, dim_ffn=2 * dim, heads=8 if dim <= 512 else dim // 64, enc_depth=1, dec_depth=2, vocab=1024,
                                   decoder_autoreg="rnn" if rnn else "self-attention")
     nets = []
     for seed in (3, 4):
@@ -80,3 +80,22 @@ def test_parameters_at_any_float_address(cuda_device):
             check(lib().mi8d_set_param(stepper.h, name.encode(), room[1:].data_ptr()))
     assert len(moved) > 8
     assert _search(net, stepper, 2, ids, mask) == want
+
+
+# packed8avx512: matrices that share a launch stay where they are, with their columns' scales, zero points and offsets (a tile per CTA and the CTA-pair
+# kernel: the encoder of 40 sentences x 50 tokens; an odd number of weight tiles)
+@pytest.mark.parametrize("dim,rnn,batch,beam,longest", [(256, True, 3, 1, 9), (256, False, 4, 2, 9), (256, False, 40, 1, 49), (768, False, 60, 1, 49)])
+def test_packed8_rewritten_in_place(cuda_device, dim, rnn, batch, beam, longest):
+    cfg, (net, other) = _models(cuda_device, "packed8avx512", rnn, dim)
+    ids, mask = _batch(cfg, batch, longest, batch)
+    stepper = _stepper(net, batch, beam, longest)
+    before = _search(net, stepper, beam, ids, mask)
+    for name, p in net.p.items():
+        if name != "Wemb":
+            p.copy_(other.p[name])
+    for name, w in net.w.items():
+        w.item.copy_(other.w[name].item)          # (scales, zero points and offsets are its tail)
+        w.bt.copy_(other.w[name].bt)
+    after = _search(net, stepper, beam, ids, mask)
+    assert after != before
+    assert after == _search(net, _stepper(net, batch, beam, longest), beam, ids, mask)
