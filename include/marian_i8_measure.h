@@ -71,8 +71,11 @@ int mi8_trace_end(void);
  * `withhold_item` (0 = its first 128-byte K block), so the roles waiting for those bytes give up after
  * `spin_limit` polls (0 = the default of about a million), raise a status word 101..104 (mi8_poll_status),
  * drain what is in flight, release their tensor memory and return; the output of such a launch is undefined.
+ * withhold_item == MI8_TEST_ONE_WARP: instead, one of the eight write-back warps of every CTA of the GEMMs gives up its wait for the
+ * first accumulator while the others do not.
  * mi8_test_wait_fault(-1, 0) restores normal operation; afterwards mi8_workspace_init + mi8_clear_status make
  * the next call exact again.  Process-wide; not for use beside production calls. */
+#define MI8_TEST_ONE_WARP (-2)
 void mi8_test_wait_fault(int withhold_item, unsigned spin_limit);
 
 /* Host-side timing of mi8d_search (marian_i8_decode.h), accumulated per decoder since the last reset:

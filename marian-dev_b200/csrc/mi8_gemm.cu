@@ -42,6 +42,7 @@ constexpr int kMmaK = 32;       // K per tcgen05.mma kind::i8
 constexpr int kThreads = 320;
 constexpr int kEpilogueThreads = 256;
 constexpr int kMaxStages = 8;
+constexpr int kWithholdWarp = MI8_TEST_ONE_WARP;
 constexpr int kPairTileCode = 512;  // force_tile_m value that selects the CTA-pair kernel
 
 template <int TM>
@@ -128,9 +129,26 @@ struct GemmParams {
   const float* seg_bias[kMaxSegments];
   void* seg_c[kMaxSegments];
   int* rows_computed;       // optional (measurement): receives the number of activation rows this launch really computed
-  int withhold_item;        // test hook: the producer leaves out the loads of this pipeline item (-1 = none)
+  int withhold_item;        // test hook: the producer leaves out the loads of this pipeline item (-1 = none; or kWithholdWarp)
   uint32_t spin_limit;      // bound of every barrier wait of this launch
 };
+
+// Named barrier at which the threads also agree: true in all of them when `ok` held in all of them.  (A write-back warp whose bounded wait ran
+// out must not leave the others behind at a barrier, which has no bound: it arrives too, and all leave the loop together.)
+__device__ __forceinline__ bool named_bar_all(int id, int count, bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, %2, %3, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all)
+      : "r"(static_cast<uint32_t>(ok)), "r"(id), "r"(count)
+      : "memory");
+  return all != 0;
+}
+// Bound of a write-back warp's wait for its accumulator (test hook: one warp of every CTA gives up at once).
+__device__ __forceinline__ uint32_t accumulator_limit(const GemmParams& p, int warp) { return p.withhold_item == kWithholdWarp && warp == 3 ? 0u : p.spin_limit; }
 
 template <bool kP8>
 struct WeightMaps {
@@ -595,10 +613,13 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
       const uint32_t as = acc_it & 1u;
       const uint32_t aph = (acc_it >> 1) & 1u;
       if(lane == 0)
-        ok = mbar_wait_bounded(&ctl->tmem_full[as], aph, abort_flag, p.spin_limit);
+        ok = mbar_wait_bounded(&ctl->tmem_full[as], aph, abort_flag, accumulator_limit(p, warp));
       ok = __shfl_sync(0xffffffffu, ok, 0);
-      if(!ok)
+      if(!ok) {
+        if(!kDuo && (kBlocks || p.splits > 1))   // (the tile's first barrier)
+          named_bar_all(1, kEpilogueThreads, false);
         break;
+      }
       tc_fence_after_sync();
 
       const uint32_t t_addr = tmem_base + as * T::kAccStride + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -781,7 +802,9 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
           }
         }
         __threadfence();
-        named_bar_sync(1, kEpilogueThreads);
+        ok = named_bar_all(1, kEpilogueThreads, true);
+        if(!ok)
+          break;
         if(epi_tid == 0) {
           const unsigned old = atomicAdd(&p.tile_counters[wi.tile], 1u);
           const int last = (old == static_cast<unsigned>(p.splits - 1)) ? 1 : 0;
@@ -824,7 +847,9 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
         tc_fence_before_sync();
         mbar_arrive(&ctl->tmem_empty[as]);
         ++acc_it;
-        named_bar_sync(1, kEpilogueThreads);
+        ok = named_bar_all(1, kEpilogueThreads, true);
+        if(!ok)
+          break;
         const int block_cols = min(kTileN, p.N - wi.n_tile * kTileN);
         for(int j = warp - 2; j < cols_valid; j += kEpilogueThreads / 32) {
           float4* at = reinterpret_cast<float4*>(parked + j * kLogitPitch) + lane;
@@ -1180,10 +1205,12 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __gri
       const uint32_t as = acc_it & 1u;
       const uint32_t aph = (acc_it >> 1) & 1u;
       if(lane == 0)
-        ok = mbar_wait_bounded(&ctl->tmem_full[as], aph, abort_flag, p.spin_limit);
+        ok = mbar_wait_bounded(&ctl->tmem_full[as], aph, abort_flag, accumulator_limit(p, warp));
       ok = __shfl_sync(0xffffffffu, ok, 0);
-      if(!ok)
+      if(!ok) {
+        named_bar_all(1, kEpilogueThreads, false);   // (the tile's barrier)
         break;
+      }
       tc_fence_after_sync();
 
       const uint32_t t_addr = tmem_base + as * T::kAccStride + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -1238,7 +1265,9 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __gri
       }
       // hand the accumulator buffer back: all epilogue warps of this CTA meet, then one arrival per CTA
       tc_fence_before_sync();
-      named_bar_sync(1, kEpilogueThreads);
+      ok = named_bar_all(1, kEpilogueThreads, true);
+      if(!ok)
+        break;
       if(epi_tid == 0)
         mbar_arrive_cluster(mapa_shared(smem_u32(&ctl->tmem_empty[as]), 0u));
       ++acc_it;
