@@ -66,13 +66,13 @@ void mi8_launch_count_reset(void);
 int mi8_trace_begin(unsigned long long* device_buf, int capacity);
 int mi8_trace_end(void);
 
-/* Test aid: makes a bounded wait inside the GEMM kernels run out on purpose, without faulting anything.
+/* Test aid: makes a bounded wait inside the GEMM kernels and decoder_rows_kernel run out on purpose, without faulting anything.
  * While withhold_item >= 0, every CTA's TMA producer leaves out the loads of its pipeline item number
- * `withhold_item` (0 = its first 128-byte K block), so the roles waiting for those bytes give up after
+ * `withhold_item` (0 = its first 128-byte K block; decoder_rows_kernel: every warp's unit of that number), so the roles waiting for those bytes give up after
  * `spin_limit` polls (0 = the default of about a million), raise a status word 101..104 (mi8_poll_status),
  * drain what is in flight, release their tensor memory and return; the output of such a launch is undefined.
  * withhold_item == MI8_TEST_ONE_WARP: instead, one of the eight write-back warps of every CTA of the GEMMs gives up its wait for the
- * first accumulator while the others do not.
+ * first accumulator (decoder_rows_kernel: one warp its waits for weights) while the others do not.
  * mi8_test_wait_fault(-1, 0) restores normal operation; afterwards mi8_workspace_init + mi8_clear_status make
  * the next call exact again.  Process-wide; not for use beside production calls. */
 #define MI8_TEST_ONE_WARP (-2)

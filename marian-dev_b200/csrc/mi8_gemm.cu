@@ -42,7 +42,6 @@ constexpr int kMmaK = 32;       // K per tcgen05.mma kind::i8
 constexpr int kThreads = 320;
 constexpr int kEpilogueThreads = 256;
 constexpr int kMaxStages = 8;
-constexpr int kWithholdWarp = MI8_TEST_ONE_WARP;
 constexpr int kPairTileCode = 512;  // force_tile_m value that selects the CTA-pair kernel
 
 template <int TM>
@@ -1878,8 +1877,7 @@ thread_local ProfileState t_profile;
 
 // Fields every launcher sets the same way.
 void finish_params(GemmParams& p) {
-  p.withhold_item = g_test_withhold_item;
-  p.spin_limit = g_test_spin_limit != 0 ? g_test_spin_limit : kSpinLimit;
+  test_wait_limits(&p.withhold_item, &p.spin_limit);
   p.rows_computed = nullptr;
   if(t_profile.on && t_profile.d_rows != nullptr && t_profile.records.size() < t_profile.capacity)
     p.rows_computed = t_profile.d_rows + t_profile.records.size();
@@ -2061,6 +2059,10 @@ MI8_DEFINE_TRACE_SETTER(trace_set_gemm)
 
 int rows_weight_map(CUtensorMap* map, const int8_t* bt, int N, int K) { return encode_kmajor_map(map, bt, N, K, 16); }
 
+void test_wait_limits(int* withhold_item, uint32_t* spin_limit) {
+  *withhold_item = g_test_withhold_item;
+  *spin_limit = g_test_spin_limit != 0 ? g_test_spin_limit : kSpinLimit;
+}
 void test_wait_fault(int withhold_item, unsigned spin_limit) {
   g_test_withhold_item = withhold_item;
   g_test_spin_limit = spin_limit;
@@ -2537,8 +2539,7 @@ int launch_gemm_cq(const CqCall& g) {
   p.ln_slot = g.ln_slot;
   p.ln_slot2 = g.ln_slot2;
   p.status = device_status_ptr();
-  p.withhold_item = g_test_withhold_item;
-  p.spin_limit = g_test_spin_limit != 0 ? g_test_spin_limit : kSpinLimit;
+  test_wait_limits(&p.withhold_item, &p.spin_limit);
   p.rows_computed = nullptr;
   if(t_profile.on && t_profile.d_rows != nullptr && t_profile.records.size() < t_profile.capacity)
     p.rows_computed = t_profile.d_rows + t_profile.records.size();

@@ -276,7 +276,9 @@ struct DecoderRowsParams {
   int8_t* out_q = nullptr;      // [rows, d] the last LayerNorm's result, quantised, and its multiplier
   float* out_qm = nullptr;
   int* status = nullptr;
-  int ring = 0, inv_mt_ffn1 = 0, inv_nf4 = 0, inv_batch = 0, inv_rows = 0;   // set by the launcher (as `status`)
+  int withhold_item = -1;       // (test hook, as in the GEMMs; `status`, these two and the next line are set by the launcher)
+  uint32_t spin_limit = 0;
+  int ring = 0, inv_mt_ffn1 = 0, inv_nf4 = 0, inv_batch = 0, inv_rows = 0;
   // n_ctrl > 0: the control words (hypothesis rows, previous words, path scores, batch rows), used from here and brought to `ctrl`
   int ctrl_words[4 * kDecoderRowsMax];
   DecoderRowsVectors vec[kDecoderRowsLayers];
@@ -284,6 +286,9 @@ struct DecoderRowsParams {
   CUtensorMap map[kDecoderRowsLayers][5];
 };
 static_assert(sizeof(DecoderRowsParams) <= 4096, "kernel parameters");
+// What mi8_test_wait_fault asked for: the item whose loads are left out (-1: none; kWithholdWarp) and the bound of every wait.
+constexpr int kWithholdWarp = MI8_TEST_ONE_WARP;
+void test_wait_limits(int* withhold_item, uint32_t* spin_limit);
 int rows_weight_map(CUtensorMap* map, const int8_t* bt, int N, int K);
 bool decoder_rows_supported(int rows, int d, int f, int heads, int layers, int src);
 int launch_decoder_rows(DecoderRowsParams& p, int d, int heads, cudaStream_t stream);

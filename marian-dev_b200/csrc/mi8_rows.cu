@@ -230,7 +230,9 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
       }
     }
   }
-  auto request = [&](int slot) {   // by the lane that knows the unit
+  auto request = [&](int slot) {   // by the lane that knows the unit (test hook: a withheld unit never arrives)
+    if(lane == p.withhold_item)
+      return;
     mbar_arrive_expect_tx(&full[warp][slot], kUnitBytes);
     tma_load_2d(ring + (warp * ring_n + slot) * kUnitBytes, my_map, (my_unit >> 16) * 128, my_row, &full[warp][slot]);
   };
@@ -264,9 +266,10 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
         break;
       const int mt = (unit >> 8) & 0xff, kb = unit >> 16;
       if(ok)
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[warp][slot], parity, abort_flag));
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[warp][slot], parity, abort_flag,
+                                                     p.withhold_item == kWithholdWarp && warp == 3 ? 0u : p.spin_limit));   // (test hook: one warp gives up at once)
       if(!ok) {
-        if(lane == 0 && !*abort_flag) {
+        if(lane == 0) {
           *abort_flag = 1;
           atomicMax(p.status, static_cast<int>(kDevTimeoutMma));
         }
@@ -690,7 +693,7 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
   }
   if(!ok)   // (a wait ran out: no copy may land after the CTA has gone)
     for(int no_abort = 0; used < requested; ++used)
-      mbar_wait_bounded(&full[warp][used % ring_n], (used / ring_n) & 1, &no_abort);
+      mbar_wait_bounded(&full[warp][used % ring_n], (used / ring_n) & 1, &no_abort, p.spin_limit);
   // ---- the output layer's operand
 #pragma unroll
   for(int i = 0; i < kRw; ++i) {
@@ -802,6 +805,7 @@ bool decoder_rows_supported(int rows, int d, int f, int heads, int layers, int s
 int launch_decoder_rows(DecoderRowsParams& p, int d, int heads, cudaStream_t stream) {
   if(!decoder_rows_supported(p.rows, d, p.ffn, heads, p.layers, p.src))
     return MI8_ERR_UNSUPPORTED;
+  test_wait_limits(&p.withhold_item, &p.spin_limit);
   p.status = device_status_ptr();
   if(p.status == nullptr)
     return MI8_ERR_LAUNCH;

@@ -55,8 +55,11 @@ def test_multiply(cuda_device, oracle, m, k, n, tile, kind):
 
 
 # the first step of up to 32 rows: its output layer reduces the blocks of the log-softmax at such barriers (tiles of 16 and of 32 rows, both schemes)
+# the first step of a few rows of an SSRU decoder: the cluster launch of all layers, one warp giving up or a unit of every warp's weights never arriving (with
+# and without units behind it that are waited for before the CTA leaves)
 @pytest.mark.parametrize("scheme,rnn,rows,items", [("intgemm8", False, 3, (ONE_WARP,)), ("intgemm8", False, 20, (ONE_WARP,)),
-                                                   ("packed8avx512", False, 5, (ONE_WARP,))])
+                                                   ("packed8avx512", False, 5, (ONE_WARP,)), ("intgemm8", True, 1, (ONE_WARP, 0, 1)),
+                                                   ("intgemm8", True, 30, (ONE_WARP, 2))])
 def test_decoder_step(cuda_device, scheme, rnn, rows, items):
     from marian_dev_b200 import decoder, model, ops
     from marian_dev_b200.binding import lib
@@ -74,6 +77,11 @@ def test_decoder_step(cuda_device, scheme, rnn, rows, items):
         return stepper.step(None, None, None, None, 1, rows, 2)
     want = first_step()
     assert ops.poll_status() == 0
+    if rnn:                                           # (all layers in one launch)
+        first_step()
+        L.mi8_launch_count_reset()
+        first_step()
+        assert L.mi8_launch_count() < 12
     for item in items:
         try:
             L.mi8_test_wait_fault(item, 1 << 14)
