@@ -31,10 +31,11 @@ def test_packed8_model_decodes_like_the_checker(cuda_device, cfg_name, beam, upl
     batches = model.make_batches(corpus, 18)
     items = _items(cfg, params)
     ref = OracleTransformer(cfg, params, threads=8, scheme="packed8avx512", packed_items=items)
-    want = {}
+    want, scores = {}, {}
     for sent_ids, ids, mask in batches:
-        for s, (toks, _s) in zip(sent_ids, beam_search(ref, ids, mask, beam=beam)):
+        for s, (toks, score) in zip(sent_ids, beam_search(ref, ids, mask, beam=beam)):
             want[int(s)] = toks
+            scores[int(s)] = np.float32(score)
     if upload_items:      # the model as read from a converted file: the same item bytes on both sides
         gpu_params = {k: v for k, v in params.items() if k not in items}
         gpu_params.update({k: packed8.Packed8Weight(it.packed, it.K, it.N, device=cuda_device) for k, it in items.items()})
@@ -48,6 +49,9 @@ def test_packed8_model_decodes_like_the_checker(cuda_device, cfg_name, beam, upl
     assert min(lens) < max(lens)
     diff = [k for k in want if want[k] != got[k]]
     assert not diff, f"{cfg_name} beam {beam}: {len(diff)} of {len(want)} sentences differ"
+    for sent_ids, ids, mask in batches:
+        res = decoder.BeamSearch(gpu, beam, native=stepper).search(ids, mask)
+        assert [np.float32(score) for _t, score in res] == [scores[int(s)] for s in sent_ids]
 
 
 def test_mixing_schemes_is_refused(cuda_device):
