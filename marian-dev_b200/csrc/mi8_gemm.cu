@@ -950,15 +950,9 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
       const float* seg_bias = p.seg_bias[seg];
       const int ldc = p.seg_n, m0 = wi.m_tile * TM + group * T::kChunk;
       const bool paired = p.out_f16 && (ldc & 1) == 0 && (reinterpret_cast<uintptr_t>(p.seg_c[seg]) & 3u) == 0 && __all_sync(0xffffffffu, n_ok);
-      unsigned out_max = 0u;
       if(n_ok)
-        out_max = write_back_chunk<T::kChunk>(p, v, static_cast<size_t>(m0) * ldc + n_loc, p.M - m0, unquant, seg_bias != nullptr ? __ldg(seg_bias + n_loc) : 0.0f,
-                                              out_max, p.seg_c[seg], ldc, seg_bias != nullptr, paired);
-      if(p.absmax_out != nullptr) {
-        out_max = __reduce_max_sync(0xffffffffu, out_max);
-        if(lane == 0 && out_max != 0u)
-          atomicMax(p.absmax_out, out_max);
-      }
+        write_back_chunk<T::kChunk>(p, v, static_cast<size_t>(m0) * ldc + n_loc, p.M - m0, unquant, seg_bias != nullptr ? __ldg(seg_bias + n_loc) : 0.0f, 0u,
+                                    p.seg_c[seg], ldc, seg_bias != nullptr, paired);
     }
   }
 
@@ -2287,9 +2281,10 @@ int launch_gemm_call(const GemmCall& g) {
     if(g.ws == nullptr || g.ws_bytes < kWsHeaderBytes + plan.partial_bytes)
       return MI8_ERR_WORKSPACE;
   }
-  // (after the check above: a call without the workspace that the other plan needs stays refused)
+  // (after the check above: a call without the workspace that the other plan needs stays refused.  No caller wants max|C| of such a product.)
   GemmPlan duo;
-  if(!blocks && g.skip_a == nullptr && M > 64 && K > 15 * kTileKBytes && make_gemm_plan(M, N, K, g.force_tile_m, g.force_splits, &duo, true) == MI8_OK && duo.duo)
+  if(!blocks && g.skip_a == nullptr && g.absmax_out == nullptr && M > 64 && K > 15 * kTileKBytes &&
+     make_gemm_plan(M, N, K, g.force_tile_m, g.force_splits, &duo, true) == MI8_OK && duo.duo)
     plan = duo;
   WeightMaps<false> tw;
   CUtensorMap ta;

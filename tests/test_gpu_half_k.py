@@ -36,22 +36,3 @@ def test_half_of_k_per_cta(cuda_device, oracle, m, k, n, half, bias, relu):
 def test_several_matrices(cuda_device, oracle, m, k, n_each, count, half):
     from tests.test_gpu_multi_weight import _run
     _run(cuda_device, oracle, m, k, n_each, count, with_bias=True, relu=half, out_dtype=torch.float16 if half else torch.float32)
-
-
-def test_maximum_for_the_next_quantisation(cuda_device):
-    """The first feed-forward affine of a wide model also reduces max|h| (two CTAs per tile: 65 rows x 2048 x 2560); the same searches with
-    64-row tiles on one CTA each, and the same bits."""
-    from marian_dev_b200 import decoder, model, ops
-    cfg = model.TransformerConfig(dim_emb=2048, dim_ffn=2560, heads=32, enc_depth=1, dec_depth=2, vocab=515)
-    net = decoder.Int8Transformer(cfg, model.random_init(cfg, 7), cuda_device)
-    rng = np.random.default_rng(7)
-    ids = torch.from_numpy(rng.integers(4, cfg.vocab, size=(65, 6)))
-    ids[:, -1] = cfg.eos_id
-    results = []
-    for tile in (0, 64):
-        stepper = decoder.NativeStepper(net, max_batch=65, beam=1, max_src=6, max_steps=10)
-        stepper.set_option("gemm_tile_rows", tile)
-        res = decoder.BeamSearch(net, 1, 1.5, 1.0, native=stepper).search(ids, torch.ones(65, 6))
-        results.append([(list(t), np.float32(s)) for t, s in res])
-        assert ops.poll_status() == 0
-    assert results[0] == results[1]
