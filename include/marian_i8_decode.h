@@ -177,8 +177,10 @@ int mi8d_history_reuse(mi8d_decoder* d, unsigned out[2], int reset);
  *   MI8D_OPT_SIDE_STREAM (default 1): the re-projection of the earlier history slabs runs on an internal stream;
  *   MI8D_OPT_ATTENTION_UNROLL (8 or 16, default 8; process-wide): key/value rows a thread keeps in flight;
  *   MI8D_OPT_ATTENTION_BLOCK_HEADS (default 8, 0 = all; process-wide): heads one block of the decoder attention serves;
- *     a divisor of the head count splits every query row over several smaller blocks.  (Both: self-attention of one
- *     hypothesis or more than eight, and attention too long for the kernels that serve a sentence's hypotheses together;)
+ *     a divisor of the head count splits every query row over several smaller blocks.  (Both: where the next switch does not
+ *     apply, and attention too long for the kernels that serve a sentence's hypotheses together;)
+ *   MI8D_OPT_SHARED_HISTORY (default 1): the decoder's self-attention serves the hypotheses of a sentence together (two to four,
+ *     up to 32 sentences also five and six) and reads each distinct history row once; 0: every hypothesis reads its own;
  *   MI8D_OPT_CLUSTER_AFFINE (default 0): affines whose activation comes with an abs-max slot run as ONE launch of the
  *     cluster GEMM (mi8g_affine_slot) instead of a quantisation launch and a GEMM launch.  Off by default: 74 to 98
  *     launches per step of the transformer-big decoder, which then had 122 (113 now), but 5 to 20 % fewer tokens per second (the
@@ -208,7 +210,8 @@ enum mi8d_option {
   MI8D_OPT_CLUSTER_SIZE = 10,
   MI8D_OPT_CLUSTER_MAX_K = 11,
   MI8D_OPT_GEMM_TILE_ROWS = 12,
-  MI8D_OPT_BLOCKING_WAIT = 13
+  MI8D_OPT_BLOCKING_WAIT = 13,
+  MI8D_OPT_SHARED_HISTORY = 14
 };
 int mi8d_set_option(mi8d_decoder* d, int option, int value);   /* d may be NULL for the process-wide switches */
 

@@ -169,7 +169,7 @@ struct mi8d_decoder {
   int opt_blocking_wait = 0;
   bool overlap = false;
   // tuning switches (mi8d_set_option)
-  int opt_fuse = 1, opt_quant_in_gemm = 0, opt_fused_out_rows = 0, opt_side_stream = 1;
+  int opt_fuse = 1, opt_quant_in_gemm = 0, opt_fused_out_rows = 0, opt_side_stream = 1, opt_shared_history = 1;
   int opt_gemm_tile = 0;
   int opt_cluster = 0, opt_fused_ln = 1, opt_cluster_max_rows = 1024, opt_cluster_size = 0, opt_cluster_max_k = 2048;
   // host-side timing of mi8d_search
@@ -750,6 +750,7 @@ int mi8d_set_option(mi8d_decoder* d, int option, int value) {
     case MI8D_OPT_QUANT_IN_GEMM: d->opt_quant_in_gemm = value != 0; break;
     case MI8D_OPT_FUSED_OUTPUT_MAX_ROWS: d->opt_fused_out_rows = value; break;
     case MI8D_OPT_SIDE_STREAM: d->opt_side_stream = value != 0; break;
+    case MI8D_OPT_SHARED_HISTORY: d->opt_shared_history = value != 0; break;
     case MI8D_OPT_CLUSTER_AFFINE: d->opt_cluster = value != 0; break;
     case MI8D_OPT_FUSED_LAYERNORM: d->opt_fused_ln = value != 0; break;
     case MI8D_OPT_CLUSTER_MAX_ROWS: d->opt_cluster_max_rows = value; break;
@@ -1171,7 +1172,7 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
       rowmax[l] = d->layers[l].rowmax;
       hslot[l] = d->layer_slot(l, kSlotHistory);
     }
-    lists.batch = attention_hist_supported(beam, dm / c.heads, t + 1) ? batch : 0;
+    lists.batch = d->opt_shared_history && attention_hist_supported(beam, batch, dm / c.heads, t + 1) ? batch : 0;
     MI8D_TRY(launch_embed_ancestors(d->wemb, words, pos, emb_scale, dm, x, d->layers[0].rowmax + static_cast<size_t>(t) * SR, d->input_slot(0),
                                     d->layer_slot(0, kSlotHistory), d->anc[d->anc_cur], d->anc[anc_new], hyp_idx, t, R, SR, s,
                                     d->p8 ? 0 : c.dec_depth, rowmax, hslot, lists));

@@ -18,7 +18,8 @@ namespace {
 constexpr int kRowThreads = 256;
 constexpr int kMaxVec = 4;  // float4 per thread: rows of up to 4096 floats
 constexpr int kMaxHistLayers = 16;
-constexpr int kMaxHistBeams = 8;   // hypotheses of a sentence that attention_hist_kernel serves together
+constexpr int kMaxHistBeams = 6;   // hypotheses of a sentence that attention_hist_kernel serves together; from kHistBeams on for so many sentences only:
+constexpr int kHistBeams = 4, kMaxHistSentences = 32;
 
 __device__ __forceinline__ unsigned abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
 
@@ -1829,13 +1830,19 @@ size_t attention_hist_smem(int beams, int dim_head, int len) {
   return kCrossStages * kCrossRows * 32 * sizeof(float4) + sizeof(float) * (static_cast<size_t>(beams) * (128 / dim_head) * ((len + 3) & ~3) + 2 * static_cast<size_t>(beams) * len);
 }
 }  // namespace
-bool attention_hist_supported(int beams, int dim_head, int len) {
-  return beams >= 2 && beams <= kMaxHistBeams && (dim_head == 64 || dim_head == 32) && attention_hist_smem(beams, dim_head, len) <= 48 * 1024;
+// Two to four hypotheses, five and six up to 32 sentences: a wider beam's hypotheses share less, and its warps wait for one another at every stage.
+// Whole mini-batches, this kernel against attention1_kernel on one box: transformer-base, beam 4, 4 to 64 sentences x 8 to 36 words 0 to -2 %; beam 6
+// 4 x 36 -2.0 %, 16 x 36 -2.8 %, 32 x 30 -2.2 %, 48 x 30 -1.8 %, 64 x 24 +1.2 %; beam 7 8 x 30 +1.2 %, 16 x 30 -2.6 %; beam 8 4 x 30 +2.0 %,
+// 8 x 30 +1.2 %, 64 x 8 +1.7 %; transformer-big, beam 5 64 x 30 +1.0 %; beam 6 16 x 36 -3.0 %, 32 x 30 -2.6 %, 48 x 30 +1.3 %, 64 x 24 +2.0 %; beam 8
+// 8 x 30 +1.9 %, 32 x 24 +2.2 %.
+bool attention_hist_supported(int beams, int sentences, int dim_head, int len) {
+  return beams >= 2 && (beams <= kHistBeams || (beams <= kMaxHistBeams && sentences <= kMaxHistSentences)) && (dim_head == 64 || dim_head == 32) &&
+         attention_hist_smem(beams, dim_head, len) <= 48 * 1024;
 }
 int launch_attention_hist(const float* q, const float* k, const float* v, int rows, int heads, int dim_head, int len, float* out, unsigned* slot,
                           cudaStream_t s, const HistLists& lists) {
   const int beams = lists.batch > 0 ? rows / lists.batch : 0;
-  if(rows <= 0 || heads <= 0 || len <= 0 || beams * lists.batch != rows || !attention_hist_supported(beams, dim_head, len))
+  if(rows <= 0 || heads <= 0 || len <= 0 || beams * lists.batch != rows || !attention_hist_supported(beams, lists.batch, dim_head, len))
     return MI8_ERR_UNSUPPORTED;
   const float scale = 1.0f / sqrtf(static_cast<float>(dim_head));
   const int warp_heads = 128 / dim_head;

@@ -227,7 +227,7 @@ int launch_embed_ancestors(const float* wemb, const int* words, const float* pos
                            unsigned* slot2, const int* anc_old, int* anc_new, const int* hyp, int t, int rows, int stride, cudaStream_t s,
                            int hist_layers, const float* const* hist_rowmax, unsigned* const* hist_slot, const HistLists& lists = HistLists());
 // decoder self-attention (mode 0 with an ancestor table) for all hypotheses of a sentence together, from the lists of this step
-bool attention_hist_supported(int beams, int dim_head, int len);
+bool attention_hist_supported(int beams, int sentences, int dim_head, int len);
 int launch_attention_hist(const float* q, const float* k, const float* v, int rows, int heads, int dim_head, int len, float* out, unsigned* slot,
                           cudaStream_t s, const HistLists& lists);
 // layer input x and the self-attention history quantised by one launch (see quantize_dual_kernel)
