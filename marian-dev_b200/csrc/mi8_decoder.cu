@@ -169,7 +169,7 @@ struct mi8d_decoder {
   int opt_blocking_wait = 0;
   bool overlap = false;
   // tuning switches (mi8d_set_option)
-  int opt_fuse = 1, opt_quant_in_gemm = 0, opt_fused_out_rows = 0, opt_side_stream = 1, opt_shared_history = 1;
+  int opt_fuse = 1, opt_quant_in_gemm = 0, opt_fused_out_rows = 0, opt_side_stream = 1, opt_shared_history = 1, opt_one_launch_rows = kDecoderRowsMax;
   int opt_gemm_tile = 0;
   int opt_cluster = 0, opt_fused_ln = 1, opt_cluster_max_rows = 1024, opt_cluster_size = 0, opt_cluster_max_k = 2048;
   // host-side timing of mi8d_search
@@ -568,7 +568,7 @@ bool ln_quantises(const mi8d_decoder* d, int rows) {
 // Whether launch_decoder_rows runs the layers of a step of `rows` rows.
 bool decoder_rows_apply(const mi8d_decoder* d, int rows) {
   const mi8d_config& c = d->cfg;
-  return d->rows_ready && d->opt_fuse && !d->opt_cluster && !d->opt_quant_in_gemm &&
+  return rows <= d->opt_one_launch_rows && d->rows_ready && d->opt_fuse && !d->opt_cluster && !d->opt_quant_in_gemm &&
          decoder_rows_supported(rows, c.dim_emb, c.dim_ffn, c.heads, c.dec_depth, d->src);
 }
 int add_ln_quant(mi8d_decoder* d, const float* a, const float* resid, const Norm& n, int rows, float* out, int8_t* q, cudaStream_t s) {
@@ -751,6 +751,7 @@ int mi8d_set_option(mi8d_decoder* d, int option, int value) {
     case MI8D_OPT_FUSED_OUTPUT_MAX_ROWS: d->opt_fused_out_rows = value; break;
     case MI8D_OPT_SIDE_STREAM: d->opt_side_stream = value != 0; break;
     case MI8D_OPT_SHARED_HISTORY: d->opt_shared_history = value != 0; break;
+    case MI8D_OPT_ONE_LAUNCH_ROWS: d->opt_one_launch_rows = value; break;
     case MI8D_OPT_CLUSTER_AFFINE: d->opt_cluster = value != 0; break;
     case MI8D_OPT_FUSED_LAYERNORM: d->opt_fused_ln = value != 0; break;
     case MI8D_OPT_CLUSTER_MAX_ROWS: d->opt_cluster_max_rows = value; break;

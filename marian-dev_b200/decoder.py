@@ -151,7 +151,7 @@ class NativeStepper:
 
     OPTIONS = {"fuse_weights": 1, "quant_in_gemm": 2, "fused_output_max_rows": 3, "side_stream": 4, "attention_unroll": 5, "attention_block_heads": 6,
                "cluster_affine": 7, "fused_layernorm": 8, "cluster_max_rows": 9, "cluster_size": 10, "cluster_max_k": 11, "gemm_tile_rows": 12, "blocking_wait": 13,
-               "shared_history": 14}
+               "shared_history": 14, "one_launch_rows": 15}
 
     def set_option(self, name: str, value: int):
         """mi8d_set_option: tuning switches of the step driver (every setting computes the same bits)."""
@@ -383,6 +383,12 @@ class SearchPool:
             for st in self.steppers:
                 st.set_option("gemm_tile_rows", shared_gpu_tile_rows)
                 st.set_option("blocking_wait", 2)     # the workers' host threads poll and yield instead of spinning on a core each
+                if len(self.steppers) > 2:
+                    # The cluster that runs an SSRU step's layers needs 16 free SMs of one partition of the GPU.  Student, 18 to 24 words, up
+                    # to 32 / up to 24 rows in one launch (medians of 13, two runs): four searches, 32 rows (8 sentences x beam 4) 53.9 and
+                    # 54.7 / 46.9 and 47.9 ms, 32 sentences 56.5 and 56.4 / 51.9 and 52.6, 28 rows 51.8 and 51.6 / 47.5 and 48.3; two
+                    # searches, 26 to 28 rows 37 to 40 / 39 to 42, 32 rows level.
+                    st.set_option("one_launch_rows", 24)
 
     @property
     def h2d_bytes(self):

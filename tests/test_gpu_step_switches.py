@@ -48,3 +48,34 @@ def test_hypotheses_share_their_history(cuda_device, dim, heads, beam, batch, sh
     assert on[0] == off[0]
     assert any("attention_hist_kernel" in n for n in on[1]) == shared
     assert not any("attention_hist_kernel" in n for n in off[1])
+
+
+# rows around what the cluster launch takes, and around the limit that a pool of several searches sets
+@pytest.mark.parametrize("dim,batch,limit,one", [(256, 32, None, True), (256, 33, None, False), (256, 24, 24, True), (256, 25, 24, False), (512, 16, None, True),
+                                                 (512, 17, None, False), (256, 1, 0, False)])
+def test_layers_of_a_step_in_one_launch(cuda_device, dim, batch, limit, one):
+    got, apart = _searches(cuda_device, dim, 8, True, 1, batch, "one_launch_rows", (limit, 0))
+    assert got[0] == apart[0]
+    # (sentences end, so later steps may be of few rows again: the first step decides, by its embedding)
+    steps = [n for k, n in got[1].items() if "decoder_rows_kernel" in k]
+    if limit == 0:
+        assert not steps
+    elif one:
+        assert sum(n for k, n in got[1].items() if "embed_kernel" in k) == 1     # (the encoder's only)
+    else:
+        assert sum(n for k, n in got[1].items() if "embed_kernel" in k) > 1
+    assert not any("decoder_rows_kernel" in k for k in apart[1])
+
+
+@pytest.mark.parametrize("workers,rows", [(2, 32), (3, 24), (4, 24)])
+def test_pools_limit_the_rows(cuda_device, workers, rows):
+    """Several searches on one GPU: from three on the cluster launch is for up to 24 rows (a step of 25 rows takes a launch per operation)."""
+    from marian_dev_b200 import decoder, model
+    cfg = model.TransformerConfig(dim_emb=256, dim_ffn=512, heads=8, enc_depth=1, dec_depth=2, vocab=515, decoder_autoreg="rnn")
+    net = decoder.Int8Transformer(cfg, model.random_init(cfg, 1), cuda_device)
+    pool = decoder.SearchPool(net, workers, beam=1, max_batch=32, max_src=9, max_steps=18)
+    for batch in (24, 25, 32):
+        for stepper in pool.steppers:
+            stepper.start(torch.randn(batch, 7, cfg.dim_emb, device=cuda_device), torch.zeros(batch, 7, device=cuda_device))
+            _out, names = _kernels(lambda: stepper.step(None, None, None, None, 1, batch, 1))
+            assert any("decoder_rows_kernel" in n for n in names) == (batch <= rows)
