@@ -11,7 +11,9 @@
  *
  * Memory: the caller owns everything.  It passes one arena (mi8d_arena_bytes) for activations and
  * decoder state and one int8 workspace (mi8_workspace_bytes(0,0,0), zero-filled); parameters are
- * registered by pointer under Marian's parameter names and must stay alive.
+ * registered by pointer under Marian's parameter names and must stay alive.  They are read where they lie, so values
+ * rewritten in place count from the next step on, with one exception: intgemm8 matrices that share a launch
+ * (MI8D_OPT_FUSE_WEIGHTS) are copied at the first step after a registration; register such a matrix again to change it.
  */
 #ifndef MARIAN_I8_DECODE_H_
 #define MARIAN_I8_DECODE_H_
@@ -169,11 +171,13 @@ int mi8d_history_reuse(mi8d_decoder* d, unsigned out[2], int reset);
 /* Tuning switches of the step driver; every setting computes the same values, bit for bit.
  *   MI8D_OPT_FUSE_WEIGHTS (default 1): matrices that multiply the same activation (Wk|Wv of a context attention, Wq|Wk|Wv of
  *     an encoder layer, the SSRU's W|Wf) run as ONE GEMM launch over copies stored one behind the other, and so do Wq|Wk|Wv of the
- *     decoder's self-attention, whose query takes its own quantisation of the layer input;
+ *     decoder's self-attention, whose query takes its own quantisation of the layer input.  (packed8avx512 matrices need no copies.)
+ *     0 also gives the few-row steps of an SSRU decoder, whose layers are one launch otherwise, a launch per operation;
  *   MI8D_OPT_QUANT_IN_GEMM (default 0): affines with K <= 1024 whose tiles fit one wave of CTAs quantise their
  *     activation while loading it (mi8_multiply_f32_slot) instead of through a quantisation launch;
- *   MI8D_OPT_FUSED_OUTPUT_MAX_ROWS (default 0): up to this many rows the output layer reduces its logits inside
- *     the GEMM's write-back, above it the logits are written and read back by the log-softmax / top-k kernel;
+ *   MI8D_OPT_FUSED_OUTPUT_MAX_ROWS (default 0): up to this many rows the output layer reduces its logits to the rows' candidates
+ *     inside the GEMM's write-back and does not write them.  Above it the logits are written, and the log-softmax / top-k kernel
+ *     reads them back; up to 32 rows it takes the blocks' maxima and sums from the write-back and reads the best blocks only;
  *   MI8D_OPT_SIDE_STREAM (default 1): the re-projection of the earlier history slabs runs on an internal stream;
  *   MI8D_OPT_ATTENTION_UNROLL (8 or 16, default 8; process-wide): key/value rows a thread keeps in flight;
  *   MI8D_OPT_ATTENTION_BLOCK_HEADS (default 8, 0 = all; process-wide): heads one block of the decoder attention serves;

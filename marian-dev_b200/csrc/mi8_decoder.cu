@@ -1318,8 +1318,8 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
   unsigned* x_slot = d->input_slot(c.dec_depth);
   if(!lq)
     MI8D_TRY(quantize_act(d, x, R, dm, x_slot, d->aq, s));
-  // The plain GEMM followed by the log-softmax / top-k kernel is the faster route at every row count since that kernel scans
-  // without candidate lists (beam 6, 2 sentences of transformer-base: 16.2 ms a mini-batch with the reducing write-back, 15.2 ms
+  // Beyond kBlockRows rows the plain GEMM followed by the scanning log-softmax / top-k kernel is the faster route since that kernel
+  // scans without candidate lists (beam 6, 2 sentences of transformer-base: 16.2 ms a mini-batch with the reducing write-back, 15.2 ms
   // without; student, 16 sentences x beam 4: 7.3 and 7.0; 64 x 4 and 128 x 4 rows: level).  opt_fused_out_rows > 0 brings the other back.
   const bool fused_output = !d->p8 && !d->keep_logits && R <= d->opt_fused_out_rows && n_best >= 2;
   const bool merge_apart = !step_end_fits(beam, n_best);

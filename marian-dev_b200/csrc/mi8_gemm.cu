@@ -296,8 +296,8 @@ __device__ __forceinline__ float p8_value(int acc, int zp_a, int sum_a, float sc
 // (m_first is a multiple of 16 and the arrays are 16-byte aligned; a warp reads the same address, so each
 // load is one broadcast transaction); the ragged last chunk of a tile takes the element-wise path.
 template <int CH>
-__device__ __forceinline__ void write_back_chunk_p8(const GemmParams& p, const int32_t (&v)[CH], size_t base, int valid, int m_first, float* c, int ldc, bool has_bias, float scale_b,
-                                                    int zp_b, int off_b, float bias_n) {
+__device__ __forceinline__ void write_back_chunk_p8(const GemmParams& p, const int32_t (&v)[CH], size_t base, int valid, int m_first, float* c, int ldc,
+                                                    bool has_bias, float scale_b, int zp_b, int off_b, float bias_n) {
   float* dst = c + base;
   int32_t* acc_dst = p.acc_out != nullptr ? p.acc_out + base : nullptr;   // (single-segment launches only: ldc == N)
   if(valid >= CH) {
@@ -341,7 +341,8 @@ __device__ __forceinline__ void write_back_chunk_p8(const GemmParams& p, const i
 // of logits it stores, the block's maximum and its sum of exponentials in ascending order; what is left of the log-softmax reads two
 // numbers per block (lse_topk_kernel).  The reduction runs on the write-back warps beside the next tile's MMAs.
 // With it a row's log-softmax / top-k no longer scans 32000 logits on one SM (14 us at one row, 17 at 16): student, one sentence 2.82 -> 2.54 ms
-// a mini-batch, 16 sentences 3.94 -> 3.67; packed8avx512 (kP8): student 4.60 -> 4.45 and 5.38 -> 5.20, transformer-base, 4 x beam 4 14.86 -> 14.71.  Up to 32 rows (kBlockRows): a wider tile's values would not fit beside the ring.
+// a mini-batch, 16 sentences 3.94 -> 3.67; packed8avx512 (kP8): student 4.60 -> 4.45 and 5.38 -> 5.20, transformer-base, 4 x beam 4 14.86 -> 14.71.
+// Up to 32 rows (kBlockRows): a wider tile's values would not fit beside the ring.
 // kDuo (long inner dimensions of a few hundred rows): the two CTAs of a cluster take one half of K each for the same 64-row tile.  Each keeps 32 of the
 // tile's rows, gets their other partial sums from its pair through distributed shared memory and writes them back.  One tile per CTA.
 template <int TM, bool kQuantA, int kTopK = 0, bool kP8 = false, bool kBlocks = false, bool kDuo = false>
@@ -2159,8 +2160,8 @@ int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, Gemm
     return MI8_OK;
   }
   // Long inner dimensions: 64-row tiles, two CTAs each, where that is one wave of at least half of the SMs.  512 x 4096 x 1024 on 128 CTAs 11.5 us with
-  // 32-row tiles, 9.4 now, 200 x 4096 x 2000 11.6 and 9.5, 500 x 2048 x 1024 7.5 and 7.3 (transformer-big, 128 x beam 4, whose W2 this is: 43.3 ->
-  // 42.5 ms a mini-batch).  On fewer SMs the plan below is as good or better: 128 x 4096 x 1024 on 32 CTAs 8.4, 7.9 below, 256 x 2048 x 512 6.3 against
+  // 32-row tiles, 9.4 now, 200 x 4096 x 2000 11.6 and 9.5, 500 x 2048 x 1024 7.5 and 7.3; 24 shapes over the rule's range 0.78 to 0.96 of the time
+  // (transformer-big, 128 x beam 4, whose W2 this is, gains less than its runs differ).  On fewer SMs the plan below is as good or better: 128 x 4096 x 1024 on 32 CTAs 8.4, 7.9 below, 256 x 2048 x 512 6.3 against
   // 7.7 back to back, but transformer-base 35.3 against 35.15 ms.
   const long long duo_tiles = static_cast<long long>((N + kTileN - 1) / kTileN) * ((M + 63) / 64);
   if(allow_duo && tm == 0 && force_splits == 0 && M > 64 && (K + kTileKBytes - 1) / kTileKBytes >= 16 && 2 * duo_tiles <= sms && 4 * duo_tiles >= sms) {

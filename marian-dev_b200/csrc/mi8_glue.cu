@@ -875,8 +875,8 @@ attention_cross_kernel(const float* __restrict__ q, const float* __restrict__ k,
 // consecutive four-element slices per block, rows through the ring.  The rows are the sentence's distinct history rows (history_list), in
 // the order of their positions; a warp takes from every stage of the ring the positions whose row lies in it.  attention1_kernel reads
 // every ancestor row once per hypothesis, which L2 bounds: 512 rows x 24 positions x 8 KB are 100 MB a launch.
-// Two to eight hypotheses (one shares nothing).  Whole mini-batches: transformer-base, 64 x beam 4 36.8 -> 35.1 ms, transformer-big, 128 x beam 4
-// 43.9 -> 43.3 ms, four searches of big 215.3 -> 209.2 ms.
+// Two to six hypotheses (one shares nothing; attention_hist_supported).  Whole mini-batches: transformer-base, 64 x beam 4 36.8 -> 35.1 ms; what
+// transformer-big gains at 128 x beam 4, alone and four searches at once, is within the spread of runs.
 template <int DH>
 __global__ void __launch_bounds__(kMaxHistBeams * 32)
 attention_hist_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, int heads, int len, int batch, float scale,
@@ -1702,7 +1702,8 @@ int launch_quantize_slot(const float* x, size_t n, const unsigned* slot, int8_t*
 int launch_embed_ancestors(const float* wemb, const int* words, const float* pos, float scale, int dim, float* out, float* rowmax, unsigned* slot,
                            unsigned* slot2, const int* anc_old, int* anc_new, const int* hyp, int t, int rows, int stride, cudaStream_t s,
                            int hist_layers, const float* const* hist_rowmax, unsigned* const* hist_slot, const HistLists& lists) {
-  if(lists.batch > 0 && (rows % lists.batch != 0 || rows / lists.batch > kMaxHistBeams || lists.list == nullptr || lists.which == nullptr || lists.count == nullptr))
+  if(lists.batch > 0 && (rows % lists.batch != 0 || rows / lists.batch > kMaxHistBeams || lists.list == nullptr || lists.which == nullptr ||
+                         lists.count == nullptr))
     return MI8_ERR_BAD_ARG;
   if(rows <= 0 || dim <= 0 || dim % 4 != 0 || dim > kRowThreads * 4 * kMaxVec || out == nullptr || pos == nullptr)
     return MI8_ERR_BAD_ARG;
@@ -1827,7 +1828,8 @@ int launch_attention1(const float* q, const float* k, const float* v, const floa
 
 namespace {
 size_t attention_hist_smem(int beams, int dim_head, int len) {
-  return kCrossStages * kCrossRows * 32 * sizeof(float4) + sizeof(float) * (static_cast<size_t>(beams) * (128 / dim_head) * ((len + 3) & ~3) + 2 * static_cast<size_t>(beams) * len);
+  return kCrossStages * kCrossRows * 32 * sizeof(float4) +
+         sizeof(float) * (static_cast<size_t>(beams) * (128 / dim_head) * ((len + 3) & ~3) + 2 * static_cast<size_t>(beams) * len);
 }
 }  // namespace
 // Two to four hypotheses, five and six up to 32 sentences: a wider beam's hypotheses share less, and its warps wait for one another at every stage.

@@ -390,7 +390,8 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
       }
     }
   };
-  // LayerNorm of x in place (kDim is a power of two: the product with 1 / kDim is the quotient), sums in the order of add_layernorm_kernel (its 256 threads' warps are the v here)
+  // LayerNorm of x in place (kDim is a power of two: the product with 1 / kDim is the quotient), sums in the order of add_layernorm_kernel
+  // (its 256 threads' warps are the v here)
   auto layernorm = [&](const float* gamma) {   // (the biases lie behind the scales)
     float4 gm[kNv], bt[kNv];
 #pragma unroll
