@@ -132,20 +132,6 @@ struct GemmParams {
   uint32_t spin_limit;      // bound of every barrier wait of this launch
 };
 
-// Named barrier at which the threads also agree: true in all of them when `ok` held in all of them.  (A write-back warp whose bounded wait ran
-// out must not leave the others behind at a barrier, which has no bound: it arrives too, and all leave the loop together.)
-__device__ __forceinline__ bool named_bar_all(int id, int count, bool ok) {
-  uint32_t all;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.and.pred q, %2, %3, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(all)
-      : "r"(static_cast<uint32_t>(ok)), "r"(id), "r"(count)
-      : "memory");
-  return all != 0;
-}
 // Bound of a write-back warp's wait for its accumulator (test hook: one warp of every CTA gives up at once).
 __device__ __forceinline__ uint32_t accumulator_limit(const GemmParams& p, int warp) { return p.withhold_item == kWithholdWarp && warp == 3 ? 0u : p.spin_limit; }
 
@@ -537,7 +523,8 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
     uint32_t acc_it = 0;
     uint32_t conv_it = 0;
     const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
-    for(int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x) {
+    int w = blockIdx.x;
+    for(; w < p.total_work && ok; w += gridDim.x) {
       const WorkItem wi = decode_work(p, w);
       if(skip_on && (wi.m_tile + 1) * TM <= p.skip_rows_below)
         continue;
@@ -615,11 +602,8 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
       if(lane == 0)
         ok = mbar_wait_bounded(&ctl->tmem_full[as], aph, abort_flag, accumulator_limit(p, warp));
       ok = __shfl_sync(0xffffffffu, ok, 0);
-      if(!ok) {
-        if(!kDuo && (kBlocks || p.splits > 1))   // (the tile's first barrier)
-          named_bar_all(1, kEpilogueThreads, false);
+      if(!ok)
         break;
-      }
       tc_fence_after_sync();
 
       const uint32_t t_addr = tmem_base + as * T::kAccStride + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -802,9 +786,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
           }
         }
         __threadfence();
-        ok = named_bar_all(1, kEpilogueThreads, true);
-        if(!ok)
-          break;
+        named_bar_sync(1, kEpilogueThreads);
         if(epi_tid == 0) {
           const unsigned old = atomicAdd(&p.tile_counters[wi.tile], 1u);
           const int last = (old == static_cast<unsigned>(p.splits - 1)) ? 1 : 0;
@@ -847,9 +829,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
         tc_fence_before_sync();
         mbar_arrive(&ctl->tmem_empty[as]);
         ++acc_it;
-        ok = named_bar_all(1, kEpilogueThreads, true);
-        if(!ok)
-          break;
+        named_bar_sync(1, kEpilogueThreads);
         const int block_cols = min(kTileN, p.N - wi.n_tile * kTileN);
         for(int j = warp - 2; j < cols_valid; j += kEpilogueThreads / 32) {
           float4* at = reinterpret_cast<float4*>(parked + j * kLogitPitch) + lane;
@@ -924,6 +904,14 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
       *abort_flag = 1;
       if(lane == 0)
         atomicMax(p.status, static_cast<int>(kDevTimeoutEpilogue));
+      if(!kDuo && (kBlocks || p.splits > 1)) {
+        // The others may not have given up: they meet this warp at the two barriers, which have no bound, of every tile from this one on.
+        for(; w < p.total_work; w += gridDim.x)
+          if(!skip_on || (decode_work(p, w).m_tile + 1) * TM > p.skip_rows_below) {
+            named_bar_sync(1, kEpilogueThreads);
+            named_bar_sync(1, kEpilogueThreads);
+          }
+      }
     }
   }
 
@@ -1192,7 +1180,8 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __gri
     float unquant = kP8 ? 1.0f : __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(qa, *p.seg_qb[0])), p.scale);
     uint32_t acc_it = 0;
     const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
-    for(int w = pair_id; w < p.total_work && ok; w += n_pairs) {
+    int w = pair_id;
+    for(; w < p.total_work && ok; w += n_pairs) {
       const WorkItem wi = decode_work(p, w);
       if(skip_on && (wi.m_tile + 1) * T::kTM <= p.skip_rows_below)
         continue;
@@ -1201,10 +1190,8 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __gri
       if(lane == 0)
         ok = mbar_wait_bounded(&ctl->tmem_full[as], aph, abort_flag, accumulator_limit(p, warp));
       ok = __shfl_sync(0xffffffffu, ok, 0);
-      if(!ok) {
-        named_bar_all(1, kEpilogueThreads, false);   // (the tile's barrier)
+      if(!ok)
         break;
-      }
       tc_fence_after_sync();
 
       const uint32_t t_addr = tmem_base + as * T::kAccStride + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -1259,9 +1246,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __gri
       }
       // hand the accumulator buffer back: all epilogue warps of this CTA meet, then one arrival per CTA
       tc_fence_before_sync();
-      ok = named_bar_all(1, kEpilogueThreads, true);
-      if(!ok)
-        break;
+      named_bar_sync(1, kEpilogueThreads);
       if(epi_tid == 0)
         mbar_arrive_cluster(mapa_shared(smem_u32(&ctl->tmem_empty[as]), 0u));
       ++acc_it;
@@ -1272,6 +1257,9 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __gri
         st_cluster_u32(peer_abort, 1u);
         atomicMax(p.status, static_cast<int>(kDevTimeoutEpilogue));
       }
+      for(; w < p.total_work; w += n_pairs)   // (the tiles' barriers, as in the single-CTA kernel)
+        if(!skip_on || (decode_work(p, w).m_tile + 1) * T::kTM > p.skip_rows_below)
+          named_bar_sync(1, kEpilogueThreads);
     }
   }
 
