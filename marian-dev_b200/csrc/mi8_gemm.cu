@@ -105,14 +105,11 @@ struct GemmParams {
   const unsigned* skip_a;   // when both are set and *skip_a == *skip_b, tiles that lie entirely below
   const unsigned* skip_b;   // row skip_rows_below are not computed (their previous results still hold)
   int skip_rows_below;
-  // packed8avx512 scheme (kP8): the activation is uint8 with a scale, zero point and row sum per ROW,
-  // the weights int8 with a scale, zero point and column offset per COLUMN (d_qa / d_qb / scale unused)
+  // packed8avx512 scheme (kP8): the activation is uint8 with a scale, zero point and row sum per ROW (the weights' per column: WeightMaps; d_qa, d_qb
+  // and scale unused)
   const float* p8_scale_a;
   const int32_t* p8_zp_a;
   const int32_t* p8_sum_a;
-  const float* p8_scale_b[kMaxSegments];
-  const int32_t* p8_zp_b[kMaxSegments];
-  const int32_t* p8_off_b[kMaxSegments];
   int* status;
   // Several weight matrices of the same shape [seg_n, K] stored one behind the other and multiplied with the
   // same activation in one launch (Wk|Wv of an attention block, Wq|Wk|Wv of the encoder): segment s covers
@@ -132,12 +129,17 @@ struct GemmParams {
   uint32_t spin_limit;      // bound of every barrier wait of this launch
 };
 
-// Bound of a write-back warp's wait for its accumulator (test hook: one warp of every CTA gives up at once).
-__device__ __forceinline__ uint32_t accumulator_limit(const GemmParams& p, int warp) { return p.withhold_item == kWithholdWarp && warp == 3 ? 0u : p.spin_limit; }
-
 template <bool kP8>
 struct WeightMaps {
-  CUtensorMap map[kP8 ? kMaxSegments : 1];
+  CUtensorMap map[1];
+};
+template <>
+struct WeightMaps<true> {
+  CUtensorMap map[kMaxSegments];
+  // per column of each matrix
+  const float* scale_b[kMaxSegments];
+  const int32_t* zp_b[kMaxSegments];
+  const int32_t* off_b[kMaxSegments];
 };
 // The weight rows from row n on: their matrix's map and the row in it (beyond the last matrix's rows: zeros).
 struct WeightRows {
@@ -523,6 +525,8 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
     uint32_t acc_it = 0;
     uint32_t conv_it = 0;
     const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
+    if(p.withhold_item == kWithholdWarp && warp == 3)   // (test hook: this warp of every CTA gives up at once)
+      ok = false;
     int w = blockIdx.x;
     for(; w < p.total_work && ok; w += gridDim.x) {
       const WorkItem wi = decode_work(p, w);
@@ -600,7 +604,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
       const uint32_t as = acc_it & 1u;
       const uint32_t aph = (acc_it >> 1) & 1u;
       if(lane == 0)
-        ok = mbar_wait_bounded(&ctl->tmem_full[as], aph, abort_flag, accumulator_limit(p, warp));
+        ok = mbar_wait_bounded(&ctl->tmem_full[as], aph, abort_flag, p.spin_limit);
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if(!ok)
         break;
@@ -761,9 +765,9 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
       int p8_zp_b = 0, p8_off_b = 0;
       if constexpr(kP8) {
         if(n_ok) {
-          p8_scale_b = __ldg(p.p8_scale_b[seg] + n_loc);
-          p8_zp_b = __ldg(p.p8_zp_b[seg] + n_loc);
-          p8_off_b = __ldg(p.p8_off_b[seg] + n_loc);
+          p8_scale_b = __ldg(tmap_w.scale_b[seg] + n_loc);
+          p8_zp_b = __ldg(tmap_w.zp_b[seg] + n_loc);
+          p8_off_b = __ldg(tmap_w.off_b[seg] + n_loc);
         }
       }
       // Split-K: every split adds its partial accumulators into one int32 buffer per tile with
@@ -1180,6 +1184,8 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __gri
     float unquant = kP8 ? 1.0f : __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(qa, *p.seg_qb[0])), p.scale);
     uint32_t acc_it = 0;
     const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
+    if(p.withhold_item == kWithholdWarp && warp == 3)   // (test hook: as above, one warp of every CTA gives up at once)
+      ok = false;
     int w = pair_id;
     for(; w < p.total_work && ok; w += n_pairs) {
       const WorkItem wi = decode_work(p, w);
@@ -1188,7 +1194,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __gri
       const uint32_t as = acc_it & 1u;
       const uint32_t aph = (acc_it >> 1) & 1u;
       if(lane == 0)
-        ok = mbar_wait_bounded(&ctl->tmem_full[as], aph, abort_flag, accumulator_limit(p, warp));
+        ok = mbar_wait_bounded(&ctl->tmem_full[as], aph, abort_flag, p.spin_limit);
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if(!ok)
         break;
@@ -1216,9 +1222,9 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __gri
       int p8_zp_b = 0, p8_off_b = 0;
       if constexpr(kP8) {
         if(n_ok) {
-          p8_scale_b = __ldg(p.p8_scale_b[seg] + n_loc);
-          p8_zp_b = __ldg(p.p8_zp_b[seg] + n_loc);
-          p8_off_b = __ldg(p.p8_off_b[seg] + n_loc);
+          p8_scale_b = __ldg(tmap_w.scale_b[seg] + n_loc);
+          p8_zp_b = __ldg(tmap_w.zp_b[seg] + n_loc);
+          p8_off_b = __ldg(tmap_w.off_b[seg] + n_loc);
         }
       }
       unsigned out_max = 0u;
@@ -2616,9 +2622,9 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
   p.nseg = nseg;
   p.seg_n = N / nseg;
   for(int i = 0; i < nseg; ++i) {
-    p.p8_scale_b[i] = sg.scale_b[i];
-    p.p8_zp_b[i] = sg.zp_b[i];
-    p.p8_off_b[i] = sg.off_b[i];
+    tw.scale_b[i] = sg.scale_b[i];
+    tw.zp_b[i] = sg.zp_b[i];
+    tw.off_b[i] = sg.off_b[i];
     p.seg_bias[i] = sg.bias[i];
     p.seg_c[i] = sg.c[i];
   }
