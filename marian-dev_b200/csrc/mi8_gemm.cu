@@ -129,26 +129,27 @@ struct GemmParams {
   uint32_t spin_limit;      // bound of every barrier wait of this launch
 };
 
-template <bool kP8>
+// (A launch of one matrix carries one map: what a launch's parameters take is paid by each of a decoder's launches.)
+template <bool kP8, int kMaps>
 struct WeightMaps {
   CUtensorMap map[1];
 };
-template <>
-struct WeightMaps<true> {
-  CUtensorMap map[kMaxSegments];
+template <int kMaps>
+struct WeightMaps<true, kMaps> {
+  CUtensorMap map[kMaps];
   // per column of each matrix
-  const float* scale_b[kMaxSegments];
-  const int32_t* zp_b[kMaxSegments];
-  const int32_t* off_b[kMaxSegments];
+  const float* scale_b[kMaps];
+  const int32_t* zp_b[kMaps];
+  const int32_t* off_b[kMaps];
 };
 // The weight rows from row n on: their matrix's map and the row in it (beyond the last matrix's rows: zeros).
 struct WeightRows {
   const CUtensorMap* map;
   int row;
 };
-template <bool kP8>
-__device__ __forceinline__ WeightRows weight_rows(const WeightMaps<kP8>& maps, int nseg, int seg_n, int n) {
-  const int seg = kP8 && nseg > 1 ? min(n / seg_n, nseg - 1) : 0;
+template <bool kP8, int kMaps>
+__device__ __forceinline__ WeightRows weight_rows(const WeightMaps<kP8, kMaps>& maps, int nseg, int seg_n, int n) {
+  const int seg = kP8 && kMaps > 1 ? min(n / seg_n, nseg - 1) : 0;
   return {&maps.map[seg], n - seg * seg_n};
 }
 
@@ -333,9 +334,9 @@ __device__ __forceinline__ void write_back_chunk_p8(const GemmParams& p, const i
 // Up to 32 rows (kBlockRows): a wider tile's values would not fit beside the ring.
 // kDuo (long inner dimensions of a few hundred rows): the two CTAs of a cluster take one half of K each for the same 64-row tile.  Each keeps 32 of the
 // tile's rows, gets their other partial sums from its pair through distributed shared memory and writes them back.  One tile per CTA.
-template <int TM, bool kQuantA, int kTopK = 0, bool kP8 = false, bool kBlocks = false, bool kDuo = false>
+template <int TM, bool kQuantA, int kTopK = 0, bool kP8 = false, bool kBlocks = false, bool kDuo = false, int kMaps = 1>
 __global__ void __launch_bounds__(kThreads, 1)
-mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
+mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
   using T = TileCfg<TM>;
   constexpr int kConvWarps = kEpilogueThreads / 32;
   extern __shared__ uint8_t smem_raw[];
@@ -635,7 +636,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_con
       const int cols_valid = min(TM, p.M - m0);  // activation rows of this tile that exist
       // the weight segment this tile belongs to: its multiplier, bias, output matrix and the column inside it
       int seg = 0, n_loc = n;
-      if(kTopK == 0 && p.nseg > 1) {
+      if(kTopK == 0 && (kP8 ? kMaps > 1 : p.nseg > 1)) {
         seg = (wi.n_tile * kTileN) / p.seg_n;
         n_loc = n - seg * p.seg_n;
         if(!kP8)
@@ -999,9 +1000,9 @@ struct PairCfg {
 };
 constexpr int smem_bytes_pair() { return PairCfg::kStages * PairCfg::kStageBytes + static_cast<int>(sizeof(Control)) + 1024; }
 
-template <bool kP8>
+template <bool kP8, int kMaps>
 __global__ void __launch_bounds__(kThreads, 1)
-mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
+mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
   using T = PairCfg;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;  // same in both CTAs
@@ -1206,7 +1207,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8> tmap_w, const __gri
       const int m0 = wi.m_tile * T::kTM;
       const int cols_valid = min(T::kTM, p.M - m0);
       int seg = 0, n_loc = n;
-      if(p.nseg > 1) {
+      if(kP8 ? kMaps > 1 : p.nseg > 1) {
         // (an odd number of 128-row weight tiles: the second CTA of the last pair has none, and stores nothing (n_ok))
         seg = min(((2 * wi.n_tile + static_cast<int>(rank)) * kTileN) / p.seg_n, p.nseg - 1);
         n_loc = n - seg * p.seg_n;
@@ -1883,14 +1884,14 @@ void single_segment(GemmParams& p) {
   }
 }
 
-template <int TM, bool kQuantA = false, int kTopK = 0, bool kP8 = false, bool kBlocks = false>
-int launch_cfg(const WeightMaps<kP8>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
+template <int TM, bool kQuantA = false, int kTopK = 0, bool kP8 = false, bool kBlocks = false, int kMaps = 1>
+int launch_cfg(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   constexpr int smem = smem_bytes_for<TM, kBlocks>();
   if(dev >= 0 && dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(mi8_gemm_kernel<TM, kQuantA, kTopK, kP8, kBlocks>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(mi8_gemm_kernel<TM, kQuantA, kTopK, kP8, kBlocks, false, kMaps>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if(e != cudaSuccess) {
       set_last_cuda_error(e);
       return MI8_ERR_LAUNCH;
@@ -1905,7 +1906,7 @@ int launch_cfg(const WeightMaps<kP8>& tw, const CUtensorMap& ta, const GemmParam
     if(rec.start != nullptr && rec.stop != nullptr)
       cudaEventRecord(rec.start, stream);
   }
-  cudaError_t le = launch_kernel(mi8_gemm_kernel<TM, kQuantA, kTopK, kP8, kBlocks>, dim3(plan.grid), dim3(kThreads), smem, stream, tw, ta, p);
+  cudaError_t le = launch_kernel(mi8_gemm_kernel<TM, kQuantA, kTopK, kP8, kBlocks, false, kMaps>, dim3(plan.grid), dim3(kThreads), smem, stream, tw, ta, p);
   if(le != cudaSuccess) {
     set_last_cuda_error(le);
     return MI8_ERR_LAUNCH;
@@ -1919,7 +1920,7 @@ int launch_cfg(const WeightMaps<kP8>& tw, const CUtensorMap& ta, const GemmParam
 }
 
 // Launch of kDuo: clusters of two CTAs, one tile each.
-int launch_duo(const WeightMaps<false>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
+int launch_duo(const WeightMaps<false, 1>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1972,8 +1973,8 @@ int launch_duo(const WeightMaps<false>& tw, const CUtensorMap& ta, const GemmPar
 }
 
 // Launch of the CTA-pair kernel: clusters of two CTAs, as many as can be resident at once.
-template <bool kP8 = false>
-int launch_pair(const WeightMaps<kP8>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
+template <bool kP8 = false, int kMaps = 1>
+int launch_pair(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
   static bool attr_set[64] = {};
   static int max_clusters[64] = {};
   int dev = 0;
@@ -1994,7 +1995,7 @@ int launch_pair(const WeightMaps<kP8>& tw, const CUtensorMap& ta, const GemmPara
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   if(!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(mi8_gemm_pair_kernel<kP8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(mi8_gemm_pair_kernel<kP8, kMaps>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if(e != cudaSuccess) {
       set_last_cuda_error(e);
       return MI8_ERR_LAUNCH;
@@ -2003,7 +2004,7 @@ int launch_pair(const WeightMaps<kP8>& tw, const CUtensorMap& ta, const GemmPara
     cfg.gridDim = dim3(2 * (sm_count() / 2));
     cfg.numAttrs = 1;
     int n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, mi8_gemm_pair_kernel<kP8>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&n, mi8_gemm_pair_kernel<kP8, kMaps>, &cfg);
     if(e != cudaSuccess || n <= 0) {
       set_last_cuda_error(e);
       cudaGetLastError();
@@ -2025,9 +2026,9 @@ int launch_pair(const WeightMaps<kP8>& tw, const CUtensorMap& ta, const GemmPara
   const bool timed = kernel_times_on();
   if(timed) {
     cfg.numAttrs = 1;   // no launch overlap while per-kernel times are taken
-    kernel_times_before(reinterpret_cast<const void*>(mi8_gemm_pair_kernel<kP8>), stream);
+    kernel_times_before(reinterpret_cast<const void*>(mi8_gemm_pair_kernel<kP8, kMaps>), stream);
   }
-  cudaError_t le = cudaLaunchKernelEx(&cfg, mi8_gemm_pair_kernel<kP8>, tw, ta, p);
+  cudaError_t le = cudaLaunchKernelEx(&cfg, mi8_gemm_pair_kernel<kP8, kMaps>, tw, ta, p);
   if(timed)
     kernel_times_after(stream);
   if(le != cudaSuccess) {
@@ -2040,6 +2041,19 @@ int launch_pair(const WeightMaps<kP8>& tw, const CUtensorMap& ta, const GemmPara
   }
   count_launch();
   return check_launch();
+}
+
+template <int kMaps>
+int launch_p8(const WeightMaps<true, kMaps>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
+  if(plan.pair)
+    return launch_pair<true, kMaps>(tw, ta, p, plan, stream);
+  switch(plan.tile_m) {
+    case 16: return launch_cfg<16, false, 0, true, false, kMaps>(tw, ta, p, plan, stream);
+    case 32: return launch_cfg<32, false, 0, true, false, kMaps>(tw, ta, p, plan, stream);
+    case 64: return launch_cfg<64, false, 0, true, false, kMaps>(tw, ta, p, plan, stream);
+    case 128: return launch_cfg<128, false, 0, true, false, kMaps>(tw, ta, p, plan, stream);
+    default: return launch_cfg<256, false, 0, true, false, kMaps>(tw, ta, p, plan, stream);
+  }
 }
 
 }  // namespace
@@ -2281,7 +2295,7 @@ int launch_gemm_call(const GemmCall& g) {
   if(!blocks && g.skip_a == nullptr && g.absmax_out == nullptr && M > 64 && K > 15 * kTileKBytes &&
      make_gemm_plan(M, N, K, g.force_tile_m, g.force_splits, &duo, true) == MI8_OK && duo.duo)
     plan = duo;
-  WeightMaps<false> tw;
+  WeightMaps<false, 1> tw;
   CUtensorMap ta;
   rc = get_kmajor_map(&tw.map[0], g.bt, N, K, kTileN);
   if(rc != MI8_OK)
@@ -2584,7 +2598,7 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
     return rc;
   if(plan.splits > 1 && (ws == nullptr || ws_bytes < kWsHeaderBytes + plan.partial_bytes))
     return MI8_ERR_WORKSPACE;
-  WeightMaps<true> tw{};
+  WeightMaps<true, kMaxSegments> tw{};
   CUtensorMap ta;
   for(int i = 0; i < nseg; ++i) {
     rc = get_kmajor_map(&tw.map[i], sg.bt[i], N / nseg, K, kTileN);
@@ -2629,21 +2643,14 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
     p.seg_c[i] = sg.c[i];
   }
   finish_params(p);
+  const WeightMaps<true, 1> tw1{{tw.map[0]}, {tw.scale_b[0]}, {tw.zp_b[0]}, {tw.off_b[0]}};
   if(blocks) {
     p.lg_max = block_max;
     p.lg_sum = block_sum;
     p.lg_blocks = plan.n_tiles;
-    return plan.tile_m == 16 ? launch_cfg<16, false, 0, true, true>(tw, ta, p, plan, stream) : launch_cfg<32, false, 0, true, true>(tw, ta, p, plan, stream);
+    return plan.tile_m == 16 ? launch_cfg<16, false, 0, true, true>(tw1, ta, p, plan, stream) : launch_cfg<32, false, 0, true, true>(tw1, ta, p, plan, stream);
   }
-  if(plan.pair)
-    return launch_pair<true>(tw, ta, p, plan, stream);
-  switch(plan.tile_m) {
-    case 16: return launch_cfg<16, false, 0, true>(tw, ta, p, plan, stream);
-    case 32: return launch_cfg<32, false, 0, true>(tw, ta, p, plan, stream);
-    case 64: return launch_cfg<64, false, 0, true>(tw, ta, p, plan, stream);
-    case 128: return launch_cfg<128, false, 0, true>(tw, ta, p, plan, stream);
-    default: return launch_cfg<256, false, 0, true>(tw, ta, p, plan, stream);
-  }
+  return nseg > 1 ? launch_p8(tw, ta, p, plan, stream) : launch_p8(tw1, ta, p, plan, stream);
 }
 
 // Tile width for the quantise-in-kernel variant: one tile per CTA, tiles as narrow as still fit on the
@@ -2679,7 +2686,7 @@ int launch_gemm_quant_a(const float* a_f32, const unsigned* a_slot, float* qa_ou
   int rc = make_gemm_plan(M, N, K, tm, 1, &plan);
   if(rc != MI8_OK)
     return rc;
-  WeightMaps<false> tw;
+  WeightMaps<false, 1> tw;
   rc = get_kmajor_map(&tw.map[0], bt, N, K, kTileN);
   if(rc != MI8_OK)
     return rc;
@@ -2748,7 +2755,7 @@ int launch_gemm_logits(const int8_t* aq, const float* d_qa, const int8_t* wq, co
   int rc = make_gemm_plan(vocab, rows, K, 256, 1, &plan);
   if(rc != MI8_OK)
     return rc;
-  WeightMaps<false> tw;
+  WeightMaps<false, 1> tw;
   CUtensorMap ta;
   rc = get_kmajor_map(&tw.map[0], aq, rows, K, kTileN);
   if(rc != MI8_OK)
