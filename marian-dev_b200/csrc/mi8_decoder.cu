@@ -490,7 +490,7 @@ GemmCall fused_call(mi8d_decoder* d, const int8_t* a, const Fused& f, int M, int
 }
 
 // the same activation against all matrices of a fused group; outs[i] receives [M, f.n].  (packed8avx512, a launch per matrix before: transformer-base,
-// 16 sentences x beam 4 18.6 -> 16.7 ms a mini-batch, transformer-big, 8 x 4 20.1 -> 18.0, student, 4 x 4 5.6 -> 5.3.)
+// 16 sentences x beam 4 19.4 -> 17.2 ms a mini-batch, transformer-big, 8 x 4 20.6 -> 18.4, student, 4 x 4 5.7 -> 5.2.)
 int gemm_fused(mi8d_decoder* d, const int8_t* a, const float* qa, int M, const Fused& f, float* const* outs, cudaStream_t s) {
   if(d->p8) {
     P8Segments segs = f.p8;
