@@ -1833,7 +1833,7 @@ size_t attention_hist_smem(int beams, int dim_head, int len) {
 }
 }  // namespace
 // Two to four hypotheses, five and six up to 32 sentences: a wider beam's hypotheses share less, and its warps wait for one another at every stage.
-// Whole mini-batches, this kernel against attention1_kernel on one box: transformer-base, beam 4, 4 to 64 sentences x 8 to 36 words 0 to -2 %; beam 6
+// Whole mini-batches, this kernel against attention1_kernel, in turn: transformer-base, beam 4, 4 to 64 sentences x 8 to 36 words 0 to -2 %; beam 6
 // 4 x 36 -2.0 %, 16 x 36 -2.8 %, 32 x 30 -2.2 %, 48 x 30 -1.8 %, 64 x 24 +1.2 %; beam 7 8 x 30 +1.2 %, 16 x 30 -2.6 %; beam 8 4 x 30 +2.0 %,
 // 8 x 30 +1.2 %, 64 x 8 +1.7 %; transformer-big, beam 5 64 x 30 +1.0 %; beam 6 16 x 36 -3.0 %, 32 x 30 -2.6 %, 48 x 30 +1.3 %, 64 x 24 +2.0 %; beam 8
 // 8 x 30 +1.9 %, 32 x 24 +2.2 %.
