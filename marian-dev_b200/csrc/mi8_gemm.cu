@@ -46,10 +46,10 @@ constexpr int kPairTileCode = 512;  // force_tile_m value that selects the CTA-p
 
 template <int TM>
 struct TileCfg {
-  static constexpr int kStages = TM == 256 ? 4 : (TM == 128 ? 6 : 8);
+  static constexpr int kRingBlocks = TM == 256 ? 4 : (TM == 128 ? 6 : 8);   // K blocks in the ring
   static constexpr int kWBytes = kTileN * kTileKBytes;
   static constexpr int kABytes = TM * kTileKBytes;
-  static constexpr int kStageBytes = kWBytes + kABytes;
+  static constexpr int kBlockBytes = kWBytes + kABytes;
   static constexpr int kAccStride = TM < 32 ? 32 : TM;  // TMEM columns between the two accumulators
   static constexpr int kTmemCols = 2 * kAccStride;
   static constexpr int kChunk = TM < 32 ? TM : 32;
@@ -72,7 +72,7 @@ static_assert(sizeof(Control) <= kParkedOffset, "");
 constexpr int kDuoBytes = 32 * kTileN * static_cast<int>(sizeof(int32_t));   // the partial sums a CTA receives from its pair (kDuo)
 template <int TM, bool kBlocks = false, bool kDuo = false>
 constexpr int smem_bytes_for() {
-  return TileCfg<TM>::kStages * TileCfg<TM>::kStageBytes + static_cast<int>(sizeof(Control)) + 1024 +
+  return TileCfg<TM>::kRingBlocks * TileCfg<TM>::kBlockBytes + static_cast<int>(sizeof(Control)) + 1024 +
          (kBlocks ? kParkedOffset + 2 * TM * kLogitPitch * static_cast<int>(sizeof(float)) : 0) + (kDuo ? kParkedOffset + kDuoBytes : 0);
 }
 
@@ -339,11 +339,18 @@ __global__ void __launch_bounds__(kThreads, 1)
 mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
   using T = TileCfg<TM>;
   constexpr int kConvWarps = kEpilogueThreads / 32;
+  // K blocks per stage of the ring.  A wait for a stage and its commit cost the issuing warp as much as the MMAs of a block (clock stamps: 520 cycles
+  // a block, about 260 of them the four MMAs and the commit, whatever the tile's width), so narrow tiles ran at the pace of the barriers, not of their
+  // operands.  With two blocks per stage, and the next stage looked at before this one's MMAs are issued: transformer-base 64 x beam 4 33.85 -> 33.3 ms,
+  // transformer-big 128 x 4 38.85 -> 37.7, packed8avx512 256 x 1024 x 4096 9.19 -> 8.53 us.  256-row tiles have no room for it beside four
+  // blocks in flight, and their MMAs take that long anyway.
+  constexpr int kPer = TM <= 128 && !kQuantA ? 2 : 1;
+  constexpr int kStages = T::kRingBlocks / kPer, kStageBytes = kPer * T::kBlockBytes;
   extern __shared__ uint8_t smem_raw[];
   // 128-byte swizzled tiles must start on a 1024-byte boundary.
   const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
   uint8_t* tiles = smem_raw + pad;
-  Control* ctl = reinterpret_cast<Control*>(tiles + T::kStages * T::kStageBytes);
+  Control* ctl = reinterpret_cast<Control*>(tiles + T::kRingBlocks * T::kBlockBytes);
   volatile int* abort_flag = &ctl->abort;
 
   const int warp = threadIdx.x >> 5;
@@ -358,7 +365,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
   if(threadIdx.x == 0) {
     tma_prefetch_desc(weight_rows(tmap_w, p.nseg, p.seg_n, decode_work(p, blockIdx.x).n_tile * kTileN).map);
     tma_prefetch_desc(&tmap_a);
-    for(int s = 0; s < T::kStages; ++s) {
+    for(int s = 0; s < kStages; ++s) {
       mbar_init(&ctl->full[s], kQuantA ? 1 + kConvWarps : 1);   // producer (+ one arrival per quantising warp)
       mbar_init(&ctl->empty[s], 1);
     }
@@ -395,12 +402,13 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
     if(p.skip_a == nullptr && kTopK == 0 && p.withhold_item < 0) {   // (output-layer variant: the M-side operand is the activation, nothing to prefetch)
       const WorkItem w0 = decode_work(p, blockIdx.x);
       const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, w0.n_tile * kTileN);
-      const int n_pre = min(T::kStages, w0.kb_end - w0.kb_begin);
+      const int blocks = w0.kb_end - w0.kb_begin, n_pre = min(kStages, (blocks + kPer - 1) / kPer);
       if(elect_one()) {
         for(int i = 0; i < n_pre; ++i) {
-          uint8_t* st = tiles + i * T::kStageBytes;
-          mbar_arrive_expect_tx(&ctl->full[i], kQuantA ? T::kWBytes : T::kStageBytes);
-          tma_load_2d(st, wr.map, (w0.kb_begin + i) * kTileKBytes, wr.row, &ctl->full[i]);
+          const int n_blocks = min(kPer, blocks - i * kPer);
+          mbar_arrive_expect_tx(&ctl->full[i], n_blocks * (kQuantA ? T::kWBytes : T::kBlockBytes));
+          for(int b = 0; b < n_blocks; ++b)
+            tma_load_2d(tiles + i * kStageBytes + b * T::kBlockBytes, wr.map, (w0.kb_begin + i * kPer + b) * kTileKBytes, wr.row, &ctl->full[i]);
         }
       }
       __syncwarp();
@@ -416,9 +424,9 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
         continue;
       const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, wi.n_tile * kTileN);
       const int a_row0 = p.seg_row0[p.nseg > 1 ? (wi.n_tile * kTileN) / p.seg_n : 0];
-      for(int kb = wi.kb_begin; kb < wi.kb_end; ++kb, ++it) {
-        const uint32_t s = it % T::kStages;
-        const uint32_t ph = (it / T::kStages) & 1u;
+      for(int kb = wi.kb_begin; kb < wi.kb_end; kb += kPer, ++it) {
+        const uint32_t s = it % kStages;
+        const uint32_t ph = (it / kStages) & 1u;
         const bool pre = it < prefetched;
         if(!pre)
           ok = mbar_wait_bounded(&ctl->empty[s], ph ^ 1u, abort_flag, p.spin_limit);   // every lane polls: the branch stays warp-uniform
@@ -427,13 +435,16 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
           break;
         // (test hook: a withheld item's operands never arrive, so the roles that wait for them run out of patience)
         if(elect_one() && static_cast<int>(it) != p.withhold_item) {
-          uint8_t* st = tiles + s * T::kStageBytes;
-          if(!pre) {
-            mbar_arrive_expect_tx(&ctl->full[s], kQuantA ? T::kWBytes : T::kStageBytes);
-            tma_load_2d(st, wr.map, kb * kTileKBytes, wr.row, &ctl->full[s]);
+          const int n_blocks = min(kPer, wi.kb_end - kb);
+          if(!pre)
+            mbar_arrive_expect_tx(&ctl->full[s], n_blocks * (kQuantA ? T::kWBytes : T::kBlockBytes));
+          for(int b = 0; b < n_blocks; ++b) {
+            uint8_t* st = tiles + s * kStageBytes + b * T::kBlockBytes;
+            if(!pre)
+              tma_load_2d(st, wr.map, (kb + b) * kTileKBytes, wr.row, &ctl->full[s]);
+            if(!kQuantA)
+              tma_load_2d(st + T::kWBytes, &tmap_a, (kb + b) * kTileKBytes, a_row0 + wi.m_tile * TM, &ctl->full[s]);
           }
-          if(!kQuantA)
-            tma_load_2d(st + T::kWBytes, &tmap_a, kb * kTileKBytes, a_row0 + wi.m_tile * TM, &ctl->full[s]);
         }
         __syncwarp();
       }
@@ -443,10 +454,10 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
       if(lane == 0) {
         atomicMax(p.status, static_cast<int>(kDevTimeoutProducer));
         // Wait (bounded) for the copies already issued, so none lands after the CTA has gone.
-        const uint32_t first = it > static_cast<uint32_t>(T::kStages) ? it - T::kStages : 0u;
+        const uint32_t first = it > static_cast<uint32_t>(kStages) ? it - kStages : 0u;
         int no_abort = 0;
         for(uint32_t j = first; j < it; ++j)
-          mbar_wait_bounded(&ctl->full[j % T::kStages], (j / T::kStages) & 1u, &no_abort, p.spin_limit);
+          mbar_wait_bounded(&ctl->full[j % kStages], (j / kStages) & 1u, &no_abort, p.spin_limit);
       }
       __syncwarp();
     }
@@ -454,6 +465,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
     // ------------------------------------------------------------ MMA issuer
     constexpr uint32_t idesc = kP8 ? make_idesc_i8_ub(TM) : make_idesc_i8(TM);
     uint32_t it = 0, acc_it = 0;
+    bool ready = false;   // the next stage, when it was last looked at
     // No MMA can be issued before the activation tiles arrive, and those are requested after the producer's
     // pdl_wait(): waiting here as well costs nothing and keeps the predecessor's run time out of the bounded
     // waits below (it also orders the read of the skip words, which earlier kernels of the stream write).
@@ -472,20 +484,28 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
         break;
       tc_fence_after_sync();
       const uint32_t d_tmem = tmem_base + as * T::kAccStride;
-      for(int kb = wi.kb_begin; kb < wi.kb_end; ++kb, ++it) {
-        const uint32_t s = it % T::kStages;
-        const uint32_t ph = (it / T::kStages) & 1u;
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&ctl->full[s], ph, abort_flag, p.spin_limit));
+      for(int kb = wi.kb_begin; kb < wi.kb_end; kb += kPer, ++it) {
+        const uint32_t s = it % kStages;
+        const uint32_t ph = (it / kStages) & 1u;
+        if(!__all_sync(0xffffffffu, ready))
+          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&ctl->full[s], ph, abort_flag, p.spin_limit));
         if(!ok)
           break;
         tc_fence_after_sync();
-        const uint32_t w_addr = smem_u32(tiles + s * T::kStageBytes);
-        const uint32_t a_addr = w_addr + T::kWBytes;
+        // (looked at before this stage's MMAs are issued, so that the answer is there behind them)
+        ready = mbar_test_wait(&ctl->full[(it + 1) % kStages], ((it + 1) / kStages) & 1u);
+        const uint32_t w_addr = smem_u32(tiles + s * kStageBytes);
+        const bool both = kPer > 1 && kb + 1 < wi.kb_end;
         if(elect_one()) {
 #pragma unroll
-          for(int k = 0; k < kTileKBytes / kMmaK; ++k) {
-            tc_mma_i8(d_tmem, make_kmajor_sw128_desc(w_addr + k * kMmaK), make_kmajor_sw128_desc(a_addr + k * kMmaK), idesc,
-                      (kb > wi.kb_begin || k > 0) ? 1u : 0u);
+          for(int b = 0; b < kPer; ++b) {
+            if(b == 0 || both) {
+#pragma unroll
+              for(int k = 0; k < kTileKBytes / kMmaK; ++k) {
+                const uint32_t at = w_addr + b * T::kBlockBytes + k * kMmaK;
+                tc_mma_i8(d_tmem, make_kmajor_sw128_desc(at), make_kmajor_sw128_desc(at + T::kWBytes), idesc, (kb > wi.kb_begin || b > 0 || k > 0) ? 1u : 0u);
+              }
+            }
           }
           tc_commit(&ctl->empty[s]);  // frees the smem slot once these MMAs have read it
         }
@@ -572,11 +592,11 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
 #pragma unroll
           for(int b = 0; b < kBatch; ++b) {
             if(kb0 + b < wi.kb_end && ok) {
-              const uint32_t s = conv_it % T::kStages;
-              const uint32_t ph = (conv_it / T::kStages) & 1u;
+              const uint32_t s = conv_it % kStages;
+              const uint32_t ph = (conv_it / kStages) & 1u;
               ok = __all_sync(0xffffffffu, mbar_wait_bounded(&ctl->empty[s], ph ^ 1u, abort_flag, p.spin_limit));
               if(ok) {
-                uint8_t* a_tile = tiles + s * T::kStageBytes + T::kWBytes;
+                uint8_t* a_tile = tiles + s * kStageBytes + T::kWBytes;
 #pragma unroll
                 for(int q = 0; q < kCpt; ++q) {
                   const int c = epi_tid + q * kEpilogueThreads;
@@ -2175,7 +2195,7 @@ int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, Gemm
   if(allow_duo && tm == 0 && force_splits == 0 && M > 64 && (K + kTileKBytes - 1) / kTileKBytes >= 16 && 2 * duo_tiles <= sms && 4 * duo_tiles >= sms) {
     plan->duo = 1;
     plan->tile_m = 64;
-    plan->stages = TileCfg<64>::kStages;
+    plan->stages = TileCfg<64>::kRingBlocks;
     plan->n_tiles = (N + kTileN - 1) / kTileN;
     plan->m_tiles = (M + 63) / 64;
     plan->kb_total = (K + kTileKBytes - 1) / kTileKBytes;

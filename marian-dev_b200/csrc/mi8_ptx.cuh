@@ -130,6 +130,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// The same without suspending the thread: whether the phase has completed already.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Default spin limit of a barrier wait.  A healthy pipeline completes a wait in well under a
 // microsecond (every role first waits for the preceding kernel with pdl_wait(), so the limit only
 // measures this kernel's own pipeline); it exists so that a broken one returns an error instead of hanging.
