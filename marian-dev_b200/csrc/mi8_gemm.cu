@@ -1007,27 +1007,44 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
 //     arrival per CTA (after that CTA's epilogue warps met at a named barrier).
 //   * The cluster barrier brackets the kernel: no remote arrival before the barriers exist, no CTA
 //     leaves (or frees TMEM) while its peer may still read its shared memory.
+//   * kResident (K of up to 1024, results too large for L2): the weights' tile stays in shared memory (16 KB per K block and CTA), only
+//     activation tiles run through the ring, and a pair walks the activation tiles of its weights.  Results that stream through L2 push out
+//     what is not read again at once: with a wave of pairs side by side along N every activation tile fetched all weights from HBM again; this
+//     way they are fetched once and the activation, which all pairs read all the time, stays in L2.  4096 x 1024 x 32000 into half / float
+//     122 -> 109 / 153 -> 133 us (the order alone 115 / 140), 2000 x 1024 x 32000 78 -> 72, 4096 x 1024 x 12000 57.6 -> 56.3; results of up to
+//     L2's size are level or 1 to 3 % slower (512 x 1024 x 32000 26.2 -> 26.9).  What is left: without its stores the first takes 77 us.
+//     A held block is overwritten without a barrier of its own: the ring has no more stages than the tile has pairs of K blocks, so the wait
+//     for a ring stage covers the last MMA that read the block.
 struct PairCfg {
   static constexpr int kTM = 256;             // activation rows per pair tile (MMA N)
   static constexpr int kHalfRows = 128;       // activation rows each CTA loads
-  static constexpr int kStages = 6;
+  static constexpr int kRingBlocks = 6;
   static constexpr int kWBytes = kTileN * kTileKBytes;
   static constexpr int kABytes = kHalfRows * kTileKBytes;
-  static constexpr int kStageBytes = kWBytes + kABytes;
+  static constexpr int kBlockBytes = kWBytes + kABytes;
   static constexpr int kAccStride = 256;
   static constexpr int kTmemCols = 512;
   static constexpr int kChunk = 32;
+  static constexpr int kResidentBlocks = 8;   // K blocks of held weights beside the ring
 };
-constexpr int smem_bytes_pair() { return PairCfg::kStages * PairCfg::kStageBytes + static_cast<int>(sizeof(Control)) + 1024; }
+constexpr int smem_bytes_pair(bool resident = false) {
+  return (resident ? (PairCfg::kRingBlocks + PairCfg::kResidentBlocks) * PairCfg::kWBytes : PairCfg::kRingBlocks * PairCfg::kBlockBytes) +
+         static_cast<int>(sizeof(Control)) + 1024;
+}
+static_assert(PairCfg::kABytes == PairCfg::kWBytes && smem_bytes_pair(true) <= 227 * 1024, "");
 
-template <bool kP8, int kMaps>
+template <bool kP8, int kMaps, bool kResident>
 __global__ void __launch_bounds__(kThreads, 1)
 mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
   using T = PairCfg;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;  // same in both CTAs
   uint8_t* tiles = smem_raw + pad;
-  Control* ctl = reinterpret_cast<Control*>(tiles + T::kStages * T::kStageBytes);
+  // (two K blocks per stage where the ring's blocks are small)
+  constexpr int kPer = kResident ? 2 : 1, kRingBlock = kResident ? T::kABytes : T::kBlockBytes, kStageBytes = kPer * kRingBlock;
+  constexpr int kStages = T::kRingBlocks / kPer;
+  uint8_t* const resident = tiles + kStages * kStageBytes;   // kResident: the weights, a block of 128 rows x 128 bytes per K block
+  Control* ctl = reinterpret_cast<Control*>(resident + (kResident ? T::kResidentBlocks * T::kWBytes : 0));
   volatile int* abort_flag = &ctl->abort;
 
   const int warp = threadIdx.x >> 5;
@@ -1036,6 +1053,26 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
   const bool leader = rank == 0;
   const int pair_id = blockIdx.x >> 1;
   const int n_pairs = gridDim.x >> 1;
+  const uint32_t stages = kResident ? static_cast<uint32_t>(min(kStages, (p.kb_total + kPer - 1) / kPer)) : kStages;
+  // The pair's tiles: every n_pairs-th one, or (kResident) an even share of neighbours, those of the same weights first.
+  struct Tiles {
+    int first, end, step, m_first, m_count;
+  };
+  auto my_tiles = [&](bool skip_on) -> Tiles {
+    const int skipped = skip_on ? min(p.m_tiles, max(p.skip_rows_below, 0) / T::kTM) : 0, left = p.m_tiles - skipped;
+    const long long count = static_cast<long long>(left) * p.n_tiles;
+    if(!kResident)
+      return {pair_id, static_cast<int>(count), n_pairs, skipped, left};
+    return {static_cast<int>(count * pair_id / n_pairs), static_cast<int>(count * (pair_id + 1) / n_pairs), 1, skipped, left};
+  };
+  struct Tile {
+    int n_tile, m_tile;
+  };
+  auto tile_at = [&](const Tiles& t, int w) -> Tile {
+    if(kResident)
+      return {w / t.m_count, t.m_first + w % t.m_count};
+    return {w % p.n_tiles, t.m_first + w / p.n_tiles};
+  };
   const uint32_t peer_abort = mapa_shared(smem_u32(&ctl->abort), rank ^ 1u);
 
   pdl_launch_dependents();
@@ -1044,9 +1081,9 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
   const unsigned long long trace_extra = static_cast<unsigned long long>(p.N) | (static_cast<unsigned long long>(p.K) << 20) |
                                          (static_cast<unsigned long long>(p.M) << 40);
   if(threadIdx.x == 0) {
-    tma_prefetch_desc(weight_rows(tmap_w, p.nseg, p.seg_n, (2 * decode_work(p, pair_id).n_tile + static_cast<int>(rank)) * kTileN).map);
+    tma_prefetch_desc(weight_rows(tmap_w, p.nseg, p.seg_n, (2 * tile_at(my_tiles(false), my_tiles(false).first).n_tile + static_cast<int>(rank)) * kTileN).map);
     tma_prefetch_desc(&tmap_a);
-    for(int s = 0; s < T::kStages; ++s) {
+    for(int s = 0; s < kStages; ++s) {
       mbar_init(&ctl->full[s], 1);
       mbar_init(&ctl->empty[s], 1);
     }
@@ -1072,21 +1109,24 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
 
   if(warp == 0) {
     // ------------------------------------------------------------ TMA producer (one per CTA)
-    uint32_t it = 0;
+    uint32_t it = 0, s = 0, ph = 0;   // item, its ring stage and that stage's parity
     uint32_t prefetched = 0;
+    int held = -1;                    // kResident: the weights' tile in shared memory
     // copies of both CTAs are credited to full[s] of the rank-0 CTA
     auto full_addr = [&](uint32_t s) { return mapa_shared(smem_u32(&ctl->full[s]), 0u); };
-    if(p.skip_a == nullptr && pair_id < p.total_work && p.withhold_item < 0) {
+    if(p.skip_a == nullptr && my_tiles(false).first < my_tiles(false).end && p.withhold_item < 0) {
       // weights do not depend on the previous kernel: request the first pipeline fill before waiting for it
-      const WorkItem w0 = decode_work(p, pair_id);
+      const Tile w0 = tile_at(my_tiles(false), my_tiles(false).first);
       const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, (2 * w0.n_tile + static_cast<int>(rank)) * kTileN);
-      const int n_pre = min(T::kStages, w0.kb_end - w0.kb_begin);
+      const int n_pre = min(static_cast<int>(stages), (p.kb_total + kPer - 1) / kPer);
       if(elect_one()) {
         for(int i = 0; i < n_pre; ++i) {
-          uint8_t* st = tiles + i * T::kStageBytes;
+          const int n_blocks = min(kPer, p.kb_total - i * kPer);
           if(leader)
-            mbar_arrive_expect_tx(&ctl->full[i], 2 * T::kStageBytes);
-          tma_load_2d_pair(st, wr.map, (w0.kb_begin + i) * kTileKBytes, wr.row, full_addr(i));
+            mbar_arrive_expect_tx(&ctl->full[i], 2 * n_blocks * T::kBlockBytes);
+          for(int b = 0; b < n_blocks; ++b)
+            tma_load_2d_pair(kResident ? resident + (i * kPer + b) * T::kWBytes : tiles + i * kStageBytes + b * kRingBlock, wr.map, (i * kPer + b) * kTileKBytes,
+                             wr.row, full_addr(i));
         }
       }
       __syncwarp();
@@ -1096,16 +1136,16 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
     const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
     if(p.rows_computed != nullptr && blockIdx.x == 0 && lane == 0)
       *p.rows_computed = p.M - (skip_on ? min(p.M, (p.skip_rows_below / T::kTM) * T::kTM) : 0);
-    for(int w = pair_id; w < p.total_work && ok; w += n_pairs) {
-      const WorkItem wi = decode_work(p, w);
-      if(skip_on && (wi.m_tile + 1) * T::kTM <= p.skip_rows_below)
-        continue;
+    const Tiles mine = my_tiles(skip_on);
+    for(int w = mine.first; w < mine.end && ok; w += mine.step) {
+      const Tile wi = tile_at(mine, w);
       // (both CTAs' weight rows lie in one segment, or all segments share the activation: launch_gemm_call sees to it)
       const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, (2 * wi.n_tile + static_cast<int>(rank)) * kTileN);
       const int a_row0 = p.seg_row0[p.nseg > 1 ? (2 * wi.n_tile * kTileN) / p.seg_n : 0];
-      for(int kb = wi.kb_begin; kb < wi.kb_end; ++kb, ++it) {
-        const uint32_t s = it % T::kStages;
-        const uint32_t ph = (it / T::kStages) & 1u;
+      const int a_row = a_row0 + wi.m_tile * T::kTM;
+      const bool fetch_w = !kResident || held != wi.n_tile;
+      held = wi.n_tile;
+      for(int kb = 0; kb < p.kb_total; kb += kPer, ++it) {
         const bool pre = it < prefetched;
         if(!pre)
           ok = mbar_wait_bounded(&ctl->empty[s], ph ^ 1u, abort_flag, p.spin_limit);
@@ -1113,16 +1153,21 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
         if(!ok)
           break;
         if(elect_one() && static_cast<int>(it) != p.withhold_item) {   // (test hook: both CTAs of the pair leave a withheld item out)
-          uint8_t* st = tiles + s * T::kStageBytes;
-          if(!pre) {
-            if(leader)
-              mbar_arrive_expect_tx(&ctl->full[s], 2 * T::kStageBytes);
-            tma_load_2d_pair(st, wr.map, kb * kTileKBytes, wr.row, full_addr(s));
+          const int n_blocks = min(kPer, p.kb_total - kb);
+          if(!pre && leader)
+            mbar_arrive_expect_tx(&ctl->full[s], 2 * n_blocks * (fetch_w ? T::kBlockBytes : T::kABytes));
+          for(int b = 0; b < n_blocks; ++b) {
+            uint8_t* const st = tiles + s * kStageBytes + b * kRingBlock;
+            if(!pre && fetch_w)
+              tma_load_2d_pair(kResident ? resident + (kb + b) * T::kWBytes : st, wr.map, (kb + b) * kTileKBytes, wr.row, full_addr(s));
+            tma_load_2d_pair(kResident ? st : st + T::kWBytes, &tmap_a, (kb + b) * kTileKBytes, a_row + static_cast<int>(rank) * T::kHalfRows, full_addr(s));
           }
-          tma_load_2d_pair(st + T::kWBytes, &tmap_a, kb * kTileKBytes,
-                           a_row0 + wi.m_tile * T::kTM + static_cast<int>(rank) * T::kHalfRows, full_addr(s));
         }
         __syncwarp();
+        if(++s == stages) {
+          s = 0;
+          ph ^= 1u;
+        }
       }
     }
     if(!ok) {
@@ -1132,10 +1177,10 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
         atomicMax(p.status, static_cast<int>(kDevTimeoutProducer));
         if(leader) {
           // Wait (bounded) for the copies of both CTAs already announced, so none lands after the pair has gone.
-          const uint32_t first = it > static_cast<uint32_t>(T::kStages) ? it - T::kStages : 0u;
+          const uint32_t first = it > stages ? it - stages : 0u;
           int no_abort = 0;
           for(uint32_t j = first; j < it; ++j)
-            mbar_wait_bounded(&ctl->full[j % T::kStages], (j / T::kStages) & 1u, &no_abort, p.spin_limit);
+            mbar_wait_bounded(&ctl->full[j % stages], (j / stages) & 1u, &no_abort, p.spin_limit);
         }
       }
       __syncwarp();
@@ -1144,13 +1189,12 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
     // ------------------------------------------------------------ MMA issuer (rank 0 only; rank 1 owns its TMEM half)
     if(leader) {
       constexpr uint32_t idesc = kP8 ? make_idesc_i8_ub(T::kTM, 256) : make_idesc_i8(T::kTM, 256);
-      uint32_t it = 0, acc_it = 0;
+      uint32_t s = 0, ph = 0, acc_it = 0;
+      bool ready = false;   // the next stage, when it was last looked at
       pdl_wait();   // as in the single-CTA kernel: keeps the predecessor's run time out of the bounded waits
       const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
-      for(int w = pair_id; w < p.total_work && ok; w += n_pairs) {
-        const WorkItem wi = decode_work(p, w);
-        if(skip_on && (wi.m_tile + 1) * T::kTM <= p.skip_rows_below)
-          continue;
+      const Tiles mine = my_tiles(skip_on);
+      for(int w = mine.first; w < mine.end && ok; w += mine.step) {
         const uint32_t as = acc_it & 1u;
         const uint32_t aph = (acc_it >> 1) & 1u;
         ok = __all_sync(0xffffffffu, mbar_wait_bounded(&ctl->tmem_empty[as], aph ^ 1u, abort_flag, p.spin_limit));
@@ -1158,24 +1202,32 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
           break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + as * T::kAccStride;
-        for(int kb = wi.kb_begin; kb < wi.kb_end; ++kb, ++it) {
-          const uint32_t s = it % T::kStages;
-          const uint32_t ph = (it / T::kStages) & 1u;
-          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&ctl->full[s], ph, abort_flag, p.spin_limit));
+        for(int kb = 0; kb < p.kb_total; kb += kPer) {
+          if(!__all_sync(0xffffffffu, ready))
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&ctl->full[s], ph, abort_flag, p.spin_limit));
           if(!ok)
             break;
           tc_fence_after_sync();
-          const uint32_t w_addr = smem_u32(tiles + s * T::kStageBytes);
-          const uint32_t a_addr = w_addr + T::kWBytes;
+          const uint32_t s_next = s + 1 == stages ? 0 : s + 1, ph_next = s + 1 == stages ? ph ^ 1u : ph;
+          ready = mbar_test_wait(&ctl->full[s_next], ph_next);
+          const uint32_t st = smem_u32(tiles + s * kStageBytes);
+          const uint32_t w_addr = kResident ? smem_u32(resident + kb * T::kWBytes) : st, a_addr = kResident ? st : st + T::kWBytes;
+          const bool both = kPer > 1 && kb + 1 < p.kb_total;
           if(elect_one()) {
 #pragma unroll
-            for(int k = 0; k < kTileKBytes / kMmaK; ++k) {
-              tc_mma_i8_pair(d_tmem, make_kmajor_sw128_desc(w_addr + k * kMmaK), make_kmajor_sw128_desc(a_addr + k * kMmaK), idesc,
-                             (kb > wi.kb_begin || k > 0) ? 1u : 0u);
+            for(int b = 0; b < kPer; ++b) {
+              if(b == 0 || both) {
+#pragma unroll
+                for(int k = 0; k < kTileKBytes / kMmaK; ++k)
+                  tc_mma_i8_pair(d_tmem, make_kmajor_sw128_desc(w_addr + b * T::kWBytes + k * kMmaK), make_kmajor_sw128_desc(a_addr + b * T::kABytes + k * kMmaK),
+                                 idesc, (kb > 0 || b > 0 || k > 0) ? 1u : 0u);
+              }
             }
             tc_commit_pair(&ctl->empty[s], 3);  // frees this slot in both CTAs once the MMAs have read it
           }
           __syncwarp();
+          s = s_next;
+          ph = ph_next;
         }
         if(!ok)
           break;
@@ -1207,11 +1259,10 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
     const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
     if(p.withhold_item == kWithholdWarp && warp == 3)   // (test hook: as above, one warp of every CTA gives up at once)
       ok = false;
-    int w = pair_id;
-    for(; w < p.total_work && ok; w += n_pairs) {
-      const WorkItem wi = decode_work(p, w);
-      if(skip_on && (wi.m_tile + 1) * T::kTM <= p.skip_rows_below)
-        continue;
+    const Tiles mine = my_tiles(skip_on);
+    int w = mine.first;
+    for(; w < mine.end && ok; w += mine.step) {
+      const Tile wi = tile_at(mine, w);
       const uint32_t as = acc_it & 1u;
       const uint32_t aph = (acc_it >> 1) & 1u;
       if(lane == 0)
@@ -1284,9 +1335,8 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
         st_cluster_u32(peer_abort, 1u);
         atomicMax(p.status, static_cast<int>(kDevTimeoutEpilogue));
       }
-      for(; w < p.total_work; w += n_pairs)   // (the tiles' barriers, as in the single-CTA kernel)
-        if(!skip_on || (decode_work(p, w).m_tile + 1) * T::kTM > p.skip_rows_below)
-          named_bar_sync(1, kEpilogueThreads);
+      for(; w < mine.end; w += mine.step)   // (the tiles' barriers, as in the single-CTA kernel)
+        named_bar_sync(1, kEpilogueThreads);
     }
   }
 
@@ -1993,15 +2043,15 @@ int launch_duo(const WeightMaps<false, 1>& tw, const CUtensorMap& ta, const Gemm
 }
 
 // Launch of the CTA-pair kernel: clusters of two CTAs, as many as can be resident at once.
-template <bool kP8 = false, int kMaps = 1>
-int launch_pair(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
+template <bool kP8, int kMaps, bool kResident>
+int launch_pair_as(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
   static bool attr_set[64] = {};
   static int max_clusters[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if(dev < 0 || dev >= 64)
     return MI8_ERR_UNSUPPORTED;
-  constexpr int smem = smem_bytes_pair();
+  constexpr int smem = smem_bytes_pair(kResident);
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
@@ -2015,7 +2065,7 @@ int launch_pair(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const G
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   if(!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(mi8_gemm_pair_kernel<kP8, kMaps>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(mi8_gemm_pair_kernel<kP8, kMaps, kResident>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if(e != cudaSuccess) {
       set_last_cuda_error(e);
       return MI8_ERR_LAUNCH;
@@ -2024,7 +2074,7 @@ int launch_pair(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const G
     cfg.gridDim = dim3(2 * (sm_count() / 2));
     cfg.numAttrs = 1;
     int n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, mi8_gemm_pair_kernel<kP8, kMaps>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&n, mi8_gemm_pair_kernel<kP8, kMaps, kResident>, &cfg);
     if(e != cudaSuccess || n <= 0) {
       set_last_cuda_error(e);
       cudaGetLastError();
@@ -2046,9 +2096,9 @@ int launch_pair(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const G
   const bool timed = kernel_times_on();
   if(timed) {
     cfg.numAttrs = 1;   // no launch overlap while per-kernel times are taken
-    kernel_times_before(reinterpret_cast<const void*>(mi8_gemm_pair_kernel<kP8, kMaps>), stream);
+    kernel_times_before(reinterpret_cast<const void*>(mi8_gemm_pair_kernel<kP8, kMaps, kResident>), stream);
   }
-  cudaError_t le = cudaLaunchKernelEx(&cfg, mi8_gemm_pair_kernel<kP8, kMaps>, tw, ta, p);
+  cudaError_t le = cudaLaunchKernelEx(&cfg, mi8_gemm_pair_kernel<kP8, kMaps, kResident>, tw, ta, p);
   if(timed)
     kernel_times_after(stream);
   if(le != cudaSuccess) {
@@ -2061,6 +2111,15 @@ int launch_pair(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const G
   }
   count_launch();
   return check_launch();
+}
+
+template <bool kP8 = false, int kMaps = 1>
+int launch_pair(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
+  // held weights where the results are more than fills L2 (126 MB; figures at the kernel)
+  const size_t result = static_cast<size_t>(p.M) * p.N * (p.out_f16 ? 2 : 4);
+  if(p.kb_total <= PairCfg::kResidentBlocks && p.M <= p.N && result >= (size_t{144} << 20))
+    return launch_pair_as<kP8, kMaps, true>(tw, ta, p, plan, stream);
+  return launch_pair_as<kP8, kMaps, false>(tw, ta, p, plan, stream);
 }
 
 template <int kMaps>
@@ -2172,7 +2231,7 @@ int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, Gemm
       return MI8_ERR_BAD_ARG;
     plan->pair = 1;
     plan->tile_m = PairCfg::kTM;
-    plan->stages = PairCfg::kStages;
+    plan->stages = PairCfg::kRingBlocks;
     plan->n_tiles = (N + 2 * kTileN - 1) / (2 * kTileN);
     plan->m_tiles = (M + PairCfg::kTM - 1) / PairCfg::kTM;
     plan->kb_total = (K + kTileKBytes - 1) / kTileKBytes;
