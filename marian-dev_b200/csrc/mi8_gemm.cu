@@ -23,6 +23,7 @@
 // kernel whose write-back reduces every 128-word block to its maximum, sum of exponentials and best
 // entries (kTopK), and the CTA-pair kernel (tcgen05.mma.cta_group::2, 256 x 256 tile per cluster of two
 // CTAs) that the plan picks for large M.
+#include <algorithm>
 #include <cfloat>
 #include <cuda_fp16.h>
 
@@ -2298,34 +2299,38 @@ int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, Gemm
   const long long tiles = static_cast<long long>(plan->n_tiles) * plan->m_tiles;
   if(tiles > 0x7fffffffLL / 64)
     return MI8_ERR_UNSUPPORTED;
-  int splits = force_splits;
-  if(splits == 0) {
-    splits = 1;
+  auto no_empty = [&](int n) {   // the same blocks per split, and no split without any
+    const int per = (plan->kb_total + n - 1) / n;
+    return (plan->kb_total + per - 1) / per;
+  };
+  int splits = force_splits, brought = force_splits;
+  if(force_splits == 0) {
+    // K across idle SMs, every split at least eight 128-byte K blocks.
+    brought = 1;
     if(tiles < sms) {
-      // Split K across idle SMs, but leave every split at least eight 128-byte K blocks: below that
-      // the fence + arrival counter of the split path costs more than the shorter stream saves.
-      int by_sms = static_cast<int>(sms / tiles);
-      int by_depth = plan->kb_total / 8 > 1 ? plan->kb_total / 8 : 1;
-      splits = by_sms < by_depth ? by_sms : by_depth;
-      if(splits > plan->kb_total)
-        splits = plan->kb_total;
-      if(splits < 1)
-        splits = 1;
+      const int by_sms = static_cast<int>(sms / tiles);
+      const int by_depth = plan->kb_total / 8 > 1 ? plan->kb_total / 8 : 1;
+      brought = std::max(1, std::min(std::min(by_sms, by_depth), plan->kb_total));
     }
+    // Beyond 64 rows only where that saves a CTA more than sixteen blocks: the fence, the atomics and the arrival counter of the split path cost 2.3 us, a
+    // block 0.15 us.  Launches in a graph, us, 1 / 2 / 4 splits: 256 x 2048 x 512 5.31, 6.66, 6.28; 128 x 2048 x 512 5.29, 6.50, 6.02; 128 x 4096 x 1024 7.91,
+    // 7.98, 6.74; 256 x 4096 x 1024 8.08, 8.25.  transformer-base, 64 x beam 4, 33.25 -> 32.8 ms.  (Up to 64 rows 2048 x 512 is 0.5 to 1.8 us faster without
+    // splits too; there the tests of the no-allocation entry point hold the plan's splits.)  The workspace that a call brings does not follow this rule.
+    splits = M <= 64 || plan->kb_total - plan->kb_total / brought > 16 ? brought : 1;
   }
   if(splits < 1 || splits > plan->kb_total)
     return MI8_ERR_BAD_ARG;
+  plan->splits = splits = no_empty(splits);
   plan->kb_per_split = (plan->kb_total + splits - 1) / splits;
-  splits = (plan->kb_total + plan->kb_per_split - 1) / plan->kb_per_split;  // no empty split
-  plan->splits = splits;
-  if(splits > 1 && tiles > kWsMaxTileCounters)
+  brought = no_empty(brought);
+  if(brought > 1 && tiles > kWsMaxTileCounters)
     return MI8_ERR_UNSUPPORTED;
   const long long work = tiles * splits;
   plan->grid = static_cast<int>(work < sms ? work : sms);
   plan->smem_bytes = tm == 256 ? smem_bytes_for<256>()
                                : tm == 128 ? smem_bytes_for<128>()
                                            : tm == 64 ? smem_bytes_for<64>() : tm == 32 ? smem_bytes_for<32>() : smem_bytes_for<16>();
-  plan->partial_bytes = splits > 1 ? static_cast<size_t>(tiles) * kTileN * tm * sizeof(int32_t) : 0;
+  plan->partial_bytes = brought > 1 ? static_cast<size_t>(tiles) * kTileN * tm * sizeof(int32_t) : 0;
   return MI8_OK;
 }
 
@@ -2365,7 +2370,7 @@ int launch_gemm_call(const GemmCall& g) {
     rc = make_gemm_plan(M, N, K, 256, g.force_splits, &plan);
   if(rc != MI8_OK)
     return rc;
-  if(plan.splits > 1) {
+  if(plan.partial_bytes > 0) {
     if(g.ws == nullptr || g.ws_bytes < kWsHeaderBytes + plan.partial_bytes)
       return MI8_ERR_WORKSPACE;
   }
@@ -2675,7 +2680,7 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
   int rc = make_gemm_plan(M, N, K, force_tile_m, force_splits, &plan);
   if(rc != MI8_OK)
     return rc;
-  if(plan.splits > 1 && (ws == nullptr || ws_bytes < kWsHeaderBytes + plan.partial_bytes))
+  if(plan.partial_bytes > 0 && (ws == nullptr || ws_bytes < kWsHeaderBytes + plan.partial_bytes))
     return MI8_ERR_WORKSPACE;
   WeightMaps<true, kMaxSegments> tw{};
   CUtensorMap ta;

@@ -48,7 +48,7 @@ struct GemmPlan {
   int kb_per_split;
   int grid;
   int smem_bytes;
-  size_t partial_bytes;
+  size_t partial_bytes;   // behind the workspace's header: what a call brings, of which a product that is not split uses nothing
 };
 int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, GemmPlan* plan, bool allow_duo = false);
 
