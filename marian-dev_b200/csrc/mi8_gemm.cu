@@ -2276,9 +2276,9 @@ int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, Gemm
       if(tiles256 >= sms) {
         tm = 256;
       } else {
-        // The main loop of a CTA is bound by what one SM can pull from L2 (~64 bytes per clock), so the
-        // narrowest tile that still gives every tile its own SM finishes first (512 x 1024 x 1024: 5.2 us
-        // with 32-row tiles on 128 CTAs, 6.1 us with 128-row tiles on 32 CTAs).
+        // The narrowest tile that still gives every tile its own SM finishes first: its operands, MMAs and write-back are the shortest
+        // (launches in a graph, us, 32 / 64 / 128 rows: 256 x 512 x 512 3.41, 3.83, 4.72; 256 x 1024 x 1024 4.05, 4.51, 5.56; 512 x 1024 x 1024
+        // 4.55, 4.56, 5.56).
         tm = 128;
         for(int cand : {32, 64}) {
           if(static_cast<long long>((N + kTileN - 1) / kTileN) * ((M + cand - 1) / cand) <= sms) {
