@@ -2121,9 +2121,18 @@ int launch_pair_as(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, cons
 
 template <bool kP8 = false, int kMaps = 1>
 int launch_pair(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
-  // held weights where the results are more than fills L2 (126 MB; figures at the kernel)
-  const size_t result = static_cast<size_t>(p.M) * p.N * (p.out_f16 ? 2 : 4);
-  if(p.kb_total <= PairCfg::kResidentBlocks && p.M <= p.N && result >= (size_t{144} << 20))
+  // Held weights where the results are more than fills L2 (126 MB; figures at the kernel) and have no more rows than columns: with more the activation is
+  // the larger operand and every pair of weights streams it (20000 x 1024 x 4096 into half 71.4 us, 69.4 held, but 12000 x 1024 x 4096 53.1 and 55.8,
+  // 32768 x 1024 x 2048 73.4 and 78.2, 40000 x 1024 x 4000 into half 140 and 151).  Only where a row of the results is whole 32-byte sectors: of a row that is not,
+  // a tile's first and last sector are another tile's as well, which in this order is written much later: L2 reads each back to merge it (4096 x 1024 x 31999
+  // into float: 33 MB more read from HBM, 13 MB more written, and far more time than that traffic takes.  4096 x 1024 x N
+  // into float, before held weights / with them: N = 31992 153 / 138 us, 31996 162 / 186, 31999 182 / 236; into half 31984 122 / 110, 31992 124 / 130,
+  // 31999 141 / 159).
+  const size_t elem = p.out_f16 ? 2 : 4, result = static_cast<size_t>(p.M) * p.N * elem;
+  uintptr_t edges = p.seg_n * elem;
+  for(int i = 0; i < p.nseg; ++i)
+    edges |= reinterpret_cast<uintptr_t>(p.seg_c[i]);
+  if(p.kb_total <= PairCfg::kResidentBlocks && p.M <= p.N && result >= (size_t{144} << 20) && (edges & 31u) == 0)
     return launch_pair_as<kP8, kMaps, true>(tw, ta, p, plan, stream);
   return launch_pair_as<kP8, kMaps, false>(tw, ta, p, plan, stream);
 }

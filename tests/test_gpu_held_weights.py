@@ -1,5 +1,8 @@
 """The CTA-pair kernel that holds its weights' tile in shared memory (results of 144 MB and more, K of up to 1024) against the same product in blocks of
 rows, which are too small for it and take the general route: the results are whole sums and two roundings, so they are equal bit for bit."""
+import ctypes
+import re
+
 import pytest
 import torch
 
@@ -11,6 +14,21 @@ def _operands(dev, m, k, n, unsigned=False):
     a = torch.randint(0, 256, (m, k), generator=g, device=dev, dtype=torch.uint8) if unsigned else torch.randint(-127, 128, (m, k), generator=g, device=dev).to(torch.int8)
     w = torch.randint(-127, 128, (n, k), generator=g, device=dev).to(torch.int8)
     return g, a, w, torch.randn(n, generator=g, device=dev)
+
+
+def _route(call):
+    """The kernel of the one product that `call` launches: "held", "pair" (the CTA-pair kernel that streams both operands) or its name."""
+    from marian_dev_b200.binding import Mi8KernelTime, check, lib
+    check(lib().mi8_kernel_times_begin())
+    try:
+        call()
+    finally:
+        records, count = (Mi8KernelTime * 4)(), ctypes.c_int(0)
+        check(lib().mi8_kernel_times_end(records, 4, ctypes.byref(count)))
+    assert count.value == 1 and records[0].launches == 1
+    name = records[0].name.decode()
+    pair = re.search(r"mi8_gemm_pair_kernelILb[01]ELi\dELb([01])E", name)
+    return name if pair is None else "held" if pair.group(1) == "1" else "pair"
 
 
 def _status():
@@ -89,4 +107,32 @@ def test_packed8(cuda_device):
     product(0, m, got)
     for r in range(0, m, 448):
         product(r, min(m, r + 448), want)
+    assert torch.equal(got, want) and _status() == 0
+
+
+# held only where every row of the results is whole 32-byte sectors; other rows' sectors at the tiles' edges would go to memory twice (`shift`: bytes between
+# a sector's start and the results')
+@pytest.mark.parametrize("m,n,half,shift,route", [(1536, 25000, False, 0, "held"), (1536, 25004, False, 0, "pair"), (1536, 25001, False, 0, "pair"),
+                                                  (1536, 25000, False, 16, "pair"), (2560, 31984, True, 0, "held"), (2560, 31992, True, 0, "pair"),
+                                                  (2560, 31985, True, 0, "pair"), (2560, 31984, True, 2, "pair")])
+def test_rows_of_whole_sectors(cuda_device, m, n, half, shift, route):
+    from marian_dev_b200.binding import check, lib
+    from marian_dev_b200 import ops
+    k = 1024
+    _, a, w, bias = _operands(cuda_device, m, k, n)
+    q = torch.tensor([31.7, 211.3], device=cuda_device)
+    ws = ops.default_workspace(cuda_device)
+    stream = torch.cuda.current_stream().cuda_stream
+    dtype, skip = (torch.float16, shift // 2) if half else (torch.float32, shift // 4)
+
+    def product(rows, out):
+        check(lib().mi8_multiply_i8(rows.data_ptr(), w.data_ptr(), rows.shape[0], n, k, q.data_ptr(), q[1:].data_ptr(), 1.0, bias.data_ptr(), 0,
+                                    out.data_ptr(), 1 if half else 0, None, ws.ptr, ws.nbytes, stream))
+
+    got = torch.full((m * n + skip,), float("nan"), dtype=dtype, device=cuda_device)[skip:].view(m, n)
+    assert got.data_ptr() % 32 == shift
+    assert _route(lambda: product(a, got)) == route
+    want = torch.empty((m, n), dtype=dtype, device=cuda_device)
+    for r in range(0, m, 512):
+        product(a[r:r + 512], want[r:r + 512])
     assert torch.equal(got, want) and _status() == 0
