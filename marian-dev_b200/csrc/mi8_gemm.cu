@@ -2125,14 +2125,15 @@ int launch_pair(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const G
   // the larger operand and every pair of weights streams it (20000 x 1024 x 4096 into half 71.4 us, 69.4 held, but 12000 x 1024 x 4096 53.1 and 55.8,
   // 32768 x 1024 x 2048 73.4 and 78.2, 40000 x 1024 x 4000 into half 140 and 151).  Only where a row of the results is whole 32-byte sectors: of a row that is not,
   // a tile's first and last sector are another tile's as well, which in this order is written much later: L2 reads each back to merge it (4096 x 1024 x 31999
-  // into float: 33 MB more read from HBM, 13 MB more written, and far more time than that traffic takes.  4096 x 1024 x N
-  // into float, before held weights / with them: N = 31992 153 / 138 us, 31996 162 / 186, 31999 182 / 236; into half 31984 122 / 110, 31992 124 / 130,
-  // 31999 141 / 159).
+  // into float: 33 MB more read from HBM, 13 MB more written, and far more time than that traffic takes.  4096 x 1024 x N into float, before held
+  // weights / with them: N = 31992 153 / 138 us, 31996 162 / 186, 31999 182 / 236; into half 31984 122 / 110, 31992 124 / 130, 31999 141 / 159).  And not where
+  // more than a ninth of the activation tiles is padding, whose MMAs every share has to do (into float, before / held / the general kernel now:
+  // 1300 x 1024 x 29104 48.5, 50.2, 47.0 us, 1285 x 1024 x 30200 49.5, 51.2, 48.2, 1793 x 1024 x 25432 55.4, 55.3, 54.1, 1550 x 1024 x 31824 61.8, 59.6, 60.4).
   const size_t elem = p.out_f16 ? 2 : 4, result = static_cast<size_t>(p.M) * p.N * elem;
   uintptr_t edges = p.seg_n * elem;
   for(int i = 0; i < p.nseg; ++i)
     edges |= reinterpret_cast<uintptr_t>(p.seg_c[i]);
-  if(p.kb_total <= PairCfg::kResidentBlocks && p.M <= p.N && result >= (size_t{144} << 20) && (edges & 31u) == 0)
+  if(p.kb_total <= PairCfg::kResidentBlocks && p.M <= p.N && result >= (size_t{144} << 20) && (edges & 31u) == 0 && 8LL * p.m_tiles * PairCfg::kTM <= 9LL * p.M)
     return launch_pair_as<kP8, kMaps, true>(tw, ta, p, plan, stream);
   return launch_pair_as<kP8, kMaps, false>(tw, ta, p, plan, stream);
 }

@@ -110,12 +110,13 @@ def test_packed8(cuda_device):
     assert torch.equal(got, want) and _status() == 0
 
 
-# held only where every row of the results is whole 32-byte sectors; other rows' sectors at the tiles' edges would go to memory twice (`shift`: bytes between
-# a sector's start and the results')
+# held only where every row of the results is whole 32-byte sectors, the parts of other rows' sectors at the tiles' edges being written too far apart (`shift`:
+# bytes between a sector's start and the results'), and where no more than a ninth of the activation tiles is padding
 @pytest.mark.parametrize("m,n,half,shift,route", [(1536, 25000, False, 0, "held"), (1536, 25004, False, 0, "pair"), (1536, 25001, False, 0, "pair"),
                                                   (1536, 25000, False, 16, "pair"), (2560, 31984, True, 0, "held"), (2560, 31992, True, 0, "pair"),
-                                                  (2560, 31985, True, 0, "pair"), (2560, 31984, True, 2, "pair")])
-def test_rows_of_whole_sectors(cuda_device, m, n, half, shift, route):
+                                                  (2560, 31985, True, 0, "pair"), (2560, 31984, True, 2, "pair"),
+                                                  (1366, 29104, False, 0, "held"), (1365, 29104, False, 0, "pair"), (1281, 30720, False, 0, "pair")])
+def test_which_results(cuda_device, m, n, half, shift, route):
     from marian_dev_b200.binding import check, lib
     from marian_dev_b200 import ops
     k = 1024
