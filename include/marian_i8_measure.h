@@ -67,8 +67,9 @@ int mi8_trace_begin(unsigned long long* device_buf, int capacity);
 int mi8_trace_end(void);
 
 /* Test aid: makes a bounded wait inside the GEMM kernels and decoder_rows_kernel run out on purpose, without faulting anything.
- * While withhold_item >= 0, every CTA's TMA producer leaves out the loads of its pipeline item number
- * `withhold_item` (0 = its first 128-byte K block; decoder_rows_kernel: every warp's unit of that number), so the roles waiting for those bytes give up after
+ * While withhold_item >= 0, every CTA's TMA producer leaves out the loads of its 128-byte K block number
+ * `withhold_item` (counted from 0 over its tiles, each as long as the longest share of K; where a pipeline stage holds two blocks, the other one's too;
+ * decoder_rows_kernel: every warp's unit of that number), so the roles waiting for those bytes give up after
  * `spin_limit` polls (0 = the default of about a million), raise a status word 101..104 (mi8_poll_status),
  * drain what is in flight, release their tensor memory and return; the output of such a launch is undefined.
  * withhold_item == MI8_TEST_ONE_WARP: instead, one of the eight write-back warps of every CTA of the GEMMs gives up its wait for the

@@ -77,6 +77,8 @@ constexpr int smem_bytes_for() {
          (kBlocks ? kParkedOffset + 2 * TM * kLogitPitch * static_cast<int>(sizeof(float)) : 0) + (kDuo ? kParkedOffset + kDuoBytes : 0);
 }
 
+__host__ __device__ constexpr int blocks_per_stage(int tile_m) { return tile_m <= 128 ? 2 : 1; }   // K blocks in a stage of the ring (why: at the kernel)
+
 struct GemmParams {
   int M, N, K;
   int n_tiles, m_tiles, splits, kb_total, kb_per_split, total_work;
@@ -126,7 +128,7 @@ struct GemmParams {
   const float* seg_bias[kMaxSegments];
   void* seg_c[kMaxSegments];
   int* rows_computed;       // optional (measurement): receives the number of activation rows this launch really computed
-  int withhold_item;        // test hook: the producer leaves out the loads of this pipeline item (-1 = none; or kWithholdWarp)
+  int withhold_item;        // test hook: the producer leaves out the loads of this one of its stages (-1 = none; or kWithholdWarp)
   uint32_t spin_limit;      // bound of every barrier wait of this launch
 };
 
@@ -345,7 +347,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
   // operands.  With two blocks per stage, and the next stage looked at before this one's MMAs are issued: transformer-base 64 x beam 4 33.85 -> 33.3 ms,
   // transformer-big 128 x 4 38.85 -> 37.7, packed8avx512 256 x 1024 x 4096 9.19 -> 8.53 us.  256-row tiles have no room for it beside four
   // blocks in flight, and their MMAs take that long anyway.
-  constexpr int kPer = TM <= 128 && !kQuantA ? 2 : 1;
+  constexpr int kPer = kQuantA ? 1 : blocks_per_stage(TM);
   constexpr int kStages = T::kRingBlocks / kPer, kStageBytes = kPer * T::kBlockBytes;
   extern __shared__ uint8_t smem_raw[];
   // 128-byte swizzled tiles must start on a 1024-byte boundary.
@@ -1032,6 +1034,7 @@ struct PairCfg {
   static constexpr int kTmemCols = 512;
   static constexpr int kChunk = 32;
   static constexpr int kResidentBlocks = 8;   // K blocks of held weights beside the ring
+  static constexpr int kResidentPer = 2;      // and K blocks per stage there, where the ring's blocks are small
 };
 constexpr int smem_bytes_pair(bool resident = false) {
   return (resident ? (PairCfg::kRingBlocks + PairCfg::kResidentBlocks) * PairCfg::kWBytes : PairCfg::kRingBlocks * PairCfg::kBlockBytes) +
@@ -1046,8 +1049,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;  // same in both CTAs
   uint8_t* tiles = smem_raw + pad;
-  // (two K blocks per stage where the ring's blocks are small)
-  constexpr int kPer = kResident ? 2 : 1, kRingBlock = kResident ? T::kABytes : T::kBlockBytes, kStageBytes = kPer * kRingBlock;
+  constexpr int kPer = kResident ? PairCfg::kResidentPer : 1, kRingBlock = kResident ? T::kABytes : T::kBlockBytes, kStageBytes = kPer * kRingBlock;
   constexpr int kStages = T::kRingBlocks / kPer;
   uint8_t* const resident = tiles + kStages * kStageBytes;   // kResident: the weights, a block of 128 rows x 128 bytes per K block
   Control* ctl = reinterpret_cast<Control*>(resident + (kResident ? T::kResidentBlocks * T::kWBytes : 0));
@@ -1941,9 +1943,11 @@ struct ProfileState {
 };
 thread_local ProfileState t_profile;
 
-// Fields every launcher sets the same way.
-void finish_params(GemmParams& p) {
+// Fields every launcher sets the same way.  `per`: K blocks in a stage of the ring.
+void finish_params(GemmParams& p, int per) {
   test_wait_limits(&p.withhold_item, &p.spin_limit);
+  if(p.withhold_item >= 0)   // the hook names a K block: the stage of the kernel's ring that holds it
+    p.withhold_item = p.withhold_item / p.kb_per_split * ((p.kb_per_split + per - 1) / per) + p.withhold_item % p.kb_per_split / per;
   p.rows_computed = nullptr;
   if(t_profile.on && t_profile.d_rows != nullptr && t_profile.records.size() < t_profile.capacity)
     p.rows_computed = t_profile.d_rows + t_profile.records.size();
@@ -2048,6 +2052,23 @@ int launch_duo(const WeightMaps<false, 1>& tw, const CUtensorMap& ta, const Gemm
   return check_launch();
 }
 
+// Held weights in the CTA-pair kernel: where the results are more than fills L2 (126 MB; figures at the kernel) and have no more rows than columns.  With
+// more rows the activation is the larger operand and every pair of weights streams it (20000 x 1024 x 4096 into half 71.4 us, 69.4 held, but 12000 x 1024 x 4096
+// 53.1 and 55.8, 32768 x 1024 x 2048 73.4 and 78.2, 40000 x 1024 x 4000 into half 140 and 151).
+// Only where a row of the results is whole 32-byte sectors: of a row that is not, a tile's first and last sector are another tile's as well, which in this order is
+// written much later: L2 reads each back to merge it (4096 x 1024 x 31999 into float: 33 MB more read from HBM, 13 MB more written, and far more time than
+// that traffic takes.  4096 x 1024 x N into float, before held weights / with them: N = 31992 153 / 138 us, 31996 162 / 186, 31999 182 / 236; into half
+// 31984 122 / 110, 31992 124 / 130, 31999 141 / 159).
+// And not where more than a ninth of the activation tiles is padding, whose MMAs every share has to do (into float, before / held / the general kernel now:
+// 1300 x 1024 x 29104 48.5, 50.2, 47.0 us, 1285 x 1024 x 30200 49.5, 51.2, 48.2, 1793 x 1024 x 25432 55.4, 55.3, 54.1, 1550 x 1024 x 31824 61.8, 59.6, 60.4).
+bool holds_weights(const GemmParams& p) {
+  const size_t elem = p.out_f16 ? 2 : 4, result = static_cast<size_t>(p.M) * p.N * elem;
+  uintptr_t edges = p.seg_n * elem;
+  for(int i = 0; i < p.nseg; ++i)
+    edges |= reinterpret_cast<uintptr_t>(p.seg_c[i]);
+  return p.kb_total <= PairCfg::kResidentBlocks && p.M <= p.N && result >= (size_t{144} << 20) && (edges & 31u) == 0 && 8LL * p.m_tiles * PairCfg::kTM <= 9LL * p.M;
+}
+
 // Launch of the CTA-pair kernel: clusters of two CTAs, as many as can be resident at once.
 template <bool kP8, int kMaps, bool kResident>
 int launch_pair_as(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
@@ -2121,21 +2142,7 @@ int launch_pair_as(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, cons
 
 template <bool kP8 = false, int kMaps = 1>
 int launch_pair(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
-  // Held weights where the results are more than fills L2 (126 MB; figures at the kernel) and have no more rows than columns: with more the activation is
-  // the larger operand and every pair of weights streams it (20000 x 1024 x 4096 into half 71.4 us, 69.4 held, but 12000 x 1024 x 4096 53.1 and 55.8,
-  // 32768 x 1024 x 2048 73.4 and 78.2, 40000 x 1024 x 4000 into half 140 and 151).  Only where a row of the results is whole 32-byte sectors: of a row that is not,
-  // a tile's first and last sector are another tile's as well, which in this order is written much later: L2 reads each back to merge it (4096 x 1024 x 31999
-  // into float: 33 MB more read from HBM, 13 MB more written, and far more time than that traffic takes.  4096 x 1024 x N into float, before held
-  // weights / with them: N = 31992 153 / 138 us, 31996 162 / 186, 31999 182 / 236; into half 31984 122 / 110, 31992 124 / 130, 31999 141 / 159).  And not where
-  // more than a ninth of the activation tiles is padding, whose MMAs every share has to do (into float, before / held / the general kernel now:
-  // 1300 x 1024 x 29104 48.5, 50.2, 47.0 us, 1285 x 1024 x 30200 49.5, 51.2, 48.2, 1793 x 1024 x 25432 55.4, 55.3, 54.1, 1550 x 1024 x 31824 61.8, 59.6, 60.4).
-  const size_t elem = p.out_f16 ? 2 : 4, result = static_cast<size_t>(p.M) * p.N * elem;
-  uintptr_t edges = p.seg_n * elem;
-  for(int i = 0; i < p.nseg; ++i)
-    edges |= reinterpret_cast<uintptr_t>(p.seg_c[i]);
-  if(p.kb_total <= PairCfg::kResidentBlocks && p.M <= p.N && result >= (size_t{144} << 20) && (edges & 31u) == 0 && 8LL * p.m_tiles * PairCfg::kTM <= 9LL * p.M)
-    return launch_pair_as<kP8, kMaps, true>(tw, ta, p, plan, stream);
-  return launch_pair_as<kP8, kMaps, false>(tw, ta, p, plan, stream);
+  return holds_weights(p) ? launch_pair_as<kP8, kMaps, true>(tw, ta, p, plan, stream) : launch_pair_as<kP8, kMaps, false>(tw, ta, p, plan, stream);
 }
 
 template <int kMaps>
@@ -2452,7 +2459,7 @@ int launch_gemm_call(const GemmCall& g) {
     p.seg_row0[i] = g.seg_row0[i] < 0 ? g.a_row0 : g.seg_row0[i];
     p.seg_qa[i] = g.seg_qa[i] != nullptr ? g.seg_qa[i] : g.d_qa;
   }
-  finish_params(p);
+  finish_params(p, !plan.pair ? blocks_per_stage(plan.tile_m) : holds_weights(p) ? PairCfg::kResidentPer : 1);
 
   if(blocks)
     return plan.tile_m == 16 ? launch_cfg<16, false, 0, false, true>(tw, ta, p, plan, g.stream) : launch_cfg<32, false, 0, false, true>(tw, ta, p, plan, g.stream);
@@ -2741,7 +2748,7 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
     p.seg_bias[i] = sg.bias[i];
     p.seg_c[i] = sg.c[i];
   }
-  finish_params(p);
+  finish_params(p, !plan.pair ? blocks_per_stage(plan.tile_m) : holds_weights(p) ? PairCfg::kResidentPer : 1);
   const WeightMaps<true, 1> tw1{{tw.map[0]}, {tw.scale_b[0]}, {tw.zp_b[0]}, {tw.off_b[0]}};
   if(blocks) {
     p.lg_max = block_max;
@@ -2824,7 +2831,7 @@ int launch_gemm_quant_a(const float* a_f32, const unsigned* a_slot, float* qa_ou
   if(p.status == nullptr)
     return MI8_ERR_LAUNCH;
   single_segment(p);
-  finish_params(p);
+  finish_params(p, 1);
   switch(tm) {   // the weight map stands in for the unused activation map
     case 16: return launch_cfg<16, true>(tw, tw.map[0], p, plan, stream);
     case 32: return launch_cfg<32, true>(tw, tw.map[0], p, plan, stream);
@@ -2899,7 +2906,7 @@ int launch_gemm_logits(const int8_t* aq, const float* d_qa, const int8_t* wq, co
   if(p.status == nullptr)
     return MI8_ERR_LAUNCH;
   single_segment(p);
-  finish_params(p);
+  finish_params(p, blocks_per_stage(256));
   p.rows_computed = nullptr;   // (in this launch p.M counts vocabulary entries, not activation rows)
   return k_top == 4 ? launch_cfg<256, false, 4>(tw, ta, p, plan, stream) : launch_cfg<256, false, 8>(tw, ta, p, plan, stream);
 }

@@ -13,7 +13,9 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("m,k,n,tile", [(48, 512, 384, 0), (200, 1024, 256, 0), (300, 1024, 512, 512)])
+# (256: the withheld block is the tile's last, and every stage's second in tiles of up to 128 rows)
+@pytest.mark.parametrize("m,k,n,tile", [(48, 512, 384, 0), (200, 1024, 256, 0), (300, 1024, 512, 512), (48, 256, 384, 0), (100, 256, 512, 128),
+                                        (300, 256, 512, 256), (300, 256, 512, 512)])
 def test_wait_runs_out_and_the_library_recovers(cuda_device, oracle, m, k, n, tile):
     from marian_dev_b200 import ops
     from marian_dev_b200.binding import check, lib
