@@ -199,7 +199,10 @@ int mi8_multiply_i8_static(const int8_t* aq, const int8_t* bt, int M, int N, int
 
 /* How mi8_multiply_i8 would tile a problem on the current device:
  * out[0]=tile_m, out[1]=pipeline stages, out[2]=splits, out[3]=tiles along N, out[4]=tiles along M,
- * out[5]=CTAs launched, out[6]=dynamic shared memory bytes, out[7]=SM count. */
+ * out[5]=CTAs launched, out[6]=dynamic shared memory bytes, out[7]=SM count.
+ * A stage holds two 128-byte K blocks in tiles of up to 128 rows and one in the others.  The type of the result
+ * is not known here: a CTA-pair product (tile_m 512) of a large result keeps its weights in shared memory and
+ * then runs with three stages of two blocks and 32 KB more than out[6]. */
 int mi8_multiply_plan(int M, int N, int K, int force_tile_m, int force_splits, int out[8]);
 
 /* Programmatic dependent launch: when enabled (the default) every kernel of the library is launched so

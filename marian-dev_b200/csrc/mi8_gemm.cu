@@ -2277,7 +2277,7 @@ int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, Gemm
   if(allow_duo && tm == 0 && force_splits == 0 && M > 64 && (K + kTileKBytes - 1) / kTileKBytes >= 16 && 2 * duo_tiles <= sms && 4 * duo_tiles >= sms) {
     plan->duo = 1;
     plan->tile_m = 64;
-    plan->stages = TileCfg<64>::kRingBlocks;
+    plan->stages = TileCfg<64>::kRingBlocks / blocks_per_stage(64);
     plan->n_tiles = (N + kTileN - 1) / kTileN;
     plan->m_tiles = (M + 63) / 64;
     plan->kb_total = (K + kTileKBytes - 1) / kTileKBytes;
@@ -2314,7 +2314,7 @@ int make_gemm_plan(int M, int N, int K, int force_tile_m, int force_splits, Gemm
   if(tm != 16 && tm != 32 && tm != 64 && tm != 128 && tm != 256)
     return MI8_ERR_BAD_ARG;
   plan->tile_m = tm;
-  plan->stages = tm == 256 ? 4 : (tm == 128 ? 6 : 8);
+  plan->stages = (tm == 256 ? 4 : (tm == 128 ? 6 : 8)) / blocks_per_stage(tm);
   plan->n_tiles = (N + kTileN - 1) / kTileN;
   plan->m_tiles = (M + tm - 1) / tm;
   plan->kb_total = (K + kTileKBytes - 1) / kTileKBytes;

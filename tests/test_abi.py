@@ -79,6 +79,18 @@ def test_plan_cta_pair_choice():
     assert multiply_plan(300, 384, 256, 512)["n_tiles"] == 2
 
 
+@pytest.mark.parametrize("tile,blocks", [(16, 2), (32, 2), (64, 2), (128, 2), (256, 1), (512, 1)])
+def test_plan_stages_fill_the_ring(tile, blocks):
+    """The reported stages, of so many 128-byte K blocks of 128 weight rows and the CTA's activation rows each, are the shared memory but for its control words."""
+    from marian_dev_b200 import multiply_plan
+    p = multiply_plan(600, 512, 1024, tile)
+    rows = 128 if tile == 512 else tile
+    assert p["tile_m"] == tile and 0 < p["smem_bytes"] - p["stages"] * blocks * 128 * (128 + rows) < 2048
+    # K long enough for two CTAs per tile
+    duo = multiply_plan(200, 1664, 2048)
+    assert duo["splits"] == 2 and duo["tile_m"] == 64 and duo["stages"] == multiply_plan(600, 512, 1024, 64)["stages"]
+
+
 def test_plan_covers_k_without_empty_splits():
     from marian_dev_b200 import multiply_plan
     for k in (64, 128, 192, 1040, 4096):
