@@ -56,7 +56,10 @@ int mi8_last_cuda_error(void);
 const char* mi8_last_cuda_error_string(void);
 
 /* Bytes of workspace a call with exactly these dimensions needs; mi8_workspace_bytes(0,0,0) is the
- * upper bound that covers every shape (about 21 MB). */
+ * upper bound that covers every shape (about 21 MB).  Products of more than 64 rows whose K could be split
+ * over idle SMs have to bring the scratch for it even where the kernel does not split them (the plan's out[2]
+ * is 1), and mi8_multiply_i8_static refuses them where it is more than 2 MiB: sizes that callers have fixed
+ * and shapes that are refused do not change with the plan. */
 size_t mi8_workspace_bytes(int M, int N, int K);
 /* Zero-fills the whole workspace (stream-ordered).  Needed once after allocation, and again after a
  * call that ended with MI8_ERR_DEVICE. */
