@@ -233,8 +233,8 @@ __device__ __forceinline__ unsigned write_back_chunk(const GemmParams& p, const 
       // Two rows at a time: neighbouring lanes hold neighbouring columns, so one exchange gives the even lane both columns of the
       // first row and the odd lane both of the second, and each stores four bytes.  Half the store instructions, one conversion
       // per two values and no test per row.  Affines into half precision, before -> after: 4096 x 512 x 32000 367 -> 141 us,
-      // 4096 x 256 x 32000 226 -> 114 us, 3937 x 1024 x 4096 58 -> 47 us, 4096 x 1024 x 32000 161 -> 157 us (this kernel's share there 120 us
-      // at 1965 MHz; no unit is saturated: tensor pipe 59 %, issue 42 %, L2 38 %, DRAM 29 %).
+      // 4096 x 256 x 32000 226 -> 114 us, 3937 x 1024 x 4096 58 -> 47 us, 4096 x 1024 x 32000 161 -> 157 us (all of the build that brought it, before the
+      // held weights of the last).
       const bool odd = threadIdx.x & 1;
       __half* pair_dst = odd ? dst - 1 + ldc : dst;
 #pragma unroll
@@ -346,7 +346,9 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
   // a block, about 260 of them the four MMAs and the commit, whatever the tile's width), so narrow tiles ran at the pace of the barriers, not of their
   // operands.  With two blocks per stage, and the next stage looked at before this one's MMAs are issued: transformer-base 64 x beam 4 33.85 -> 33.3 ms,
   // transformer-big 128 x 4 38.85 -> 37.7, packed8avx512 256 x 1024 x 4096 9.19 -> 8.53 us.  256-row tiles have no room for it beside four
-  // blocks in flight, and their MMAs take that long anyway.
+  // blocks in flight, and their MMAs take that long anyway.  A tile of one K block fills half of each stage and an odd number of blocks half of its last;
+  // nothing is lost by it (launches in a graph, 4 to 8192 rows by 512 to 32000 columns, geometric means: K of 128 0.94 of the time before, of 384 0.94,
+  // of 1152 0.85, no shape of 272 above 1.01).
   constexpr int kPer = kQuantA ? 1 : blocks_per_stage(TM);
   constexpr int kStages = T::kRingBlocks / kPer, kStageBytes = kPer * T::kBlockBytes;
   extern __shared__ uint8_t smem_raw[];
@@ -626,8 +628,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
           break;
       }
       // The column's parameters are fetched while the MMAs run: behind them their round trip to L2 stood alone, 0.3 us of each launch of one tile per CTA
-      // (transformer-base, 64 x beam 4, 32.7 -> 31.85 ms, transformer-big, 128 x 4, 40.3 -> 39.5, four searches 209.6 -> 205.9; 512 x 1024 x 32000
-      // 26.3 -> 25.7 us).
+      // (transformer-base, 64 x beam 4, 32.7 -> 31.85 ms, transformer-big, 128 x 4, 40.3 -> 39.5; 512 x 1024 x 32000 26.3 -> 25.7 us).
       const int n = wi.n_tile * kTileN + row;
       const bool n_ok = n < p.N;
       const int m0 = wi.m_tile * TM;
@@ -1015,12 +1016,16 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
 //     arrival per CTA (after that CTA's epilogue warps met at a named barrier).
 //   * The cluster barrier brackets the kernel: no remote arrival before the barriers exist, no CTA
 //     leaves (or frees TMEM) while its peer may still read its shared memory.
-//   * kResident (K of up to 1024, results too large for L2): the weights' tile stays in shared memory (16 KB per K block and CTA), only
+//   * The next stage is looked at before this one's MMAs are issued, and the column's parameters are fetched while they run: 40000 x 1024 x 4000 into half
+//     146 -> 140 us, 20000 x 1024 x 4096 into half 73.9 -> 71.4, 32768 x 1024 x 2048 into float 74.0 -> 73.4.
+//   * kResident (K of up to 1024, results too large for L2; which ones: holds_weights): the weights' tile stays in shared memory (16 KB per K block and CTA), only
 //     activation tiles run through the ring, and a pair walks the activation tiles of its weights.  Results that stream through L2 push out
-//     what is not read again at once: with a wave of pairs side by side along N every activation tile fetched all weights from HBM again; this
-//     way they are fetched once and the activation, which all pairs read all the time, stays in L2.  4096 x 1024 x 32000 into half / float
-//     122 -> 109 / 153 -> 133 us (the order alone 115 / 140), 2000 x 1024 x 32000 78 -> 72, 4096 x 1024 x 12000 57.6 -> 56.3; results of up to
-//     L2's size are level or 1 to 3 % slower (512 x 1024 x 32000 26.2 -> 26.9).  What is left: without its stores the first takes 77 us.
+//     what is not read again at once: with a wave of pairs side by side along N every activation tile fetched all weights from HBM again (4096 x 1024 x 31992 into
+//     float: 157 MB read); this way they are fetched once and the activation, which all pairs read all the time, stays in L2 (58 MB).  4096 x 1024 x 32000 into
+//     half / float 123 -> 107 / 153 -> 133 us (the order alone, at a build of 109 / 133: 115 / 140), 2000 x 1024 x 32000 76.5 -> 68.5, 4096 x 1024 x 12000 55.2 ->
+//     52.8; results of up to L2's size are level or 1 to 3 % slower (512 x 1024 x 32000 26.2 -> 26.9).  What is left: without its stores the first takes 77 us.
+//     The plan takes the pair kernel from eight K blocks on, so by itself it comes here with K of 897 to 1024; with fewer blocks, which a caller's tile width
+//     asks for, it is at 4096 x 768 x 32000 into half 94.5 us against 104.6 of the 256-row tiles that the plan takes, at 4096 x 512 x 16000 into float level.
 //     A held block is overwritten without a barrier of its own: the ring has no more stages than the tile has pairs of K blocks, so the wait
 //     for a ring stage covers the last MMA that read the block.
 struct PairCfg {

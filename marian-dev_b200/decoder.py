@@ -379,7 +379,9 @@ class SearchPool:
         self.streams = [torch.cuda.Stream(device=model.device) for _ in self.steppers]
         if len(self.steppers) > 1 and shared_gpu_tile_rows:
             # With the GPU shared, an affine need not spread over every SM to be done soonest: wide tiles on few SMs read each
-            # weight tile fewer times (measured on transformer-big, 4 workers: 187 k -> 218 k tokens/s).  Same values either way.
+            # weight tile fewer times.  Same values either way.  Beam 4, the plan's tiles / 64 / 128 / 256 rows, ms: transformer-big, 128 sentences,
+            # four workers 231 / 215 / 206 / 206, two 129 / 126 / 126 / 132; transformer-base, 64 sentences, four workers 121 / 116 / 117 / 122,
+            # two 90 / 91 / 95 / 102 (the narrower ones gained most from two K blocks per stage, after this width was chosen).
             for st in self.steppers:
                 st.set_option("gemm_tile_rows", shared_gpu_tile_rows)
                 st.set_option("blocking_wait", 2)     # the workers' host threads poll and yield instead of spinning on a core each
