@@ -200,21 +200,24 @@ __device__ __forceinline__ float quant_mult_from_bits(unsigned bits) {
 }
 
 // Block `block` of `blocks` quantises its share of n floats (a multiple of four) at x into q: four 16-byte loads in flight per thread, the lanes of a warp
-// side by side in each.  (A thread that took 64 consecutive bytes spread every load of its warp over 2 KB.)
+// side by side in each.  (A thread that took 64 consecutive bytes spread every load of its warp over 2 KB.)  The distance of a thread's vectors is a constant:
+// from blockDim launches of up to 500000 floats were slower than with 64 consecutive bytes (16384 floats 1.52 us then, 1.63 with blockDim, 1.46 so; 524288
+// 2.07, 2.11, 1.82; 4 M 3.87, 3.52, 2.97).
+constexpr int kQuantizeThreads = 256;
 __device__ __forceinline__ void quantize_range(const float* __restrict__ x, int8_t* __restrict__ q, size_t n, float qm, unsigned block, unsigned blocks) {
   const size_t n4 = n / 4;
   const float4* x4 = reinterpret_cast<const float4*>(x);
   unsigned* q4 = reinterpret_cast<unsigned*>(q);
-  for(size_t base = static_cast<size_t>(block) * blockDim.x * 4 + threadIdx.x; base < n4; base += static_cast<size_t>(blocks) * blockDim.x * 4) {
+  for(size_t base = static_cast<size_t>(block) * (4 * kQuantizeThreads) + threadIdx.x; base < n4; base += static_cast<size_t>(blocks) * (4 * kQuantizeThreads)) {
     float4 v[4];
 #pragma unroll
     for(int e = 0; e < 4; ++e)
-      if(base + e * blockDim.x < n4)
-        v[e] = __ldg(x4 + base + e * blockDim.x);
+      if(base + e * kQuantizeThreads < n4)
+        v[e] = __ldg(x4 + base + e * kQuantizeThreads);
 #pragma unroll
     for(int e = 0; e < 4; ++e)
-      if(base + e * blockDim.x < n4)
-        q4[base + e * blockDim.x] = pack4(v[e], qm);
+      if(base + e * kQuantizeThreads < n4)
+        q4[base + e * kQuantizeThreads] = pack4(v[e], qm);
   }
 }
 
