@@ -355,8 +355,8 @@ int launch_quantize(const float* x, size_t n, const float* d_quant_mult, int8_t*
 
 int launch_prepare(const float* x, size_t n, float* d_quant_mult, int8_t* q, void* ws, size_t ws_bytes, cudaStream_t stream) {
   // Up to kOneCtaMaxN floats one CTA, up to kClusterMaxN the cluster (beyond, eight SMs read for longer than the other launch costs).
-  // Launches back to back, in us: one CTA 1.61 at 4096 floats, 2.08 at 8192; cluster 1.82 at 8208, 1.90 at 16384, 2.11 at 32752, 5.39 at
-  // 262144; the two kernels 5.25, 5.23 and 5.60 at 8208, 16384 and 32752 floats, 5.75 at 262160.
+  // Launches back to back, in us: one CTA 1.23 at 4096 floats, 1.51 at 8192; cluster 1.57 at 8448, 1.75 at 32768, 3.91 at 256000; the two kernels
+  // 4.51 at 307200 (and 5.2 to 5.7 from 8208 to 262160 when the lines were drawn).
   if(n == 0 || n % 16 != 0 || n > kClusterMaxN) {
     const int rc = launch_max_absolute(x, n, nullptr, d_quant_mult, ws, ws_bytes, stream);
     return rc != MI8_OK ? rc : launch_quantize(x, n, d_quant_mult, q, stream);
