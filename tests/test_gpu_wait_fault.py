@@ -2,7 +2,7 @@
 
 Every wait inside the GEMM kernels (on a shared-memory barrier fed by TMA copies or by the tensor core) gives up after a
 limited number of polls, raises a status word, lets the other roles of the CTA leave, drains what is in flight, frees its
-tensor memory and returns.  mi8_test_wait_fault makes the producer leave out the loads of one pipeline item, so the roles
+tensor memory and returns.  mi8_test_wait_fault makes the producer leave out the stage that holds one K block, so the roles
 waiting for those bytes time out - nothing traps, faults or spins for ever.  The test checks what the host sees (the error
 contract of the reference is "report and stop", src/common/logging.h:100-140): the launch returns, mi8_poll_status reports
 MI8_ERR_DEVICE with a 10x code, and after mi8_workspace_init + mi8_clear_status the next call is bit-exact again."""
