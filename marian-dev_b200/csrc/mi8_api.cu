@@ -204,13 +204,9 @@ int mi8_prepare_b_f32(const float* w, int K, int N, int w_is_nk, int8_t* bt, flo
                       size_t workspace_bytes, void* stream) {
   if(K <= 0 || N <= 0 || d_quant_mult == nullptr)
     return MI8_ERR_BAD_ARG;
-  const size_t n = static_cast<size_t>(K) * static_cast<size_t>(N);
   if(w_is_nk)
-    return launch_prepare(w, n, d_quant_mult, bt, workspace, workspace_bytes, as_stream(stream));
-  int rc = launch_max_absolute(w, n, nullptr, d_quant_mult, workspace, workspace_bytes, as_stream(stream));
-  if(rc != MI8_OK)
-    return rc;
-  return launch_transpose_quantize(w, K, N, d_quant_mult, bt, as_stream(stream));
+    return launch_prepare(w, static_cast<size_t>(K) * static_cast<size_t>(N), d_quant_mult, bt, workspace, workspace_bytes, as_stream(stream), true);
+  return launch_convert(w, K, N, d_quant_mult, bt, workspace, workspace_bytes, as_stream(stream));
 }
 
 int mi8_transpose_f32(const float* in, int batch, int rows, int cols, float* out, void* stream) {

@@ -62,9 +62,10 @@ int profile_end(mi8_gemm_record* out, int capacity, int* count);
 int launch_max_absolute(const float* x, size_t n, float* d_absmax, float* d_quant_mult, void* ws, size_t ws_bytes,
                         cudaStream_t stream);
 int launch_quantize(const float* x, size_t n, const float* d_quant_mult, int8_t* q, cudaStream_t stream);
-// both in turn (d_quant_mult = 127 / max|x|, q = x quantised with it); one launch for small tensors
-int launch_prepare(const float* x, size_t n, float* d_quant_mult, int8_t* q, void* ws, size_t ws_bytes, cudaStream_t stream);
-int launch_transpose_quantize(const float* w, int K, int N, const float* d_quant_mult, int8_t* bt, cudaStream_t stream);
+// both in turn (d_quant_mult = 127 / max|x|, q = x quantised with it); one launch for small tensors.  `weight`: q is a product's weight
+int launch_prepare(const float* x, size_t n, float* d_quant_mult, int8_t* q, void* ws, size_t ws_bytes, cudaStream_t stream, bool weight = false);
+// W [K, N] -> Bt [N, K] and its multiplier
+int launch_convert(const float* w, int K, int N, float* d_quant_mult, int8_t* bt, void* ws, size_t ws_bytes, cudaStream_t stream);
 int launch_transpose_f32(const float* in, int batch, int rows, int cols, float* out, cudaStream_t stream);
 
 // GEMM (mi8_gemm.cu)
