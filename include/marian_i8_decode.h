@@ -188,6 +188,8 @@ int mi8d_history_reuse(mi8d_decoder* d, unsigned out[2], int reset);
  *   MI8D_OPT_ONE_LAUNCH_ROWS (default 32): up to this many rows (32 of 256 floats, 16 of 512) the layers of an SSRU decoder's step run in one
  *     launch of a cluster of 16 CTAs; 0: a launch per operation.  Where four searches share a GPU 24 is better: the cluster needs 16 free
  *     SMs of one partition at once, and its wait for them then costs more than the launches it saves;
+ *   MI8D_OPT_STEP_AHEAD (default 1): mi8d_search launches a step whose layers are one launch before it has seen the lists of the step in front,
+ *     with control words that the device leaves (not with MI8D_OPT_BLOCKING_WAIT 1, which sleeps); 0: step by step;
  *   MI8D_OPT_CLUSTER_AFFINE (default 0): affines whose activation comes with an abs-max slot run as ONE launch of the
  *     cluster GEMM (mi8g_affine_slot) instead of a quantisation launch and a GEMM launch.  Off by default: 74 to 98
  *     launches per step of the transformer-big decoder, which then had 122 (113 now), but 5 to 20 % fewer tokens per second (the
@@ -219,7 +221,8 @@ enum mi8d_option {
   MI8D_OPT_GEMM_TILE_ROWS = 12,
   MI8D_OPT_BLOCKING_WAIT = 13,
   MI8D_OPT_SHARED_HISTORY = 14,
-  MI8D_OPT_ONE_LAUNCH_ROWS = 15
+  MI8D_OPT_ONE_LAUNCH_ROWS = 15,
+  MI8D_OPT_STEP_AHEAD = 16
 };
 int mi8d_set_option(mi8d_decoder* d, int option, int value);   /* d may be NULL for the process-wide switches */
 

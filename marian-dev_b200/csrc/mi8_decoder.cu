@@ -8,6 +8,7 @@
 // src/translator/beam_search.cpp:249-538), so a mini-batch is translated by one call.
 #include <thread>
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -147,9 +148,13 @@ struct mi8d_decoder {
   float* log_mask[2] = {nullptr, nullptr};
   int* anc[2] = {nullptr, nullptr};
   // beam-search bookkeeping (mi8d_search): per-step control words and n-best lists, device side and pinned host side
-  int* s_ctrl = nullptr;            // [3 * max_rows + max_batch]: hypothesis rows, previous words, path scores (as bits), batch rows
+  int* s_ctrl[2] = {nullptr, nullptr};   // [3 * max_rows + max_batch]: hypothesis rows, previous words, path scores (as bits), batch rows; steps in turn
   int* h_ctrl = nullptr;            // pinned; read by the step's first kernel
-  int* h_out = nullptr;             // pinned, [3][max_batch * 8]: scores (as bits), beams, words, written by the step's last kernel
+  int* h_out = nullptr;             // pinned, [2][3][max_batch * 8]: scores (as bits), beams, words, written by the step's last kernel; steps in turn
+  unsigned long long* h_tagged = nullptr;   // pinned, [2][kDecoderRowsMax * 2]: StepEnd::tagged; steps in turn
+  unsigned* stops = nullptr;        // [2] StepEnd::next_stop
+  unsigned long long* s_tagged = nullptr;   // [2][kDecoderRowsMax * 2] the same on the device, on its way through the step behind
+  unsigned tag = 0;
   float *blk_max = nullptr, *blk_sum = nullptr, *blk_topv = nullptr;   // per (row, 128-word block) partials of the output layer
   int* blk_topi = nullptr;
   bool keep_logits = false;
@@ -169,7 +174,7 @@ struct mi8d_decoder {
   int opt_blocking_wait = 0;
   bool overlap = false;
   // tuning switches (mi8d_set_option)
-  int opt_fuse = 1, opt_quant_in_gemm = 0, opt_fused_out_rows = 0, opt_side_stream = 1, opt_shared_history = 1, opt_one_launch_rows = kDecoderRowsMax;
+  int opt_fuse = 1, opt_quant_in_gemm = 0, opt_fused_out_rows = 0, opt_side_stream = 1, opt_shared_history = 1, opt_one_launch_rows = kDecoderRowsMax, opt_step_ahead = 1;
   int opt_gemm_tile = 0;
   int opt_cluster = 0, opt_fused_ln = 1, opt_cluster_max_rows = 1024, opt_cluster_size = 0, opt_cluster_max_k = 2048;
   // host-side timing of mi8d_search
@@ -224,7 +229,10 @@ struct mi8d_decoder {
     blk_sum = arena.take<float>(R * nb);
     blk_topv = arena.take<float>(R * nb * 8);
     blk_topi = arena.take<int>(R * nb * 8);
-    s_ctrl = arena.take<int>(3 * R + B);   // (the arena rounds every array up to 256 bytes)
+    for(int*& ctrl : s_ctrl)
+      ctrl = arena.take<int>(3 * R + B);   // (the arena rounds every array up to 256 bytes)
+    stops = arena.take<unsigned>(2);
+    s_tagged = arena.take<unsigned long long>(4 * kDecoderRowsMax);
     cand_score = arena.take<float>(R * 8);
     cand_word = arena.take<int>(R * 8);
     for(int i = 0; i < 2; ++i) {
@@ -650,13 +658,16 @@ int mi8d_create(const mi8d_config* cfg, void* arena, size_t arena_bytes, void* w
     cudaMemset(d->reuse_stats, 0, 2 * sizeof(unsigned));
   {
     // pinned host staging for the beam search's per-step upload and download
-    const size_t nc = 3 * static_cast<size_t>(cfg->max_rows) + cfg->max_batch + 3, no = 3 * static_cast<size_t>(cfg->max_batch) * 8;
+    const size_t nc = 3 * static_cast<size_t>(cfg->max_rows) + cfg->max_batch + 3, no = 2 * 3 * static_cast<size_t>(cfg->max_batch) * 8;
     if(cudaHostAlloc(reinterpret_cast<void**>(&d->h_ctrl), nc * sizeof(int), cudaHostAllocDefault) != cudaSuccess ||
-       cudaHostAlloc(reinterpret_cast<void**>(&d->h_out), no * sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+       cudaHostAlloc(reinterpret_cast<void**>(&d->h_out), no * sizeof(int) + 4 * kDecoderRowsMax * sizeof(unsigned long long), cudaHostAllocDefault) != cudaSuccess) {
       cudaGetLastError();
       if(d->h_ctrl)
         cudaFreeHost(d->h_ctrl);
       d->h_ctrl = d->h_out = nullptr;   // mi8d_search then reports MI8_ERR_WORKSPACE; stepping by hand still works
+    } else {
+      d->h_tagged = reinterpret_cast<unsigned long long*>(d->h_out + no);   // (an even number of words behind)
+      std::fill(d->h_tagged, d->h_tagged + 4 * kDecoderRowsMax, 0ull);
     }
   }
   if(!cfg->ssru) {
@@ -752,6 +763,7 @@ int mi8d_set_option(mi8d_decoder* d, int option, int value) {
     case MI8D_OPT_SIDE_STREAM: d->opt_side_stream = value != 0; break;
     case MI8D_OPT_SHARED_HISTORY: d->opt_shared_history = value != 0; break;
     case MI8D_OPT_ONE_LAUNCH_ROWS: d->opt_one_launch_rows = value; break;
+    case MI8D_OPT_STEP_AHEAD: d->opt_step_ahead = value != 0; break;
     case MI8D_OPT_CLUSTER_AFFINE: d->opt_cluster = value != 0; break;
     case MI8D_OPT_FUSED_LAYERNORM: d->opt_fused_ln = value != 0; break;
     case MI8D_OPT_CLUSTER_MAX_ROWS: d->opt_cluster_max_rows = value; break;
@@ -1052,8 +1064,25 @@ int mi8d_encode(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
   return MI8_OK;
 }
 
-int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const int* batch_idx, const float* prev_scores, int beam,
-              int batch, int n_best, float* out_score, int* out_beam, int* out_word, void* stream) {
+}  // extern "C"
+
+namespace {
+
+// How a step of mi8d_search is tied to the one behind it (StepEnd has the words' meaning): `end` carries them to the step's last kernel.
+struct StepLink {
+  const unsigned* stop = nullptr;
+  unsigned* next_stop = nullptr;
+  int* next_ctrl = nullptr;
+  unsigned long long *tagged = nullptr, *host_lists = nullptr;   // where the last kernel leaves the lists; where the first brings those of the step in front
+  const unsigned long long* lists = nullptr;
+  int n_lists = 0;
+  unsigned tag = 0;
+  int eos = 0;
+  unsigned char hyps[kDecoderRowsMax] = {};
+};
+
+int run_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const int* batch_idx, const float* prev_scores, int beam, int batch, int n_best,
+             float* out_score, int* out_beam, int* out_word, void* stream, const StepLink& link) {
   if(d == nullptr || beam <= 0 || batch <= 0 || n_best <= 0 || n_best > 8 || out_score == nullptr || out_beam == nullptr ||
      out_word == nullptr)
     return MI8_ERR_BAD_ARG;
@@ -1081,7 +1110,7 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
   const bool rows_path = decoder_rows_apply(d, R);
   const bool begin_apart = !rows_path || batch != d->batch;
   if(begin_apart)
-    MI8D_TRY(launch_step_begin(d->step_ctrl, d->s_ctrl, d->n_step_ctrl, d->slots, d->n_slots, s));
+    MI8D_TRY(launch_step_begin(d->step_ctrl, d->s_ctrl[t & 1], d->n_step_ctrl, d->slots, d->n_slots, s));
 
   // sentences that finished leave the batch: compact the encoder context, recompute cross K/V
   if(batch != d->batch) {
@@ -1150,7 +1179,12 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
     p.log_mask = lmask;
     p.words = words;
     p.hyp = t == 0 ? nullptr : hyp_idx;
-    p.ctrl = d->s_ctrl;
+    p.ctrl = d->s_ctrl[t & 1];
+    p.stop = link.stop;
+    p.next_stop = link.next_stop;
+    p.lists = link.lists;
+    p.host_lists = link.host_lists;
+    p.n_lists = link.n_lists;
     p.n_ctrl = begin_apart ? 0 : d->n_step_ctrl;
     std::copy(d->step_ctrl, d->step_ctrl + p.n_ctrl, p.ctrl_words);   // (3 R + batch words, batch <= R <= kDecoderRowsMax)
     p.slots = d->slots;
@@ -1330,6 +1364,13 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
   end.out_score = out_score;
   end.out_beam = out_beam;
   end.out_word = out_word;
+  end.stop = link.stop;
+  end.next_stop = link.next_stop;
+  end.next_ctrl = link.next_ctrl;
+  end.tagged = link.tagged;
+  end.tag = link.tag;
+  end.eos = link.eos;
+  std::copy(link.hyps, link.hyps + kDecoderRowsMax, end.hyps);
   if(!c.ssru && !d->p8) {   // remember which abs-max the stored keys/values of every layer now belong to
     end.layers = c.dec_depth;
     end.first = 1 + kSlotHistory;
@@ -1380,6 +1421,15 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
   return MI8_OK;
 }
 
+}  // namespace
+
+extern "C" {
+
+int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const int* batch_idx, const float* prev_scores, int beam,
+              int batch, int n_best, float* out_score, int* out_beam, int* out_word, void* stream) {
+  return run_step(d, hyp_idx, prev_words, batch_idx, prev_scores, beam, batch, n_best, out_score, out_beam, out_word, stream, StepLink());
+}
+
 // Beam search over one mini-batch: the bookkeeping of BeamSearch::search (src/translator/beam_search.cpp:249-538)
 // around mi8d_encode / mi8d_step.  Per step: every sentence still in the batch contributes its surviving
 // hypotheses (beam-major rows, dummy slots with EOS and score -inf), the n-best lists come back, each sentence keeps
@@ -1387,7 +1437,10 @@ int mi8d_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const 
 // ((pathScore - wordPenalty * length) / length^normalize, src/translator/history.h:22-35) and leave the beam, a
 // sentence whose beam is empty leaves the batch (purgeBeams, :224-245), and everything stops at
 // length >= max_length_factor * width (:521-531).  The best finished hypothesis of every sentence is traced back
-// through the per-step parent links.  One stream synchronisation per step (the n-best download).
+// through the per-step parent links.  One wait per step (the n-best download).
+// Where a step's layers are one launch (few rows of an SSRU decoder), step t + 1 is launched before the host has seen step t's lists, with the control
+// words that step t's last kernel leaves on the device (StepEnd): the GPU no longer waits for the host's turn, 12 of 58 us of a step of one sentence.
+// Those words hold while no hypothesis ends; otherwise the three launches do nothing or only fill scratch, and the host launches step t + 1 anew.
 int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batch, int width, const mi8d_search_config* sc,
                 int* out_tokens, int max_out, int* out_len, float* out_score, unsigned long long* h2d_bytes, unsigned long long* d2h_bytes,
                 void* stream) {
@@ -1420,6 +1473,49 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
 
   using clk = std::chrono::steady_clock;
   auto secs = [](clk::time_point a, clk::time_point b) { return std::chrono::duration<double>(b - a).count(); };
+  const auto last_step = [&](int t) { return static_cast<double>(t + 1) >= static_cast<double>(sc->max_length_factor) * width; };
+  const bool may_run_ahead = d->opt_step_ahead && d->opt_blocking_wait != 1 && d->opt_fused_out_rows == 0 && !d->keep_logits;
+  // Step t + 1 may be launched before step t's lists are seen: both take the cluster launch, with nothing between them but the control words.
+  const auto ahead_of = [&](int t, int nb, int max_beam) {
+    return may_run_ahead && !last_step(t) && t + 1 < c.max_steps && max_beam * nb <= kBlockRows && decoder_rows_apply(d, max_beam * nb) &&
+           (t > 0 || decoder_rows_apply(d, nb));
+  };
+  // What step t needs to know of its neighbours, while `active` and W are those of step t
+  const auto link_of = [&](int t, int nb, int max_beam, bool launched_ahead) {
+    StepLink link;
+    const int own = (t & 1) * 2 * kDecoderRowsMax, front = 2 * kDecoderRowsMax - own;
+    const bool ahead = ahead_of(t, nb, max_beam);
+    if(launched_ahead) {
+      link.stop = d->stops + (t & 1);
+      link.lists = d->s_tagged + front;
+      link.host_lists = d->h_tagged + front;
+      link.n_lists = 2 * nb * max_beam;
+    }
+    if(launched_ahead || ahead) {
+      link.tagged = (ahead ? d->s_tagged : d->h_tagged) + own;
+      d->tag = d->tag == 0xffffffffu ? 1u : d->tag + 1u;
+      link.tag = d->tag;
+    }
+    if(ahead) {
+      link.next_stop = d->stops + ((t + 1) & 1);
+      link.next_ctrl = d->s_ctrl[(t + 1) & 1];
+      link.eos = eos;
+      for(int a = 0; a < nb; ++a)
+        link.hyps[a] = static_cast<unsigned char>(W[active[a]]);
+    }
+    return link;
+  };
+  // Launches step t: hypotheses from the control words in s_ctrl[t & 1] (t > 0); the lists go to the step's half of h_out
+  const auto launch = [&](int t, int nb, int max_beam, const StepLink& link) {
+    const int tensor_beam = t == 0 ? 1 : max_beam, R = tensor_beam * nb, cells = nb * max_beam;
+    int *ctrl = d->s_ctrl[t & 1], *out = d->h_out + (t & 1) * 3 * c.max_batch * 8;
+    return run_step(d, t > 0 ? ctrl : nullptr, t > 0 ? ctrl + R : nullptr, t > 0 ? ctrl + 3 * R : nullptr,
+                    t > 0 ? reinterpret_cast<const float*>(ctrl + 2 * R) : nullptr, tensor_beam, nb, max_beam, reinterpret_cast<float*>(out), out + cells,
+                    out + 2 * cells, stream, link);
+  };
+  StepLink link, next_link;   // of the running step, and of the one launched ahead of it
+  bool launched = false;      // the running step was launched ahead, and stands
+  bool loose_end = false;     // the stream may still be at work
   clk::time_point mark = clk::now();
   for(int t = 0;; ++t) {
     int max_beam = 0;
@@ -1435,9 +1531,7 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
     const int n_best = max_beam;
     const int tensor_beam = t == 0 ? 1 : max_beam;
     const int R = tensor_beam * nb;
-    const int *hyp = nullptr, *pw = nullptr, *bidx = nullptr;
-    const float* ps = nullptr;
-    if(t > 0) {
+    if(t > 0 && !launched) {
       int* hc = d->h_ctrl;
       for(int j = 0; j < max_beam; ++j) {
         for(int a = 0; a < nb; ++a) {
@@ -1456,24 +1550,54 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
       d->step_ctrl = hc;
       d->n_step_ctrl = 3 * R + nb;
       up_bytes += n_up;
-      hyp = d->s_ctrl;
-      pw = d->s_ctrl + R;
-      ps = reinterpret_cast<const float*>(d->s_ctrl + 2 * R);
-      bidx = d->s_ctrl + 3 * R;
     }
     const int cells = nb * n_best;
-    // the step's last kernel writes the n-best lists straight into pinned host memory
-    float* o_score = reinterpret_cast<float*>(d->h_out);
-    int* o_beam = d->h_out + cells;
-    int* o_word = d->h_out + 2 * cells;
     const clk::time_point t_a = clk::now();
-    rc = mi8d_step(d, hyp, pw, bidx, ps, tensor_beam, nb, n_best, o_score, o_beam, o_word, stream);
-    d->step_ctrl = nullptr;
-    d->n_step_ctrl = 0;
-    if(rc != MI8_OK)
-      return rc;
+    if(launched) {
+      link = next_link;
+    } else {
+      link = link_of(t, nb, max_beam, false);
+      rc = launch(t, nb, max_beam, link);
+      d->step_ctrl = nullptr;
+      d->n_step_ctrl = 0;
+      if(rc != MI8_OK)
+        return rc;
+    }
+    const int was_t = d->t, was_cell = d->cell_cur, was_anc = d->anc_cur;
+    const bool ahead = link.next_ctrl != nullptr;
+    if(ahead) {
+      next_link = link_of(t + 1, nb, max_beam, true);
+      rc = launch(t + 1, nb, max_beam, next_link);
+      if(rc != MI8_OK)
+        return rc;
+    }
     const clk::time_point t_b = clk::now();
-    if(d->opt_blocking_wait == 2 && d->ev_step != nullptr) {
+    int* out = d->h_out + (t & 1) * 3 * c.max_batch * 8;
+    if(link.tagged != nullptr) {
+      const volatile unsigned long long* word = d->h_tagged + (t & 1) * 2 * kDecoderRowsMax;
+      const auto arrived = [&](int i) { return static_cast<unsigned>(word[i] >> 32) == link.tag; };
+      loose_end = true;
+      int i = 0;
+      for(unsigned spins = 1; i < 2 * cells; ++spins) {
+        while(i < 2 * cells && arrived(i))
+          ++i;
+        if(d->opt_blocking_wait == 2)
+          std::this_thread::yield();
+        if(i < 2 * cells && spins % 4096 == 0) {   // (a failed launch never writes the words)
+          const cudaError_t qe = cudaStreamQuery(s);
+          if(qe != cudaSuccess && qe != cudaErrorNotReady)
+            MI8D_CUDA(qe);
+          if(qe == cudaSuccess && !arrived(2 * cells - 1) && !arrived(i))
+            return MI8_ERR_DEVICE;
+        }
+      }
+      for(int e = 0; e < cells; ++e) {
+        const unsigned score = static_cast<unsigned>(word[2 * e]), key = static_cast<unsigned>(word[2 * e + 1]);
+        memcpy(out + e, &score, sizeof(float));
+        out[cells + e] = static_cast<int>(key / static_cast<unsigned>(c.vocab));
+        out[2 * cells + e] = static_cast<int>(key % static_cast<unsigned>(c.vocab));
+      }
+    } else if(d->opt_blocking_wait == 2 && d->ev_step != nullptr) {
       // several searches (and ranks) share the host's cores: poll, and hand the core to another thread between polls - as
       // quick as spinning while cores are free, fair when there are more waiting threads than cores
       MI8D_CUDA(cudaEventRecord(d->ev_step, s));
@@ -1481,12 +1605,15 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
       while((qe = cudaEventQuery(d->ev_step)) == cudaErrorNotReady)
         std::this_thread::yield();
       MI8D_CUDA(qe);
+      loose_end = false;
     } else if(d->opt_blocking_wait && d->ev_step != nullptr) {
       // sleep until the step's results have arrived (an interrupt wakes the thread: tens of microseconds later than polling)
       MI8D_CUDA(cudaEventRecord(d->ev_step, s));
       MI8D_CUDA(cudaEventSynchronize(d->ev_step));
+      loose_end = false;
     } else {
       MI8D_CUDA(cudaStreamSynchronize(s));
+      loose_end = false;
     }
     const clk::time_point t_c = clk::now();
     d->t_host += secs(mark, t_a);
@@ -1495,9 +1622,9 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
     d->n_steps += 1;
     mark = t_c;
     down_bytes += static_cast<size_t>(3 * cells) * sizeof(int);
-    const float* nv = reinterpret_cast<const float*>(d->h_out);
-    const int* nbm = d->h_out + cells;
-    const int* nw = d->h_out + 2 * cells;
+    const float* nv = reinterpret_cast<const float*>(out);
+    const int* nbm = out + cells;
+    const int* nw = out + 2 * cells;
 
     // toHyps: every sentence keeps its current number of hypotheses, skipping invalid scores
     std::fill(new_n.begin(), new_n.end(), 0);
@@ -1520,7 +1647,8 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
     }
     // purgeBeams and History::add
     const int length = t + 1;
-    const bool max_len_reached = static_cast<double>(length) >= static_cast<double>(sc->max_length_factor) * width;
+    const bool max_len_reached = last_step(t);
+    bool one_ended = false;   // (or one without a successor: what finish_step takes as a reason to stop)
     StepRecord rec;
     rec.words = new_words;
     rec.prev = new_prev;
@@ -1532,6 +1660,7 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
         if(new_words[o * beam + j] != eos)
           ++surv;
       new_W[o] = surv;
+      one_ended = one_ended || surv != W[o];
       const bool last = surv == 0 || max_len_reached;
       int rank = 0;
       for(int j = 0; j < new_n[o]; ++j) {
@@ -1546,6 +1675,12 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
       }
     }
     history.push_back(std::move(rec));
+    launched = ahead && !one_ended;
+    if(ahead && one_ended) {   // the step launched ahead is launched anew: its words were not these
+      d->t = was_t;
+      d->cell_cur = was_cell;
+      d->anc_cur = was_anc;
+    }
     if(max_len_reached)
       break;
     const StepRecord& cur = history.back();
@@ -1566,6 +1701,9 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
       step_map[active[a]] = a;
     prev_dim = nb;
   }
+
+  if(loose_end)
+    MI8D_CUDA(cudaStreamSynchronize(s));
 
   // best finished hypothesis per sentence (highest score; ties to the earlier step, then the earlier position), traced back
   for(int o = 0; o < B0; ++o) {

@@ -1162,6 +1162,7 @@ __device__ __forceinline__ void topk_block_merge(float* s_v, int* s_i) {
 // candidates before it; places that stay empty get score -inf, beam 0, word 0.  Block 0 also remembers, per layer, the history
 // abs-max the stored keys/values now belong to (prev_bits[l] = slots[first + l * stride]; stats: pairs unchanged, all pairs).
 // In place of two launches, each of a launch's hand-over (6 us together in a transformer-base step).
+// It also leaves the next step's control words where that step is launched already (StepEnd::next_ctrl).
 // The sentence's candidates lie in c_v / c_i: beam * k <= kStepEndCandidates (both launchers refuse more; mi8d_step then merges the
 // n-best lists with nbest_merge_kernel, which has no such limit).
 __device__ __forceinline__ void finish_step(const StepEnd& e, int r, int k, int vocab, const float* cand_score, const int* cand_word, float* c_v,
@@ -1189,6 +1190,17 @@ __device__ __forceinline__ void finish_step(const StepEnd& e, int r, int k, int 
   }
   if(threadIdx.x >= 32)
     return;
+  const auto store_entry = [&](int place, float score, int from, int word, int key) {
+    if(e.tagged != nullptr) {
+      volatile unsigned long long* at = e.tagged + 2 * (b * k + place);
+      at[0] = static_cast<unsigned long long>(e.tag) << 32 | __float_as_uint(score);
+      at[1] = static_cast<unsigned long long>(e.tag) << 32 | static_cast<unsigned>(key);
+    } else {
+      e.out_score[b * k + place] = score;
+      e.out_beam[b * k + place] = from;
+      e.out_word[b * k + place] = word;
+    }
+  };
   const int n = e.beam * k;
   int valid = 0;
   for(int c0 = 0; c0 < n; c0 += 32) {
@@ -1215,16 +1227,35 @@ __device__ __forceinline__ void finish_step(const StepEnd& e, int r, int k, int 
       for(int o = 0; o < n; ++o)
         place += (c_v[o] > -FLT_MAX && better(c_v[o], c_i[o], v, key)) ? 1 : 0;
       if(place < k) {
-        e.out_score[b * k + place] = v;
-        e.out_beam[b * k + place] = key / vocab;
-        e.out_word[b * k + place] = key % vocab;
+        const int from = key / vocab, word = key % vocab;
+        store_entry(place, v, from, word, key);
+        if(e.next_ctrl != nullptr && place < e.hyps[b]) {
+          int* next = e.next_ctrl + place * e.batch + b;
+          next[0] = from * e.batch + b;
+          next[k * e.batch] = word;
+          next[2 * k * e.batch] = __float_as_int(v);
+          if(word == e.eos)
+            *e.next_stop = 1u;
+        }
       }
     }
   }
   for(int c = valid + threadIdx.x; c < k; c += 32) {
-    e.out_score[b * k + c] = -INFINITY;
-    e.out_beam[b * k + c] = 0;
-    e.out_word[b * k + c] = 0;
+    store_entry(c, -INFINITY, 0, 0, 0);
+  }
+  if(e.next_ctrl != nullptr) {
+    const int alive = e.hyps[b];
+    for(int c = alive + threadIdx.x; c < k; c += 32) {   // (no hypothesis: end of sentence and score -inf)
+      int* next = e.next_ctrl + c * e.batch + b;
+      next[0] = 0;
+      next[k * e.batch] = e.eos;
+      next[2 * k * e.batch] = __float_as_int(-INFINITY);
+    }
+    if(threadIdx.x == 0) {
+      e.next_ctrl[3 * k * e.batch + b] = b;
+      if(valid < alive)
+        *e.next_stop = 1u;
+    }
   }
 }
 
@@ -1288,6 +1319,8 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
   pdl_wait();
+  if(end.stop != nullptr && *end.stop != 0u)
+    return;
   trace_stamp_start(th, kTrLseTopk);
   extern __shared__ float lse_blocks[];   // [nb] block maxima, [nb] block sums
   static_assert(kStepEndCandidates <= kMaxK * 128, "finish_step reuses these arrays");

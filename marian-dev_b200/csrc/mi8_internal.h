@@ -176,6 +176,7 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
                    float* c, int32_t* acc_out, void* ws, size_t ws_bytes, cudaStream_t stream, int force_tile_m, int force_splits,
                    const P8Segments* segs = nullptr, float* block_max = nullptr, float* block_sum = nullptr);
 
+constexpr int kDecoderRowsMax = 32;   // rows of a step that launch_decoder_rows takes
 // What the last kernel of a decoder step does besides the rows' candidates: the n-best lists of the sentences (arrivals != nullptr; one
 // zeroed counter per sentence; the outputs may be pinned host memory) and the record of the history abs-max per layer (layers > 0).
 struct StepEnd {
@@ -188,6 +189,19 @@ struct StepEnd {
   const unsigned* slots = nullptr;
   unsigned* prev_bits = nullptr;
   unsigned* stats = nullptr;
+  // A step whose successor is launched before the host has seen its n-best lists (mi8d_search, few rows): the control words of the successor, which are
+  // those of the lists as long as no hypothesis ends - otherwise `next_stop` is set, and the successor does nothing.  hyps: hypotheses of each sentence that
+  // are alive, of k.  stop: this step itself is such a successor.  tagged ([batch * k][2], in the place of the three lists): an entry's score and its
+  // beam * vocab + word, each below `tag`, so that the host sees when a word is new.  With a successor they stay on the device and its first kernel brings
+  // them to the host (DecoderRowsParams::lists): stores to the host held the end of this kernel, and with it the successor, up (student, one sentence: 9.0 us
+  // with a fence and a flag behind them, 7.8 with tagged words alone, 6.9 so).
+  int* next_ctrl = nullptr;   // hypothesis rows, previous words, path scores [k * batch] each, batch rows [batch]
+  unsigned* next_stop = nullptr;
+  const unsigned* stop = nullptr;
+  unsigned long long* tagged = nullptr;
+  unsigned tag = 0;
+  int eos = 0;
+  unsigned char hyps[kDecoderRowsMax] = {};
 };
 // Candidates of one sentence (beam x k) that the row kernels' shared memory holds; wider beams end with launch_nbest_merge.
 constexpr int kStepEndCandidates = 1024;
@@ -254,7 +268,7 @@ int launch_ssru_cell(const float* cell_old, const int* hyp, const float* xw, con
                      float* h_out, cudaStream_t s);
 
 // The layers of an SSRU decoder's step for few rows in one launch (mi8_rows.cu).
-constexpr int kDecoderRowsLayers = 4, kDecoderRowsMax = 32, kRowsMultipliers = 6;
+constexpr int kDecoderRowsLayers = 4, kRowsMultipliers = 6;
 // A layer's parameters apart from the matrices, read from here by every launch; 16-byte aligned but for the multipliers.
 struct DecoderRowsVectors {
   const float* qb[kRowsMultipliers];   // multipliers of W, Wf, Wq, Wo, W1, W2
@@ -274,6 +288,11 @@ struct DecoderRowsParams {
   int* ctrl = nullptr;
   int n_ctrl = 0, n_slots = 0;
   unsigned* slots = nullptr;    // zeroed
+  const unsigned* stop = nullptr;   // optional: the launch does nothing where this word is set (StepEnd)
+  unsigned* next_stop = nullptr;    // optional: zeroed
+  const unsigned long long* lists = nullptr;   // optional: what the step in front left for the host (StepEnd::tagged), and where it goes
+  unsigned long long* host_lists = nullptr;
+  int n_lists = 0;
   int8_t* out_q = nullptr;      // [rows, d] the last LayerNorm's result, quantised, and its multiplier
   float* out_qm = nullptr;
   int* status = nullptr;

@@ -153,57 +153,7 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
   pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
 
-  pdl_wait();
-  trace_stamp_start(th, kTrDecoderRows);
-  // (Nothing is gained by set-up before the wait: the host has waited for the preceding step.  The loads go first, the set-up hides them.)
-  // ---- embedding * sqrt(d) + position, and the cells' previous state.  The control words come with the launch's parameters, which are
-  // there at once (reads of pinned memory by every CTA went over PCIe lane by lane: 16 rows 250 us), or from the device.
-  const bool with_words = p.n_ctrl > 0;
-  float4 x[kRw][kNv];
-#pragma unroll
-  for(int i = 0; i < kRw; ++i) {
-    const int r = warp + i * kWarps;
-    if(r < R) {
-      const int word = with_words ? p.ctrl_words[R + r] : (p.words ? p.words[r] : -1);
-      const float4* src = reinterpret_cast<const float4*>(p.wemb + static_cast<size_t>(max(word, 0)) * kDim) + lane;
-#pragma unroll
-      for(int v = 0; v < kNv; ++v)
-        x[i][v] = word >= 0 ? __ldg(src + 32 * v) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-#pragma unroll 1
-  for(int l = 0; l < p.layers; ++l)
-#pragma unroll 1
-    for(int i = threadIdx.x; i < R * (kNd / 4); i += kThreads) {
-      const int r = i / (kNd / 4), c = 4 * (i % (kNd / 4));
-      const int src = with_words ? p.ctrl_words[r] : (p.hyp ? p.hyp[r] : r);
-      copy_async16(cell + (l * R + r) * kNd + c, p.cell_old + l * p.layer_stride + static_cast<size_t>(src) * kDim + rank * kNd + c);
-    }
-  // The LayerNorms, this CTA's columns of the biases and the weights' multipliers, from where they were registered: a caller may rewrite
-  // them between steps.
-#pragma unroll 1
-  for(int l = 0; l < p.layers; ++l) {
-    const DecoderRowsVectors& v = p.vec[l];
-    float* own = prm + l * T::params(f);
-    constexpr int kLn = kDim / 4, kOwn = kNd / 4;   // 16-byte chunks
-#pragma unroll 1
-    for(int i = threadIdx.x; i < 6 * kLn + 3 * kOwn + (kNq + nf) / 4; i += kThreads) {
-      const int c = i - 6 * kLn, q = c - 3 * kOwn;
-      if(c < 0)
-        copy_async16(norms + l * T::kNorms + 4 * i, v.ln[i / kLn] + 4 * (i % kLn));
-      else if(q < 0)
-        copy_async16(own + 4 * c, v.own[c / kOwn] + rank * kNd + 4 * (c % kOwn));
-      else
-        copy_async16(own + 4 * c, q < kNq / 4 ? v.b_q + head0 * kDh + 4 * q : v.b_1 + rank * nf + 4 * q - kNq);
-    }
-    if(threadIdx.x < kRowsMultipliers)
-      copy_async4(own + 3 * kNd + kNq + nf + threadIdx.x, v.qb[threadIdx.x]);
-  }
-  float4 pv[kNv];
-#pragma unroll
-  for(int v = 0; v < kNv; ++v)
-    pv[v] = __ldg(reinterpret_cast<const float4*>(p.pos) + 32 * v + lane);
-
+  // ---- what does not depend on the kernel in front
   // ---- the weight stream: lane k knows the warp's k-th unit
   const CUtensorMap* my_map = nullptr;
   int my_row = 0, my_unit = -1;   // first weight row; phase | m tile << 8 | K block << 16, phase counted over the layers
@@ -248,11 +198,85 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
   uint32_t parity = 0;
   bool ok = true;
 
+  // The LayerNorms, this CTA's columns of the biases and the weights' multipliers, from where they were registered: a caller may rewrite
+  // them between steps (the kernels in front of a step do not write them).
+#pragma unroll 1
+  for(int l = 0; l < p.layers; ++l) {
+    const DecoderRowsVectors& v = p.vec[l];
+    float* own = prm + l * T::params(f);
+    constexpr int kLn = kDim / 4, kOwn = kNd / 4;   // 16-byte chunks
+#pragma unroll 1
+    for(int i = threadIdx.x; i < 6 * kLn + 3 * kOwn + (kNq + nf) / 4; i += kThreads) {
+      const int c = i - 6 * kLn, q = c - 3 * kOwn;
+      if(c < 0)
+        copy_async16(norms + l * T::kNorms + 4 * i, v.ln[i / kLn] + 4 * (i % kLn));
+      else if(q < 0)
+        copy_async16(own + 4 * c, v.own[c / kOwn] + rank * kNd + 4 * (c % kOwn));
+      else
+        copy_async16(own + 4 * c, q < kNq / 4 ? v.b_q + head0 * kDh + 4 * q : v.b_1 + rank * nf + 4 * q - kNq);
+    }
+    if(threadIdx.x < kRowsMultipliers)
+      copy_async4(own + 3 * kNd + kNq + nf + threadIdx.x, v.qb[threadIdx.x]);
+  }
+  float4 pv[kNv];
+#pragma unroll
+  for(int v = 0; v < kNv; ++v)
+    pv[v] = __ldg(reinterpret_cast<const float4*>(p.pos) + 32 * v + lane);
+
 #pragma unroll 1
   for(int i = threadIdx.x; i < Rp * (T::acc_cols(f) + 4) / 4; i += kThreads)
     reinterpret_cast<int4*>(acc)[i] = make_int4(0, 0, 0, 0);
   if(threadIdx.x == 0)
     abort_word = 0;
+  pdl_wait();
+  trace_stamp_start(th, kTrDecoderRows);
+  // ---- embedding * sqrt(d) + position, and the cells' previous state.  The control words come with the launch's parameters, which are
+  // there at once (reads of pinned memory by every CTA went over PCIe lane by lane: 16 rows 250 us), or from the device, where the step in front left
+  // them (StepEnd::next_ctrl): launched before the host has seen that step's words, this one has its weights under way when they come.
+  const bool with_words = p.n_ctrl > 0;
+  int word[kRw];
+  const unsigned stopped = p.stop != nullptr ? *p.stop : 0u;   // (looked at once the loads beside it are under way)
+#pragma unroll
+  for(int i = 0; i < kRw; ++i) {
+    const int r = min(warp + i * kWarps, R - 1);
+    word[i] = with_words ? p.ctrl_words[R + r] : (p.words ? p.words[r] : -1);
+  }
+  const int own_row = min(static_cast<int>(threadIdx.x) / (kNd / 4), R - 1);
+  const int own_src = with_words ? p.ctrl_words[own_row] : (p.hyp ? p.hyp[own_row] : own_row);
+  const bool brings = rank == kCtas - 1 && static_cast<int>(threadIdx.x) < p.n_lists;
+  const unsigned long long entry = brings ? p.lists[threadIdx.x] : 0ull;
+  auto bring = [&]() {   // the lists of the step in front, to the host
+    if(brings)
+      const_cast<volatile unsigned long long*>(p.host_lists)[threadIdx.x] = entry;
+  };
+  if(stopped != 0u) {   // (the same word for every CTA) a hypothesis has ended: the host launches this step anew
+    int no_abort = 0;
+    for(int i = 0; i < requested; ++i)
+      mbar_wait_bounded(&full[warp][i], 0u, &no_abort, p.spin_limit);
+    copy_async_wait();
+    bring();
+    return;
+  }
+  float4 x[kRw][kNv];
+#pragma unroll
+  for(int i = 0; i < kRw; ++i) {
+    const int r = warp + i * kWarps;
+    if(r < R) {
+      const float4* src = reinterpret_cast<const float4*>(p.wemb + static_cast<size_t>(max(word[i], 0)) * kDim) + lane;
+#pragma unroll
+      for(int v = 0; v < kNv; ++v)
+        x[i][v] = word[i] >= 0 ? __ldg(src + 32 * v) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+#pragma unroll 1
+  for(int l = 0; l < p.layers; ++l)
+#pragma unroll 1
+    for(int i = threadIdx.x; i < R * (kNd / 4); i += kThreads) {
+      const int r = i / (kNd / 4), c = 4 * (i % (kNd / 4));
+      const int src = i < kThreads ? own_src : with_words ? p.ctrl_words[r] : (p.hyp ? p.hyp[r] : r);
+      copy_async16(cell + (l * R + r) * kNd + c, p.cell_old + l * p.layer_stride + static_cast<size_t>(src) * kDim + rank * kNd + c);
+    }
+  bring();
   __syncthreads();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (this CTA runs: the others may store into it)
 
@@ -322,6 +346,8 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
   if(rank == 0) {   // for the kernels behind this one
     for(int i = threadIdx.x; i < p.n_ctrl; i += kThreads)
       p.ctrl[i] = p.ctrl_words[i];
+    if(threadIdx.x == 0 && p.next_stop != nullptr)
+      *p.next_stop = 0u;
     for(int i = threadIdx.x; i < p.n_slots; i += kThreads)
       p.slots[i] = 0u;
   }
