@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cuda_fp16.h>
+#include <type_traits>
 
 #include <vector>
 
@@ -130,6 +131,7 @@ struct GemmParams {
   int* rows_computed;       // optional (measurement): receives the number of activation rows this launch really computed
   int withhold_item;        // test hook: the producer leaves out the loads of this one of its stages (-1 = none; or kWithholdWarp)
   uint32_t spin_limit;      // bound of every barrier wait of this launch
+  int pair_items, pair_whole;   // kHalves: the CTA-pair kernel's items, and how many of them are whole tiles
 };
 
 // (A launch of one matrix carries one map: what a launch's parameters take is paid by each of a decoder's launches.)
@@ -1028,6 +1030,10 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
 //     asks for, it is at 4096 x 768 x 32000 into half 94.5 us against 104.6 of the 256-row tiles that the plan takes, at 4096 x 512 x 16000 into float level.
 //     A held block is overwritten without a barrier of its own: the ring has no more stages than the tile has pairs of K blocks, so the wait
 //     for a ring stage covers the last MMA that read the block.
+//   * kHalves: where the last wave of tiles has one for no more than half of the pairs, each of those is two items of 128 activation rows (MMAs of half the
+//     width; both CTAs still load a box of 128 rows and use half of it), so that the wave is shorter: 5000 x 2048 x 2048 24.4 -> 23.45 us, 512 x 1024 x 32000
+//     24.5 -> 23.5, 3937 x 1024 x 4096 22.2 -> 21.7, 6000 x 1024 x 1024 13.25 -> 12.4.  A kernel of its own: as a case of the one above it cost every launch
+//     0.2 us.  A half takes more than half a tile's time: with the first wave in halves as well, whose stores then begin earlier, 22.2 -> 23.8.
 struct PairCfg {
   static constexpr int kTM = 256;             // activation rows per pair tile (MMA N)
   static constexpr int kHalfRows = 128;       // activation rows each CTA loads
@@ -1047,7 +1053,7 @@ constexpr int smem_bytes_pair(bool resident = false) {
 }
 static_assert(PairCfg::kABytes == PairCfg::kWBytes && smem_bytes_pair(true) <= 227 * 1024, "");
 
-template <bool kP8, int kMaps, bool kResident>
+template <bool kP8, int kMaps, bool kResident, bool kHalves>
 __global__ void __launch_bounds__(kThreads, 1)
 mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
   using T = PairCfg;
@@ -1069,22 +1075,26 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
   const uint32_t stages = kResident ? static_cast<uint32_t>(min(kStages, (p.kb_total + kPer - 1) / kPer)) : kStages;
   // The pair's tiles: every n_pairs-th one, or (kResident) an even share of neighbours, those of the same weights first.
   struct Tiles {
-    int first, end, step, m_first, m_count;
+    int first, end, step, m_first, m_count, whole;   // whole: items below it are whole tiles
   };
   auto my_tiles = [&](bool skip_on) -> Tiles {
+    if(kHalves)
+      return {pair_id, p.pair_items, n_pairs, 0, p.m_tiles, p.pair_whole};
     const int skipped = skip_on ? min(p.m_tiles, max(p.skip_rows_below, 0) / T::kTM) : 0, left = p.m_tiles - skipped;
     const long long count = static_cast<long long>(left) * p.n_tiles;
     if(!kResident)
-      return {pair_id, static_cast<int>(count), n_pairs, skipped, left};
-    return {static_cast<int>(count * pair_id / n_pairs), static_cast<int>(count * (pair_id + 1) / n_pairs), 1, skipped, left};
+      return {pair_id, static_cast<int>(count), n_pairs, skipped, left, 0x7fffffff};
+    return {static_cast<int>(count * pair_id / n_pairs), static_cast<int>(count * (pair_id + 1) / n_pairs), 1, skipped, left, 0x7fffffff};
   };
   struct Tile {
-    int n_tile, m_tile;
+    int n_tile, m0, rows;   // first activation row, and how many
   };
   auto tile_at = [&](const Tiles& t, int w) -> Tile {
     if(kResident)
-      return {w / t.m_count, t.m_first + w % t.m_count};
-    return {w % p.n_tiles, t.m_first + w / p.n_tiles};
+      return {w / t.m_count, (t.m_first + w % t.m_count) * T::kTM, T::kTM};
+    const bool half = kHalves && w >= t.whole;
+    const int at = half ? t.whole + ((w - t.whole) >> 1) : w;
+    return {at % p.n_tiles, (t.m_first + at / p.n_tiles) * T::kTM + (half && ((w - t.whole) & 1) ? T::kTM / 2 : 0), half ? T::kTM / 2 : T::kTM};
   };
   const uint32_t peer_abort = mapa_shared(smem_u32(&ctl->abort), rank ^ 1u);
 
@@ -1155,7 +1165,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
       // (both CTAs' weight rows lie in one segment, or all segments share the activation: launch_gemm_call sees to it)
       const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, (2 * wi.n_tile + static_cast<int>(rank)) * kTileN);
       const int a_row0 = p.seg_row0[p.nseg > 1 ? (2 * wi.n_tile * kTileN) / p.seg_n : 0];
-      const int a_row = a_row0 + wi.m_tile * T::kTM;
+      const int a_row = a_row0 + wi.m0 + static_cast<int>(rank) * (kHalves ? wi.rows / 2 : T::kHalfRows);   // this CTA's half of the tile's rows (of a half tile's box the first half is used)
       const bool fetch_w = !kResident || held != wi.n_tile;
       held = wi.n_tile;
       for(int kb = 0; kb < p.kb_total; kb += kPer, ++it) {
@@ -1173,7 +1183,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
             uint8_t* const st = tiles + s * kStageBytes + b * kRingBlock;
             if(!pre && fetch_w)
               tma_load_2d_pair(kResident ? resident + (kb + b) * T::kWBytes : st, wr.map, (kb + b) * kTileKBytes, wr.row, full_addr(s));
-            tma_load_2d_pair(kResident ? st : st + T::kWBytes, &tmap_a, (kb + b) * kTileKBytes, a_row + static_cast<int>(rank) * T::kHalfRows, full_addr(s));
+            tma_load_2d_pair(kResident ? st : st + T::kWBytes, &tmap_a, (kb + b) * kTileKBytes, a_row, full_addr(s));
           }
         }
         __syncwarp();
@@ -1201,7 +1211,8 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
   } else if(warp == 1) {
     // ------------------------------------------------------------ MMA issuer (rank 0 only; rank 1 owns its TMEM half)
     if(leader) {
-      constexpr uint32_t idesc = kP8 ? make_idesc_i8_ub(T::kTM, 256) : make_idesc_i8(T::kTM, 256);
+      constexpr uint32_t idesc_whole = kP8 ? make_idesc_i8_ub(T::kTM, 256) : make_idesc_i8(T::kTM, 256);
+      constexpr uint32_t idesc_half = kP8 ? make_idesc_i8_ub(T::kTM / 2, 256) : make_idesc_i8(T::kTM / 2, 256);
       uint32_t s = 0, ph = 0, acc_it = 0;
       bool ready = false;   // the next stage, when it was last looked at
       pdl_wait();   // as in the single-CTA kernel: keeps the predecessor's run time out of the bounded waits
@@ -1215,33 +1226,39 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
           break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + as * T::kAccStride;
-        for(int kb = 0; kb < p.kb_total; kb += kPer) {
-          if(!__all_sync(0xffffffffu, ready))
-            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&ctl->full[s], ph, abort_flag, p.spin_limit));
-          if(!ok)
-            break;
-          tc_fence_after_sync();
-          const uint32_t s_next = s + 1 == stages ? 0 : s + 1, ph_next = s + 1 == stages ? ph ^ 1u : ph;
-          ready = mbar_test_wait(&ctl->full[s_next], ph_next);
-          const uint32_t st = smem_u32(tiles + s * kStageBytes);
-          const uint32_t w_addr = kResident ? smem_u32(resident + kb * T::kWBytes) : st, a_addr = kResident ? st : st + T::kWBytes;
-          const bool both = kPer > 1 && kb + 1 < p.kb_total;
-          if(elect_one()) {
+        auto blocks = [&](auto idesc) {   // (the descriptor a constant: a register would be moved to the uniform ones for every MMA)
+          for(int kb = 0; kb < p.kb_total; kb += kPer) {
+            if(!__all_sync(0xffffffffu, ready))
+              ok = __all_sync(0xffffffffu, mbar_wait_bounded(&ctl->full[s], ph, abort_flag, p.spin_limit));
+            if(!ok)
+              break;
+            tc_fence_after_sync();
+            const uint32_t s_next = s + 1 == stages ? 0 : s + 1, ph_next = s + 1 == stages ? ph ^ 1u : ph;
+            ready = mbar_test_wait(&ctl->full[s_next], ph_next);
+            const uint32_t st = smem_u32(tiles + s * kStageBytes);
+            const uint32_t w_addr = kResident ? smem_u32(resident + kb * T::kWBytes) : st, a_addr = kResident ? st : st + T::kWBytes;
+            const bool both = kPer > 1 && kb + 1 < p.kb_total;
+            if(elect_one()) {
 #pragma unroll
-            for(int b = 0; b < kPer; ++b) {
-              if(b == 0 || both) {
+              for(int b = 0; b < kPer; ++b) {
+                if(b == 0 || both) {
 #pragma unroll
-                for(int k = 0; k < kTileKBytes / kMmaK; ++k)
-                  tc_mma_i8_pair(d_tmem, make_kmajor_sw128_desc(w_addr + b * T::kWBytes + k * kMmaK), make_kmajor_sw128_desc(a_addr + b * T::kABytes + k * kMmaK),
-                                 idesc, (kb > 0 || b > 0 || k > 0) ? 1u : 0u);
+                  for(int k = 0; k < kTileKBytes / kMmaK; ++k)
+                    tc_mma_i8_pair(d_tmem, make_kmajor_sw128_desc(w_addr + b * T::kWBytes + k * kMmaK), make_kmajor_sw128_desc(a_addr + b * T::kABytes + k * kMmaK),
+                                   decltype(idesc)::value, (kb > 0 || b > 0 || k > 0) ? 1u : 0u);
+                }
               }
+              tc_commit_pair(&ctl->empty[s], 3);  // frees this slot in both CTAs once the MMAs have read it
             }
-            tc_commit_pair(&ctl->empty[s], 3);  // frees this slot in both CTAs once the MMAs have read it
+            __syncwarp();
+            s = s_next;
+            ph = ph_next;
           }
-          __syncwarp();
-          s = s_next;
-          ph = ph_next;
-        }
+        };
+        if(!kHalves || w < mine.whole)
+          blocks(std::integral_constant<uint32_t, idesc_whole>());
+        else
+          blocks(std::integral_constant<uint32_t, idesc_half>());
         if(!ok)
           break;
         if(elect_one())
@@ -1278,8 +1295,8 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
       const Tile wi = tile_at(mine, w);
       const int n = (2 * wi.n_tile + static_cast<int>(rank)) * kTileN + row;
       const bool n_ok = n < p.N;
-      const int m0 = wi.m_tile * T::kTM;
-      const int cols_valid = min(T::kTM, p.M - m0);
+      const int m0 = wi.m0;
+      const int cols_valid = min(kHalves ? wi.rows : T::kTM, p.M - m0);
       int seg = 0, n_loc = n;
       if(kP8 ? kMaps > 1 : p.nseg > 1) {
         // (an odd number of 128-row weight tiles: the second CTA of the last pair has none, and stores nothing (n_ok))
@@ -2075,7 +2092,7 @@ bool holds_weights(const GemmParams& p) {
 }
 
 // Launch of the CTA-pair kernel: clusters of two CTAs, as many as can be resident at once.
-template <bool kP8, int kMaps, bool kResident>
+template <bool kP8, int kMaps, bool kResident, bool kHalves>
 int launch_pair_as(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
   static bool attr_set[64] = {};
   static int max_clusters[64] = {};
@@ -2097,7 +2114,7 @@ int launch_pair_as(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, cons
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   if(!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(mi8_gemm_pair_kernel<kP8, kMaps, kResident>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(mi8_gemm_pair_kernel<kP8, kMaps, kResident, kHalves>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if(e != cudaSuccess) {
       set_last_cuda_error(e);
       return MI8_ERR_LAUNCH;
@@ -2106,7 +2123,7 @@ int launch_pair_as(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, cons
     cfg.gridDim = dim3(2 * (sm_count() / 2));
     cfg.numAttrs = 1;
     int n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, mi8_gemm_pair_kernel<kP8, kMaps, kResident>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&n, mi8_gemm_pair_kernel<kP8, kMaps, kResident, kHalves>, &cfg);
     if(e != cudaSuccess || n <= 0) {
       set_last_cuda_error(e);
       cudaGetLastError();
@@ -2128,9 +2145,9 @@ int launch_pair_as(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, cons
   const bool timed = kernel_times_on();
   if(timed) {
     cfg.numAttrs = 1;   // no launch overlap while per-kernel times are taken
-    kernel_times_before(reinterpret_cast<const void*>(mi8_gemm_pair_kernel<kP8, kMaps, kResident>), stream);
+    kernel_times_before(reinterpret_cast<const void*>(mi8_gemm_pair_kernel<kP8, kMaps, kResident, kHalves>), stream);
   }
-  cudaError_t le = cudaLaunchKernelEx(&cfg, mi8_gemm_pair_kernel<kP8, kMaps, kResident>, tw, ta, p);
+  cudaError_t le = cudaLaunchKernelEx(&cfg, mi8_gemm_pair_kernel<kP8, kMaps, kResident, kHalves>, tw, ta, p);
   if(timed)
     kernel_times_after(stream);
   if(le != cudaSuccess) {
@@ -2147,7 +2164,18 @@ int launch_pair_as(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, cons
 
 template <bool kP8 = false, int kMaps = 1>
 int launch_pair(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
-  return holds_weights(p) ? launch_pair_as<kP8, kMaps, true>(tw, ta, p, plan, stream) : launch_pair_as<kP8, kMaps, false>(tw, ta, p, plan, stream);
+  if(holds_weights(p))
+    return launch_pair_as<kP8, kMaps, true, false>(tw, ta, p, plan, stream);
+  if constexpr(!kP8) {
+    const int pairs = plan.grid / 2, all = p.n_tiles * p.m_tiles, last = all % pairs;
+    if(p.skip_a == nullptr && all > pairs && last > 0 && 2 * last <= pairs) {
+      GemmParams halves = p;
+      halves.pair_items = all + last;
+      halves.pair_whole = all - last;
+      return launch_pair_as<kP8, kMaps, false, true>(tw, ta, halves, plan, stream);
+    }
+  }
+  return launch_pair_as<kP8, kMaps, false, false>(tw, ta, p, plan, stream);
 }
 
 template <int kMaps>
