@@ -363,7 +363,6 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  pdl_launch_dependents();  // the next kernel on the stream may begin its own set-up now
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
   constexpr int kTraceId = kTopK > 0 ? kTrGemmLogits : (kQuantA ? kTrGemmQuantA : kTrGemm);
@@ -421,7 +420,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
       __syncwarp();
       prefetched = n_pre;
     }
-    pdl_wait();
+    pdl_wait_and_launch();
     const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
     if(p.rows_computed != nullptr && blockIdx.x == 0 && lane == 0)
       *p.rows_computed = p.M - (skip_on ? min(p.M, (p.skip_rows_below / TM) * TM) : 0);
@@ -476,7 +475,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
     // No MMA can be issued before the activation tiles arrive, and those are requested after the producer's
     // pdl_wait(): waiting here as well costs nothing and keeps the predecessor's run time out of the bounded
     // waits below (it also orders the read of the skip words, which earlier kernels of the stream write).
-    pdl_wait();
+    pdl_wait_and_launch();
     const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
     for(int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x) {
       const WorkItem wi = decode_work(p, w);
@@ -541,7 +540,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
     constexpr int kChunks = TM / T::kChunk;
     constexpr int kChunkStep = kChunks > 1 ? 2 : 1;
     const bool has_chunks = kChunks > 1 || group == 0;
-    pdl_wait();  // the activation multiplier (or abs-max slot) is written by the previous kernel
+    pdl_wait_and_launch();  // the activation multiplier (or abs-max slot) is written by the previous kernel
     trace_stamp_start(th, kTraceId, trace_extra);
     // kQuantA: the multiplier comes from the abs-max slot, which is read only after the first fp32 loads of the
     // activation have been issued (below), so the two round trips to L2 overlap instead of following one another.
@@ -1098,7 +1097,6 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
   };
   const uint32_t peer_abort = mapa_shared(smem_u32(&ctl->abort), rank ^ 1u);
 
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
   const unsigned long long trace_extra = static_cast<unsigned long long>(p.N) | (static_cast<unsigned long long>(p.K) << 20) |
@@ -1155,7 +1153,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
       __syncwarp();
       prefetched = n_pre;
     }
-    pdl_wait();
+    pdl_wait_and_launch();
     const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
     if(p.rows_computed != nullptr && blockIdx.x == 0 && lane == 0)
       *p.rows_computed = p.M - (skip_on ? min(p.M, (p.skip_rows_below / T::kTM) * T::kTM) : 0);
@@ -1215,7 +1213,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
       constexpr uint32_t idesc_half = kP8 ? make_idesc_i8_ub(T::kTM / 2, 256) : make_idesc_i8(T::kTM / 2, 256);
       uint32_t s = 0, ph = 0, acc_it = 0;
       bool ready = false;   // the next stage, when it was last looked at
-      pdl_wait();   // as in the single-CTA kernel: keeps the predecessor's run time out of the bounded waits
+      pdl_wait_and_launch();   // as in the single-CTA kernel: keeps the predecessor's run time out of the bounded waits
       const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
       const Tiles mine = my_tiles(skip_on);
       for(int w = mine.first; w < mine.end && ok; w += mine.step) {
@@ -1281,7 +1279,7 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
     const int row = quarter * 32 + lane;
     const int epi_tid = threadIdx.x - 64;
     constexpr int kChunks = T::kTM / T::kChunk;
-    pdl_wait();
+    pdl_wait_and_launch();
     trace_stamp_start(th, kTrGemmPair, trace_extra);
     const float qa = kP8 ? 1.0f : *p.d_qa;
     float unquant = kP8 ? 1.0f : __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(qa, *p.seg_qb[0])), p.scale);
@@ -1505,7 +1503,6 @@ mi8_gemm_cq_kernel(const __grid_constant__ CUtensorMap tmap_w, const CqParams p)
   const int n_tile = blockIdx.x;
   const int m0 = blockIdx.y * TM;
 
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
   const unsigned long long trace_extra = static_cast<unsigned long long>(p.N) | (static_cast<unsigned long long>(p.K) << 20);
@@ -1593,7 +1590,7 @@ mi8_gemm_cq_kernel(const __grid_constant__ CUtensorMap tmap_w, const CqParams p)
     const int quarter = warp & 3;
     const int group = (warp - 2) >> 2;
     const int row = quarter * 32 + lane;
-    pdl_wait();   // the activation and its abs-max slot are the preceding kernel's output
+    pdl_wait_and_launch();   // the activation and its abs-max slot are the preceding kernel's output
     trace_stamp_start(th, kTrGemmCq, trace_extra);
     if(p.rows_computed != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && epi_tid == 0)
       *p.rows_computed = p.M;

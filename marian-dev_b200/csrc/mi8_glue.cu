@@ -75,10 +75,9 @@ __device__ __forceinline__ void embed_row(int r, const float* __restrict__ wemb,
 __global__ void __launch_bounds__(kRowThreads)
 embed_kernel(const float* __restrict__ wemb, const int* __restrict__ words, const float* __restrict__ pos, int pos_mod, float scale,
              int dim, float* __restrict__ out, float* __restrict__ rowmax, unsigned* absmax_slot) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrEmbed);
   __shared__ unsigned red[kRowThreads / 32];
   embed_row(blockIdx.x, wemb, words, pos, pos_mod, scale, dim, out, rowmax, absmax_slot, nullptr, red);
@@ -93,9 +92,8 @@ embed_kernel(const float* __restrict__ wemb, const int* __restrict__ words, cons
 // student, 16 x beam 4 6.80 -> 6.55 ms; transformer-base, 16 x beam 4 19.27 -> 19.08 ms; transformer-big level.
 __global__ void __launch_bounds__(1024)
 step_begin_kernel(const int* host_ctrl, int* __restrict__ ctrl, int n_ctrl, unsigned* __restrict__ slots, int n_slots) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrStepBegin);
   for(int i = threadIdx.x; i < n_slots; i += blockDim.x)
     slots[i] = 0u;
@@ -115,14 +113,17 @@ step_begin_kernel(const int* host_ctrl, int* __restrict__ ctrl, int n_ctrl, unsi
 //   s_t = sum_j ((y0 + y1) + (y2 + y3));  mean = block256_sum(s) / dim;
 //   q_t = sum_j fma(d0,d0, fma(d1,d1, fma(d2,d2, d3*d3))), d = y - mean;  var = block256_sum(q) / dim;
 //   out = ((y - mean) / sqrt(var + eps)) * gamma + beta.
+constexpr unsigned kEarlyRows = 320;   // beyond, the next kernel may begin at once: transformer-big, 128 x beam 4 (512 rows) 39.05 ms, 39.35 behind the wait; 200 rows of it
+                                       // 15.32 and 15.17, transformer-base, 64 x beam 4 (256 rows) 30.6 and 30.43
 __global__ void __launch_bounds__(kRowThreads)
 add_layernorm_kernel(const float* __restrict__ a, const float* __restrict__ resid, const float* __restrict__ gamma,
                      const float* __restrict__ beta, float eps, int dim, float* __restrict__ out, float* __restrict__ rowmax,
                      unsigned* absmax_slot, unsigned* absmax_slot2) {
-  pdl_launch_dependents();
+  if(gridDim.x > kEarlyRows)
+    pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrAddLn);
   __shared__ float redf[kRowThreads / 32];
   __shared__ unsigned redu[kRowThreads / 32];
@@ -226,7 +227,7 @@ __device__ __forceinline__ void quantize_range(const float* __restrict__ x, int8
 __global__ void __launch_bounds__(256)
 quantize_slot_kernel(const float* __restrict__ x, size_t n, const unsigned* __restrict__ absmax_slot, int8_t* __restrict__ q,
                      float* __restrict__ d_quant_mult, int* status) {
-  pdl_launch_dependents();
+  pdl_launch_dependents();   // (early: the GEMM behind it has a longer set-up than this kernel work)
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
   pdl_wait();
@@ -265,7 +266,6 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(1024)
 add_layernorm_quant_kernel(const float* __restrict__ a, const SsruArgs cell, const float* __restrict__ resid, const float* __restrict__ gamma,
                            const float* __restrict__ beta, float eps, int rows, int dim, int group_warps, float* __restrict__ out,
                            int8_t* __restrict__ q, float* __restrict__ d_quant_mult, int* status) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
   __shared__ float red[32];
@@ -273,7 +273,7 @@ add_layernorm_quant_kernel(const float* __restrict__ a, const SsruArgs cell, con
   __shared__ unsigned cta_max[kCtas];
   if(kCtas > 1)
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (this CTA runs: the others may write to cta_max)
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrAddLnQuant);
   const int rank = kCtas > 1 ? static_cast<int>(blockIdx.x) : 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = static_cast<int>(blockDim.x) >> 5;
@@ -368,10 +368,9 @@ quantize_dual_kernel(const float* __restrict__ x, size_t n, const unsigned* __re
                      float* __restrict__ qm_x, int* status, int blocks_x, const float* __restrict__ slabs, int slab_rows, int steps,
                      int rows_new, int dim, const unsigned* __restrict__ slot_h, const unsigned* __restrict__ prev_bits,
                      int8_t* __restrict__ hq, float* __restrict__ qm_h) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrQuantDual);
   if(static_cast<int>(blockIdx.x) < blocks_x) {
     const unsigned bits = *slot_x;
@@ -499,10 +498,9 @@ embed_ancestors_kernel(const float* __restrict__ wemb, const int* __restrict__ w
                        float* __restrict__ out, float* __restrict__ rowmax, unsigned* absmax_slot, unsigned* absmax_slot2,
                        const int* __restrict__ anc_old, int* __restrict__ anc_new, const int* __restrict__ hyp, int t, int rows, int stride,
                        const HistMaxArgs hist, const HistLists lists) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrEmbed);
   __shared__ unsigned red[kRowThreads / 32];
   if(static_cast<int>(blockIdx.x) < rows)
@@ -565,10 +563,9 @@ __global__ void __launch_bounds__(256)
 attention1_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                   const float* __restrict__ log_mask, int heads, int len, int rows, int batch, int mode, float scale,
                   float* __restrict__ out, unsigned* absmax_slot, const int* __restrict__ anc, int anc_stride, int kv_rows) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrAttention1);
   extern __shared__ float sc_smem[];  // [heads][len] scores, then probabilities
   constexpr int G = DH / 4;
@@ -720,7 +717,6 @@ __global__ void __launch_bounds__(kCrossMaxBeams * 32)
 attention_cross_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                        const float* __restrict__ log_mask, int heads, int len, int rows, int batch, float scale, float* __restrict__ out,
                        unsigned* absmax_slot) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
   constexpr int G = DH / 4, U = kCrossU, SR = kCrossRows;
@@ -766,7 +762,7 @@ attention_cross_kernel(const float* __restrict__ q, const float* __restrict__ k,
     for(int i = threadIdx.x; i < 2 * len; i += blockDim.x)
       prefetch_l2((i < len ? k : v) + (static_cast<size_t>(b) * len + (i < len ? i : i - len)) * dim + blockIdx.y * 128, bytes);
   }
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrAttentionCross);
 #pragma unroll
   for(int i = 0; i < kCrossStages - 1; ++i)
@@ -877,7 +873,6 @@ template <int DH>
 __global__ void __launch_bounds__(kMaxHistBeams * 32)
 attention_hist_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, int heads, int len, int batch, float scale,
                       float* __restrict__ out, unsigned* absmax_slot, const HistLists lists) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
   constexpr int G = DH / 4, U = kCrossU, SR = kCrossRows;
@@ -894,7 +889,7 @@ attention_hist_kernel(const float* __restrict__ q, const float* __restrict__ k, 
   float* sc = scores + (warp * kWarpHeads + lane / G) * len4;
   int* list = reinterpret_cast<int*>(scores + beams * kWarpHeads * len4);
   int* which = list + beams * len + warp * len;
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrAttentionHist);
   const float4 qv = active ? __ldg(reinterpret_cast<const float4*>(q + static_cast<size_t>(r) * dim) + slice) : make_float4(0.f, 0.f, 0.f, 0.f);
   const int n_rows = lists.count[b];
@@ -1034,10 +1029,9 @@ __global__ void __launch_bounds__(128)
 attention_enc_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                      const float* __restrict__ log_mask, int heads, int len, float scale, float* __restrict__ out,
                      unsigned* absmax_slot) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrAttentionEnc);
   extern __shared__ float enc_smem[];
   constexpr int G = DH / 4;
@@ -1315,10 +1309,9 @@ template <int kThreads, bool kFromBlocks = false>
 __global__ void __launch_bounds__(kThreads, 1024 / kThreads)
 lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float* __restrict__ prev_scores, float* cand_score, int* cand_word,
                 const StepEnd end, const float* __restrict__ block_max, const float* __restrict__ block_sum) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
-  pdl_wait();
+  pdl_wait_and_launch();
   if(end.stop != nullptr && *end.stop != 0u)
     return;
   trace_stamp_start(th, kTrLseTopk);
@@ -1511,10 +1504,9 @@ __global__ void __launch_bounds__(256)
 lse_merge_kernel(const float* __restrict__ blk_max, const float* __restrict__ blk_sum, const float* __restrict__ blk_topv,
                  const int* __restrict__ blk_topi, int nb, int k, const float* __restrict__ prev_scores, float* cand_score, int* cand_word, int vocab,
                  const StepEnd end) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrLseMerge);
   static_assert(kStepEndCandidates <= 256 * KT, "finish_step reuses these arrays");
   extern __shared__ float lse_blocks[];
@@ -1564,10 +1556,9 @@ lse_merge_kernel(const float* __restrict__ blk_max, const float* __restrict__ bl
 template <int K>
 __global__ void nbest_merge_kernel(const float* __restrict__ cand_score, const int* __restrict__ cand_word, int beam, int batch,
                                    int vocab, float* __restrict__ out_score, int* __restrict__ out_beam, int* __restrict__ out_word) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrNbest);
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if(b >= batch) {
@@ -1606,10 +1597,9 @@ __global__ void nbest_merge_kernel(const float* __restrict__ cand_score, const i
 
 // rows gather: out[i,:] = in[idx[i],:]  (16-byte copies when the row length allows it)
 __global__ void gather_rows_kernel(const float* __restrict__ in, const int* __restrict__ idx, int dim, float* __restrict__ out) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrGather);
   const int r = blockIdx.x;
   const float* src = in + static_cast<size_t>(idx[r]) * dim;
@@ -1631,10 +1621,9 @@ __global__ void gather_rows_kernel(const float* __restrict__ in, const int* __re
 // Writes the new cell state and y = LayerNorm(h + resid) * gamma + beta is done by add_layernorm on h.
 __global__ void ssru_cell_kernel(const float* __restrict__ cell_old, const int* __restrict__ hyp, const float* __restrict__ xw,
                                  const float* __restrict__ f, int dim, float* __restrict__ cell_new, float* __restrict__ h_out) {
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrSsru);
   const int r = blockIdx.x;
   const float* c = cell_old + static_cast<size_t>(hyp ? hyp[r] : r) * dim;

@@ -29,6 +29,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // barrier/TMEM set-up and loads of constant weights qualify.  Without the launch attribute both are no-ops.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Both, the wait first: the form of most kernels.  When every kernel lets its successor start at its own start, a chain of five to seven of them lies on the
+// SMs waiting for one another, and each hand-over takes longer (2.2 us instead of 1.4 to 1.6 between a decoder step's kernels); with the next one alone set up
+// beside the running one nothing of that is lost, as long as the running one works for as long as the next one's set-up takes.  Decodes, start / behind the
+// wait, ms: transformer-base, 64 x beam 4 31.4 / 30.4, 4 x 4 14.1 / 13.5, four searches of 20 x 4 66.9 / 60.0; transformer-big, 8 x 4 25.0 / 23.7; student,
+// 16 sentences 3.27 / 3.13, 40 x 4 5.96 / 5.67.
+__device__ __forceinline__ void pdl_wait_and_launch() { asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------- in-situ timeline (measurement aid)
 // While a trace buffer is installed (mi8_trace_begin), one thread of block 0 of every kernel stamps the

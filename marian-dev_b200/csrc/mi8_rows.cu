@@ -150,7 +150,6 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
   float* norms = prm + p.layers * T::params(f);                                 // [layers][6][d] LayerNorm scales and biases
   float* sc = norms + p.layers * T::kNorms + warp * T::scores(S);               // this warp's scores, then the head's output
 
-  pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
 
   // ---- what does not depend on the kernel in front
@@ -228,7 +227,7 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
     reinterpret_cast<int4*>(acc)[i] = make_int4(0, 0, 0, 0);
   if(threadIdx.x == 0)
     abort_word = 0;
-  pdl_wait();
+  pdl_wait_and_launch();
   trace_stamp_start(th, kTrDecoderRows);
   // ---- embedding * sqrt(d) + position, and the cells' previous state.  The control words come with the launch's parameters, which are
   // there at once (reads of pinned memory by every CTA went over PCIe lane by lane: 16 rows 250 us), or from the device, where the step in front left
