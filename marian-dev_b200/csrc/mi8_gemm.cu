@@ -363,6 +363,10 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  // packed8avx512: the quantisation of rows behind this triggers late itself and is the longer for its set-up (256 x 1024 x 4096 9.05 us with both late, 8.55 so;
+  // transformer-base, 64 x beam 4 17.35 -> 17.1 ms)
+  if(kP8)
+    pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
   constexpr int kTraceId = kTopK > 0 ? kTrGemmLogits : (kQuantA ? kTrGemmQuantA : kTrGemm);

@@ -24,7 +24,7 @@ constexpr int kRi = 4;      // consecutive rows stored together (row interleave)
 // threads read consecutive words of the item and write bt[n][4 * kq .. 4 * kq + 3].
 __global__ void __launch_bounds__(kBlock)
 p8_unpack_bt_kernel(const uint32_t* __restrict__ packed, int K, int N, uint32_t* __restrict__ bt) {
-  pdl_wait();
+  pdl_wait_and_launch();
   const size_t words = static_cast<size_t>(K) * N / kRi;
   const size_t stride = static_cast<size_t>(gridDim.x) * kBlock;
   constexpr int kBlockWords = kKcb * kNcb / kRi;
@@ -49,7 +49,7 @@ p8_unpack_bt_kernel(const uint32_t* __restrict__ packed, int K, int N, uint32_t*
 __global__ void __launch_bounds__(kBlock)
 p8_prepare_b_kernel(const float* __restrict__ w, int K, int N, uint32_t* __restrict__ packed, float* __restrict__ scale_b,
                     int32_t* __restrict__ zp_b, int32_t* __restrict__ off_b) {
-  pdl_wait();
+  pdl_wait_and_launch();
   __shared__ float s_min[kBlock / 32][kNcb], s_max[kBlock / 32][kNcb];
   __shared__ int s_sum[kBlock / 32][kNcb];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -127,8 +127,7 @@ __device__ __forceinline__ float block_reduce(float v, float* smem, bool is_max)
 __global__ void __launch_bounds__(kBlock)
 p8_quantize_rows_kernel(const float* __restrict__ a, int K, uint8_t* __restrict__ aq, float* __restrict__ scale_a, int32_t* __restrict__ zp_a,
                         int32_t* __restrict__ sum_a, int* status) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait_and_launch();
   __shared__ float red[kBlock / 32];
   __shared__ int red_i[kBlock / 32];
   const int m = blockIdx.x;
@@ -193,8 +192,7 @@ template <int kVec>
 __global__ void __launch_bounds__(kBlock)
 p8_quantize_rows_warp_kernel(const float* __restrict__ a, int M, int K, uint8_t* __restrict__ aq, float* __restrict__ scale_a,
                              int32_t* __restrict__ zp_a, int32_t* __restrict__ sum_a, int* status) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait_and_launch();
   const int lane = threadIdx.x & 31;
   const int m = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
   if(m >= M)
