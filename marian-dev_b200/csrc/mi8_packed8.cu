@@ -24,7 +24,7 @@ constexpr int kRi = 4;      // consecutive rows stored together (row interleave)
 // threads read consecutive words of the item and write bt[n][4 * kq .. 4 * kq + 3].
 __global__ void __launch_bounds__(kBlock)
 p8_unpack_bt_kernel(const uint32_t* __restrict__ packed, int K, int N, uint32_t* __restrict__ bt) {
-  pdl_wait_and_launch();
+  pdl_wait();   // (no trigger: a product behind this fetches the weight in front of its own wait)
   const size_t words = static_cast<size_t>(K) * N / kRi;
   const size_t stride = static_cast<size_t>(gridDim.x) * kBlock;
   constexpr int kBlockWords = kKcb * kNcb / kRi;
@@ -49,7 +49,7 @@ p8_unpack_bt_kernel(const uint32_t* __restrict__ packed, int K, int N, uint32_t*
 __global__ void __launch_bounds__(kBlock)
 p8_prepare_b_kernel(const float* __restrict__ w, int K, int N, uint32_t* __restrict__ packed, float* __restrict__ scale_b,
                     int32_t* __restrict__ zp_b, int32_t* __restrict__ off_b) {
-  pdl_wait_and_launch();
+  pdl_wait();
   __shared__ float s_min[kBlock / 32][kNcb], s_max[kBlock / 32][kNcb];
   __shared__ int s_sum[kBlock / 32][kNcb];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
