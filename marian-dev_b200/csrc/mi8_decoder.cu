@@ -464,6 +464,17 @@ int wide_tile(const mi8d_decoder* d, int M) {
   return t;
 }
 
+// Few rows: 16-row tiles for up to 64 of them, where that is one wave of CTAs (the plan takes the smallest tile that holds all rows), and inner dimensions of up
+// to 2048 unsplit (the plan splits 2048).  A tile's operands, MMAs and write-back are then the shortest, and the split path's fence, atomics and counter cost more
+// than eight K blocks.  Whole mini-batches, the plan / 16-row tiles / those and no splits: transformer-base, 4 x beam 4 13.5 / 13.5 / 13.25 ms, 10 x 4 15.0 /
+// 14.5 / 14.4, 16 x 4 15.5 / 14.95 / 14.75; transformer-big, 10 x 4 17.25 / 16.75 / 16.75, 16 x 4 17.2 / 16.9 / 16.9; student, 40 sentences 4.95 / 4.8 / 4.8.
+// (32-row tiles: 10 x 4 14.55 and 16.95.  No splits of 4096: transformer-big, 4 x 4 15.3 -> 15.8.)
+constexpr int kNarrowRows = 64, kUnsplitK = 2048;
+int narrow_tile(int M, int N) {
+  return M > 16 && M <= kNarrowRows && static_cast<long long>((N + 127) / 128) * ((M + 15) / 16) <= sm_count() ? 16 : 0;
+}
+int few_rows_splits(int M, int K) { return M <= kNarrowRows && K <= kUnsplitK ? 1 : 0; }
+
 // aq (already quantised, multiplier behind the data) x weight -> c
 int gemm(mi8d_decoder* d, const int8_t* a, int M, const Aff& w, bool relu, float* c, cudaStream_t s, unsigned* absmax_out = nullptr,
          int force_splits = 0, int force_tile_m = 0) {
@@ -473,6 +484,10 @@ int gemm(mi8d_decoder* d, const int8_t* a, int M, const Aff& w, bool relu, float
     force_tile_m = wide_tile(d, M);
     force_splits = 1;
   }
+  if(force_tile_m == 0)
+    force_tile_m = narrow_tile(M, w.N);
+  if(force_splits == 0 && w.N <= 8192)
+    force_splits = few_rows_splits(M, w.K);
   return launch_gemm(a, w.bt, M, w.N, w.K, qa, w.qm, 1.0f, w.bias, relu ? 1 : 0, c, MI8_F32, nullptr, d->ws, d->ws_bytes, s, force_tile_m,
                      force_splits, absmax_out);
 }
@@ -494,6 +509,8 @@ GemmCall fused_call(mi8d_decoder* d, const int8_t* a, const Fused& f, int M, int
   g.ws_bytes = d->ws_bytes;
   g.stream = s;
   g.a_rows_cap = a_rows_cap;
+  g.force_tile_m = narrow_tile(M, g.N);
+  g.force_splits = few_rows_splits(M, f.K);
   return g;
 }
 
@@ -504,7 +521,7 @@ int gemm_fused(mi8d_decoder* d, const int8_t* a, const float* qa, int M, const F
     P8Segments segs = f.p8;
     std::copy(outs, outs + f.nseg, segs.c);
     return launch_gemm_p8(reinterpret_cast<const uint8_t*>(a), d->p8_scale_a, d->p8_zp_a, d->p8_sum_a, nullptr, nullptr, nullptr, nullptr, M,
-                          f.nseg * f.n, f.K, nullptr, 0, nullptr, nullptr, d->ws, d->ws_bytes, s, 0, 0, &segs);
+                          f.nseg * f.n, f.K, nullptr, 0, nullptr, nullptr, d->ws, d->ws_bytes, s, narrow_tile(M, f.nseg * f.n), few_rows_splits(M, f.K), &segs);
   }
   GemmCall g = fused_call(d, a, f, M, 0, f.nseg, 0, s);
   g.d_qa = qa;
@@ -527,7 +544,8 @@ int gemm_act(mi8d_decoder* d, const int8_t* q, int M, const Aff& w, bool relu, f
              int force_splits = 0) {
   if(w.p8)
     return launch_gemm_p8(reinterpret_cast<const uint8_t*>(q), d->p8_scale_a, d->p8_zp_a, d->p8_sum_a, w.bt, w.scale_b, w.zp_b, w.off_b, M, w.N,
-                          w.K, w.bias, relu ? 1 : 0, c, nullptr, d->ws, d->ws_bytes, s, 0, force_splits);
+                          w.K, w.bias, relu ? 1 : 0, c, nullptr, d->ws, d->ws_bytes, s, narrow_tile(M, w.N),
+                          force_splits != 0 || w.N > 8192 ? force_splits : few_rows_splits(M, w.K));
   return gemm(d, q, M, w, relu, c, s, absmax_out, force_splits);
 }
 
@@ -1309,8 +1327,10 @@ int run_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const i
         g.seg_c[0] = d->qbuf;
         g.seg_c[1] = kv_new[0];
         g.seg_c[2] = kv_new[1];
-        g.force_tile_m = wide_tile(d, R);
-        g.force_splits = g.force_tile_m != 0 ? 1 : 0;
+        if(wide_tile(d, R) != 0) {
+          g.force_tile_m = wide_tile(d, R);
+          g.force_splits = 1;
+        }
         MI8D_TRY(launch_gemm_call(g));
       } else {
         const int8_t* a_new = L.hq + static_cast<size_t>(t) * slab_stride;
