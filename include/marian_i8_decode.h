@@ -178,7 +178,8 @@ int mi8d_history_reuse(mi8d_decoder* d, unsigned out[2], int reset);
  *   MI8D_OPT_FUSED_OUTPUT_MAX_ROWS (default 0): up to this many rows the output layer reduces its logits to the rows' candidates
  *     inside the GEMM's write-back and does not write them.  Above it the logits are written, and the log-softmax / top-k kernel
  *     reads them back; up to 32 rows it takes the blocks' maxima and sums from the write-back and reads the best blocks only;
- *   MI8D_OPT_SIDE_STREAM (default 1): the re-projection of the earlier history slabs runs on an internal stream;
+ *   MI8D_OPT_SIDE_STREAM (default 1): the re-projection of the earlier history slabs is part of the newest slab's launch while they are
+ *     short, and runs on an internal stream beside it when they are not; 0: a launch of its own in front of it;
  *   MI8D_OPT_ATTENTION_UNROLL (8 or 16, default 8; process-wide): key/value rows a thread keeps in flight;
  *   MI8D_OPT_ATTENTION_BLOCK_HEADS (default 8, 0 = all; process-wide): heads one block of the decoder attention serves;
  *     a divisor of the head count splits every query row over several smaller blocks.  (Both: where the next switch does not

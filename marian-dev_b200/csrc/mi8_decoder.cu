@@ -475,6 +475,22 @@ int narrow_tile(int M, int N) {
 }
 int few_rows_splits(int M, int K) { return M <= kNarrowRows && K <= kUnsplitK ? 1 : 0; }
 
+// The tile of the launch that projects a step's newest history slab and, when the history's abs-max changed, the earlier slabs as well (GemmCall::rows_below), or 0
+// for a launch of their own beside it (`below`: floats of the earlier slabs).  Together as long as the earlier slabs are short: the launch has one tile width, which
+// the newest slab wants narrow and they want wide, and a launch of their own runs beside the newest slab's.  They are what a beam's reordering changes often and what
+// one hypothesis per sentence rarely does, so that its tiles are those of the newest slab.  Whole mini-batches, apart / together up to 2 M / 4 M / any number of
+// floats, ms: transformer-base, 4 x beam 4 (40 words) 25.5 / 23.8 / 23.8 / 23.9, 20 x 4 28.0 / 27.5 / 27.5 / 27.9, 64 x 4 30.4 / 30.4 / 30.4 / 31.3, 30 x 6 25.8 /
+// 25.6 / 26.1 / 26.9, 64 x 1 29.2 / 27.6 / 27.6 / 27.7; transformer-big, 16 x 4 16.95 / 16.6 / 16.5 / 16.7, 60 x 4 21.9 / 21.75 / 21.6 / 21.4, 128 x 4 39.1 /
+// 39.05 / 38.9 / 39.35, 20 x 1 16.1 / 15.1 / 15.1 / 15.2, 60 x 1 32.6 / 31.65 / 31.1 / 31.0.  Tiles of 16 / 32 / 64 / 128 rows: base, 4 x 4 13.3 / 12.9 / 12.9 / -,
+// 20 x 4 15.8 / 15.7 / 15.6 / 15.4, 64 x 1 14.6 / 15.2 / 15.3 / -.  Not on a GPU that several searches share: the launch has a CTA on every SM.
+int below_tile(int rows, int beam, size_t below) {
+  if(rows > 512 || below > (beam == 1 ? size_t{4} << 20 : size_t{2} << 20))
+    return 0;
+  if(beam == 1)
+    return rows <= 64 ? 16 : rows <= 128 ? 32 : 64;
+  return rows <= 64 ? 64 : 128;
+}
+
 // aq (already quantised, multiplier behind the data) x weight -> c
 int gemm(mi8d_decoder* d, const int8_t* a, int M, const Aff& w, bool relu, float* c, cudaStream_t s, unsigned* absmax_out = nullptr,
          int force_splits = 0, int force_tile_m = 0) {
@@ -1287,17 +1303,17 @@ int run_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const i
       const bool fused = d->opt_fuse && w.self_qkv.ready;
       float* kv_new[2] = {L.kslab + static_cast<size_t>(t) * slab_stride, L.vslab + static_cast<size_t>(t) * slab_stride};
       // Query, key and value projections of the newest slab are one launch (the query's segment takes its rows and multiplier from
-      // another place of hq).  The earlier slabs' keys and values, recomputed only when the abs-max changed, run before it, or
-      // beside it on the internal stream.  The internal stream gains where re-projections
-      // happen: transformer-base 64 x 4 37.4 against 37.9 ms on one stream, 16 x 4 18.1 against 18.8, transformer-big 44.2 against 44.9.
+      // another place of hq).  The earlier slabs' keys and values, recomputed only when the abs-max changed, are in it as well (below_tile), or run
+      // beside it on the internal stream, or in front of it.
       // (As three launches, the query's on its own stream beside the others with tiles for half of the SMs each: 38.4, 19.1 and 45.7 ms.)
-      const bool side = d->overlap && d->opt_side_stream && t > 0;
+      const int below = fused && t > 0 && d->opt_gemm_tile == 0 && d->opt_side_stream ? below_tile(R, beam, static_cast<size_t>(t) * SR * dm) : 0;
+      const bool side = d->overlap && d->opt_side_stream && t > 0 && below == 0;
       cudaStream_t so = side ? d->side : s;
       if(side) {
         MI8D_CUDA(cudaEventRecord(d->ev_fork, s));
         MI8D_CUDA(cudaStreamWaitEvent(so, d->ev_fork, 0));
       }
-      if(t > 0) {
+      if(t > 0 && below == 0) {
         // all tiles skipped when the stored results still hold; no split-K: the two streams must not share the workspace's counters
         if(fused) {
           GemmCall g = fused_call(d, L.hq, w.self_qkv, t * SR, 1, 3, cap_rows + c.max_rows, so);
@@ -1327,7 +1343,14 @@ int run_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const i
         g.seg_c[0] = d->qbuf;
         g.seg_c[1] = kv_new[0];
         g.seg_c[2] = kv_new[1];
-        if(wide_tile(d, R) != 0) {
+        if(below != 0) {
+          g.rows_below = true;
+          g.force_tile_m = below;
+          g.force_splits = 1;
+          g.skip_a = d->prev_bits + l;
+          g.skip_b = sh;
+          g.skip_rows_below = t * SR;
+        } else if(wide_tile(d, R) != 0) {
           g.force_tile_m = wide_tile(d, R);
           g.force_splits = 1;
         }

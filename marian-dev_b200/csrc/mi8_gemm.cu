@@ -173,6 +173,23 @@ __device__ __forceinline__ WorkItem decode_work(const GemmParams& p, int w) {
   return it;
 }
 
+// kBelow: behind the tiles of the launch's own rows come those of the rows in front of them, of all segments but the first.
+__device__ __forceinline__ int below_tiles(const GemmParams& p) { return p.n_tiles - p.n_tiles / p.nseg; }
+__device__ __forceinline__ WorkItem decode_work_below(const GemmParams& p, int w) {
+  const int own = p.n_tiles * p.m_tiles;
+  if(w < own)
+    return decode_work(p, w);
+  const int v = w - own, n = below_tiles(p);
+  WorkItem it;
+  it.split = 0;
+  it.tile = w;
+  it.n_tile = p.n_tiles / p.nseg + v % n;
+  it.m_tile = v / n;
+  it.kb_begin = 0;
+  it.kb_end = p.kb_total;
+  return it;
+}
+
 __device__ __forceinline__ void named_bar_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
@@ -339,7 +356,10 @@ __device__ __forceinline__ void write_back_chunk_p8(const GemmParams& p, const i
 // Up to 32 rows (kBlockRows): a wider tile's values would not fit beside the ring.
 // kDuo (long inner dimensions of a few hundred rows): the two CTAs of a cluster take one half of K each for the same 64-row tile.  Each keeps 32 of the
 // tile's rows, gets their other partial sums from its pair through distributed shared memory and writes them back.  One tile per CTA.
-template <int TM, bool kQuantA, int kTopK = 0, bool kP8 = false, bool kBlocks = false, bool kDuo = false, int kMaps = 1>
+// kBelow (query, key and value projections of the newest history slab): the key and value segments also take the skip_rows_below rows in front of their own, operand
+// and results, unless *skip_a == *skip_b; those tiles come behind the launch's own.  As a launch beside this one, on a stream of its own, they held up the kernel
+// behind both by a fork and a join (9 of the 57 us of a layer of few rows) even where they had nothing to do (which rows: mi8_decoder.cu).
+template <int TM, bool kQuantA, int kTopK = 0, bool kP8 = false, bool kBlocks = false, bool kDuo = false, int kMaps = 1, bool kBelow = false>
 __global__ void __launch_bounds__(kThreads, 1)
 mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
   using T = TileCfg<TM>;
@@ -362,6 +382,13 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  auto work_item = [&](int w) -> WorkItem {
+    if constexpr(kBelow)
+      return decode_work_below(p, w);
+    return decode_work(p, w);
+  };
+  auto is_below = [&](int w) { return kBelow && w >= p.n_tiles * p.m_tiles; };
+  auto items = [&](bool skip_on) { return kBelow && skip_on ? p.n_tiles * p.m_tiles : p.total_work; };   // what this launch has to do
 
   // packed8avx512: the quantisation of rows behind this triggers late itself and is the longer for its set-up (256 x 1024 x 4096 9.05 us with both late, 8.55 so;
   // transformer-base, 64 x beam 4 17.35 -> 17.1 ms)
@@ -373,7 +400,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
   const unsigned long long trace_extra = static_cast<unsigned long long>(p.N) | (static_cast<unsigned long long>(p.K) << 20) |
                                          (static_cast<unsigned long long>(p.M) << 40);
   if(threadIdx.x == 0) {
-    tma_prefetch_desc(weight_rows(tmap_w, p.nseg, p.seg_n, decode_work(p, blockIdx.x).n_tile * kTileN).map);
+    tma_prefetch_desc(weight_rows(tmap_w, p.nseg, p.seg_n, work_item(blockIdx.x).n_tile * kTileN).map);
     tma_prefetch_desc(&tmap_a);
     for(int s = 0; s < kStages; ++s) {
       mbar_init(&ctl->full[s], kQuantA ? 1 + kConvWarps : 1);   // producer (+ one arrival per quantising warp)
@@ -409,7 +436,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
     // are requested before waiting for it, the activation tiles (its output) after.
     uint32_t it = 0;
     uint32_t prefetched = 0;  // stages whose weight tile is already in flight
-    if(p.skip_a == nullptr && kTopK == 0 && p.withhold_item < 0) {   // (output-layer variant: the M-side operand is the activation, nothing to prefetch)
+    if((kBelow ? !is_below(blockIdx.x) : p.skip_a == nullptr) && kTopK == 0 && p.withhold_item < 0) {   // (output-layer variant: the M-side operand is the activation, nothing to prefetch)
       const WorkItem w0 = decode_work(p, blockIdx.x);
       const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, w0.n_tile * kTileN);
       const int blocks = w0.kb_end - w0.kb_begin, n_pre = min(kStages, (blocks + kPer - 1) / kPer);
@@ -427,13 +454,13 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
     pdl_wait_and_launch();
     const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
     if(p.rows_computed != nullptr && blockIdx.x == 0 && lane == 0)
-      *p.rows_computed = p.M - (skip_on ? min(p.M, (p.skip_rows_below / TM) * TM) : 0);
-    for(int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x) {
-      const WorkItem wi = decode_work(p, w);
-      if(skip_on && (wi.m_tile + 1) * TM <= p.skip_rows_below)
+      *p.rows_computed = kBelow ? p.M + (skip_on ? 0 : p.skip_rows_below * (p.nseg - 1) / p.nseg) : p.M - (skip_on ? min(p.M, (p.skip_rows_below / TM) * TM) : 0);
+    for(int w = blockIdx.x; w < items(skip_on) && ok; w += gridDim.x) {
+      const WorkItem wi = work_item(w);
+      if(!kBelow && skip_on && (wi.m_tile + 1) * TM <= p.skip_rows_below)
         continue;
       const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, wi.n_tile * kTileN);
-      const int a_row0 = p.seg_row0[p.nseg > 1 ? (wi.n_tile * kTileN) / p.seg_n : 0];
+      const int a_row0 = p.seg_row0[p.nseg > 1 ? (wi.n_tile * kTileN) / p.seg_n : 0] - (is_below(w) ? p.skip_rows_below : 0);
       for(int kb = wi.kb_begin; kb < wi.kb_end; kb += kPer, ++it) {
         const uint32_t s = it % kStages;
         const uint32_t ph = (it / kStages) & 1u;
@@ -481,9 +508,9 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
     // waits below (it also orders the read of the skip words, which earlier kernels of the stream write).
     pdl_wait_and_launch();
     const bool skip_on = p.skip_a != nullptr && *p.skip_a == *p.skip_b;
-    for(int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x) {
-      const WorkItem wi = decode_work(p, w);
-      if(skip_on && (wi.m_tile + 1) * TM <= p.skip_rows_below)
+    for(int w = blockIdx.x; w < items(skip_on) && ok; w += gridDim.x) {
+      const WorkItem wi = work_item(w);
+      if(!kBelow && skip_on && (wi.m_tile + 1) * TM <= p.skip_rows_below)
         continue;
       const uint32_t as = acc_it & 1u;
       const uint32_t aph = (acc_it >> 1) & 1u;
@@ -559,9 +586,9 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
     if(p.withhold_item == kWithholdWarp && warp == 3)   // (test hook: this warp of every CTA gives up at once)
       ok = false;
     int w = blockIdx.x;
-    for(; w < p.total_work && ok; w += gridDim.x) {
-      const WorkItem wi = decode_work(p, w);
-      if(skip_on && (wi.m_tile + 1) * TM <= p.skip_rows_below)
+    for(; w < items(skip_on) && ok; w += gridDim.x) {
+      const WorkItem wi = work_item(w);
+      if(!kBelow && skip_on && (wi.m_tile + 1) * TM <= p.skip_rows_below)
         continue;
       if(kQuantA) {
         // Quantise this tile's activation rows, one 128-byte K block per pipeline stage.  A thread
@@ -637,7 +664,7 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
       const int n = wi.n_tile * kTileN + row;
       const bool n_ok = n < p.N;
       const int m0 = wi.m_tile * TM;
-      const int cols_valid = min(TM, p.M - m0);  // activation rows of this tile that exist
+      const int cols_valid = min(TM, (is_below(w) ? p.skip_rows_below : p.M) - m0);  // activation rows of this tile that exist
       // the weight segment this tile belongs to: its multiplier, bias, output matrix and the column inside it
       int seg = 0, n_loc = n;
       if(kTopK == 0 && (kP8 ? kMaps > 1 : p.nseg > 1)) {
@@ -647,8 +674,10 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
           unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(*p.seg_qa[seg], *p.seg_qb[seg])), p.scale);
       }
       const float* seg_bias = p.seg_bias[seg];
-      void* seg_c = p.seg_c[seg];
       const int ldc = p.seg_n;
+      void* seg_c = p.seg_c[seg];
+      if(is_below(w))
+        seg_c = static_cast<float*>(seg_c) - static_cast<size_t>(p.skip_rows_below) * ldc;
       // (segments are 128 columns wide or more: n_loc has the parity of the lane)
       const bool paired = p.out_f16 && (ldc & 1) == 0 && (reinterpret_cast<uintptr_t>(seg_c) & 3u) == 0 && __all_sync(0xffffffffu, n_ok);
       float bias_n = 0.0f;
@@ -1987,14 +2016,14 @@ void single_segment(GemmParams& p) {
   }
 }
 
-template <int TM, bool kQuantA = false, int kTopK = 0, bool kP8 = false, bool kBlocks = false, int kMaps = 1>
+template <int TM, bool kQuantA = false, int kTopK = 0, bool kP8 = false, bool kBlocks = false, int kMaps = 1, bool kBelow = false>
 int launch_cfg(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const GemmParams& p, const GemmPlan& plan, cudaStream_t stream) {
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   constexpr int smem = smem_bytes_for<TM, kBlocks>();
   if(dev >= 0 && dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(mi8_gemm_kernel<TM, kQuantA, kTopK, kP8, kBlocks, false, kMaps>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(mi8_gemm_kernel<TM, kQuantA, kTopK, kP8, kBlocks, false, kMaps, kBelow>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if(e != cudaSuccess) {
       set_last_cuda_error(e);
       return MI8_ERR_LAUNCH;
@@ -2009,7 +2038,7 @@ int launch_cfg(const WeightMaps<kP8, kMaps>& tw, const CUtensorMap& ta, const Ge
     if(rec.start != nullptr && rec.stop != nullptr)
       cudaEventRecord(rec.start, stream);
   }
-  cudaError_t le = launch_kernel(mi8_gemm_kernel<TM, kQuantA, kTopK, kP8, kBlocks, false, kMaps>, dim3(plan.grid), dim3(kThreads), smem, stream, tw, ta, p);
+  cudaError_t le = launch_kernel(mi8_gemm_kernel<TM, kQuantA, kTopK, kP8, kBlocks, false, kMaps, kBelow>, dim3(plan.grid), dim3(kThreads), smem, stream, tw, ta, p);
   if(le != cudaSuccess) {
     set_last_cuda_error(le);
     return MI8_ERR_LAUNCH;
@@ -2420,8 +2449,16 @@ int launch_gemm_call(const GemmCall& g) {
   if(blocks && (M > kBlockRows || g.block_sum == nullptr || g.nseg != 1 || g.relu || g.out_dtype != MI8_F32 || g.acc_out != nullptr || g.absmax_out != nullptr ||
                 g.skip_a != nullptr || g.force_tile_m != 0))
     return MI8_ERR_UNSUPPORTED;
+  if(g.rows_below) {   // (up to 128-row tiles, unsplit; every segment but the first has the rows in front of its own)
+    if(g.nseg < 2 || g.skip_a == nullptr || g.skip_b == nullptr || g.skip_rows_below <= 0 || g.out_dtype != MI8_F32 || g.absmax_out != nullptr ||
+       g.force_tile_m < 16 || g.force_tile_m > 128 || blocks)
+      return MI8_ERR_UNSUPPORTED;
+    for(int i = 1; i < g.nseg; ++i)
+      if((g.seg_row0[i] < 0 ? g.a_row0 : g.seg_row0[i]) < g.skip_rows_below)
+        return MI8_ERR_BAD_ARG;
+  }
   GemmPlan plan;
-  int rc = make_gemm_plan(M, N, K, blocks ? (M <= 16 ? 16 : 32) : g.force_tile_m, blocks ? 1 : g.force_splits, &plan);
+  int rc = make_gemm_plan(M, N, K, blocks ? (M <= 16 ? 16 : 32) : g.force_tile_m, blocks || g.rows_below ? 1 : g.force_splits, &plan);
   if(rc == MI8_OK && plan.pair && own_rows && (N / g.nseg) % (2 * kTileN) != 0)   // a pair's 256 weight rows share their activation tile
     rc = make_gemm_plan(M, N, K, 256, g.force_splits, &plan);
   if(rc != MI8_OK)
@@ -2495,6 +2532,19 @@ int launch_gemm_call(const GemmCall& g) {
   }
   finish_params(p, !plan.pair ? blocks_per_stage(plan.tile_m) : holds_weights(p) ? PairCfg::kResidentPer : 1);
 
+  if(g.rows_below) {
+    const long long below = static_cast<long long>(plan.n_tiles - plan.n_tiles / g.nseg) * ((g.skip_rows_below + plan.tile_m - 1) / plan.tile_m);
+    if(p.total_work + below > 0x7fffffffLL / 64)
+      return MI8_ERR_UNSUPPORTED;
+    p.total_work += static_cast<int>(below);
+    plan.grid = std::min(p.total_work, sm_count());
+    switch(plan.tile_m) {
+      case 16: return launch_cfg<16, false, 0, false, false, 1, true>(tw, ta, p, plan, g.stream);
+      case 32: return launch_cfg<32, false, 0, false, false, 1, true>(tw, ta, p, plan, g.stream);
+      case 64: return launch_cfg<64, false, 0, false, false, 1, true>(tw, ta, p, plan, g.stream);
+      default: return launch_cfg<128, false, 0, false, false, 1, true>(tw, ta, p, plan, g.stream);
+    }
+  }
   if(blocks)
     return plan.tile_m == 16 ? launch_cfg<16, false, 0, false, true>(tw, ta, p, plan, g.stream) : launch_cfg<32, false, 0, false, true>(tw, ta, p, plan, g.stream);
   if(plan.duo)

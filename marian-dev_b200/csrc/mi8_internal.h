@@ -100,6 +100,9 @@ struct GemmCall {
   const unsigned* skip_a = nullptr;
   const unsigned* skip_b = nullptr;
   int skip_rows_below = 0;
+  // with the three above: the segments from the second on also take the skip_rows_below rows in front of their own (of the operand's buffer and of their results,
+  // which continue there), unless the two words are equal.  Needs force_tile_m of 16 to 128.
+  bool rows_below = false;
   // optional, up to kBlockRows rows of one fp32 result: per (row, block of 128 columns) the maximum and the sum of exponentials [M][ceil(N / 128)]
   float* block_max = nullptr;
   float* block_sum = nullptr;
