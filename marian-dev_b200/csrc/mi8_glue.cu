@@ -1007,12 +1007,16 @@ attention_hist_kernel(const float* __restrict__ q, const float* __restrict__ k, 
   trace_stamp(th.last, kTrAttentionHist, 3);
 }
 
-// Encoder self-attention (mode 2) with the keys and values of one (sentence, head) staged in shared memory: block
-// (b, h), thread = one query position (128 at a time).  attention1_kernel re-reads every key/value row once per
-// query; here they cross L2 -> SM once per sentence and head.  The arithmetic per (row, head) is that of
-// attention1_kernel restated for one thread: the G = DH/4 four-element partial dot products are combined in the
+// Encoder self-attention (mode 2): block (b, h, i) has 32 query positions of one (sentence, head), a lane each, and its keys and values in shared memory.
+// attention1_kernel re-reads every key/value row once per query; here they cross L2 -> SM once per 32 queries.  The eight warps share the key positions out
+// (position p is warp p % 8's: its scores, exponentials and the interleaved partial sums they belong to) and then the elements of the output.
+// The arithmetic per (row, head) is that of attention1_kernel restated for one lane: the G = DH/4 four-element partial dot products are combined in the
 // butterfly's order (pairs G/2 apart first), the softmax sum as G interleaved partial sums combined the same way,
 // the output as a fused-multiply-add chain over the positions in ascending order.
+// Bound by one warp's chain of instructions where blocks are few, by shared-memory reads (a broadcast of four floats feeds four multiply-adds) where they are many.
+// With a thread per query position, one or two warps of a block at work on all key positions, before: a layer of transformer-big, 128 sentences of 31 words,
+// 95 -> 43 us (47 with registers for two blocks per SM instead of three), of transformer-base, 64 of 38 words, 42 -> 27, of the student, one sentence 9 -> 3.7,
+// 16 sentences 14 -> 4.6; student, 16 sentences, a mini-batch 3.14 -> 3.035 ms, one sentence 2.22 -> 2.135.
 template <int G>
 __device__ __forceinline__ float butterfly_order_sum(float (&a)[G]) {
 #pragma unroll
@@ -1024,8 +1028,13 @@ __device__ __forceinline__ float butterfly_order_sum(float (&a)[G]) {
   return a[0];
 }
 
+constexpr int kEncWarps = 8, kEncRows = 32;
+constexpr size_t attention_enc_smem(int dim_head, size_t len) {   // keys, values, scores, mask; queries; partial sums; maxima
+  return sizeof(float) * (len * (2 * dim_head + kEncRows + 1) + kEncRows * (dim_head + 4) + kEncRows * (dim_head / 4) + kEncRows * kEncWarps + 4);
+}
+
 template <int DH>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kEncWarps * 32, DH == 64 ? 3 : 2)
 attention_enc_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                      const float* __restrict__ log_mask, int heads, int len, float scale, float* __restrict__ out,
                      unsigned* absmax_slot) {
@@ -1033,93 +1042,118 @@ attention_enc_kernel(const float* __restrict__ q, const float* __restrict__ k, c
   unsigned long long* const tb = th.first;
   pdl_wait_and_launch();
   trace_stamp_start(th, kTrAttentionEnc);
-  extern __shared__ float enc_smem[];
-  constexpr int G = DH / 4;
-  const int b = blockIdx.x, h = blockIdx.y;
-  const int dim = heads * DH;
-  float* ks = enc_smem;                     // [len][DH]
-  float* vs = ks + static_cast<size_t>(len) * DH;
-  float* sc = vs + static_cast<size_t>(len) * DH;   // [len][128] scores / probabilities, position-major
+  extern __shared__ float4 enc_smem[];
+  constexpr int G = DH / 4, W = kEncWarps, kQPitch = DH + 4, kOwn = DH / W;   // (a row of queries 4 floats longer: eight lanes' reads on different banks)
+  static_assert(G % W == 0 && kOwn % 4 == 0, "");
+  const int b = blockIdx.x, h = blockIdx.y, q0 = blockIdx.z * kEncRows;
+  const int dim = heads * DH, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* ks = reinterpret_cast<float*>(enc_smem);   // [len][DH]
+  float* vs = ks + static_cast<size_t>(len) * DH;   // [len][DH]
+  float* qs = vs + static_cast<size_t>(len) * DH;   // [32][DH + 4]
+  float* parts = qs + kEncRows * kQPitch;           // [G][32]
+  float* maxima = parts + G * kEncRows;             // [W][32]
+  float* sc = maxima + W * kEncRows;                // [len][32] scores / probabilities
+  float* ms = sc + static_cast<size_t>(len) * kEncRows;   // [len]
   const size_t row0 = static_cast<size_t>(b) * len;
-  for(int i = threadIdx.x; i < len * (DH / 4); i += blockDim.x) {
-    const int p = i / (DH / 4), c = i % (DH / 4);
-    const size_t off = (row0 + p) * dim + h * DH + 4 * c;
+  for(int i = threadIdx.x; i < len * G; i += W * 32) {
+    const size_t off = (row0 + i / G) * dim + h * DH + 4 * (i % G);
     reinterpret_cast<float4*>(ks)[i] = __ldg(reinterpret_cast<const float4*>(k + off));
     reinterpret_cast<float4*>(vs)[i] = __ldg(reinterpret_cast<const float4*>(v + off));
   }
+  for(int i = threadIdx.x; i < kEncRows * G; i += W * 32)   // (beyond the end the last query once more)
+    *reinterpret_cast<float4*>(qs + (i / G) * kQPitch + 4 * (i % G)) =
+        __ldg(reinterpret_cast<const float4*>(q + (row0 + min(q0 + i / G, len - 1)) * dim + h * DH + 4 * (i % G)));
+  for(int i = threadIdx.x; i < len; i += W * 32)
+    ms[i] = log_mask ? __ldg(log_mask + row0 + i) : 0.f;
   __syncthreads();
-  const float* mask = log_mask ? log_mask + row0 : nullptr;
-  unsigned m_abs = 0u;
-  for(int q0 = 0; q0 < len; q0 += 128) {
-    const int qi = q0 + threadIdx.x;
-    const bool active = qi < len;
-    float qv[DH];
-    {
-      const float4* q4 = reinterpret_cast<const float4*>(q + (row0 + (active ? qi : 0)) * dim + h * DH);
+  float qv[DH];
 #pragma unroll
-      for(int c = 0; c < DH / 4; ++c) {
-        const float4 t = __ldg(q4 + c);
-        qv[4 * c] = t.x; qv[4 * c + 1] = t.y; qv[4 * c + 2] = t.z; qv[4 * c + 3] = t.w;
-      }
-    }
-    float mx = -FLT_MAX;
-    for(int p = 0; p < len; ++p) {
-      const float* kr = ks + p * DH;
-      float a[G];
+  for(int c = 0; c < G; ++c) {
+    const float4 t = *reinterpret_cast<const float4*>(qs + lane * kQPitch + 4 * c);
+    qv[4 * c] = t.x; qv[4 * c + 1] = t.y; qv[4 * c + 2] = t.z; qv[4 * c + 3] = t.w;
+  }
+  float mx = -FLT_MAX;
+  for(int p = warp; p < len; p += W) {
+    const float4* kr = reinterpret_cast<const float4*>(ks + p * DH);
+    float a[G];
 #pragma unroll
-      for(int j = 0; j < G; ++j) {
-        float d = __fmul_rn(qv[4 * j], kr[4 * j]);
-        d = __fmaf_rn(qv[4 * j + 1], kr[4 * j + 1], d);
-        d = __fmaf_rn(qv[4 * j + 2], kr[4 * j + 2], d);
-        d = __fmaf_rn(qv[4 * j + 3], kr[4 * j + 3], d);
-        a[j] = d;
-      }
-      float sv = __fmul_rn(butterfly_order_sum<G>(a), scale);
-      if(mask)
-        sv = __fadd_rn(sv, mask[p]);
-      sc[p * 128 + threadIdx.x] = sv;
-      mx = fmaxf(mx, sv);
+    for(int j = 0; j < G; ++j) {
+      const float4 t = kr[j];
+      a[j] = __fmul_rn(qv[4 * j], t.x);
+      a[j] = __fmaf_rn(qv[4 * j + 1], t.y, a[j]);
+      a[j] = __fmaf_rn(qv[4 * j + 2], t.z, a[j]);
+      a[j] = __fmaf_rn(qv[4 * j + 3], t.w, a[j]);
     }
-    float part[G];
+    float sv = __fmul_rn(butterfly_order_sum<G>(a), scale);
+    if(log_mask)
+      sv = __fadd_rn(sv, ms[p]);
+    sc[p * kEncRows + lane] = sv;
+    mx = fmaxf(mx, sv);
+  }
+  maxima[warp * kEncRows + lane] = mx;
+  __syncthreads();
+#pragma unroll
+  for(int w = 0; w < W; ++w)
+    mx = fmaxf(mx, maxima[w * kEncRows + lane]);
+#pragma unroll
+  for(int j = 0; j < G; j += W) {   // partial sum j + warp: positions j + warp, j + warp + G, ...
+    float part = 0.f;
+    for(int p = j + warp; p < len; p += G) {
+      const float e = det_expf(__fadd_rn(sc[p * kEncRows + lane], -mx));
+      sc[p * kEncRows + lane] = e;
+      part = __fadd_rn(part, e);
+    }
+    parts[(j + warp) * kEncRows + lane] = part;
+  }
+  __syncthreads();
+  {
+    float a[G];
 #pragma unroll
     for(int j = 0; j < G; ++j)
-      part[j] = 0.f;
-    for(int p0 = 0; p0 < len; p0 += G) {
+      a[j] = parts[j * kEncRows + lane];
+    const float total = butterfly_order_sum<G>(a);
+    for(int p = warp; p < len; p += W)
+      sc[p * kEncRows + lane] = __fdiv_rn(sc[p * kEncRows + lane], total);
+  }
+  __syncthreads();
+  float acc[kOwn];
 #pragma unroll
-      for(int j = 0; j < G; ++j) {
-        if(p0 + j < len) {
-          const float e = det_expf(__fadd_rn(sc[(p0 + j) * 128 + threadIdx.x], -mx));
-          sc[(p0 + j) * 128 + threadIdx.x] = e;
-          part[j] = __fadd_rn(part[j], e);
-        }
-      }
-    }
-    const float total = butterfly_order_sum<G>(part);
-    float acc[DH];
+  for(int e = 0; e < kOwn; ++e)
+    acc[e] = 0.f;
+#pragma unroll 4
+  for(int p = 0; p < len; ++p) {
+    const float w = sc[p * kEncRows + lane];
+    const float4* vr = reinterpret_cast<const float4*>(vs + p * DH + warp * kOwn);
 #pragma unroll
-    for(int e = 0; e < DH; ++e)
-      acc[e] = 0.f;
-    for(int p = 0; p < len; ++p) {
-      const float w = __fdiv_rn(sc[p * 128 + threadIdx.x], total);
-      const float* vr = vs + p * DH;
-#pragma unroll
-      for(int e = 0; e < DH; ++e)
-        acc[e] = __fmaf_rn(w, vr[e], acc[e]);
-    }
-    if(active) {
-      float4* o4 = reinterpret_cast<float4*>(out + (row0 + qi) * dim + h * DH);
-#pragma unroll
-      for(int c = 0; c < DH / 4; ++c) {
-        const float4 t = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
-        o4[c] = t;
-        m_abs = max4u(m_abs, t);
-      }
+    for(int c = 0; c < kOwn / 4; ++c) {
+      const float4 t = vr[c];
+      acc[4 * c] = __fmaf_rn(w, t.x, acc[4 * c]);
+      acc[4 * c + 1] = __fmaf_rn(w, t.y, acc[4 * c + 1]);
+      acc[4 * c + 2] = __fmaf_rn(w, t.z, acc[4 * c + 2]);
+      acc[4 * c + 3] = __fmaf_rn(w, t.w, acc[4 * c + 3]);
     }
   }
-  if(absmax_slot) {
+  unsigned m_abs = 0u;
+  if(q0 + lane < len) {
+    float4* o4 = reinterpret_cast<float4*>(out + (row0 + q0 + lane) * dim + h * DH + warp * kOwn);
+#pragma unroll
+    for(int c = 0; c < kOwn / 4; ++c) {
+      const float4 t = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+      o4[c] = t;
+      m_abs = max4u(m_abs, t);
+    }
+  }
+  if(absmax_slot) {   // one atomic per block: all go to one address
     m_abs = __reduce_max_sync(0xffffffffu, m_abs);
-    if((threadIdx.x & 31) == 0 && m_abs != 0u)
-      atomicMax(absmax_slot, m_abs);
+    unsigned* red = reinterpret_cast<unsigned*>(maxima);   // (used up)
+    if(lane == 0)
+      red[warp] = m_abs;
+    __syncthreads();
+    if(warp == 0) {
+      m_abs = __reduce_max_sync(0xffffffffu, lane < W ? red[lane] : 0u);
+      if(lane == 0 && m_abs != 0u)
+        atomicMax(absmax_slot, m_abs);
+    }
   }
   trace_stamp(tb, kTrAttentionEnc, 2);
   trace_stamp(th.last, kTrAttentionEnc, 3);
@@ -1775,8 +1809,8 @@ int launch_attention1(const float* q, const float* k, const float* v, const floa
   if(dim > 1024)
     return MI8_ERR_UNSUPPORTED;
   if(mode == 2 && batch > 0 && rows == batch * len && anc == nullptr && (dim_head == 64 || dim_head == 32)) {
-    // encoder: keys/values of a (sentence, head) staged in shared memory, one thread per query position
-    const size_t esmem = (static_cast<size_t>(len) * dim_head * 2 + static_cast<size_t>(len) * 128) * sizeof(float);
+    // encoder: keys/values of a (sentence, head) staged in shared memory
+    const size_t esmem = attention_enc_smem(dim_head, len);
     if(esmem <= 200 * 1024) {
       static bool attr_set[64][2] = {};
       int dev = 0;
@@ -1791,10 +1825,11 @@ int launch_attention1(const float* q, const float* k, const float* v, const floa
         }
         attr_set[dev][which] = true;
       }
+      const dim3 egrid(batch, heads, (len + kEncRows - 1) / kEncRows);
       if(which == 0)
-        launch_kernel(attention_enc_kernel<64>, dim3(batch, heads), dim3(128), esmem, s, q, k, v, log_mask, heads, len, scale, out, slot);
+        launch_kernel(attention_enc_kernel<64>, egrid, dim3(kEncWarps * 32), esmem, s, q, k, v, log_mask, heads, len, scale, out, slot);
       else
-        launch_kernel(attention_enc_kernel<32>, dim3(batch, heads), dim3(128), esmem, s, q, k, v, log_mask, heads, len, scale, out, slot);
+        launch_kernel(attention_enc_kernel<32>, egrid, dim3(kEncWarps * 32), esmem, s, q, k, v, log_mask, heads, len, scale, out, slot);
       count_launch();
       return check_launch();
     }
