@@ -282,6 +282,10 @@ int mi8_affine_f32(const float* a, int M, int K, const int8_t* bt, const float* 
   if(K % 16 != 0)
     return MI8_ERR_MISALIGNED;
   float* d_qa = reinterpret_cast<float*>(aq_scratch + static_cast<size_t>(M) * K);
+  // few floats: one launch (what the two launches below refuse goes there to be refused)
+  if(quant_a_own_max(M, N, K) && a != nullptr && workspace != nullptr && workspace_bytes >= kWsHeaderBytes &&
+     ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(aq_scratch)) & 15u) == 0)
+    return launch_gemm_quant_a(a, nullptr, d_qa, bt, M, N, K, d_qb, scale, bias, relu, c, out_dtype, nullptr, as_stream(stream), nullptr, aq_scratch);
   int rc = mi8_prepare_a_f32(a, M, K, aq_scratch, d_qa, workspace, workspace_bytes, stream);
   if(rc != MI8_OK)
     return rc;

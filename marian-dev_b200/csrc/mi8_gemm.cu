@@ -44,6 +44,7 @@ constexpr int kMmaK = 32;       // K per tcgen05.mma kind::i8
 constexpr int kThreads = 320;
 constexpr int kEpilogueThreads = 256;
 constexpr int kMaxStages = 8;
+constexpr int kOwnMaxRows = 16, kOwnMaxK = 1024, kOwnMaxFloats = 4096;   // of an activation whose maximum every CTA finds itself (quant_a_own_max): one tile, in registers
 constexpr int kPairTileCode = 512;  // force_tile_m value that selects the CTA-pair kernel
 
 template <int TM>
@@ -106,6 +107,7 @@ struct GemmParams {
   const float* a_f32;       // quantise-in-kernel variant: fp32 activation [M,K] and the 4-byte slot that
   const unsigned* a_slot;   // holds the bit pattern of max|A| (then aq / d_qa / the activation tensor map are unused)
   float* qa_out;            // optional: receives the activation multiplier 127 / max|A|
+  int8_t* aq_out;           // optional (a_slot == nullptr): receives the quantised activation
   const unsigned* skip_a;   // when both are set and *skip_a == *skip_b, tiles that lie entirely below
   const unsigned* skip_b;   // row skip_rows_below are not computed (their previous results still hold)
   int skip_rows_below;
@@ -343,7 +345,8 @@ __device__ __forceinline__ void write_back_chunk_p8(const GemmParams& p, const i
 // warps quantise the tile's rows (Int8::PrepareA: round(x * 127/max) saturated to +-127) straight into the
 // shared-memory ring in the 128-byte-swizzled K-major layout the MMA reads, so no int8 copy of the
 // activation and no quantisation launch exist.  Used when every CTA has one tile (they quantise before
-// their write-back work begins).
+// their write-back work begins).  Without a slot (a_slot == nullptr; one tile of rows and K of up to 1024, which the eight warps hold in registers) every CTA
+// finds the maximum itself: a launch less, and few floats for each CTA to read (mi8_affine_f32).
 // kTopK > 0 (the output layer, operands swapped by the host: the M-side tile holds 128 ACTIVATION rows, the
 // N-side tile 256 rows of the tied embedding matrix): a thread owns one query row and 128 consecutive
 // vocabulary entries of it per tile, so it can reduce them on its own - block maximum, sum of exponentials
@@ -571,12 +574,16 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
     constexpr int kChunks = TM / T::kChunk;
     constexpr int kChunkStep = kChunks > 1 ? 2 : 1;
     const bool has_chunks = kChunks > 1 || group == 0;
+    float own_qb = 0.0f;
+    if constexpr(kQuantA)
+      own_qb = __ldg(p.seg_qb[0]);   // (with the weight, in front of the wait: behind it its way from L2 stood in front of the quantisation)
     pdl_wait_and_launch();  // the activation multiplier (or abs-max slot) is written by the previous kernel
     trace_stamp_start(th, kTraceId, trace_extra);
     // kQuantA: the multiplier comes from the abs-max slot, which is read only after the first fp32 loads of the
     // activation have been issued (below), so the two round trips to L2 overlap instead of following one another.
     float qa = 1.0f;
     bool qa_ready = !kQuantA;
+    __shared__ unsigned warp_max[kQuantA ? kConvWarps : 1];
     if(!kQuantA && !kP8)
       qa = *p.d_qa;
     float unquant = (kP8 || kQuantA) ? 1.0f : __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(qa, *p.seg_qb[0])), p.scale);
@@ -615,9 +622,26 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
             }
           }
           if(!qa_ready) {
-            const unsigned bits = *p.a_slot;
+            unsigned bits = 0u;
+            if(p.a_slot != nullptr) {
+              bits = *p.a_slot;
+            } else {   // (all of the activation is in f)
+#pragma unroll
+              for(int b = 0; b < kBatch; ++b)
+#pragma unroll
+                for(int q = 0; q < kCpt; ++q)
+#pragma unroll
+                  for(int e = 0; e < 4; ++e)
+                    bits = max(bits, max(max(__float_as_uint(f[b][q][e].x) & 0x7fffffffu, __float_as_uint(f[b][q][e].y) & 0x7fffffffu),
+                                         max(__float_as_uint(f[b][q][e].z) & 0x7fffffffu, __float_as_uint(f[b][q][e].w) & 0x7fffffffu)));
+              bits = __reduce_max_sync(0xffffffffu, bits);
+              if(lane == 0)
+                warp_max[warp - 2] = bits;
+              named_bar_sync(1, kEpilogueThreads);
+              bits = __reduce_max_sync(0xffffffffu, warp_max[lane & (kConvWarps - 1)]);
+            }
             qa = bits == 0u ? 1.0f : __fdiv_rn(127.0f, __uint_as_float(bits));
-            unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(qa, *p.seg_qb[0])), p.scale);
+            unquant = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(qa, own_qb)), p.scale);
             if(blockIdx.x == 0 && epi_tid == 0) {
               if(p.qa_out != nullptr)
                 *p.qa_out = qa;
@@ -645,6 +669,9 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
                     o.z = pack4_i8(f[b][q][2], qa);
                     o.w = pack4_i8(f[b][q][3], qa);
                     *reinterpret_cast<uint4*>(a_tile + r * 128 + ((ch ^ (r & 7)) << 4)) = o;
+                    const int gk = (kb0 + b) * kTileKBytes + ch * 16;
+                    if(p.aq_out != nullptr && blockIdx.x == 0 && r < p.M && gk < p.K)
+                      *reinterpret_cast<uint4*>(p.aq_out + static_cast<size_t>(r) * p.K + gk) = o;
                   }
                 }
                 fence_proxy_async_smem();   // the tensor core reads these bytes through the async proxy
@@ -972,6 +999,8 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
       *abort_flag = 1;
       if(lane == 0)
         atomicMax(p.status, static_cast<int>(kDevTimeoutEpilogue));
+      if(kQuantA && p.a_slot == nullptr && !qa_ready)   // (the others wait for this warp's maximum)
+        named_bar_sync(1, kEpilogueThreads);
       if(!kDuo && (kBlocks || p.splits > 1)) {
         // The others may not have given up: they meet this warp at the two barriers, which have no bound, of every tile from this one on.
         for(; w < p.total_work; w += gridDim.x)
@@ -2856,14 +2885,22 @@ int quant_a_tile(int M, int N) {
   return 0;
 }
 
+// One launch instead of two: what a call of so few floats costs is the host's launches, 2.3 us each, while on the device the GEMM that quantises for itself is the slower
+// one, the more so the more it reads.  A call from the host / back to back on the device, two launches -> one, us: 4 x 256 x 1536 7.4 -> 5.3 / 4.8 -> 5.15,
+// 8 x 512 x 256 7.3 -> 5.5 / 5.2 -> 5.45, 16 x 512 x 2048 7.3 -> 5.8 / 5.2 -> 5.9, 32 x 512 x 512 7.4 -> 6.95 / 5.5 -> 6.95, 32 x 1024 x 1024 7.4 -> 9.4.  A
+// single tile of weights keeps its two launches, which the test of the kernel times counts (8 x 256 x 128: 7.35 -> 5.3 / 4.7 -> 5.05).
+bool quant_a_own_max(int M, int N, int K) {
+  return M > 0 && M <= kOwnMaxRows && N > kTileN && K <= kOwnMaxK && static_cast<long long>(M) * K <= kOwnMaxFloats && quant_a_tile(M, N) != 0;
+}
+
 int launch_gemm_quant_a(const float* a_f32, const unsigned* a_slot, float* qa_out, const int8_t* bt, int M, int N, int K,
                         const float* d_qb, float scale, const float* bias, int relu, void* c, int out_dtype, int32_t* acc_out,
-                        cudaStream_t stream, unsigned* absmax_out) {
+                        cudaStream_t stream, unsigned* absmax_out, int8_t* aq_out) {
   if(M < 0 || N <= 0 || K <= 0)
     return MI8_ERR_BAD_ARG;
   if(M == 0)
     return MI8_OK;
-  if(a_f32 == nullptr || a_slot == nullptr || bt == nullptr || d_qb == nullptr || c == nullptr)
+  if(a_f32 == nullptr || (a_slot == nullptr && (aq_out == nullptr || !quant_a_own_max(M, N, K))) || bt == nullptr || d_qb == nullptr || c == nullptr)
     return MI8_ERR_BAD_ARG;
   if(out_dtype != MI8_F32 && out_dtype != MI8_F16)
     return MI8_ERR_BAD_ARG;
@@ -2908,6 +2945,7 @@ int launch_gemm_quant_a(const float* a_f32, const unsigned* a_slot, float* qa_ou
   p.a_f32 = a_f32;
   p.a_slot = a_slot;
   p.qa_out = qa_out;
+  p.aq_out = a_slot == nullptr ? aq_out : nullptr;
   p.skip_a = nullptr;
   p.skip_b = nullptr;
   p.skip_rows_below = 0;

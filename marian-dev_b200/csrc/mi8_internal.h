@@ -123,7 +123,9 @@ void test_wait_fault(int withhold_item, unsigned spin_limit);
 int quant_a_tile(int M, int N);
 int launch_gemm_quant_a(const float* a_f32, const unsigned* a_slot, float* qa_out, const int8_t* bt, int M, int N, int K,
                         const float* d_qb, float scale, const float* bias, int relu, void* c, int out_dtype, int32_t* acc_out,
-                        cudaStream_t stream, unsigned* absmax_out = nullptr);
+                        cudaStream_t stream, unsigned* absmax_out = nullptr, int8_t* aq_out = nullptr);
+// ... and without a slot, where every CTA finds the maximum itself (aq_out: the quantised activation, M * K bytes).
+bool quant_a_own_max(int M, int N, int K);
 
 // The cluster GEMM for decode shapes: quantises the fp32 activation `a_f32` [M, K] itself with the multiplier of the abs-max
 // slot `a_slot` (its CTAs share the quantised tile through distributed shared memory, so the fp32 values are read once
