@@ -551,7 +551,7 @@ int gemm_fused(mi8d_decoder* d, const int8_t* a, const float* qa, int M, const F
 // (src/tensors/cpu/mjdgemm/mjdgemm_avx512.cpp:195-276), kept in the decoder's per-row arrays until the next quantisation.
 int quantize_act(mi8d_decoder* d, const float* x, int M, int K, const unsigned* slot, int8_t* q, cudaStream_t s) {
   if(d->p8)
-    return launch_p8_quantize_rows(x, M, K, reinterpret_cast<uint8_t*>(q), d->p8_scale_a, d->p8_zp_a, d->p8_sum_a, s);
+    return launch_p8_quantize_rows(x, M, K, reinterpret_cast<uint8_t*>(q), d->p8_scale_a, d->p8_zp_a, d->p8_sum_a, s, false);
   return launch_quantize_slot(x, static_cast<size_t>(M) * K, slot, q, reinterpret_cast<float*>(q + static_cast<size_t>(M) * K), s);
 }
 

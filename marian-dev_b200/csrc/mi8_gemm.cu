@@ -393,8 +393,8 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
   auto is_below = [&](int w) { return kBelow && w >= p.n_tiles * p.m_tiles; };
   auto items = [&](bool skip_on) { return kBelow && skip_on ? p.n_tiles * p.m_tiles : p.total_work; };   // what this launch has to do
 
-  // packed8avx512: the quantisation of rows behind this triggers late itself and is the longer for its set-up (256 x 1024 x 4096 9.05 us with both late, 8.55 so;
-  // transformer-base, 64 x beam 4 17.35 -> 17.1 ms)
+  // packed8avx512: the quantisation of rows behind this is the longer for its set-up (256 x 1024 x 4096 9.05 us behind the wait, 8.55 so; transformer-base, 64 x beam 4
+  // 17.35 -> 17.1 ms)
   if(kP8)
     pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
