@@ -1290,12 +1290,19 @@ __device__ __forceinline__ void finish_step(const StepEnd& e, int r, int k, int 
   }
 }
 
+// mx + log(sum of the nb terms, added in ascending order).
+__device__ __forceinline__ float lse_of_terms(const float* terms, int nb, float mx) {
+  float total = 0.f;
+#pragma unroll 16
+  for(int b = 0; b < nb; ++b)   // (unrolled: the loads run ahead of the chain of additions)
+    total = __fadd_rn(total, terms[b]);
+  return __fadd_rn(mx, det_logf(total));
+}
+
 // Combines the per-block pairs (m_b, s_b) of one row, held in shared memory, into the row's log-sum-exp:
 // M = max_b m_b;  S = sum over b ascending of s_b * exp(m_b - M), product and sum rounded separately;
-// lse = M + log(S).  bm/bs: nb entries each; red: 33 floats.  Every thread returns the same value.  `beside` is called by all threads
-// while warp 0 walks the chain of additions (it may read bm).
-template <typename F>
-__device__ __forceinline__ float lse_from_blocks(const float* bm, float* bs, int nb, float* red, F&& beside) {
+// lse = M + log(S).  bm/bs: nb entries each; red: 33 floats.  Every thread returns the same value.
+__device__ __forceinline__ float lse_from_blocks(const float* bm, float* bs, int nb, float* red) {
   float mx = -FLT_MAX;
   for(int b = threadIdx.x; b < nb; b += blockDim.x)
     mx = fmaxf(mx, bm[b]);
@@ -1311,14 +1318,8 @@ __device__ __forceinline__ float lse_from_blocks(const float* bm, float* bs, int
   for(int b = threadIdx.x; b < nb; b += blockDim.x)
     bs[b] = __fmul_rn(bs[b], det_expf(__fadd_rn(bm[b], -mx)));
   __syncthreads();
-  if(threadIdx.x == 0) {
-    float total = 0.f;
-#pragma unroll 16
-    for(int b = 0; b < nb; ++b)   // (unrolled: the loads run ahead of the chain of additions)
-      total = __fadd_rn(total, bs[b]);
-    red[32] = __fadd_rn(mx, det_logf(total));
-  }
-  beside();
+  if(threadIdx.x == 0)
+    red[32] = lse_of_terms(bs, nb, mx);
   __syncthreads();
   return red[32];
 }
@@ -1326,10 +1327,16 @@ __device__ __forceinline__ float lse_from_blocks(const float* bm, float* bs, int
 constexpr size_t kLseBlockBytes = 32 * 1024;   // the blocks' maxima and sums of the widest row that is taken
 __host__ __device__ constexpr size_t lse_staged_floats(int threads, bool from_blocks) { return from_blocks ? 0 : static_cast<size_t>(threads) * 32; }
 
+__device__ __forceinline__ float warp_max(float v) {   // (no NaN)
+  float m;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(v));
+  return m;
+}
+
 // One block per row: cand_score[r][j] = (j-th largest logit - logsumexp(row)) + prev_score[r], cand_word[r][j].
 // The log-sum-exp is defined over blocks of 128 consecutive entries (the unit the output GEMM's write-back
 // owns): per block its maximum m_b and s_b = sum of det_expf(x - m_b) with the entries added one after the
-// other in ascending order; the blocks are combined by lse_from_blocks.
+// other in ascending order; the blocks are combined as lse_from_blocks does it.
 //
 // Bound by instruction issue (about 20 per logit, most of them the exponential), so the work per logit is kept small:
 //   * Four neighbouring lanes share a block of 128 entries, 32 consecutive ones each, held in registers from the one
@@ -1347,8 +1354,11 @@ __host__ __device__ constexpr size_t lse_staged_floats(int threads, bool from_bl
 // 512 rows of 32000 logits with a list of k per thread and a block of 128 per lane: 55.6 us back to back and 42.6 us inside a
 // decoder step (logits in L2); 34.0 and 24.7 us as described, 26.9 back to back with the block sizes below.
 // kThreads: 1024 (one pass over 32000 logits, one block per SM) while every row has an SM to itself, 512 (two blocks per SM) up to two
-// rows per SM, 256 (four) beyond, registers held to 64 so that they fit: 148 rows 14.9 us with the picks after the sum, 13.4 now; 256
-// rows 29.1 us with 256 threads, 18.0 now; 512 rows 33.8 us, 26.9 now.
+// rows per SM, 256 (four) beyond, registers held to 64 so that they fit: 256 rows 29.1 us with 256 threads, 18.0 with 512.
+// After the scan no warp waits for the block's maximum (each takes it from the warps' maxima), one warp picks the blocks with two warp
+// reductions a pick while another walks the chain of additions.  Back to back, against the maximum by two block-wide waits and picks by
+// shuffles: rows of 32000: one 14.0 us to 10.8, 148 14.8 to 11.7, 296 20.7 to 17.6, 512 29.7 to 26.6, 768 43.2 to 37.0.  (That warp
+// collecting the picked blocks' entries as well, while the sum runs, instead of all warps behind it: 512 rows 31.1 us.)
 // kFromBlocks: the blocks' maxima and sums were left by the output layer's write-back (few rows); no scan.
 template <int kThreads, bool kFromBlocks = false>
 __global__ void __launch_bounds__(kThreads, 1024 / kThreads)
@@ -1373,6 +1383,7 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float* row = logits + static_cast<size_t>(r) * vocab;
   const int nb = (vocab + 127) / 128;
+  float most = -FLT_MAX;   // of the blocks' maxima that this lane has seen
   float* bm = lse_smem + lse_staged_floats(kThreads, kFromBlocks);
   float* bs = bm + nb;
   const bool vec = (vocab & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15u) == 0;
@@ -1381,6 +1392,7 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
   if(kFromBlocks) {
     for(int b = threadIdx.x; b < nb; b += kThreads) {
       bm[b] = __ldg(block_max + static_cast<size_t>(r) * nb + b);
+      most = fmaxf(most, bm[b]);
       bs[b] = __ldg(block_sum + static_cast<size_t>(r) * nb + b);
     }
   }
@@ -1434,6 +1446,7 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
       m = fmaxf(m, x[j]);
     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    most = fmaxf(most, m);
     if(cnt == 32) {
 #pragma unroll
       for(int j = 0; j < 32; ++j)
@@ -1457,42 +1470,52 @@ lse_topk_kernel(const float* __restrict__ logits, int vocab, int k, const float*
       bs[b] = sum;
     }
   }
+  most = warp_max(most);
+  if(lane == 0)
+    red[warp] = most;
   __syncthreads();
-  // While warp 0 sums the blocks: the k blocks with the best maxima (warp 1), k rounds, each picks the best block that follows the
-  // last pick.
-  auto pick_blocks = [&]() {
-    if(warp != 1)
-      return;
-    float last_v = FLT_MAX;
-    int last_i = -1;
-    for(int j = 0; j < k; ++j) {
-      float v = -FLT_MAX;
-      int i = 0x7fffffff;
+  if(warp != 1) {
+    // Every warp but one: the blocks' terms of the sum; warp 0 then adds them up.
+    const float mx = warp_max(lane < kThreads / 32 ? red[lane] : -FLT_MAX);
+    for(int b = warp == 0 ? lane : threadIdx.x - 32; b < nb; b += kThreads - 32)
+      bs[b] = __fmul_rn(bs[b], det_expf(__fadd_rn(bm[b], -mx)));
+    if(warp == 0) {
+      asm volatile("bar.sync 1, %0;" ::"n"(kThreads - 32) : "memory");
+      if(lane == 0)
+        red[32] = lse_of_terms(bs, nb, mx);
+    } else {
+      asm volatile("bar.arrive 1, %0;" ::"n"(kThreads - 32) : "memory");
+    }
+  } else {
+    // Warp 1 meanwhile: the k blocks with the best maxima, k rounds, each picks the best block that follows the last pick; a lane keeps
+    // the best of its own blocks.
+    float v, last_v = FLT_MAX;
+    int i, last_i = -1;
+    auto next_own = [&]() {
+      v = -FLT_MAX;
+      i = 0x7fffffff;
       for(int b = lane; b < nb; b += 32) {
         const float bv = bm[b];
-        if((j == 0 || better(last_v, last_i, bv, b)) && better(bv, b, v, i)) {
+        if((last_i < 0 || better(last_v, last_i, bv, b)) && better(bv, b, v, i)) {
           v = bv;
           i = b;
         }
       }
-#pragma unroll
-      for(int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, i, o);
-        if(better(ov, oi, v, i)) {
-          v = ov;
-          i = oi;
-        }
-      }
-      last_v = v;
-      last_i = i;
+    };
+    next_own();
+    for(int j = 0; j < k; ++j) {
+      last_v = warp_max(v);
+      last_i = __reduce_min_sync(0xffffffffu, v == last_v ? i : 0x7fffffff);
       if(lane == 0)
-        pick[j] = i;   // 0x7fffffff: there are fewer than k blocks
+        pick[j] = last_i;   // 0x7fffffff: there are fewer than k blocks
+      if(i == last_i && i != 0x7fffffff)
+        next_own();
     }
     if(lane == 0)
       s_floor = last_v;
-  };
-  const float lse = lse_from_blocks(bm, bs, nb, red, pick_blocks);
+  }
+  __syncthreads();
+  const float lse = red[32];
   const float floor_v = s_floor;
   // Without k maxima above the lowest finite value the argument above does not hold (a block without a single number shares that
   // maximum): then the k best are searched for one by one.
@@ -1610,7 +1633,7 @@ lse_merge_kernel(const float* __restrict__ blk_max, const float* __restrict__ bl
     s_i[threadIdx.x * KT + j] = t.i[j];
   }
   __syncthreads();
-  const float lse = lse_from_blocks(bm, bs, nb, red, []() {});
+  const float lse = lse_from_blocks(bm, bs, nb, red);
   topk_block_merge<KT>(s_v, s_i);
   if(threadIdx.x < k) {
     const float ps = prev_scores ? prev_scores[r] : 0.f;
