@@ -37,7 +37,7 @@ if ROOT not in sys.path:
 KERNEL_NAMES = ["mi8_gemm_pair_kernel", "mi8_gemm_kernel", "quantize_slot_kernel", "attention1_kernel", "attention_cross_kernel", "attention_enc_kernel",
                 "add_layernorm_kernel", "add_layernorm_quant_kernel", "quantize_dual_kernel", "lse_topk_kernel",
                 "lse_merge_kernel", "nbest_merge_kernel", "step_begin_kernel", "embed_ancestors_kernel", "embed_kernel", "gather_rows_kernel",
-                "ssru_cell_kernel", "mi8_absmax_kernel", "mi8_quantize_kernel", "mi8_prepare_cluster_kernel", "mi8_transpose_quantize_kernel"]
+                "ssru_cell_kernel", "mi8_absmax_kernel", "mi8_quantize_kernel", "mi8_prepare_cluster_kernel", "mi8_convert_kernel"]
 METRIC = "int8_decode_tgt_tokens_per_sec"
 UNIT = "tokens/s"
 WORKLOAD = "transformer-big decode (6+6 layers, d=1024, ffn=4096, 16 heads, tied 32000 vocab, all affines int8), beam 4, mini-batch 128, lengths clip(N(30,12),4,128), max length 1.5x source"

@@ -1,5 +1,5 @@
 """Encoder self-attention, 32 query positions a block: lengths around a block's queries, a warp's key positions, a head's interleaved sums and what shared memory
-holds (the lengths beyond take the one-row kernel), with and without a mask; bit for bit the CPU checker's."""
+holds (the lengths beyond take the one-row kernel), with and without a mask; bit for bit the oracle's."""
 import numpy as np
 import pytest
 import torch
