@@ -124,14 +124,18 @@ __device__ __forceinline__ float block_reduce(float v, float* smem, bool is_max)
 //   q = nearest_even(min(max(fma(x, 1 / scaleA, zeroPointA), 0), 255)), sumA = sum of q.
 // A row whose values are all equal (the reference divides by zero there) first widens its range to
 // contain 0; an all-zero row takes scaleA = 1.  Inf or NaN in the row raises the non-finite status.
-// `early`: the next kernel may begin at once.  For one affine after the other (256 x 512 x 16000 12.45 us, 12.57 behind the wait; 256 x 1024 x 4096 8.47 and 8.64), not in
+// kEarly: the next kernel may begin at once.  For one affine after the other (256 x 512 x 16000 12.45 us, 12.57 behind the wait; 256 x 1024 x 4096 8.47 and 8.64), not in
 // the chain of a decoder step (transformer-base, 64 x beam 4 17.4 ms, 17.1 behind the wait).
+template <bool kEarly>
 __global__ void __launch_bounds__(kBlock)
 p8_quantize_rows_kernel(const float* __restrict__ a, int K, uint8_t* __restrict__ aq, float* __restrict__ scale_a, int32_t* __restrict__ zp_a,
-                        int32_t* __restrict__ sum_a, int* status, int early) {
-  if(early)
+                        int32_t* __restrict__ sum_a, int* status) {
+  if(kEarly) {
     pdl_launch_dependents();
-  pdl_wait_and_launch();
+    pdl_wait();
+  } else {
+    pdl_wait_and_launch();
+  }
   __shared__ float red[kBlock / 32];
   __shared__ int red_i[kBlock / 32];
   const int m = blockIdx.x;
@@ -192,13 +196,16 @@ __device__ __forceinline__ int p8_q(float x, float inv, float zf) {
 
 // The same for rows of at most 128 * kVec values: one WARP per row, the row held in registers (kVec 16-byte loads per
 // lane, all issued before the first use), statistics by shuffles - one pass over global memory and no block barrier.
-template <int kVec>
+template <int kVec, bool kEarly>
 __global__ void __launch_bounds__(kBlock)
 p8_quantize_rows_warp_kernel(const float* __restrict__ a, int M, int K, uint8_t* __restrict__ aq, float* __restrict__ scale_a,
-                             int32_t* __restrict__ zp_a, int32_t* __restrict__ sum_a, int* status, int early) {
-  if(early)
+                             int32_t* __restrict__ zp_a, int32_t* __restrict__ sum_a, int* status) {
+  if(kEarly) {
     pdl_launch_dependents();
-  pdl_wait_and_launch();
+    pdl_wait();
+  } else {
+    pdl_wait_and_launch();
+  }
   const int lane = threadIdx.x & 31;
   const int m = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
   if(m >= M)
@@ -310,15 +317,18 @@ int launch_p8_quantize_rows(const float* a, int M, int K, uint8_t* aq, float* sc
   if(status == nullptr)
     return MI8_ERR_LAUNCH;
   const int warp_grid = (M + kBlock / 32 - 1) / (kBlock / 32);
+  auto by_warps = [&](auto late, auto at_once) {
+    return launch_kernel(early ? at_once : late, dim3(warp_grid), dim3(kBlock), 0, stream, a, M, K, aq, scale_a, zp_a, sum_a, status);
+  };
   cudaError_t e;
   if(K <= 512)
-    e = launch_kernel(p8_quantize_rows_warp_kernel<4>, dim3(warp_grid), dim3(kBlock), 0, stream, a, M, K, aq, scale_a, zp_a, sum_a, status, early ? 1 : 0);
+    e = by_warps(p8_quantize_rows_warp_kernel<4, false>, p8_quantize_rows_warp_kernel<4, true>);
   else if(K <= 1024)
-    e = launch_kernel(p8_quantize_rows_warp_kernel<8>, dim3(warp_grid), dim3(kBlock), 0, stream, a, M, K, aq, scale_a, zp_a, sum_a, status, early ? 1 : 0);
+    e = by_warps(p8_quantize_rows_warp_kernel<8, false>, p8_quantize_rows_warp_kernel<8, true>);
   else if(K <= 2048)
-    e = launch_kernel(p8_quantize_rows_warp_kernel<16>, dim3(warp_grid), dim3(kBlock), 0, stream, a, M, K, aq, scale_a, zp_a, sum_a, status, early ? 1 : 0);
+    e = by_warps(p8_quantize_rows_warp_kernel<16, false>, p8_quantize_rows_warp_kernel<16, true>);
   else
-    e = launch_kernel(p8_quantize_rows_kernel, dim3(M), dim3(kBlock), 0, stream, a, K, aq, scale_a, zp_a, sum_a, status, early ? 1 : 0);
+    e = launch_kernel(early ? p8_quantize_rows_kernel<true> : p8_quantize_rows_kernel<false>, dim3(M), dim3(kBlock), 0, stream, a, K, aq, scale_a, zp_a, sum_a, status);
   if(e != cudaSuccess) {
     set_last_cuda_error(e);
     return MI8_ERR_LAUNCH;
