@@ -178,6 +178,7 @@ int mi8_multiply_i8_rows_from(const int8_t* aq, const int8_t* bt, int M, int N, 
  * (src/graph/expression_operators.cpp:554-731 dispatching to
  * src/tensors/cpu/intgemm_interface.h:46-99): prepareA into aq_scratch (M*K + 4 bytes, multiplier
  * in the last 4), then the multiply with the fused epilogue.  bias NULL = dot.
+ * `a` is read before anything is stored: c may lie over it (and so may aq_scratch); c and aq_scratch lie apart.
  */
 int mi8_affine_f32(const float* a, int M, int K, const int8_t* bt, const float* d_qb, int N,
                    const float* bias, float scale, int relu, void* c, int out_dtype,

@@ -105,6 +105,13 @@ int sm_count() {
 
 using namespace mi8;
 
+namespace {
+bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return x < y + b_bytes && y < x + a_bytes;
+}
+}  // namespace
+
 extern "C" {
 
 int mi8_version(void) { return 10200; }
@@ -282,9 +289,12 @@ int mi8_affine_f32(const float* a, int M, int K, const int8_t* bt, const float* 
   if(K % 16 != 0)
     return MI8_ERR_MISALIGNED;
   float* d_qa = reinterpret_cast<float*>(aq_scratch + static_cast<size_t>(M) * K);
-  // few floats: one launch (what the two launches below refuse goes there to be refused)
+  // few floats: one launch (what the two launches below refuse goes there to be refused).  Its CTAs read all of `a` while others already store their part of
+  // the results and CTA 0 the scratch; the two launches have read `a` before anything is stored, so they take what lies over it.
+  const size_t floats = static_cast<size_t>(M) * K, c_bytes = static_cast<size_t>(M) * N * (out_dtype == MI8_F16 ? 2 : 4);
   if(quant_a_own_max(M, N, K) && a != nullptr && workspace != nullptr && workspace_bytes >= kWsHeaderBytes &&
-     ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(aq_scratch)) & 15u) == 0)
+     ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(aq_scratch)) & 15u) == 0 && !overlap(a, 4 * floats, c, c_bytes) &&
+     !overlap(a, 4 * floats, aq_scratch, floats + 4) && !overlap(c, c_bytes, aq_scratch, floats + 4))
     return launch_gemm_quant_a(a, nullptr, d_qa, bt, M, N, K, d_qb, scale, bias, relu, c, out_dtype, nullptr, as_stream(stream), nullptr, aq_scratch);
   int rc = mi8_prepare_a_f32(a, M, K, aq_scratch, d_qa, workspace, workspace_bytes, stream);
   if(rc != MI8_OK)
