@@ -1104,6 +1104,7 @@ namespace {
 
 // How a step of mi8d_search is tied to the one behind it (StepEnd has the words' meaning): `end` carries them to the step's last kernel.
 struct StepLink {
+  bool in_search = false;   // (what lies in front of the step is the search's own)
   const unsigned* stop = nullptr;
   unsigned* next_stop = nullptr;
   int* next_ctrl = nullptr;
@@ -1231,7 +1232,7 @@ int run_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const i
     p.cell_old = first.cell[d->cell_cur];
     p.cell_new = first.cell[cell_new];
     p.layer_stride = static_cast<size_t>(next.cross_k - first.cross_k);
-    MI8D_TRY(launch_decoder_rows(p, dm, c.heads, s));
+    MI8D_TRY(launch_decoder_rows(p, dm, c.heads, s, link.in_search));
   } else if(c.ssru) {
     MI8D_TRY(launch_embed(d->wemb, words, pos, 0, emb_scale, R, dm, x, nullptr, d->input_slot(0), s));
   } else {
@@ -1526,6 +1527,7 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
   // What step t needs to know of its neighbours, while `active` and W are those of step t
   const auto link_of = [&](int t, int nb, int max_beam, bool launched_ahead) {
     StepLink link;
+    link.in_search = true;
     const int own = (t & 1) * 2 * kDecoderRowsMax, front = 2 * kDecoderRowsMax - own;
     const bool ahead = ahead_of(t, nb, max_beam);
     if(launched_ahead) {

@@ -316,7 +316,9 @@ constexpr int kWithholdWarp = MI8_TEST_ONE_WARP;
 void test_wait_limits(int* withhold_item, uint32_t* spin_limit);
 int rows_weight_map(CUtensorMap* map, const int8_t* bt, int N, int K);
 bool decoder_rows_supported(int rows, int d, int f, int heads, int layers, int src);
-int launch_decoder_rows(DecoderRowsParams& p, int d, int heads, cudaStream_t stream);
+// `params_settled`: what lies in front on the stream, as far as it has not completed when the launch is due, writes none of the registered parameters, which the kernel
+// reads in front of its wait.  Otherwise the launch is not overlapped.
+int launch_decoder_rows(DecoderRowsParams& p, int d, int heads, cudaStream_t stream, bool params_settled);
 int trace_set_rows(unsigned long long* buf);
 
 // Whether kernels are launched with programmatic dependent launch (mi8_set_pdl; on by default).

@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(kThreads, 1) decoder_rows_kernel(const __grid_
   bool ok = true;
 
   // The LayerNorms, this CTA's columns of the biases and the weights' multipliers, from where they were registered: a caller may rewrite
-  // them between steps (the kernels in front of a step do not write them).
+  // them between steps.  Like the weights above they are read in front of the wait: only mi8d_search's steps, which have its own kernels in front of them, are
+  // launched over the end of those; a step that a caller asks for starts when all in front of it has completed (launch_decoder_rows).
 #pragma unroll 1
   for(int l = 0; l < p.layers; ++l) {
     const DecoderRowsVectors& v = p.vec[l];
@@ -773,7 +774,7 @@ struct RowsKernel {
            rows * (f / kCtas / 4) <= 2 * kThreads && rows * (f / kCtas / 4) * (f / kCtas / 4) < 65536 && layers * T::units(f) <= 32 * kWarps &&
            T::smem(rows, f, layers, src, 1) <= static_cast<size_t>(kMaxDynSmem) && available();
   }
-  static int launch(DecoderRowsParams& p, cudaStream_t stream) {
+  static int launch(DecoderRowsParams& p, cudaStream_t stream, bool params_settled) {
     // as many units in flight per warp as fit, up to all of a warp's
     const int most = (p.layers * T::units(p.ffn) + kWarps - 1) / kWarps;
     p.ring = 1;
@@ -796,7 +797,7 @@ struct RowsKernel {
     cfg.stream = stream;
     cfg.attrs = attr;
     const bool timed = kernel_times_on();
-    cfg.numAttrs = pdl_enabled() && !timed ? 2 : 1;
+    cfg.numAttrs = pdl_enabled() && params_settled && !timed ? 2 : 1;
     if(timed)
       kernel_times_before(reinterpret_cast<const void*>(kernel), stream);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<const DecoderRowsParams&>(p));
@@ -828,14 +829,14 @@ bool decoder_rows_supported(int rows, int d, int f, int heads, int layers, int s
   return false;
 }
 
-int launch_decoder_rows(DecoderRowsParams& p, int d, int heads, cudaStream_t stream) {
+int launch_decoder_rows(DecoderRowsParams& p, int d, int heads, cudaStream_t stream, bool params_settled) {
   if(!decoder_rows_supported(p.rows, d, p.ffn, heads, p.layers, p.src))
     return MI8_ERR_UNSUPPORTED;
   test_wait_limits(&p.withhold_item, &p.spin_limit);
   p.status = device_status_ptr();
   if(p.status == nullptr)
     return MI8_ERR_LAUNCH;
-  return d == 256 ? Rows256::launch(p, stream) : Rows512::launch(p, stream);
+  return d == 256 ? Rows256::launch(p, stream, params_settled) : Rows512::launch(p, stream, params_settled);
 }
 
 }  // namespace mi8

@@ -1,0 +1,71 @@
+"""Parameters and weights that this library's own kernels write directly in front of the launch that reads them: the launch takes the new values, although
+launches overlap and fetch what does not change from call to call before the kernel in front is done.  (A longer kernel of the library goes first, so that the
+writer is still at work when the next launch is due.)"""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+def _copy(dst, src):
+    """dst = src, by a kernel of the library."""
+    from marian_dev_b200.binding import check, lib
+    check(lib().mi8_transpose_f32(src.data_ptr(), 1, 1, src.numel(), dst.data_ptr(), _stream()))
+
+
+def _max_into(multiplier, x, ws):
+    """*multiplier = 127 / max|x|, by a kernel of the library."""
+    from marian_dev_b200.binding import check, lib
+    check(lib().mi8_max_absolute_f32(x.data_ptr(), x.numel(), None, multiplier.data_ptr(), ws.ptr, ws.nbytes, _stream()))
+
+
+class _Busy:
+    def __init__(self, device):
+        self.x = torch.randn(2048, 2048, device=device)
+        self.y = torch.empty_like(self.x)
+
+    def __call__(self):
+        from marian_dev_b200.binding import check, lib
+        check(lib().mi8_transpose_f32(self.x.data_ptr(), 1, 2048, 2048, self.y.data_ptr(), _stream()))
+
+
+@pytest.mark.parametrize("dim,batch", [(256, 1), (256, 8), (512, 4)])
+@pytest.mark.parametrize("last", ["ffn_ffn_ln_bias", "rnn_bf", "ffn_b2", "context_Wo_ln_scale", "ffn_W1"])
+def test_decoder_step(cuda_device, dim, batch, last):
+    """A step of an SSRU decoder whose layers are one launch: the registered vector, or a matrix's multiplier, is written in front of mi8d_step."""
+    from marian_dev_b200 import decoder, model, ops
+    cfg = model.TransformerConfig(dim_emb=dim, dim_ffn=2 * dim, heads=8, enc_depth=1, dec_depth=2, vocab=515, decoder_autoreg="rnn")
+    net = decoder.Int8Transformer(cfg, model.random_init(cfg, dim), cuda_device)
+    stepper = decoder.NativeStepper(net, max_batch=batch, beam=1, max_src=5, max_steps=8)
+    g = torch.Generator(device=cuda_device).manual_seed(batch)
+    ctx, mask = torch.randn(batch, 5, dim, generator=g, device=cuda_device), torch.zeros(batch, 5, device=cuda_device)
+    name = "decoder_l2_" + last
+    matrix = name in net.w
+    assert matrix or name in net.p, sorted(net.p)
+    param = net.w[name].quant_mult if matrix else net.p[name].view(-1)
+    values = [torch.randn(64 if matrix else param.numel(), generator=g, device=cuda_device) * s + 1.0 for s in (0.3, 0.8)]
+    ws, busy = ops.default_workspace(cuda_device), _Busy(cuda_device)
+
+    def step(write):
+        stepper.start(ctx, mask)
+        write()
+        return stepper.step(None, None, None, None, 1, batch, 1)[0].copy()
+
+    def settled(v):
+        _max_into(param, v, ws) if matrix else param.copy_(v)
+        torch.cuda.synchronize()
+
+    def at_once(v):
+        busy()
+        _max_into(param, v, ws) if matrix else _copy(param, v)
+
+    want = [step(lambda: settled(v)) for v in values]
+    assert not np.array_equal(want[0], want[1])
+    for i in range(12):
+        assert np.array_equal(step(lambda: at_once(values[i & 1])), want[i & 1])
+    assert ops.poll_status() == 0
