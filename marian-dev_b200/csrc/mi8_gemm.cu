@@ -580,10 +580,10 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
     constexpr int kChunks = TM / T::kChunk;
     constexpr int kChunkStep = kChunks > 1 ? 2 : 1;
     const bool has_chunks = kChunks > 1 || group == 0;
+    wait_for_input();  // the activation multiplier (or abs-max slot) is written by the previous kernel
     float own_qb = 0.0f;
     if constexpr(kQuantA)
-      own_qb = __ldg(p.seg_qb[0]);   // (with the weight, in front of the wait: behind it its way from L2 stood in front of the quantisation)
-    wait_for_input();  // the activation multiplier (or abs-max slot) is written by the previous kernel
+      own_qb = __ldg(p.seg_qb[0]);   // (the previous kernel may have written this one too; asked for in front of the activation, whose way from L2 hides its own)
     trace_stamp_start(th, kTraceId, trace_extra);
     // kQuantA: the multiplier comes from the abs-max slot, which is read only after the first fp32 loads of the
     // activation have been issued (below), so the two round trips to L2 overlap instead of following one another.

@@ -69,3 +69,39 @@ def test_decoder_step(cuda_device, dim, batch, last):
     for i in range(12):
         assert np.array_equal(step(lambda: at_once(values[i & 1])), want[i & 1])
     assert ops.poll_status() == 0
+
+
+@pytest.mark.parametrize("m,k,n", [(4, 256, 1536), (1, 1024, 300), (16, 256, 129)])
+@pytest.mark.parametrize("entry", ["affine", "slot"])
+def test_weight_multiplier(cuda_device, m, k, n, entry):
+    """A weight's multiplier written in front of a product that quantises its activation itself."""
+    from marian_dev_b200 import ops
+    from marian_dev_b200.binding import check, lib
+    g = torch.Generator(device=cuda_device).manual_seed(n)
+    x = torch.randn(m, k, generator=g, device=cuda_device)
+    w = ops.prepareB(torch.randn(k, n, generator=g, device=cuda_device))
+    slot = ops.max_absolute(x)
+    values = [torch.randn(1 << 18, generator=g, device=cuda_device) * s for s in (0.3, 0.8)]
+    ws, busy, scratch = ops.default_workspace(cuda_device), _Busy(cuda_device), torch.empty(m * k + 64, dtype=torch.int8, device=cuda_device)
+
+    def product():
+        out = torch.empty(m, n, device=cuda_device)
+        if entry == "affine":
+            check(lib().mi8_affine_f32(x.data_ptr(), m, k, w.data.data_ptr(), w.quant_mult.data_ptr(), n, None, 1.0, 0, out.data_ptr(), 0, scratch.data_ptr(), ws.ptr,
+                                       ws.nbytes, _stream()))
+        else:
+            check(lib().mi8_multiply_f32_slot(x.data_ptr(), slot.data_ptr(), None, w.data.data_ptr(), m, n, k, w.quant_mult.data_ptr(), 1.0, None, 0, out.data_ptr(), 0,
+                                              None, _stream()))
+        return out
+
+    want = []
+    for v in values:
+        _max_into(w.quant_mult, v, ws)
+        torch.cuda.synchronize()
+        want.append(product())
+    assert not torch.equal(want[0], want[1])
+    for i in range(12):
+        busy()
+        _max_into(w.quant_mult, values[i & 1], ws)
+        assert torch.equal(product(), want[i & 1])
+    assert ops.poll_status() == 0
