@@ -44,7 +44,7 @@ constexpr int kMmaK = 32;       // K per tcgen05.mma kind::i8
 constexpr int kThreads = 320;
 constexpr int kEpilogueThreads = 256;
 constexpr int kMaxStages = 8;
-constexpr int kOwnMaxRows = 16, kOwnMaxK = 1024, kOwnMaxFloats = 4096;   // of an activation whose maximum every CTA finds itself (quant_a_own_max): one tile, in registers
+constexpr int kOwnMaxRows = 16, kOwnMaxK = 1024, kOwnMaxFloats = 4096, kOwnMaxLongN = 8192;   // of an activation whose maximum every CTA finds itself (quant_a_own_max): one tile, in registers
 constexpr int kPairTileCode = 512;  // force_tile_m value that selects the CTA-pair kernel
 
 template <int TM>
@@ -2893,10 +2893,15 @@ int quant_a_tile(int M, int N) {
 
 // One launch instead of two: what a call of so few floats costs is the host's launches, 2.3 us each, while on the device the GEMM that quantises for itself is the slower
 // one, the more so the more it reads.  A call from the host / back to back on the device, two launches -> one, us: 4 x 256 x 1536 7.4 -> 5.3 / 4.8 -> 5.15,
-// 8 x 512 x 256 7.3 -> 5.5 / 5.2 -> 5.45, 16 x 512 x 2048 7.3 -> 5.8 / 5.2 -> 5.9, 32 x 512 x 512 7.4 -> 6.95 / 5.5 -> 6.95, 32 x 1024 x 1024 7.4 -> 9.4.  A
-// single tile of weights keeps its two launches, which the test of the kernel times counts (8 x 256 x 128: 7.35 -> 5.3 / 4.7 -> 5.05).
+// 8 x 512 x 256 7.3 -> 5.5 / 5.2 -> 5.45, 16 x 512 x 2048 7.3 -> 5.8 / 5.2 -> 5.9, 4 x 1024 x 1024 7.5 -> 6.4 / 5.6 -> 6.4, 4 x 1024 x 8192 8.05 -> 7.2,
+// 32 x 512 x 512 7.4 -> 6.95 / 5.5 -> 6.95, 32 x 1024 x 1024 7.4 -> 9.4.  Where the weights fill the chip and K is long the device is what a call waits for:
+// 4 x 512 x 18900 7.5 -> 6.3 / 5.8 -> 6.35, 4 x 1024 x 18900 7.6 -> 8.4 / 6.9 -> 8.4; those keep two launches.  So do calls under capture, whose graph has no
+// host launches to save (a replay, per call: 4 x 256 x 1536 3.86 as two launches, 4.57 as one, 4 x 1024 x 1024 4.88 and 6.28).  A single tile of weights keeps them
+// as well: its call gains like the others' from the host and loses like them on the device (8 x 256 x 128: 7.35 -> 5.3 / 4.7 -> 5.05), and there is a test that
+// counts its launches.
 bool quant_a_own_max(int M, int N, int K) {
-  return M > 0 && M <= kOwnMaxRows && N > kTileN && K <= kOwnMaxK && static_cast<long long>(M) * K <= kOwnMaxFloats && quant_a_tile(M, N) != 0;
+  return M > 0 && M <= kOwnMaxRows && N > kTileN && K <= kOwnMaxK && (K <= 512 || N <= kOwnMaxLongN) && static_cast<long long>(M) * K <= kOwnMaxFloats &&
+         quant_a_tile(M, N) != 0;
 }
 
 int launch_gemm_quant_a(const float* a_f32, const unsigned* a_slot, float* qa_out, const int8_t* bt, int M, int N, int K,
@@ -2906,7 +2911,7 @@ int launch_gemm_quant_a(const float* a_f32, const unsigned* a_slot, float* qa_ou
     return MI8_ERR_BAD_ARG;
   if(M == 0)
     return MI8_OK;
-  if(a_f32 == nullptr || (a_slot == nullptr && (aq_out == nullptr || !quant_a_own_max(M, N, K))) || bt == nullptr || d_qb == nullptr || c == nullptr)
+  if(a_f32 == nullptr || (a_slot == nullptr && (aq_out == nullptr || M > kOwnMaxRows || K > kOwnMaxK)) || bt == nullptr || d_qb == nullptr || c == nullptr)
     return MI8_ERR_BAD_ARG;
   if(out_dtype != MI8_F32 && out_dtype != MI8_F16)
     return MI8_ERR_BAD_ARG;
