@@ -311,8 +311,9 @@ int mi8_affine_f32(const float* a, int M, int K, const int8_t* bt, const float* 
   int rc = mi8_prepare_a_f32(a, M, K, aq_scratch, d_qa, workspace, workspace_bytes, stream);
   if(rc != MI8_OK)
     return rc;
+  // (the quantisation lets the product start behind its own wait: what may have written the weight has completed then)
   return launch_gemm(aq_scratch, bt, M, N, K, d_qa, d_qb, scale, bias, relu, c, out_dtype, nullptr, workspace,
-                     workspace_bytes, as_stream(stream), 0, 0);
+                     workspace_bytes, as_stream(stream), 0, 0, nullptr, nullptr, nullptr, 0, true);
 }
 
 void mi8_set_pdl(int enabled) { set_pdl(enabled != 0); }

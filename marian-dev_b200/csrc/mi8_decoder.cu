@@ -464,6 +464,10 @@ int wide_tile(const mi8d_decoder* d, int M) {
   return t;
 }
 
+// The driver's products may fetch their weights in front of their wait: an encoder begins with a copy, a step with a kernel that lets the next one start behind its own
+// wait (a step in one launch sees to itself, launch_decoder_rows), so that all a caller has put in front has completed, and the driver's kernels write no weight.
+constexpr bool kOwnChain = true;
+
 // Few rows: 16-row tiles for up to 64 of them, where that is one wave of CTAs (the plan takes the smallest tile that holds all rows), and inner dimensions of up
 // to 2048 unsplit (the plan splits 2048).  A tile's operands, MMAs and write-back are then the shortest, and the split path's fence, atomics and counter cost more
 // than eight K blocks.  Whole mini-batches, the plan / 16-row tiles / those and no splits: transformer-base, 4 x beam 4 13.5 / 13.5 / 13.25 ms, 10 x 4 15.0 /
@@ -505,7 +509,7 @@ int gemm(mi8d_decoder* d, const int8_t* a, int M, const Aff& w, bool relu, float
   if(force_splits == 0 && w.N <= 8192)
     force_splits = few_rows_splits(M, w.K);
   return launch_gemm(a, w.bt, M, w.N, w.K, qa, w.qm, 1.0f, w.bias, relu ? 1 : 0, c, MI8_F32, nullptr, d->ws, d->ws_bytes, s, force_tile_m,
-                     force_splits, absmax_out);
+                     force_splits, absmax_out, nullptr, nullptr, 0, kOwnChain);
 }
 
 // M rows of `a` against the matrices [first, last) of a fused group, one launch; outputs and the activation's details are the caller's
@@ -525,6 +529,7 @@ GemmCall fused_call(mi8d_decoder* d, const int8_t* a, const Fused& f, int M, int
   g.ws_bytes = d->ws_bytes;
   g.stream = s;
   g.a_rows_cap = a_rows_cap;
+  g.weights_settled = kOwnChain;
   g.force_tile_m = narrow_tile(M, g.N);
   g.force_splits = few_rows_splits(M, f.K);
   return g;
@@ -588,12 +593,13 @@ int quant_gemm(mi8d_decoder* d, const float* x, int M, const unsigned* slot, con
     g.relu = relu ? 1 : 0;
     g.c = c;
     g.absmax_out = absmax_out;
+    g.weights_settled = kOwnChain;
     g.force_cluster = d->opt_cluster_size;
     g.stream = s;
     return launch_gemm_cq(g);
   }
   if(!w.p8 && d->opt_quant_in_gemm && w.K <= 1024 && quant_a_tile(M, w.N) != 0)
-    return launch_gemm_quant_a(x, slot, qa, w.bt, M, w.N, w.K, w.qm, 1.0f, w.bias, relu ? 1 : 0, c, MI8_F32, nullptr, s, absmax_out);
+    return launch_gemm_quant_a(x, slot, qa, w.bt, M, w.N, w.K, w.qm, 1.0f, w.bias, relu ? 1 : 0, c, MI8_F32, nullptr, s, absmax_out, nullptr, kOwnChain);
   MI8D_TRY(quantize_act(d, x, M, w.K, slot, d->aq, s));
   return gemm_act(d, d->aq, M, w, relu, c, s, absmax_out);
 }
@@ -643,6 +649,7 @@ int quant_gemm_ln(mi8d_decoder* d, const float* x, int M, const unsigned* slot, 
     g.ln_rowmax = rowmax;
     g.ln_slot = out_slot;
     g.ln_slot2 = out_slot2;
+    g.weights_settled = kOwnChain;
     g.stream = s;
     return launch_gemm_cq(g);
   }
@@ -1359,11 +1366,11 @@ int run_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const i
       } else {
         const int8_t* a_new = L.hq + static_cast<size_t>(t) * slab_stride;
         MI8D_TRY(launch_gemm(xq, w.self_q.bt, R, w.self_q.N, w.self_q.K, xq_tail, w.self_q.qm, 1.0f, w.self_q.bias, 0, d->qbuf, MI8_F32,
-                             nullptr, d->ws, d->ws_bytes, s, 0, 1));
+                             nullptr, d->ws, d->ws_bytes, s, 0, 1, nullptr, nullptr, nullptr, 0, kOwnChain));
         MI8D_TRY(launch_gemm(a_new, w.self_k.bt, R, w.self_k.N, w.self_k.K, hq_tail, w.self_k.qm, 1.0f, w.self_k.bias, 0, kv_new[0], MI8_F32,
-                             nullptr, d->ws, d->ws_bytes, s, 0, 1));
+                             nullptr, d->ws, d->ws_bytes, s, 0, 1, nullptr, nullptr, nullptr, 0, kOwnChain));
         MI8D_TRY(launch_gemm(a_new, w.self_v.bt, R, w.self_v.N, w.self_v.K, hq_tail, w.self_v.qm, 1.0f, w.self_v.bias, 0, kv_new[1], MI8_F32,
-                             nullptr, d->ws, d->ws_bytes, s, 0, 1));
+                             nullptr, d->ws, d->ws_bytes, s, 0, 1, nullptr, nullptr, nullptr, 0, kOwnChain));
       }
       if(side)
         MI8D_CUDA(cudaStreamWaitEvent(s, d->ev_join, 0));
@@ -1440,6 +1447,7 @@ int run_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const i
       g.seg_qb[0] = d->out_w.qm;
       g.seg_bias[0] = d->out_bias;
       g.seg_c[0] = d->logits;
+      g.weights_settled = kOwnChain;
       g.stream = s;
       g.block_max = d->blk_max;
       g.block_sum = d->blk_sum;

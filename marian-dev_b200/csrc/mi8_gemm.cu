@@ -133,6 +133,7 @@ struct GemmParams {
   int* rows_computed;       // optional (measurement): receives the number of activation rows this launch really computed
   int withhold_item;        // test hook: the producer leaves out the loads of this one of its stages (-1 = none; or kWithholdWarp)
   uint32_t spin_limit;      // bound of every barrier wait of this launch
+  int weights_settled;      // the weight does not come from a kernel that may still be at work (launch_gemm): fetched in front of the wait
   int pair_items, pair_whole;   // kHalves: the CTA-pair kernel's items, and how many of them are whole tiles
 };
 
@@ -441,11 +442,11 @@ mi8_gemm_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, const __g
 
   if(warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    // The weights do not depend on the previous kernel: the weight tiles of the first pipeline fill
+    // Where the weights do not depend on the previous kernel the weight tiles of the first pipeline fill
     // are requested before waiting for it, the activation tiles (its output) after.
     uint32_t it = 0;
     uint32_t prefetched = 0;  // stages whose weight tile is already in flight
-    if((kBelow ? !is_below(blockIdx.x) : p.skip_a == nullptr) && kTopK == 0 && p.withhold_item < 0) {   // (output-layer variant: the M-side operand is the activation, nothing to prefetch)
+    if((kBelow ? !is_below(blockIdx.x) : p.skip_a == nullptr) && kTopK == 0 && p.weights_settled && p.withhold_item < 0) {   // (output-layer variant: the M-side operand is the activation, nothing to prefetch)
       const WorkItem w0 = decode_work(p, blockIdx.x);
       const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, w0.n_tile * kTileN);
       const int blocks = w0.kb_end - w0.kb_begin, n_pre = min(kStages, (blocks + kPer - 1) / kPer);
@@ -1203,8 +1204,8 @@ mi8_gemm_pair_kernel(const __grid_constant__ WeightMaps<kP8, kMaps> tmap_w, cons
     int held = -1;                    // kResident: the weights' tile in shared memory
     // copies of both CTAs are credited to full[s] of the rank-0 CTA
     auto full_addr = [&](uint32_t s) { return mapa_shared(smem_u32(&ctl->full[s]), 0u); };
-    if(p.skip_a == nullptr && my_tiles(false).first < my_tiles(false).end && p.withhold_item < 0) {
-      // weights do not depend on the previous kernel: request the first pipeline fill before waiting for it
+    if(p.skip_a == nullptr && p.weights_settled && my_tiles(false).first < my_tiles(false).end && p.withhold_item < 0) {
+      // weights that do not depend on the previous kernel: request the first pipeline fill before waiting for it
       const Tile w0 = tile_at(my_tiles(false), my_tiles(false).first);
       const WeightRows wr = weight_rows(tmap_w, p.nseg, p.seg_n, (2 * w0.n_tile + static_cast<int>(rank)) * kTileN);
       const int n_pre = min(static_cast<int>(stages), (p.kb_total + kPer - 1) / kPer);
@@ -1511,6 +1512,7 @@ struct CqParams {
   int* status;
   uint32_t spin_limit;
   int withhold_item;
+  int weights_settled;      // as in GemmParams
   int* rows_computed;
 };
 
@@ -1601,7 +1603,9 @@ mi8_gemm_cq_kernel(const __grid_constant__ CUtensorMap tmap_w, const CqParams p)
   float unquant = 1.0f;
 
   if(warp == 0) {
-    // ------------------------------------------------------------ weight producer (weights never depend on the preceding kernel)
+    // ------------------------------------------------------------ weight producer
+    if(!p.weights_settled)
+      pdl_wait();
     for(int kb = 0; kb < p.kb_total; ++kb) {
       const uint32_t s = kb % p.stages;
       const uint32_t ph = (kb / p.stages) & 1u;
@@ -2550,6 +2554,7 @@ int launch_gemm_call(const GemmCall& g) {
   p.skip_a = g.skip_a;
   p.skip_b = g.skip_b;
   p.skip_rows_below = g.skip_rows_below;
+  p.weights_settled = g.weights_settled;
   p.p8_scale_a = nullptr;
   p.p8_zp_a = p.p8_sum_a = nullptr;
   p.status = device_status_ptr();
@@ -2598,7 +2603,7 @@ int launch_gemm_call(const GemmCall& g) {
 int launch_gemm(const int8_t* aq, const int8_t* bt, int M, int N, int K, const float* d_qa, const float* d_qb, float scale,
                 const float* bias, int relu, void* c, int out_dtype, int32_t* acc_out, void* ws, size_t ws_bytes,
                 cudaStream_t stream, int force_tile_m, int force_splits, unsigned* absmax_out, const unsigned* skip_a,
-                const unsigned* skip_b, int skip_rows_below) {
+                const unsigned* skip_b, int skip_rows_below, bool weights_settled) {
   if(M > 0 && (d_qb == nullptr || c == nullptr))
     return MI8_ERR_BAD_ARG;
   GemmCall g;
@@ -2625,6 +2630,7 @@ int launch_gemm(const int8_t* aq, const int8_t* bt, int M, int N, int K, const f
   g.skip_a = skip_a;
   g.skip_b = skip_b;
   g.skip_rows_below = skip_rows_below;
+  g.weights_settled = weights_settled;
   return launch_gemm_call(g);
 }
 
@@ -2767,6 +2773,7 @@ int launch_gemm_cq(const CqCall& g) {
   p.ln_rowmax = g.ln_rowmax;
   p.ln_slot = g.ln_slot;
   p.ln_slot2 = g.ln_slot2;
+  p.weights_settled = g.weights_settled;
   p.status = device_status_ptr();
   test_wait_limits(&p.withhold_item, &p.spin_limit);
   p.rows_computed = nullptr;
@@ -2854,6 +2861,7 @@ int launch_gemm_p8(const uint8_t* aq, const float* scale_a, const int32_t* zp_a,
   p.p8_scale_a = scale_a;
   p.p8_zp_a = zp_a;
   p.p8_sum_a = sum_a;
+  p.weights_settled = 1;   // (the kernels that write a weight of this scheme do not let the next one start before they are done)
   p.status = device_status_ptr();
   if(p.status == nullptr)
     return MI8_ERR_LAUNCH;
@@ -2906,7 +2914,7 @@ bool quant_a_own_max(int M, int N, int K) {
 
 int launch_gemm_quant_a(const float* a_f32, const unsigned* a_slot, float* qa_out, const int8_t* bt, int M, int N, int K,
                         const float* d_qb, float scale, const float* bias, int relu, void* c, int out_dtype, int32_t* acc_out,
-                        cudaStream_t stream, unsigned* absmax_out, int8_t* aq_out) {
+                        cudaStream_t stream, unsigned* absmax_out, int8_t* aq_out, bool weights_settled) {
   if(M < 0 || N <= 0 || K <= 0)
     return MI8_ERR_BAD_ARG;
   if(M == 0)
@@ -2957,6 +2965,7 @@ int launch_gemm_quant_a(const float* a_f32, const unsigned* a_slot, float* qa_ou
   p.a_slot = a_slot;
   p.qa_out = qa_out;
   p.aq_out = a_slot == nullptr ? aq_out : nullptr;
+  p.weights_settled = weights_settled;
   p.skip_a = nullptr;
   p.skip_b = nullptr;
   p.skip_rows_below = 0;
@@ -3035,6 +3044,7 @@ int launch_gemm_logits(const int8_t* aq, const float* d_qa, const int8_t* wq, co
   p.skip_a = nullptr;
   p.skip_b = nullptr;
   p.skip_rows_below = 0;
+  p.weights_settled = 0;   // (not looked at)
   p.status = device_status_ptr();
   if(p.status == nullptr)
     return MI8_ERR_LAUNCH;

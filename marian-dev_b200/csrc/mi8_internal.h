@@ -62,7 +62,7 @@ int profile_end(mi8_gemm_record* out, int capacity, int* count);
 int launch_max_absolute(const float* x, size_t n, float* d_absmax, float* d_quant_mult, void* ws, size_t ws_bytes,
                         cudaStream_t stream);
 int launch_quantize(const float* x, size_t n, const float* d_quant_mult, int8_t* q, cudaStream_t stream);
-// both in turn (d_quant_mult = 127 / max|x|, q = x quantised with it); one launch for small tensors.  `weight`: q is a product's weight
+// both in turn (d_quant_mult = 127 / max|x|, q = x quantised with it); one launch for small tensors.  `weight`: a conversion
 int launch_prepare(const float* x, size_t n, float* d_quant_mult, int8_t* q, void* ws, size_t ws_bytes, cudaStream_t stream, bool weight = false);
 // W [K, N] -> Bt [N, K] and its multiplier
 int launch_convert(const float* w, int K, int N, float* d_quant_mult, int8_t* bt, void* ws, size_t ws_bytes, cudaStream_t stream);
@@ -71,10 +71,12 @@ int launch_transpose_f32(const float* in, int batch, int rows, int cols, float* 
 // GEMM (mi8_gemm.cu)
 // absmax_out (optional): 4-byte slot that receives max|C| (unsigned bit pattern, atomicMax) for the
 // quantisation of C as the next affine's input.
+// weights_settled: whatever may still be at work in front of the launch on its stream does not write the weight, so that the first of it is fetched in front of the
+// kernel's wait.  Where the caller of the library orders the launches nobody knows that (a kernel that quantises a weight lets the next one start before it is done).
 int launch_gemm(const int8_t* aq, const int8_t* bt, int M, int N, int K, const float* d_qa, const float* d_qb, float scale,
                 const float* bias, int relu, void* c, int out_dtype, int32_t* acc_out, void* ws, size_t ws_bytes,
                 cudaStream_t stream, int force_tile_m, int force_splits, unsigned* absmax_out = nullptr,
-                const unsigned* skip_a = nullptr, const unsigned* skip_b = nullptr, int skip_rows_below = 0);
+                const unsigned* skip_a = nullptr, const unsigned* skip_b = nullptr, int skip_rows_below = 0, bool weights_settled = false);
 
 // The general form: one activation against up to three weight matrices of the same shape stored one behind the
 // other (N = nseg * rows of one of them), each with its own multiplier, bias and output matrix [M, N / nseg].
@@ -111,6 +113,7 @@ struct GemmCall {
   // per segment, where it differs: the first of its M activation rows (-1: a_row0) and their multiplier (null: d_qa)
   int seg_row0[3] = {-1, -1, -1};
   const float* seg_qa[3] = {nullptr, nullptr, nullptr};
+  bool weights_settled = false;
 };
 int launch_gemm_call(const GemmCall& g);
 
@@ -123,7 +126,7 @@ void test_wait_fault(int withhold_item, unsigned spin_limit);
 int quant_a_tile(int M, int N);
 int launch_gemm_quant_a(const float* a_f32, const unsigned* a_slot, float* qa_out, const int8_t* bt, int M, int N, int K,
                         const float* d_qb, float scale, const float* bias, int relu, void* c, int out_dtype, int32_t* acc_out,
-                        cudaStream_t stream, unsigned* absmax_out = nullptr, int8_t* aq_out = nullptr);
+                        cudaStream_t stream, unsigned* absmax_out = nullptr, int8_t* aq_out = nullptr, bool weights_settled = false);
 // ... and without a slot, where every CTA finds the maximum itself (aq_out: the quantised activation, M * K bytes).
 bool quant_a_own_max(int M, int N, int K);
 
@@ -157,6 +160,7 @@ struct CqCall {
   cudaStream_t stream = nullptr;
   int force_tile_m = 0;     // 0 = chosen from M and N
   int force_cluster = 0;    // 0 = the largest of 8, 4, 2, 1 that divides N / 128 (ln: N / 128)
+  bool weights_settled = false;
 };
 bool gemm_cq_supported(int M, int N, int K, bool ln);
 int launch_gemm_cq(const CqCall& g);

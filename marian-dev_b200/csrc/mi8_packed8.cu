@@ -24,7 +24,7 @@ constexpr int kRi = 4;      // consecutive rows stored together (row interleave)
 // threads read consecutive words of the item and write bt[n][4 * kq .. 4 * kq + 3].
 __global__ void __launch_bounds__(kBlock)
 p8_unpack_bt_kernel(const uint32_t* __restrict__ packed, int K, int N, uint32_t* __restrict__ bt) {
-  pdl_wait();   // (no trigger: a product behind this fetches the weight in front of its own wait)
+  pdl_wait();   // (no trigger: a product of this scheme behind this fetches the weight in front of its own wait)
   const size_t words = static_cast<size_t>(K) * N / kRi;
   const size_t stride = static_cast<size_t>(gridDim.x) * kBlock;
   constexpr int kBlockWords = kKcb * kNcb / kRi;

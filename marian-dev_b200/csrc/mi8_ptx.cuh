@@ -26,7 +26,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // predecessor on the stream is still running.  pdl_launch_dependents() lets the successor start
 // launching; pdl_wait() blocks until the predecessor has completed and its writes are visible.
 // Everything a kernel does before pdl_wait() must not depend on (or disturb) the predecessor:
-// barrier/TMEM set-up and loads of constant weights qualify.  Without the launch attribute both are no-ops.
+// barrier/TMEM set-up qualifies, and loads of what no kernel in front can still be writing: that takes a launcher who knows what is in
+// front (launch_gemm's weights_settled, launch_decoder_rows' params_settled, launch_parts).  Without the launch attribute both are no-ops.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Both, the wait first: the form of most kernels.  When every kernel lets its successor start at its own start, a chain of five to seven of them lies on the

@@ -208,7 +208,7 @@ __device__ __forceinline__ float parts_multiplier(const unsigned* partials, int 
 
 // kHeld 16-byte vectors per thread, a warp's lanes side by side in each (beyond the end the last one once more).  Three blocks per SM are resident beside
 // the search for the maximum, so kHeld is the smallest that puts the tensor into so many; beyond eight there are more blocks, whose turn comes later.
-// `early`: the next kernel may begin beside this one; not where the tensor is a weight, which a product fetches in front of its own wait.
+// `early`: the next kernel may begin beside this one; not behind a conversion, which is not part of a chain.
 template <int kHeld>
 __global__ void __launch_bounds__(kBlock)
 mi8_quantize_kernel_held(const float* __restrict__ x, size_t n, const unsigned* partials, int n_partials, float* d_quant_mult, int8_t* __restrict__ q,
@@ -316,7 +316,7 @@ constexpr size_t kNarrowMaxN = static_cast<size_t>(kPrepareCtas) * 1024 * 16, kC
 __global__ void __launch_bounds__(kBlock)
 mi8_convert_kernel(const float* __restrict__ w, int K, int N, const unsigned* partials, int n_partials, float* d_quant_mult, int8_t* __restrict__ bt,
                    int words, int vec, int* status) {
-  // (no pdl_launch_dependents(): a product behind this fetches the converted weight in front of its own wait)
+  // (no pdl_launch_dependents(): a conversion is not part of a chain)
   __shared__ unsigned tile[32][33];   // [n][k / 4]
   __shared__ unsigned red[kBlock / 32];
   const int n0 = blockIdx.x * 32, k0 = (gridDim.y - 1 - blockIdx.y) * 128;   // (the rows that the search reads last are still in L2)

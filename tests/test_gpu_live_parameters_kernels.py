@@ -105,3 +105,64 @@ def test_weight_multiplier(cuda_device, m, k, n, entry):
         _max_into(w.quant_mult, values[i & 1], ws)
         assert torch.equal(product(), want[i & 1])
     assert ops.poll_status() == 0
+
+
+@pytest.mark.parametrize("m,k,n", [(4, 256, 1536), (1, 1024, 300), (64, 512, 512), (300, 2048, 1024)])
+@pytest.mark.parametrize("writer", ["quantize", "prepare_a", "quantize_slot", "prepare_b", "prepare_b_nk"])
+@pytest.mark.parametrize("entry", ["multiply", "affine", "slot", "cluster"])
+def test_weight(cuda_device, m, k, n, writer, entry):
+    """A weight quantised by any of the entry points that write int8 matrices, directly in front of the product."""
+    from marian_dev_b200 import ops
+    from marian_dev_b200.binding import check, lib
+    g = torch.Generator(device=cuda_device).manual_seed(n)
+    x = torch.randn(m, k, generator=g, device=cuda_device)
+    if entry == "slot" and (m > 64 or k > 1024) or entry == "cluster" and n % 128:
+        pytest.skip("a shape that this entry point refuses")
+    aq, own_slot = ops.prepareA(x), ops.max_absolute(x)
+    ws, busy, scratch = ops.Workspace(cuda_device), _Busy(cuda_device), torch.empty(m * k + 64, dtype=torch.int8, device=cuda_device)
+    own = ops.Workspace(cuda_device)
+    values = [torch.randn(n, k, generator=g, device=cuda_device) for _ in range(2)]
+    slots = [ops.max_absolute(v) for v in values]
+    multipliers = [127.0 / s for s in slots]
+    turned = [v.t().contiguous() for v in values]
+    bt, qb = torch.zeros(n, k, dtype=torch.int8, device=cuda_device), torch.ones(1, device=cuda_device)
+
+    def write(i):
+        v, st = values[i], _stream()
+        if writer == "quantize":
+            check(lib().mi8_quantize_f32_i8(v.data_ptr(), v.numel(), multipliers[i].data_ptr(), bt.data_ptr(), st))
+        elif writer == "prepare_a":
+            check(lib().mi8_prepare_a_f32(v.data_ptr(), n, k, bt.data_ptr(), qb.data_ptr(), ws.ptr, ws.nbytes, st))
+        elif writer == "quantize_slot":
+            check(lib().mi8g_quantize_slot(v.data_ptr(), v.numel(), slots[i].data_ptr(), bt.data_ptr(), qb.data_ptr(), st))
+        else:
+            nk = writer == "prepare_b_nk"
+            check(lib().mi8_prepare_b_f32((v if nk else turned[i]).data_ptr(), k, n, int(nk), bt.data_ptr(), qb.data_ptr(), ws.ptr, ws.nbytes, st))
+
+    def product():
+        out = torch.empty(m, n, device=cuda_device)
+        if entry == "affine":
+            check(lib().mi8_affine_f32(x.data_ptr(), m, k, bt.data_ptr(), qb.data_ptr(), n, None, 1.0, 0, out.data_ptr(), 0, scratch.data_ptr(), own.ptr, own.nbytes,
+                                       _stream()))
+        elif entry == "slot":
+            check(lib().mi8_multiply_f32_slot(x.data_ptr(), own_slot.data_ptr(), None, bt.data_ptr(), m, n, k, qb.data_ptr(), 1.0, None, 0, out.data_ptr(), 0, None,
+                                              _stream()))
+        elif entry == "cluster":
+            check(lib().mi8g_affine_slot(x.data_ptr(), own_slot.data_ptr(), bt.data_ptr(), qb.data_ptr(), m, n, k, 1.0, None, 0, out.data_ptr(), None, 0, 0, _stream()))
+        else:
+            check(lib().mi8_multiply_i8(aq.data.data_ptr(), bt.data_ptr(), m, n, k, aq.quant_mult.data_ptr(), qb.data_ptr(), 1.0, None, 0, out.data_ptr(), 0, None,
+                                        own.ptr, own.nbytes, _stream()))
+        return out
+
+    want = []
+    for i in range(2):
+        write(i)
+        torch.cuda.synchronize()
+        want.append(product())
+        torch.cuda.synchronize()
+    assert not torch.equal(want[0], want[1])
+    for i in range(8):
+        busy()
+        write(i & 1)
+        assert torch.equal(product(), want[i & 1])
+    assert ops.poll_status() == 0
