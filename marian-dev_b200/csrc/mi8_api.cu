@@ -106,6 +106,7 @@ int sm_count() {
 using namespace mi8;
 
 namespace {
+constexpr size_t kAtOnceFloats = 4096;
 bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
   const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
   return x < y + b_bytes && y < x + a_bytes;
@@ -216,7 +217,7 @@ int mi8_prepare_a_f32(const float* a, int rows, int cols, int8_t* q, float* d_qu
   if(rows == 0)
     return MI8_OK;
   const size_t n = static_cast<size_t>(rows) * static_cast<size_t>(cols);
-  return launch_prepare(a, n, d_quant_mult, q, workspace, workspace_bytes, as_stream(stream));
+  return launch_prepare(a, n, d_quant_mult, q, workspace, workspace_bytes, as_stream(stream), Trigger::kBehindWait);
 }
 
 int mi8_prepare_b_f32(const float* w, int K, int N, int w_is_nk, int8_t* bt, float* d_quant_mult, void* workspace,
@@ -224,7 +225,7 @@ int mi8_prepare_b_f32(const float* w, int K, int N, int w_is_nk, int8_t* bt, flo
   if(K <= 0 || N <= 0 || d_quant_mult == nullptr)
     return MI8_ERR_BAD_ARG;
   if(w_is_nk)
-    return launch_prepare(w, static_cast<size_t>(K) * static_cast<size_t>(N), d_quant_mult, bt, workspace, workspace_bytes, as_stream(stream), true);
+    return launch_prepare(w, static_cast<size_t>(K) * static_cast<size_t>(N), d_quant_mult, bt, workspace, workspace_bytes, as_stream(stream), Trigger::kDone);
   return launch_convert(w, K, N, d_quant_mult, bt, workspace, workspace_bytes, as_stream(stream));
 }
 
@@ -308,12 +309,16 @@ int mi8_affine_f32(const float* a, int M, int K, const int8_t* bt, const float* 
      ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(aq_scratch)) & 15u) == 0 && !overlap(a, 4 * floats, c, c_bytes) &&
      !overlap(a, 4 * floats, aq_scratch, floats + 4) && !overlap(c, c_bytes, aq_scratch, floats + 4) && !being_captured(as_stream(stream)))
     return launch_gemm_quant_a(a, nullptr, d_qa, bt, M, N, K, d_qb, scale, bias, relu, c, out_dtype, nullptr, as_stream(stream), nullptr, aq_scratch);
-  int rc = mi8_prepare_a_f32(a, M, K, aq_scratch, d_qa, workspace, workspace_bytes, stream);
+  // The quantisation of up to kAtOnceFloats is shorter than the product's set-up and lets the product start at its own start; a larger one lets it start behind its
+  // wait: what may have written the weight has completed then, so that the product may fetch the weight in front of its own.  Replayed from a graph, at the start and
+  // the weight behind the wait / the other way round, us: 4 x 256 x 1536 3.86 / 4.16, 8 x 256 x 128 3.52 / 4.3, 4 x 1024 x 1024 4.95 / 5.46, 1 x 4096 x 1024 7.07 /
+  // 7.53; 16 x 512 x 2048 4.92 / 4.81, 8 x 1024 x 1024 5.53 / 5.43, 64 x 512 x 2048 5.84 / 5.73, 256 x 512 x 2048 6.14 / 5.84.
+  const bool at_once = floats <= kAtOnceFloats;
+  int rc = launch_prepare(a, floats, d_qa, aq_scratch, workspace, workspace_bytes, as_stream(stream), at_once ? Trigger::kAtStart : Trigger::kBehindWait);
   if(rc != MI8_OK)
     return rc;
-  // (the quantisation lets the product start behind its own wait: what may have written the weight has completed then)
   return launch_gemm(aq_scratch, bt, M, N, K, d_qa, d_qb, scale, bias, relu, c, out_dtype, nullptr, workspace,
-                     workspace_bytes, as_stream(stream), 0, 0, nullptr, nullptr, nullptr, 0, true);
+                     workspace_bytes, as_stream(stream), 0, 0, nullptr, nullptr, nullptr, 0, !at_once);
 }
 
 void mi8_set_pdl(int enabled) { set_pdl(enabled != 0); }

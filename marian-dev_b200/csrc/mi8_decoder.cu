@@ -1174,7 +1174,7 @@ int run_step(mi8d_decoder* d, const int* hyp_idx, const int* prev_words, const i
     if(d->p8) {
       MI8D_TRY(quantize_act(d, ctx, batch * S, dm, nullptr, d->cq, s));
     } else {
-      MI8D_TRY(launch_prepare(ctx, n, cq_tail, d->cq, d->ws, d->ws_bytes, s));
+      MI8D_TRY(launch_prepare(ctx, n, cq_tail, d->cq, d->ws, d->ws_bytes, s, Trigger::kBehindWait));
     }
     for(int l = 0; l < c.dec_depth; ++l) {
       const DecLayerW& w = d->dec_w[l];

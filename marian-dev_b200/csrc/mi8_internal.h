@@ -62,8 +62,10 @@ int profile_end(mi8_gemm_record* out, int capacity, int* count);
 int launch_max_absolute(const float* x, size_t n, float* d_absmax, float* d_quant_mult, void* ws, size_t ws_bytes,
                         cudaStream_t stream);
 int launch_quantize(const float* x, size_t n, const float* d_quant_mult, int8_t* q, cudaStream_t stream);
-// both in turn (d_quant_mult = 127 / max|x|, q = x quantised with it); one launch for small tensors.  `weight`: a conversion
-int launch_prepare(const float* x, size_t n, float* d_quant_mult, int8_t* q, void* ws, size_t ws_bytes, cudaStream_t stream, bool weight = false);
+// When the last kernel of launch_prepare lets the next one start: when it is done, behind its own wait (what is in front has completed then), or at its start.
+enum class Trigger { kDone, kBehindWait, kAtStart };
+// both in turn (d_quant_mult = 127 / max|x|, q = x quantised with it); one launch for small tensors
+int launch_prepare(const float* x, size_t n, float* d_quant_mult, int8_t* q, void* ws, size_t ws_bytes, cudaStream_t stream, Trigger trigger);
 // W [K, N] -> Bt [N, K] and its multiplier
 int launch_convert(const float* w, int K, int N, float* d_quant_mult, int8_t* bt, void* ws, size_t ws_bytes, cudaStream_t stream);
 int launch_transpose_f32(const float* in, int batch, int rows, int cols, float* out, cudaStream_t stream);

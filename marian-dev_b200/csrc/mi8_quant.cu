@@ -243,15 +243,17 @@ mi8_quantize_kernel_held(const float* __restrict__ x, size_t n, const unsigned* 
 // affine 256 x 512 x 2048 10.9 -> 7.9 us, 250 x 1024 x 32000 24.2 -> 21.1 us, 4 x 256 x 1536 8.8 -> 6.8 us.
 template <int kCtas>
 __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(1024)
-mi8_prepare_cluster_kernel(const float* __restrict__ x, int n16, float* d_quant_mult, int8_t* __restrict__ q, int* status, int early) {
+mi8_prepare_cluster_kernel(const float* __restrict__ x, int n16, float* d_quant_mult, int8_t* __restrict__ q, int* status, Trigger trigger) {
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
   __shared__ unsigned red[32];
   __shared__ unsigned cta_max[kCtas];
   if(kCtas > 1)
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (this CTA runs: the others may write to cta_max)
+  if(trigger == Trigger::kAtStart)
+    pdl_launch_dependents();
   pdl_wait();
-  if(early)
+  if(trigger == Trigger::kBehindWait)
     pdl_launch_dependents();
   trace_stamp_start(th, kTrQuantize);
   const int rank = kCtas > 1 ? static_cast<int>(blockIdx.x) : 0;
@@ -496,7 +498,7 @@ bool wide_cluster_fits() {
 }
 }  // namespace
 
-int launch_prepare(const float* x, size_t n, float* d_quant_mult, int8_t* q, void* ws, size_t ws_bytes, cudaStream_t stream, bool weight) {
+int launch_prepare(const float* x, size_t n, float* d_quant_mult, int8_t* q, void* ws, size_t ws_bytes, cudaStream_t stream, Trigger trigger) {
   // Up to kOneCtaMaxN floats one CTA, up to kClusterMaxN a cluster, of kWideCtas from kWideMinN on (beyond, so few SMs read for longer than the other
   // launch costs).  Launches back to back, in us: one CTA 1.23 at 4096 floats, 1.51 at 8192; clusters of eight and sixteen 1.91 and 1.95 at 16384,
   // 2.01 and 2.01 at 32768, 2.42 and 2.22 at 66000, 3.04 and 2.49 at 131072, 4.13 (two chunks per thread) and 3.24 at 256000; two kernels 3.07 at 66000,
@@ -514,7 +516,7 @@ int launch_prepare(const float* x, size_t n, float* d_quant_mult, int8_t* q, voi
   int* status = device_status_ptr();
   if(status == nullptr)
     return MI8_ERR_LAUNCH;
-  const int early = weight ? 0 : 1;
+  const int early = trigger != Trigger::kDone ? 1 : 0;   // (larger tensors: the second kernel starts behind the first one's wait, and so may the next at its start)
   if(n < 4) {   // (no whole vector)
     const int rc = launch_max_absolute(x, n, nullptr, d_quant_mult, ws, ws_bytes, stream);
     return rc != MI8_OK ? rc : launch_quantize(x, n, d_quant_mult, q, stream);
@@ -531,13 +533,13 @@ int launch_prepare(const float* x, size_t n, float* d_quant_mult, int8_t* q, voi
   }
   const int n16 = static_cast<int>(n / 16);
   if(n <= kOneCtaMaxN)
-    launch_kernel(mi8_prepare_cluster_kernel<1>, dim3(1), dim3((n16 + 31) / 32 * 32), 0, stream, x, n16, d_quant_mult, q, status, early);
+    launch_kernel(mi8_prepare_cluster_kernel<1>, dim3(1), dim3((n16 + 31) / 32 * 32), 0, stream, x, n16, d_quant_mult, q, status, trigger);
   else if(wide)
     launch_kernel(mi8_prepare_cluster_kernel<kWideCtas>, dim3(kWideCtas), dim3(((n16 + kWideCtas - 1) / kWideCtas + 31) / 32 * 32), 0, stream, x, n16,
-                  d_quant_mult, q, status, early);
+                  d_quant_mult, q, status, trigger);
   else
     launch_kernel(mi8_prepare_cluster_kernel<kPrepareCtas>, dim3(kPrepareCtas), dim3(((n16 + kPrepareCtas - 1) / kPrepareCtas + 31) / 32 * 32), 0, stream,
-                  x, n16, d_quant_mult, q, status, early);
+                  x, n16, d_quant_mult, q, status, trigger);
   count_launch();
   return check_launch();
 }
