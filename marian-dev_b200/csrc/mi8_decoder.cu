@@ -18,6 +18,7 @@
 
 #include "../../include/marian_i8_decode.h"
 #include "mi8_internal.h"
+#include "mi8_tagged.h"
 
 namespace mi8 {
 namespace {
@@ -1566,6 +1567,14 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
                     t > 0 ? reinterpret_cast<const float*>(ctrl + 2 * R) : nullptr, tensor_beam, nb, max_beam, reinterpret_cast<float*>(out), out + cells,
                     out + 2 * cells, stream, link);
   };
+  // An error behind a launch: what is in flight still writes to pinned memory and to the caller's arena
+  const auto settled = [&](int code) {
+    cudaStreamSynchronize(s);
+    if(d->side != nullptr)
+      cudaStreamSynchronize(d->side);
+    cudaGetLastError();
+    return code;
+  };
   StepLink link, next_link;   // of the running step, and of the one launched ahead of it
   bool launched = false;      // the running step was launched ahead, and stands
   bool loose_end = false;     // the stream may still be at work
@@ -1614,7 +1623,7 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
       d->step_ctrl = nullptr;
       d->n_step_ctrl = 0;
       if(rc != MI8_OK)
-        return rc;
+        return settled(rc);
     }
     const int was_t = d->t, was_cell = d->cell_cur, was_anc = d->anc_cur;
     const bool ahead = link.next_ctrl != nullptr;
@@ -1622,28 +1631,27 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
       next_link = link_of(t + 1, nb, max_beam, true);
       rc = launch(t + 1, nb, max_beam, next_link);
       if(rc != MI8_OK)
-        return rc;
+        return settled(rc);
     }
     const clk::time_point t_b = clk::now();
     int* out = d->h_out + (t & 1) * 3 * c.max_batch * 8;
     if(link.tagged != nullptr) {
       const volatile unsigned long long* word = d->h_tagged + (t & 1) * 2 * kDecoderRowsMax;
-      const auto arrived = [&](int i) { return static_cast<unsigned>(word[i] >> 32) == link.tag; };
       loose_end = true;
-      int i = 0;
-      for(unsigned spins = 1; i < 2 * cells; ++spins) {
-        while(i < 2 * cells && arrived(i))
-          ++i;
+      const auto pause = [&]() {
         if(d->opt_blocking_wait == 2)
           std::this_thread::yield();
-        if(i < 2 * cells && spins % 4096 == 0) {   // (a failed launch never writes the words)
-          const cudaError_t qe = cudaStreamQuery(s);
-          if(qe != cudaSuccess && qe != cudaErrorNotReady)
-            MI8D_CUDA(qe);
-          if(qe == cudaSuccess && !arrived(2 * cells - 1) && !arrived(i))
-            return MI8_ERR_DEVICE;
-        }
-      }
+      };
+      cudaError_t qe = cudaSuccess;
+      const auto state = [&]() {
+        qe = cudaStreamQuery(s);
+        return qe == cudaSuccess ? StreamState::kIdle : qe == cudaErrorNotReady ? StreamState::kBusy : StreamState::kFailed;
+      };
+      const TaggedWait waited = wait_for_tagged(word, 2 * cells, link.tag, 4096, pause, state);
+      if(waited == TaggedWait::kFailed)
+        MI8D_CUDA(qe);
+      if(waited == TaggedWait::kMissing)
+        return MI8_ERR_DEVICE;
       for(int e = 0; e < cells; ++e) {
         const unsigned score = static_cast<unsigned>(word[2 * e]), key = static_cast<unsigned>(word[2 * e + 1]);
         memcpy(out + e, &score, sizeof(float));
