@@ -1682,7 +1682,7 @@ int mi8d_search(mi8d_decoder* d, const int* ids, const float* log_mask, int batc
     d->t_wait += secs(t_b, t_c);
     d->n_steps += 1;
     mark = t_c;
-    down_bytes += static_cast<size_t>(3 * cells) * sizeof(int);
+    down_bytes += static_cast<size_t>(cells) * (link.tagged != nullptr ? 2 * sizeof(unsigned long long) : 3 * sizeof(int));
     const float* nv = reinterpret_cast<const float*>(out);
     const int* nbm = out + cells;
     const int* nw = out + 2 * cells;
