@@ -113,17 +113,22 @@ step_begin_kernel(const int* host_ctrl, int* __restrict__ ctrl, int n_ctrl, unsi
 //   s_t = sum_j ((y0 + y1) + (y2 + y3));  mean = block256_sum(s) / dim;
 //   q_t = sum_j fma(d0,d0, fma(d1,d1, fma(d2,d2, d3*d3))), d = y - mean;  var = block256_sum(q) / dim;
 //   out = ((y - mean) / sqrt(var + eps)) * gamma + beta.
-constexpr unsigned kEarlyRows = 320;   // beyond, the next kernel may begin at once: transformer-big, 128 x beam 4 (512 rows) 39.05 ms, 39.35 behind the wait; 200 rows of it
-                                       // 15.32 and 15.17, transformer-base, 64 x beam 4 (256 rows) 30.6 and 30.43
+// More floats than kEarlyFloats: the next kernel may begin at once instead of behind the wait, beside a kernel that works for longer than its set-up.  Medians of 4 to 6
+// passes by turns, at once / behind the wait, ms: transformer-big (1024 floats a row), 512 rows 38.9 / 39.3, 440 35.4 / 35.7, 400 36.2 / 36.6, 380 35.3 / 35.7, 336 33.5 /
+// 33.2; transformer-base (512), 480 rows 28.4 / 27.7, 400 28.1 / 27.7, 360 33.3 / 32.8, 512 level.
+constexpr unsigned kEarlyFloats = 368 * 1024;
 __global__ void __launch_bounds__(kRowThreads)
 add_layernorm_kernel(const float* __restrict__ a, const float* __restrict__ resid, const float* __restrict__ gamma,
                      const float* __restrict__ beta, float eps, int dim, float* __restrict__ out, float* __restrict__ rowmax,
                      unsigned* absmax_slot, unsigned* absmax_slot2) {
-  if(gridDim.x > kEarlyRows)
-    pdl_launch_dependents();
   const TraceHandles th = trace_open_all();
   unsigned long long* const tb = th.first;
-  pdl_wait_and_launch();
+  if(gridDim.x * static_cast<unsigned>(dim) > kEarlyFloats) {
+    pdl_launch_dependents();
+    pdl_wait();
+  } else {
+    pdl_wait_and_launch();
+  }
   trace_stamp_start(th, kTrAddLn);
   __shared__ float redf[kRowThreads / 32];
   __shared__ unsigned redu[kRowThreads / 32];
