@@ -378,13 +378,15 @@ class SearchPool:
         self.searches = [BeamSearch(model, beam, max_length_factor, normalize, native=st) for st in self.steppers]
         self.streams = [torch.cuda.Stream(device=model.device) for _ in self.steppers]
         if len(self.steppers) > 1 and shared_gpu_tile_rows:
+            # (`shared_gpu_tile_rows`: the widest tiles to take; 0: the plan's, as for a search that has the GPU to itself)
             # With the GPU shared, an affine need not spread over every SM to be done soonest: wide tiles on few SMs read each
             # weight tile fewer times.  Same values either way.  How wide depends on what the searches leave idle: beam 4, the plan's tiles / 32 / 64 / 128 /
-            # 256 rows, ms: transformer-big, 128 sentences, four workers 226.5 / 232 / 211.7 / 202.1 / 200.3, two 125.6 / 130.4 / 122.0 / 122.2 / 126.5, 32
-            # sentences, four workers 94.4 / 89.7 / 82.9 / 84.2 / 84.1; transformer-base, 64 sentences, four workers 81.3 / 81.4 / 76.2 / 76.4 / 80.1, two
-            # 56.7 / 56.6 / 55.2 / 56.9 / 61.8, 20 sentences, four workers 59.3 / 59.3 / 59.0 / 60.4 / 60.4; student, 64 sentences, four workers 24.6 / 24.5 /
+            # 256 rows, ms: transformer-big, 128 sentences, four workers 226.5 / 232 / 211.7 / 202.1 / 200.3 (again 226 / 231 / 211 / 200 / 200), three 174.6 / 180.4 /
+            # 165.7 / 158.9 / 161.3, two 125.6 / 130.4 / 122.0 / 122.2 / 126.5, 32 sentences, four workers 94.4 / 89.7 / 82.9 / 84.2 / 84.1, three 84.8 / 82.7 / 78.2 /
+            # 80.4 / 80.2; transformer-base, 64 sentences, four workers 81.3 / 81.4 / 76.2 / 76.4 / 80.1, three 74.3 / 75.4 / 72.0 / 73.4 / 77.9, two 56.7 / 56.6 /
+            # 55.2 / 56.9 / 61.8, 20 sentences, four workers 59.3 / 59.3 / 59.0 / 60.4 / 60.4; student, 64 sentences, four workers 24.6 / 24.5 /
             # 24.1 / 24.8 / 25.1.
-            widest = 64 if model.cfg.dim_emb < 1024 else 128 if len(self.steppers) == 2 else shared_gpu_tile_rows
+            widest = 64 if model.cfg.dim_emb < 1024 else 128 if len(self.steppers) <= 3 else shared_gpu_tile_rows
             for st in self.steppers:
                 st.set_option("gemm_tile_rows", min(widest, shared_gpu_tile_rows))
                 st.set_option("blocking_wait", 2)     # the workers' host threads poll and yield instead of spinning on a core each
