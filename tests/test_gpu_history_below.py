@@ -7,9 +7,9 @@ import numpy as np
 import pytest
 import torch
 
-pytestmark = pytest.mark.gpu
+from tests.kernel_args import arguments
 
-BELOW = "ELb0ELb0ELi1ELb1E"    # (the launch's template arguments end so)
+pytestmark = pytest.mark.gpu
 
 
 def _search(net, cfg, batch, beam, width, side, ids):
@@ -23,7 +23,7 @@ def _search(net, cfg, batch, beam, width, side, ids):
     search.search(ids, torch.ones(batch, width))
     buf, n = (Mi8KernelTime * 64)(), ctypes.c_int(0)
     check(lib().mi8_kernel_times_end(buf, 64, ctypes.byref(n)))
-    return out, sum(r.launches for r in buf[:n.value] if "mi8_gemm_kernel" in r.name.decode() and BELOW in r.name.decode())
+    return out, sum(r.launches for r in buf[:n.value] if (arguments("mi8_gemm_kernel", r.name.decode()) or {}).get("kBelow"))
 
 
 @pytest.mark.parametrize("dim,heads,batch,beam,width,eos_bias,launches", [
