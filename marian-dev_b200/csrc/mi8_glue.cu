@@ -1025,6 +1025,9 @@ attention_hist_kernel(const float* __restrict__ q, const float* __restrict__ k, 
 // With a thread per query position, one or two warps of a block at work on all key positions, before: a layer of transformer-big, 128 sentences of 31 words,
 // 95 -> 43 us (47 with registers for two blocks per SM instead of three), of transformer-base, 64 of 38 words, 42 -> 27, of the student, one sentence 9 -> 3.7,
 // 16 sentences 14 -> 4.6; student, 16 sentences, a mini-batch 3.14 -> 3.035 ms, one sentence 2.22 -> 2.135.
+// Longer sentences, 16 heads of 64: 16 sentences of 64 words 42 -> 21, 100 words 53 -> 49, 128 words 113 -> 68, 200 words 319 -> 261; 64 of 64 words 123 -> 67, 100
+// words 221 -> 190.  Beyond 200 words (64 floats a head; 264 of 32), which attention1_kernel had: 250 words, one sentence 89 -> 25, 16 511 -> 355; 290 words 104 -> 56
+// and 679 -> 514.  Of 142 sizes from 1 x 16 to 128 x 64 and 16 x 330 none is slower.
 template <int G>
 __device__ __forceinline__ float butterfly_order_sum(float (&a)[G]) {
 #pragma unroll
